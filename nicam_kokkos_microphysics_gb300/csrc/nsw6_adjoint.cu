@@ -852,7 +852,7 @@ __global__ void __launch_bounds__(STAGE_THREADS) adj_s4_kernel(StageIO io, Const
   __shared__ double grid[GF_COUNT * MAX_KALL];
   __shared__ double tab[FM_TABLE_DOUBLES];
   stage_smem(io.P, grid, tab);
-  const FastMath fm{tab, tab + FM_EXP_N, tab + 2 * FM_EXP_N, tab + 2 * FM_EXP_N + FM_LOG_N};
+  const FastMath fm(tab);
   tape_bind_s(tm);
   LeafLog lg;
   for (size_t c = tape().slot; c < io.NC; c += tape().nslot) {
@@ -890,7 +890,7 @@ __global__ void __launch_bounds__(STAGE_THREADS) adj_s4_hw_kernel(StageIO io, Co
   __shared__ double grid[GF_COUNT * MAX_KALL];
   __shared__ double tab[FM_TABLE_DOUBLES];
   stage_smem(io.P, grid, tab);
-  const FastMath fm{tab, tab + FM_EXP_N, tab + 2 * FM_EXP_N, tab + 2 * FM_EXP_N + FM_LOG_N};
+  const FastMath fm(tab);
   const Problem& P = io.P;
   const int K = P.kall, kmin = P.kmin, kmax = P.kmax;
   const double* afact = grid + GF_AFACT * K;
@@ -1895,7 +1895,7 @@ template <>
 struct CellMath<double> {
   using M = FastMath;
   __device__ static M make(const double* tab) {
-    return FastMath{tab, tab + FM_EXP_N, tab + 2 * FM_EXP_N, tab + 2 * FM_EXP_N + FM_LOG_N};
+    return FastMath(tab);
   }
 };
 template <>
@@ -2082,7 +2082,7 @@ __global__ void __launch_bounds__(128) tlm_cell_kernel(StageIO io, Consts C, con
     consts_with_params(C, p, CT);
   }
   __syncthreads();
-  const FastMath fm{tab, tab + FM_EXP_N, tab + 2 * FM_EXP_N, tab + 2 * FM_EXP_N + FM_LOG_N};
+  const FastMath fm(tab);
   const ADMath<Dual> mth{fm};
   const LayS& L = io.L;
   const size_t NC = io.NC;
@@ -2203,7 +2203,7 @@ __global__ void __launch_bounds__(STAGE_THREADS) tlm_s4_kernel(StageIO io, Const
   __shared__ double grid[GF_COUNT * MAX_KALL];
   __shared__ double tab[FM_TABLE_DOUBLES];
   stage_smem(io.P, grid, tab);
-  const FastMath fm{tab, tab + FM_EXP_N, tab + 2 * FM_EXP_N, tab + 2 * FM_EXP_N + FM_LOG_N};
+  const FastMath fm(tab);
   const LayS& L = io.L;
   const size_t NC = io.NC;
   double* const* x = io.x.a;

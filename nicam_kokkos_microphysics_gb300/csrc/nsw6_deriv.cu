@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(AD_THREADS) nsw6_serial_kernel(Problem P, Cons
   __shared__ double grid[GF_COUNT * KA];
   __shared__ double tab[FM_TABLE_DOUBLES];
   stage(P, grid, tab);
-  const FastMath fm{tab, tab + FM_EXP_N, tab + 2 * FM_EXP_N, tab + 2 * FM_EXP_N + FM_LOG_N};
+  const FastMath fm(tab);
   const Lay L{P.kall, P.gall, P.lall, P.prec_ld};
   const int l = blockIdx.y;
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
@@ -155,7 +155,7 @@ __global__ void __launch_bounds__(AD_THREADS) nsw6_tlm_kernel(Problem P, Consts 
   __shared__ double grid[GF_COUNT * KA];
   __shared__ double tab[FM_TABLE_DOUBLES];
   stage(P, grid, tab);
-  const FastMath fm{tab, tab + FM_EXP_N, tab + 2 * FM_EXP_N, tab + 2 * FM_EXP_N + FM_LOG_N};
+  const FastMath fm(tab);
   const ADMath<Dual> mth{fm};
   const Lay L{P.kall, P.gall, P.lall, P.prec_ld};
   const int l = blockIdx.y;
@@ -207,7 +207,7 @@ __global__ void __launch_bounds__(256) nsw6_adj_cellfwd_kernel(Problem P, Consts
   __shared__ double tab[FM_TABLE_DOUBLES];
   for (int c = threadIdx.x; c < FM_TABLE_DOUBLES; c += blockDim.x) tab[c] = P.fmtab[c];
   __syncthreads();
-  const FastMath fm{tab, tab + FM_EXP_N, tab + 2 * FM_EXP_N, tab + 2 * FM_EXP_N + FM_LOG_N};
+  const FastMath fm(tab);
   const Lay L{P.kall, P.gall, P.lall, P.prec_ld};
   const size_t NC = (size_t)P.lall * P.kall * P.gall;
   const int nint = P.kmax - P.kmin + 1;
@@ -267,7 +267,7 @@ __global__ void __launch_bounds__(AD_THREADS, 3) nsw6_adj_cell_kernel(Problem P,
   __shared__ double red[7][AD_THREADS];
   for (int c = threadIdx.x; c < FM_TABLE_DOUBLES; c += blockDim.x) tab[c] = P.fmtab[c];
   __syncthreads();
-  const FastMath fm{tab, tab + FM_EXP_N, tab + 2 * FM_EXP_N, tab + 2 * FM_EXP_N + FM_LOG_N};
+  const FastMath fm(tab);
   const ADMath<RVar> mth{fm};
   const Lay L{P.kall, P.gall, P.lall, P.prec_ld};
   const size_t NC = (size_t)P.lall * P.kall * P.gall;

@@ -331,28 +331,19 @@ Consts make_consts(const nsw6_params& p) {
   return make_consts(p, o);
 }
 
-// Fast-math tables (nsw6_fastmath.cuh), computed in extended precision:
-// [0,256) 2^(j/256) rounded; [256,512) its relative rounding error;
-// [512,768) 1/c_j; [768,1024) -log(1/c_j), where c_j is the centre of the j-th
-// of 256 mantissa intervals of [0.75, 1.5).
-void build_fastmath_tables(double* t) {
-  for (int j = 0; j < FM_EXP_N; ++j) {
-    const long double v = exp2l((long double)j / 256.0L);
-    t[j] = (double)v;
-    t[FM_EXP_N + j] = (double)(v / (long double)t[j] - 1.0L);
-  }
-  double* ic_t = t + 2 * FM_EXP_N;
-  double* lc_t = ic_t + FM_LOG_N;
-  for (int j = 0; j < FM_LOG_N; ++j) {
-    unsigned long long lo_bits = 0x3FE8000000000000ull + ((unsigned long long)j << 44);
-    unsigned long long hi_bits = lo_bits + (1ull << 44);
-    double mlo, mhi;
-    std::memcpy(&mlo, &lo_bits, 8);
-    std::memcpy(&mhi, &hi_bits, 8);
-    const long double cj = 0.5L * ((long double)mlo + (long double)mhi);
-    const double ic = (double)(1.0L / cj);
-    ic_t[j] = ic;
-    lc_t[j] = (double)(-logl((long double)ic));
+// Tables of the fixed-point exp2 and log2 (nsw6_soft.cuh, layout in
+// nsw6_fastmath.cuh), computed in extended precision.
+void build_fastmath_tables(double* tab) {
+  unsigned long long* t = reinterpret_cast<unsigned long long*>(tab);
+  unsigned long long* lt = t + SOFT_EXP_N;
+  unsigned short* ic = reinterpret_cast<unsigned short*>(lt + SOFT_LOG_N);
+  for (int j = 0; j < SOFT_EXP_N; ++j)
+    t[j] = (unsigned long long)(exp2l((long double)j / SOFT_EXP_N) * 9223372036854775808.0L + 0.5L);
+  for (int j = 0; j < SOFT_LOG_N; ++j) {
+    const int lo = SOFT_LOG_N + j;   // the interval's lower end in units of 1 / SOFT_LOG_N
+    const int n = (32768 * SOFT_LOG_N + lo - 1) / lo;
+    ic[j] = (unsigned short)n;
+    lt[j] = (unsigned long long)(-log2l((long double)n / 32768.0L) * 18446744073709551616.0L + 0.5L);
   }
 }
 
