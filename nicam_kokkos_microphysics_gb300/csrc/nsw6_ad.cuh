@@ -37,8 +37,9 @@ __device__ __forceinline__ Dual operator+(const Dual& a, const Dual& b) { return
 __device__ __forceinline__ Dual operator-(const Dual& a, const Dual& b) { return Dual(a.v - b.v, a.d - b.d); }
 __device__ __forceinline__ Dual operator*(const Dual& a, const Dual& b) { return Dual(a.v * b.v, a.d * b.v + a.v * b.d); }
 __device__ __forceinline__ Dual operator/(const Dual& a, const Dual& b) {
-  const double q = a.v / b.v;
-  return Dual(q, (a.d - q * b.d) / b.v);
+  const SoftDivisor by = soft_divisor(b.v);
+  const double q = soft_div(a.v, by, b.v);
+  return Dual(q, soft_div(a.d - q * b.d, by, b.v));
 }
 __device__ __forceinline__ Dual operator-(const Dual& a) { return Dual(-a.v, -a.d); }
 __device__ __forceinline__ Dual operator+(const Dual& a) { return a; }
@@ -67,8 +68,8 @@ __device__ __forceinline__ Dual fmaR(const Dual& a, const Dual& b, const Dual& c
   return Dual(__fma_rn(a.v, b.v, c.v), a.d * b.v + a.v * b.d + c.d);
 }
 __device__ __forceinline__ Dual sqrtR(const Dual& x) {
-  const double s = sqrt(x.v);
-  return Dual(s, s > 0.0 ? 0.5 * x.d / s : 0.0);
+  const double s = soft_sqrt(x.v);
+  return Dual(s, s > 0.0 ? soft_div(0.5 * x.d, s) : 0.0);
 }
 __device__ __forceinline__ Dual fabsR(const Dual& x) { return x.v < 0.0 ? -x : x; }
 __device__ __forceinline__ Dual dmin(const Dual& a, const Dual& b) { return (b < a) ? b : a; }
@@ -77,7 +78,6 @@ __device__ __forceinline__ Dual rate_on(const Dual& x) { return x.v > 0.0 ? x : 
 // The quotient helpers of the FP64 kernels give the correctly rounded a / b.
 __device__ __forceinline__ Dual div_rn(const Dual& a, const Dual& b, const Dual&) { return a / b; }
 __device__ __forceinline__ Dual sel(bool on, const Dual& x) { return on ? x : Dual(copysign(0.0, x.v)); }
-__device__ __forceinline__ Dual per_dt(const Dual& q, const Dual& dt, const Dual&) { return q / dt; }
 
 // ------------------------------------------------------------------ RVar
 // The per-thread tape lives in global memory, interleaved over the threads of
@@ -142,8 +142,9 @@ __device__ __forceinline__ RVar operator+(const RVar& a, const RVar& b) { return
 __device__ __forceinline__ RVar operator-(const RVar& a, const RVar& b) { return record(a.v - b.v, a.id, 1.0, b.id, -1.0); }
 __device__ __forceinline__ RVar operator*(const RVar& a, const RVar& b) { return record(a.v * b.v, a.id, b.v, b.id, a.v); }
 __device__ __forceinline__ RVar operator/(const RVar& a, const RVar& b) {
-  const double q = a.v / b.v;
-  return record(q, a.id, 1.0 / b.v, b.id, -q / b.v);
+  const SoftDivisor by = soft_divisor(b.v);
+  const double q = soft_div(a.v, by, b.v);
+  return record(q, a.id, soft_rcp(by, b.v), b.id, soft_div(-q, by, b.v));
 }
 __device__ __forceinline__ RVar operator-(const RVar& a) { return record(-a.v, a.id, -1.0, -1, 0.0); }
 __device__ __forceinline__ RVar operator+(const RVar& a) { return a; }
@@ -171,8 +172,8 @@ __device__ __forceinline__ RVar fmaR(const RVar& a, const RVar& b, const RVar& c
   return record(__fma_rn(a.v, b.v, c.v), ab.id, 1.0, c.id, 1.0);
 }
 __device__ __forceinline__ RVar sqrtR(const RVar& x) {
-  const double s = sqrt(x.v);
-  return record(s, x.id, s > 0.0 ? 0.5 / s : 0.0, -1, 0.0);
+  const double s = soft_sqrt(x.v);
+  return record(s, x.id, s > 0.0 ? soft_div(0.5, s) : 0.0, -1, 0.0);
 }
 __device__ __forceinline__ RVar fabsR(const RVar& x) { return x.v < 0.0 ? -x : x; }
 __device__ __forceinline__ RVar dmin(const RVar& a, const RVar& b) { return (b < a) ? b : a; }
@@ -180,7 +181,6 @@ __device__ __forceinline__ RVar dmax(const RVar& a, const RVar& b) { return (a <
 __device__ __forceinline__ RVar rate_on(const RVar& x) { return x.v > 0.0 ? x : RVar(dmax(x.v, 0.0)); }
 __device__ __forceinline__ RVar div_rn(const RVar& a, const RVar& b, const RVar&) { return a / b; }
 __device__ __forceinline__ RVar sel(bool on, const RVar& x) { return on ? x : RVar(copysign(0.0, x.v)); }
-__device__ __forceinline__ RVar per_dt(const RVar& q, const RVar& dt, const RVar&) { return q / dt; }
 
 // Reverse sweep of the calling thread's tape: propagates the adjoints seeded
 // in adj[] from the last entry to the first.
@@ -210,16 +210,16 @@ struct ADMath {
     const double e = fm.exp(val(x));
     return dep(e, x, e);
   }
-  __device__ __forceinline__ T log(const T& x) const { return dep(fm.log(val(x)), x, 1.0 / val(x)); }
+  __device__ __forceinline__ T log(const T& x) const { return dep(fm.log(val(x)), x, soft_div(1.0, val(x))); }
   __device__ __forceinline__ T pow(const T& x, const T& y) const {
     const double xv = val(x), yv = val(y);
     const double p = fm.pow(xv, yv);
     if (!(xv > 0.0)) return dep2(p, x, 0.0, y, 0.0);
     if constexpr (std::is_same<T, Dual>::value) {
       // a constant exponent (every pow of the scheme): no d/dy term, no log
-      if (y.d == 0.0) return Dual(p, (yv * p / xv) * x.d);
+      if (y.d == 0.0) return Dual(p, soft_div(yv * p, xv) * x.d);
     }
-    return dep2(p, x, yv * p / xv, y, p * fm.log(xv));
+    return dep2(p, x, soft_div(yv * p, xv), y, p * fm.log(xv));
   }
 };
 

@@ -286,22 +286,22 @@ __device__ void stage1(const In<T>& in, const double* gr, int k, const O& out, c
   }
   // metric factors and kinetic energy (mod_precip_transport.cpp:715-770)
   T rgs = T(0.0), kinh = T(0.0), kinv = T(0.0);
-  if (interior) rgs = xf(in, A_gam2, k) / xf(in, A_gsgam2, k);
+  if (interior) rgs = quo(xf(in, A_gam2, k), xf(in, A_gsgam2, k));
   const T vx = xf(in, A_vx, k), vy = xf(in, A_vy, k), vz = xf(in, A_vz, k);
   const T vi = vx * xc(in, A_ix) + vy * xc(in, A_iy) + vz * xc(in, A_iz);
   const T vj = vx * xc(in, A_jx) + vy * xc(in, A_jy) + vz * xc(in, A_jz);
   if (interior) {
     const T rvx = xf(in, A_rhogvx, k), rvy = xf(in, A_rhogvy, k), rvz = xf(in, A_rhogvz, k);
-    kinh = 0.5 * (rvx * rvx + rvy * rvy + rvz * rvz) / st_rhog(in, k);
+    kinh = quo(0.5 * (rvx * rvx + rvy * rvy + rvz * rvz), st_rhog(in, k));
   }
   const bool hk = (k >= kmin + 1 && k <= kmax);
   T rw = T(0.0);
   if (hk) {
     const T gh = xf(in, A_gsgam2h, k);
-    const T c2w0 = afact[k] / xf(in, A_gsgam2, k) * gh;
-    const T c2w1 = bfact[k] / xf(in, A_gsgam2, k - 1) * gh;
+    const T c2w0 = quo(afact[k], xf(in, A_gsgam2, k)) * gh;
+    const T c2w1 = quo(bfact[k], xf(in, A_gsgam2, k - 1)) * gh;
     rw = xf(in, A_rhogw, k);
-    kinv = 0.5 * (rw * rw) / (c2w0 * st_rhog(in, k) + c2w1 * st_rhog(in, k - 1));
+    kinv = quo(0.5 * (rw * rw), c2w0 * st_rhog(in, k) + c2w1 * st_rhog(in, k - 1));
   }
   out(W_KINH, kinh);
   out(W_KINV, kinv);
@@ -309,7 +309,7 @@ __device__ void stage1(const In<T>& in, const double* gr, int k, const O& out, c
   const T tem = interior ? st_tem(in, k) : T(0.0);
   const T zz = interior ? xf(in, A_z, k) : T(0.0);
   T rgsh = T(0.0);
-  if (hk) rgsh = xf(in, A_gam2h, k) / xf(in, A_gsgam2h, k);
+  if (hk) rgsh = quo(xf(in, A_gam2h, k), xf(in, A_gsgam2h, k));
   for (int t = 0; t < ntr; ++t) {
     const int nq = sed_tracer(t, ntr).nq;
     T base = T(0.0), qn = T(0.0);
@@ -391,7 +391,7 @@ __device__ void stage3(const In<T>& in, const double* gr, int k, const O& o, con
         switch (f) {
           case 0:
             dq[t] = -d;
-            if (nq == I_QR) fin(SF_GPREC, 0.0 + (-fk / dt));
+            if (nq == I_QR) fin(SF_GPREC, 0.0 + (-quo(fk, dt)));
             break;
           case 1: drhoe = drhoe - d; break;
           case 2: drhophi = drhophi - d; break;
@@ -403,15 +403,15 @@ __device__ void stage3(const In<T>& in, const double* gr, int k, const O& o, con
           switch (f) {
             case 0:
               if (nq == I_QR) {
-                acc[0] = acc[0] - fk / dt;
+                acc[0] = acc[0] - quo(fk, dt);
               } else {
-                acc[1] = acc[1] - fk / dt;
-                acc[2] = acc[2] + fk * LHF0 / dt;
+                acc[1] = acc[1] - quo(fk, dt);
+                acc[2] = acc[2] + quo(fk * LHF0, dt);
               }
               break;
-            case 1: acc[3] = acc[3] - fk / dt; break;
-            case 2: acc[4] = acc[4] - fk / dt; break;
-            case 3: acc[5] = acc[5] - fk / dt; break;
+            case 1: acc[3] = acc[3] - quo(fk, dt); break;
+            case 2: acc[4] = acc[4] - quo(fk, dt); break;
+            case 3: acc[5] = acc[5] - quo(fk, dt); break;
             default: break;
           }
         }
@@ -486,10 +486,10 @@ __device__ __forceinline__ T kinv_new(const In<T>& in, const double* gr, int j) 
   const double* afact = gr + GF_AFACT * K;
   const double* bfact = gr + GF_BFACT * K;
   const T gh = xf(in, A_gsgam2h, j);
-  const T c2w0 = afact[j] / xf(in, A_gsgam2, j) * gh;
-  const T c2w1 = bfact[j] / xf(in, A_gsgam2, j - 1) * gh;
+  const T c2w0 = quo(afact[j], xf(in, A_gsgam2, j)) * gh;
+  const T c2w1 = quo(bfact[j], xf(in, A_gsgam2, j - 1)) * gh;
   const T rw = in.w(W_RW_N, j);
-  return 0.5 * (rw * rw) / (c2w0 * in.w(W_RHOG_N, j) + c2w1 * in.w(W_RHOG_N, j - 1));
+  return quo(0.5 * (rw * rw), c2w0 * in.w(W_RHOG_N, j) + c2w1 * in.w(W_RHOG_N, j - 1));
 }
 
 // S4: KIN2EIN, thermodynamics, saturation adjustment and negative filter of
@@ -505,7 +505,7 @@ __device__ int stage4(const In<T>& in, const Consts& C, const double* gr, const 
   const bool interior = (k >= kmin && k <= kmax);
   const bool kin2kin = P.opt && C.opt_kin2kin != 0.0;
   const T rhog = in.w(W_RHOG_N, k);
-  const T rrhog = 1.0 / rhog;
+  const T rrhog = quo(1.0, rhog);
   T rhoge = in.w(W_RHOGE_N, k);
   const T gsg = xf(in, A_gsgam2, k);
   if (kin2kin) {
@@ -516,11 +516,11 @@ __device__ int stage4(const In<T>& in, const Consts& C, const double* gr, const 
     T rvx = in.w(W_RVX_N, k), rvy = in.w(W_RVY_N, k), rvz = in.w(W_RVZ_N, k), rw = in.w(W_RW_N, k);
     if (k >= kmin && k <= kmax + 1) {
       if (k <= kmax) {
-        const T kin_h0 = in.w(W_KINH_N, k) / rhog;
-        T vx_t = rvx / rhog, vy_t = rvy / rhog, vz_t = rvz / rhog;
+        const T kin_h0 = quo(in.w(W_KINH_N, k), rhog);
+        T vx_t = quo(rvx, rhog), vy_t = quo(rvy, rhog), vz_t = quo(rvz, rhog);
         const T kin_h = 0.5 * (vx_t * vx_t + vy_t * vy_t + vz_t * vz_t);
         if (val_of(kin_h) > 1.0E-20) {
-          const T r = sqrtR(fabsR(kin_h0 / kin_h));
+          const T r = sqrtR(fabsR(quo(kin_h0, kin_h)));
           vx_t = vx_t * r;
           vy_t = vy_t * r;
           vz_t = vz_t * r;
@@ -532,13 +532,13 @@ __device__ int stage4(const In<T>& in, const Consts& C, const double* gr, const 
       const double* afact = gr + GF_AFACT * K;
       const double* bfact = gr + GF_BFACT * K;
       const T gh = xf(in, A_gsgam2h, k);
-      const T c2w0 = afact[k] / gsg * gh;
-      const T c2w1 = bfact[k] / xf(in, A_gsgam2, k - 1) * gh;
+      const T c2w0 = quo(afact[k], gsg) * gh;
+      const T c2w1 = quo(bfact[k], xf(in, A_gsgam2, k - 1)) * gh;
       const T rhogh = c2w0 * rhog + c2w1 * in.w(W_RHOG_N, k - 1);
-      const T kin_v0 = in.w(W_KINV_N, k) / rhogh;
-      T w_t = rw / rhogh;
+      const T kin_v0 = quo(in.w(W_KINV_N, k), rhogh);
+      T w_t = quo(rw, rhogh);
       const T kin_v = 0.5 * (w_t * w_t);
-      if (val_of(kin_v) > 1.0E-20) w_t = w_t * sqrtR(fabsR(kin_v0 / kin_v));
+      if (val_of(kin_v) > 1.0E-20) w_t = w_t * sqrtR(fabsR(quo(kin_v0, kin_v)));
       rw = w_t * rhogh;
     }
     fin(SF_RVX, rvx);
@@ -548,7 +548,7 @@ __device__ int stage4(const In<T>& in, const Consts& C, const double* gr, const 
   } else if (interior) {
     // KIN2EIN (mod_precip_transport.cpp:991-1011): the transported kinetic
     // energy tmp2 less that of the updated state
-    const T gh = xf(in, A_gsgam2h, k + 1), rgh = 1.0 / gh;
+    const T gh = xf(in, A_gsgam2h, k + 1), rgh = quo(1.0, gh);
     const T w2c0 = div_rn(cfact[k] * gsg, gh, rgh);
     const T w2c1 = div_rn(dfact[k] * gsg, gh, rgh);
     const T tmp2 = in.w(W_KINH_N, k) + (w2c0 * in.w(W_KINV_N, k + 1) + w2c1 * in.w(W_KINV_N, k));
@@ -562,7 +562,7 @@ __device__ int stage4(const In<T>& in, const Consts& C, const double* gr, const 
   for (int n = 0; n < 6; ++n) rq[n] = in.w(W_RQ_N + n, k);
 #pragma unroll
   for (int n = 0; n < 6; ++n) q[n] = div_rn(rq[n], rhog, rrhog);
-  T rho = rhog / gsg;
+  T rho = quo(rhog, gsg);
   const T ein = div_rn(rhoge, rhog, rrhog);
   T qd = T(1.0);
 #pragma unroll
@@ -574,7 +574,7 @@ __device__ int stage4(const In<T>& in, const Consts& C, const double* gr, const 
     qdl = qdl - q[n];
   }
   cvt = cvt + qdl * CVDRY;
-  T tem = ein / cvt;
+  T tem = quo(ein, cvt);
   T pre = rho * tem * (qdl * RDRY + q[I_QV] * RVAP);
   // SATURATION_adjustment (mod_satadjust.cpp:274-362); with the switch
   // explicit_icegen = 0 cloud ice joins it (satadjust_all)
@@ -594,7 +594,7 @@ __device__ int stage4(const In<T>& in, const Consts& C, const double* gr, const 
 #pragma unroll
   for (int n = 1; n <= 5; ++n) cvtot = cvtot + q[n] * CVDRY;
   const T rho_l = rho;
-  tem = (ein_moist - q[I_QV] * LHV0) / cvtot;
+  tem = quo(ein_moist - q[I_QV] * LHV0, cvtot);
   int rc = 0;
   if (interior)
     rc = ice_adj ? satadjust_all_t(C, fm, P.itelim, ein_moist, qsum, rho_l, q, tem, iters)
@@ -622,8 +622,8 @@ __device__ int stage4(const In<T>& in, const Consts& C, const double* gr, const 
     rq[I_QV] = dmax(rq[I_QV], T(0.0));
     diffq -= rq[I_QV];
     rhog_o = rhog * (1.0 - diffq);
-    rho = rhog_o / gsg;
-    const T rrhog_o = 1.0 / rhog_o;
+    rho = quo(rhog_o, gsg);
+    const T rrhog_o = quo(1.0, rhog_o);
 #pragma unroll
     for (int n = 1; n <= 5; ++n) q[n] = div_rn(rq[n], rhog_o, rrhog_o);
     T qdf = T(1.0);
@@ -914,10 +914,10 @@ __global__ void __launch_bounds__(STAGE_THREADS) adj_s4_hw_kernel(StageIO io, Co
     const double* gsh = io.x.a[A_gsgam2h];
     // ------------------------------------------------------------ forward
     const double rhog = W(W_RHOG_N, c);
-    const double rrhog = 1.0 / rhog;
+    const double rrhog = quo(1.0, rhog);
     const double rhoge_a = W(W_RHOGE_N, c);
     const double gsg = gs[c];
-    const double rgsg = 1.0 / gsg;   // the reciprocals of gsgam2 at k - 1, k, k + 1 serve both sweeps
+    const double rgsg = quo(1.0, gsg);   // the reciprocals of gsgam2 at k - 1, k, k + 1 serve both sweeps
     double rg_up = 0.0, rg_dn = 0.0;
     double rhoge = rhoge_a;
     // KIN2EIN pieces
@@ -926,7 +926,7 @@ __global__ void __launch_bounds__(STAGE_THREADS) adj_s4_hw_kernel(StageIO io, Co
     bool hv[2] = {false, false};
     if (interior) {
       gh = gsh[c + G];
-      rgh = 1.0 / gh;
+      rgh = quo(1.0, gh);
       w2c0 = div_rn(cfact[k] * gsg, gh, rgh);
       w2c1 = div_rn(dfact[k] * gsg, gh, rgh);
       kinh = W(W_KINH_N, c);
@@ -944,14 +944,14 @@ __global__ void __launch_bounds__(STAGE_THREADS) adj_s4_hw_kernel(StageIO io, Co
         if (!hv[s2]) continue;
         const double ghj = gsh[cj];
         // afact / gs(j) and bfact / gs(j-1), correctly rounded, from the reciprocals
-        if (s2 == 0) rg_up = 1.0 / gs[cj];
-        else rg_dn = 1.0 / gs[cj - G];
+        if (s2 == 0) rg_up = quo(1.0, gs[cj]);
+        else rg_dn = quo(1.0, gs[cj - G]);
         const double rgj = s2 == 0 ? rg_up : rgsg, rgjm = s2 == 0 ? rgsg : rg_dn;
         c2a[s2] = div_rn(afact[j], gs[cj], rgj) * ghj;
         c2b[s2] = div_rn(bfact[j], gs[cj - G], rgjm) * ghj;
         rwj[s2] = W(W_RW_N, cj);
         den[s2] = c2a[s2] * W(W_RHOG_N, cj) + c2b[s2] * W(W_RHOG_N, cj - G);
-        kvu[s2] = 0.5 * (rwj[s2] * rwj[s2]) / den[s2];
+        kvu[s2] = quo(0.5 * (rwj[s2] * rwj[s2]), den[s2]);
       }
       const double tmp = tmp_h + (w2c0 * kvu[0] + w2c1 * kvu[1]);
       rhoge = rhoge_a + (tmp2 - tmp);
@@ -961,7 +961,7 @@ __global__ void __launch_bounds__(STAGE_THREADS) adj_s4_hw_kernel(StageIO io, Co
     for (int n = 0; n < 6; ++n) rq[n] = W(W_RQ_N + n, c);
 #pragma unroll
     for (int n = 0; n < 6; ++n) qo[n] = div_rn(rq[n], rhog, rrhog);
-    const double rho1 = rhog / gsg;
+    const double rho1 = quo(rhog, gsg);
     const double ein = div_rn(rhoge, rhog, rrhog);
     double qd = 1.0;
 #pragma unroll
@@ -974,7 +974,7 @@ __global__ void __launch_bounds__(STAGE_THREADS) adj_s4_hw_kernel(StageIO io, Co
       qdl = qdl - qo[n];
     }
     cvt = cvt + qdl * CVDRY;
-    const double tem0 = ein / cvt;
+    const double tem0 = quo(ein, cvt);
     const double pq0 = qdl * RDRY + qo[0] * RVAP;
     const double ein_moist = ein + qo[0] * LHV0;
     const double qsum = qo[0] + qo[1];
@@ -986,7 +986,7 @@ __global__ void __launch_bounds__(STAGE_THREADS) adj_s4_hw_kernel(StageIO io, Co
     double cvtot1 = qd * CVDRY;
 #pragma unroll
     for (int n = 1; n <= 5; ++n) cvtot1 = cvtot1 + q[n] * CVDRY;
-    const double tem_p = (ein_moist - q[0] * LHV0) / cvtot1;
+    const double tem_p = quo(ein_moist - q[0] * LHV0, cvtot1);
     double tem = tem_p;
     // saturation adjustment (satadjust_t's iteration, then its implicit derivative pieces)
     bool sat = false;
@@ -999,9 +999,9 @@ __global__ void __launch_bounds__(STAGE_THREADS) adj_s4_hw_kernel(StageIO io, Co
       // the test decided in FP32 where its margin allows (sat_screen_liq)
       sc = sat_screen_liq(tem, rho1, qsum, float(C.LovR_liq));
       if (sc < 0) {
-        const double rtem0 = 1.0 / fp_max_pos(tem, TEM_MIN);
+        const double rtem0 = quo(1.0, fp_max_pos(tem, TEM_MIN));
         const double psat0 = PSAT0 * fm.exp(C.LovR_liq * (C.RTEM00 - rtem0));
-        sc = (qsum - psat0 / (rho1 * RVAP * tem) > EPS) ? 1 : 0;
+        sc = (qsum - quo(psat0, rho1 * RVAP * tem) > EPS) ? 1 : 0;
       }
     }
     if (first) {
@@ -1030,9 +1030,9 @@ __global__ void __launch_bounds__(STAGE_THREADS) adj_s4_hw_kernel(StageIO io, Co
         int ite;
         for (ite = 0; ite < P.itelim; ++ite) {
           tprev = tv;
-          const double rtem = 1.0 / fp_max_pos(tv, TEM_MIN);
+          const double rtem = quo(1.0, fp_max_pos(tv, TEM_MIN));
           const double psat = PSAT0 * fm.exp(C.LovR_liq * (C.RTEM00 - rtem));
-          const double qsat = psat / (rho1 * RVAP * tv);
+          const double qsat = quo(psat, rho1 * RVAP * tv);
           qs_last = qsat;
           qv[I_QV] = qsat;
           qv[I_QC] = qsum - qsat;
@@ -1042,7 +1042,7 @@ __global__ void __launch_bounds__(STAGE_THREADS) adj_s4_hw_kernel(StageIO io, Co
           const double emoist_new = tv * cv + qv[I_QV] * LHV0;
           const double dqsat_dT = C.LovR_liq * rtem * rtem * qsat;
           const double demoist_dT = cv + dqsat_dT * LHV0;
-          const double dtemp = (emoist_new - ein_moist) / demoist_dT;
+          const double dtemp = quo(emoist_new - ein_moist, demoist_dT);
           tv = tv - dtemp;
           if (fp_abs_lt(dtemp, C.dtemp_criteria)) {
             converged = true;
@@ -1060,7 +1060,7 @@ __global__ void __launch_bounds__(STAGE_THREADS) adj_s4_hw_kernel(StageIO io, Co
           cvT = qd_l * CVDRY + (qsum - qsT) * CVDRY;
 #pragma unroll
           for (int n = 2; n <= 5; ++n) cvT = cvT + q[n] * CVDRY;
-          const double rts = 1.0 / ts;
+          const double rts = quo(1.0, ts);
           dqs = qsT * (C.LovR_liq * rts * rts - rts);
           FT = cvT - ts * dqs * CVDRY + dqs * LHV0;
         } else {
@@ -1109,8 +1109,8 @@ __global__ void __launch_bounds__(STAGE_THREADS) adj_s4_hw_kernel(StageIO io, Co
           if (n == I_QC ? fp_bits(q[I_QC]) != 0 : clip[n]) qf[n] = div_rn(rqf[n], rhog, rrhog);
       } else {
         rhog_o = rhog * (1.0 - d2);
-        rho_f = rhog_o / gsg;
-        rrhog_o = 1.0 / rhog_o;
+        rho_f = quo(rhog_o, gsg);
+        rrhog_o = quo(1.0, rhog_o);
 #pragma unroll
         for (int n = 1; n <= 5; ++n) qf[n] = div_rn(rqf[n], rhog_o, rrhog_o);
       }
@@ -1203,7 +1203,7 @@ __global__ void __launch_bounds__(STAGE_THREADS) adj_s4_hw_kernel(StageIO io, Co
       const double b_qsI = b_qv - b_qc;
       double b_qsT = b_qsI;
       const double b_temI = b_tem + b_qsI * dqs;
-      const double b_F = -b_temI * (1.0 / FT);
+      const double b_F = -b_temI * quo(1.0, FT);
       const double b_cvT = b_F * ts;
       b_qsT += b_F * LHV0;
       b_ein_moist -= b_F;
@@ -1219,7 +1219,7 @@ __global__ void __launch_bounds__(STAGE_THREADS) adj_s4_hw_kernel(StageIO io, Co
     }
     // tem_p = (ein_moist - qsum LHV0) / cvtot1, cvtot1 = qd CV + sum_{n >= 2} q[n] CV
     {
-      const double rcv1 = 1.0 / cvtot1;
+      const double rcv1 = quo(1.0, cvtot1);
       const double b_num = b_tem_p * rcv1;
       const double b_cv1 = -b_tem_p * tem_p * rcv1;
       b_ein_moist += b_num;
@@ -1244,7 +1244,7 @@ __global__ void __launch_bounds__(STAGE_THREADS) adj_s4_hw_kernel(StageIO io, Co
       const double b_pq0 = b_pre0 * rho1 * tem0;
       const double b_qdl0 = b_pq0 * RDRY;
       b_qo[0] += b_pq0 * RVAP;
-      const double rcvt = 1.0 / cvt;
+      const double rcvt = quo(1.0, cvt);
       b_ein += b_tem0 * rcvt;
       const double b_cvt = -b_tem0 * tem0 * rcvt;
       const double b_qdl = b_qdl0 + b_cvt * CVDRY;
@@ -1283,7 +1283,7 @@ __global__ void __launch_bounds__(STAGE_THREADS) adj_s4_hw_kernel(StageIO io, Co
         const int j = k + 1 - s2;
         const size_t cj = c + G - s2 * G;
         const double b_kvu = b_tmp * (s2 == 0 ? w2c0 : w2c1);
-        const double rden = 1.0 / den[s2];
+        const double rden = quo(1.0, den[s2]);
         WBadd(W_RW_N, cj, b_kvu * rwj[s2] * rden);
         const double b_den = -b_kvu * kvu[s2] * rden;
         WBadd(W_RHOG_N, cj, b_den * c2a[s2]);
@@ -1463,7 +1463,7 @@ __global__ void __launch_bounds__(STAGE_THREADS) adj_s1_hw_kernel(StageIO io) {
     // (recomputed for the partials only, so by reciprocals; no branch reads them)
     const size_t ck = c;   // (l, k, g) in the full-level fields
     const double gam2 = x[A_gam2][ck], gs = x[A_gsgam2][ck];
-    const double rgsr = 1.0 / gs;
+    const double rgsr = quo(1.0, gs);
     const double rgs = gam2 * rgsr;
     const double vx = x[A_vx][ck], vy = x[A_vy][ck], vz = x[A_vz][ck];
     const double ix = x[A_ix][cc], iy = x[A_iy][cc], iz = x[A_iz][cc];
@@ -1472,20 +1472,20 @@ __global__ void __launch_bounds__(STAGE_THREADS) adj_s1_hw_kernel(StageIO io) {
     const double vj = vx * jx + vy * jy + vz * jz;
     const double rvx = x[A_rhogvx][ck], rvy = x[A_rhogvy][ck], rvz = x[A_rhogvz][ck];
     const double rhog = Y(YS_RHOG, c);
-    const double rrhog = 1.0 / rhog;
+    const double rrhog = quo(1.0, rhog);
     const double kinh = 0.5 * (rvx * rvx + rvy * rvy + rvz * rvz) * rrhog;
     double gh = 0, rgh = 0, rgsm = 0, rden = 0, gsm = 0, c2w0 = 0, c2w1 = 0, rw = 0, rhogm = 0, den = 0, kinv = 0, gam2h = 0, rgsh = 0;
     if (hk) {
       gh = x[A_gsgam2h][ck];
       gsm = x[A_gsgam2][ck - G];
-      rgh = 1.0 / gh;
-      rgsm = 1.0 / gsm;
+      rgh = quo(1.0, gh);
+      rgsm = quo(1.0, gsm);
       c2w0 = afact[k] * rgsr * gh;
       c2w1 = bfact[k] * rgsm * gh;
       rw = x[A_rhogw][ck];
       rhogm = Y(YS_RHOG, c - G);
       den = c2w0 * rhog + c2w1 * rhogm;
-      rden = 1.0 / den;
+      rden = quo(1.0, den);
       kinv = 0.5 * (rw * rw) * rden;
       gam2h = x[A_gam2h][ck];
       rgsh = gam2h * rgh;

@@ -36,21 +36,10 @@
 #pragma once
 
 #include "nsw6_common.cuh"
+#include "nsw6_soft.cuh"
 #include "nsw6_fastmath.cuh"
 
 namespace nsw6 {
-
-// a / b rounded to nearest, given rb = 1 / b rounded to nearest: one product
-// and Markstein's correction step (r = a - q b is exact in an FMA, and q + r rb
-// rounds to the correctly rounded quotient).  Three FP64 instructions where a
-// division costs several times more; used where the reference divides by a
-// value the cell reuses, so that near-total consumption of a species leaves
-// the same residue as in the reference.
-__device__ __forceinline__ double div_rn(double a, double b, double rb) {
-  const double q = a * rb;
-  const double r = __fma_rn(-q, b, a);
-  return __fma_rn(r, rb, q);
-}
 
 template <class D>
 struct CellInT {
@@ -74,7 +63,7 @@ using CellOut = CellOutT<double>;
 // the plain path, FP32 in the mixed path).
 __device__ __forceinline__ double fmaR(double a, double b, double c) { return __fma_rn(a, b, c); }
 __device__ __forceinline__ float fmaR(float a, float b, float c) { return __fmaf_rn(a, b, c); }
-__device__ __forceinline__ double sqrtR(double x) { return sqrt(x); }
+__device__ __forceinline__ double sqrtR(double x) { return soft_sqrt(x); }
 __device__ __forceinline__ float sqrtR(float x) { return sqrtf(x); }
 __device__ __forceinline__ double fabsR(double x) { return fabs(x); }
 __device__ __forceinline__ float fabsR(float x) { return fabsf(x); }
@@ -96,10 +85,44 @@ __device__ __forceinline__ R rate_on(const R& x) { return dmax(x, R(0)); }
 __device__ __forceinline__ double sel(bool on, double x) { return on ? x : copysign(0.0, x); }
 __device__ __forceinline__ float sel(bool on, float x) { return on ? x : copysignf(0.0f, x); }
 
+// Quotients.  Doubles: correctly rounded on the integer pipe (nsw6_soft.cuh; a
+// division on the FP64 pipe takes 137 cycles of an SM, one of these about 35:
+// with these and the roots one 16900 x 42 region's FP64 step went 1.944 ->
+// 1.643 ms, the same bits); the other types divide natively.
+template <class A, class B>
+__device__ __forceinline__ auto quo(const A& a, const B& b) -> decltype(a / b) { return a / b; }
+__device__ __forceinline__ double quo(double a, double b) { return soft_div(a, b); }
+
+// A divisor that several quotients share: the first 32 bits of its reciprocal
+// are formed once.  div_rn: a / b, correctly rounded; rcp_of: 1 / b.
+template <class T>
+struct DivisorT {
+  T b;
+  __device__ __forceinline__ explicit DivisorT(const T& x) : b(x) {}
+};
+template <>
+struct DivisorT<double> {
+  SoftDivisor s;
+  double b;
+  __device__ __forceinline__ explicit DivisorT(double x) : s(soft_divisor(x)), b(x) {}
+};
+using Divisor = DivisorT<double>;
+template <class T>
+__device__ __forceinline__ T div_rn(const T& a, const DivisorT<T>& d) { return a / d.b; }
+__device__ __forceinline__ double div_rn(double a, const Divisor& d) { return soft_div_rn(a, d.s, d.b); }
+template <class T>
+__device__ __forceinline__ T rcp_of(const DivisorT<T>& d) { return 1.0 / d.b; }
+__device__ __forceinline__ double rcp_of(const Divisor& d) { return soft_rcp(d.s, d.b); }
+
+// The same where the caller has 1 / b too (the derivative types' form; the
+// divisor's part is common to the quotients by the same b).
+__device__ __forceinline__ double div_rn(double a, double b, double) { return soft_div_rn(a, soft_divisor(b), b); }
+
 // q / dt of the rates: the correctly rounded quotient in FP64 (the reference
 // divides), a product with 1/dt in FP32.
-__device__ __forceinline__ double per_dt(double q, double dt, double rdt) { return div_rn(q, dt, rdt); }
-__device__ __forceinline__ float per_dt(float q, float, float rdt) { return q * rdt; }
+template <class T>
+__device__ __forceinline__ T per_dt(const T& q, const DivisorT<T>& dt, const T&) { return div_rn(q, dt); }
+__device__ __forceinline__ float per_dt(float q, const DivisorT<float>&, float rdt) { return q * rdt; }
 
 // The comparisons of the cell physics with constants and the min / max they
 // select: for doubles the integer-pipe forms of nsw6_fpcmp.cuh (an FP64
@@ -199,11 +222,16 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
   rq[I_QV] = maxz(rq[I_QV]);
   diffq -= rq[I_QV];
   const D rhog = in.rhog * (1.0 - diffq);
-  const D rrhog = 1.0 / rhog;
+  const DivisorT<D> by_rhog(rhog);
+  D rrhog;   // mixed only
+  if constexpr (kMixed) rrhog = rcp_of(by_rhog);
   D qn[6];
   qn[0] = in.q0;
 #pragma unroll
-  for (int n = 1; n <= 5; ++n) qn[n] = kMixed ? rq[n] * rrhog : div_rn(rq[n], rhog, rrhog);
+  for (int n = 1; n <= 5; ++n) {
+    if constexpr (kMixed) qn[n] = rq[n] * rrhog;
+    else qn[n] = div_rn(rq[n], by_rhog);
+  }
   const D temp = in.tem;
   D rhoge;
   R pre, densR;
@@ -219,7 +247,7 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
     for (int n = 1; n <= 5; ++n) qdR = qdR - R(qn[n]);
     pre = densR * (qdR * R(RDRY) + R(qn[0]) * R(RVAP)) * R(temp);
   } else {
-    const D dens = rhog / in.gsgam2;
+    const D dens = quo(rhog, in.gsgam2);
     D qd = D(1.0);
 #pragma unroll
     for (int n = 1; n <= 5; ++n) qd = qd - qn[n];
@@ -233,10 +261,10 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
 
   // ---- psat / qsat (CPovR = 0 under EIN_TYPE "SIMPLE": the power term is 1)
   const R tempR = R(temp);
-  const R rtem = R(1.0) / maxc(tempR, R(TEM_MIN));
+  const R rtem = quo(R(1.0), maxc(tempR, R(TEM_MIN)));
   const R psatl = R(PSAT0) * mth.exp(C.LovR_liq * (C.RTEM00 - rtem));
   const R psati = R(PSAT0) * mth.exp(C.LovR_ice * (C.RTEM00 - rtem));
-  const R rdrt = R(1.0) / (densR * R(RVAP) * tempR);
+  const R rdrt = quo(R(1.0), densR * R(RVAP) * tempR);
   const R qsatl = psatl * rdrt;
   const R qsati = psati * rdrt;
 
@@ -244,17 +272,18 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
   const R Z = R(0.0), ONE = R(1.0);
   const R qv = maxz(R(qn[0])), qc = maxz(R(qn[1])), qr = maxz(R(qn[2]));
   const R qi = maxz(R(qn[3])), qs = maxz(R(qn[4])), qg = maxz(R(qn[5]));
-  const R Sliq = qv / maxc(qsatl, R(EPS));
-  const R Sice = qv / maxc(qsati, R(EPS));
-  const R Rdens = ONE / densR;
+  const R Sliq = quo(qv, maxc(qsatl, R(EPS)));
+  const R Sice = quo(qv, maxc(qsati, R(EPS)));
+  const R Rdens = quo(ONE, densR);
   const R rho_fact = sqrtR(R(DENS00) * Rdens);
   const R temc = tempR - R(TEM00);
   const bool warm = !lt_z(temc);  // iceflg = 0.5 - copysign(0.5, temc) == 0
   const bool d1 = ge_c(qr, R(1.0E-4));                          // delta1
   const bool d2 = le_c(qr, R(1.0E-4)) && le_c(qs, R(1.0E-4));       // delta2
   const bool sps = ge_c(Sice, ONE);                              // spsati
-  const R dqv_dt = per_dt(qv, dtR, rdtR), dqc_dt = per_dt(qc, dtR, rdtR), dqr_dt = per_dt(qr, dtR, rdtR);
-  const R dqi_dt = per_dt(qi, dtR, rdtR), dqs_dt = per_dt(qs, dtR, rdtR), dqg_dt = per_dt(qg, dtR, rdtR);
+  const DivisorT<R> by_dt(dtR);
+  const R dqv_dt = per_dt(qv, by_dt, rdtR), dqc_dt = per_dt(qc, by_dt, rdtR), dqr_dt = per_dt(qr, by_dt, rdtR);
+  const R dqi_dt = per_dt(qi, by_dt, rdtR), dqs_dt = per_dt(qs, by_dt, rdtR), dqg_dt = per_dt(qg, by_dt, rdtR);
 
   // The blocks of a species that is absent are skipped: every quantity they
   // would compute is then exactly zero (the reference evaluates them with a
@@ -320,7 +349,7 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
       const R lb = fmaR(fmaR(fmaR(b[3], tems, b[2]), tems, b[1]), tems, b[0]);
       mom[i] = mth.exp(fmaR(logX, lb, la));
     }
-    RMOMs_Vt = mom[5] / mom[2];
+    RMOMs_Vt = quo(mom[5], mom[2]);
   }
   const R MOMs_0 = mom[0], MOMs_1 = mom[1];
   const R MOMs_0bs = mom[2], MOMs_1bs = mom[3], MOMs_2bs = mom[4], MOMs_2ds = mom[5];
@@ -411,24 +440,24 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
     // Berry (1968), :1145-1147
     R Dc = C.Dc_berry;
     if constexpr (OPT) {
-      if (C.opt_indir != Z) Dc = R(0.146) - R(5.964E-2) * mth.log(Nc / R(2000.0));
+      if (C.opt_indir != Z) Dc = R(0.146) - R(5.964E-2) * mth.log(quo(Nc, R(2000.0)));
     }
-    Praut = Rdens * R(1.67E-5) * rhoqc * rhoqc / (R(5.0) + R(3.66E-2) * Nc / (Dc * rhoqc + R(EPS)));
+    Praut = quo(Rdens * R(1.67E-5) * rhoqc * rhoqc, R(5.0) + quo(R(3.66E-2) * Nc, Dc * rhoqc + R(EPS)));
   }
   R Psaut = rate_on(betai * (qi - C.qicrt_saut));
 
   // evaporation, sublimation, melting and freezing, :1174-1247
   const R Ka = (R(2.428E-2) + R(7.47E-5) * temc);
-  const R KdD = (R(2.222E-5) + R(1.37E-7) * temc) * R(PSTD) / pre * densR;   // Kd * dens
-  const R rNu = densR / (R(1.718E-5) + R(5.28E-8) * temc);                 // 1 / Nu
-  const R rKaT = ONE / (Ka * tempR);
+  const R KdD = quo((R(2.222E-5) + R(1.37E-7) * temc) * R(PSTD), pre) * densR;   // Kd * dens
+  const R rNu = quo(densR, R(1.718E-5) + R(5.28E-8) * temc);               // 1 / Nu
+  const R rKaT = quo(ONE, Ka * tempR);
   const R xi = KdD * qsati;
-  const R Giv = xi / (R(LHS0) * rKaT * (C.LovR_ice * rtem - ONE) * xi + ONE);
+  const R Giv = quo(xi, R(LHS0) * rKaT * (C.LovR_ice * rtem - ONE) * xi + ONE);
   const R Gil = Ka * temc * C.rLHF0;
   R Prevp = Z;
   if (rain) {
     const R xl = KdD * qsatl;
-    const R Glv = xl / (R(LHV0) * rKaT * (C.LovR_liq * rtem - ONE) * xl + ONE);
+    const R Glv = quo(xl, R(LHV0) * rKaT * (C.LovR_liq * rtem - ONE) * xl + ONE);
     const R ventr = C.K_ventr1 * RLMDr_2 + C.K_ventr2 * sqrtR(C.Cr * fr * rNu * RLMDr_5dr);
     Prevp = C.K_revp * Rdens * (ONE - minc(Sliq, ONE)) * Glv * ventr;
   }
@@ -437,7 +466,7 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
   R XNi = C.XNi_eps, Di = C.Di_eps;
   if (gt_c(rhoqi, R(EPS))) {
     XNi = minc(maxc(R(5.38E+7) * mth.pow(rhoqi, R(0.75)), R(1.0E+3)), R(1.0E+6));
-    const R XMi = rhoqi / XNi;
+    const R XMi = quo(rhoqi, XNi);
     Di = minc(C.Di_a * sqrtR(XMi), C.Di_max);
   }
   R tmp = R(4.0) * Di * XNi * Rdens * (Sice - ONE) * Giv;
@@ -477,10 +506,10 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
       const R a2 = (ONE - fact) * C.berg_a2[it] + fact * C.berg_a2[it + 1];
       const R ma2 = ONE - a2;
       const R a1 = ((ONE - fact) * C.berg_a1[it] + fact * C.berg_a1[it + 1]) * mth.pow(R(1.0E-3), ma2);
-      const R dt1 = (mth.exp(C.log_mi50 * ma2) - mth.exp(C.log_mi40 * ma2)) / (a1 * ma2);
-      const R Ni50 = qi * dtR / (C.mi50 * dt1);
+      const R dt1 = quo(mth.exp(C.log_mi50 * ma2) - mth.exp(C.log_mi40 * ma2), a1 * ma2);
+      const R Ni50 = quo(qi * dtR, C.mi50 * dt1);
       Psfw = Ni50 * (a1 * mth.pow(C.mi50, a2) + C.K_berg_w * densR * qc);
-      Psfi = qi / dt1;
+      Psfi = quo(qi, dt1);
     }
   }
 
@@ -528,7 +557,7 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
   // loss limiters, :1298-1477: fac = 1 when production >= loss - EPS,
   // else min(-dq/dt / net, 1) (the reference's (net - fac_sw) is net there)
   auto limiter = [&](R net, R dq) {
-    return is_nonneg(net + R(EPS)) ? ONE : dmin(-dq / net, ONE);
+    return is_nonneg(net + R(EPS)) ? ONE : dmin(quo(-dq, net), ONE);
   };
   // Scaling by fac = 1 is exact and skipped.  The tendencies below are the
   // nets the limiters form (same terms, same order) where no later scaling
@@ -670,7 +699,7 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
     R K_xf = C.K_xf, K_r2c = C.K_r2c;
     if constexpr (OPT) {
       if (C.opt_indir != Z) {
-        K_xf = R(1.0E-9) / Nc;
+        K_xf = quo(R(1.0E-9), Nc);
         K_r2c = C.coef_dgam * (Nc * R(1.0E+6));
       }
     }
@@ -681,12 +710,12 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
     const R r3_qr = C.coef_xf * densR * qr;
     const R r2 = r2_qc + r2_qr;
     const bool big = ge_c(r2, r2_min);
-    const R rceff = big ? (r3_qc + r3_qr) / r2 : Z;
+    const R rceff = big ? quo(r3_qc + r3_qr, r2) : Z;
     const bool top = !big && ge_c(qc + qr, q_min);
     o.rceff = D(rceff);
     o.rctop = top ? D(rceff) : D(UNDEF);
     o.tctop = top ? temp : D(UNDEF);
-    o.rceff_cld = ge_c(r2_qc, r2_min) ? D(r3_qc / r2_qc) : D(0.0);
+    o.rceff_cld = ge_c(r2_qc, r2_min) ? D(quo(r3_qc, r2_qc)) : D(0.0);
   }
 
   // ---- TagUpdateRHOGQ / RHOGE / MassConc / TEM, mod_mp_nsw6.cpp:692-744
@@ -701,14 +730,14 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
     o.tem = rhoge * rrhog * (1.0 / CVDRY);
   } else {
 #pragma unroll
-    for (int n = 1; n <= 5; ++n) o.q[n] = div_rn(rq[n], rhog, rrhog);
+    for (int n = 1; n <= 5; ++n) o.q[n] = div_rn(rq[n], by_rhog);
     D qd2 = D(1.0);
 #pragma unroll
     for (int n = 1; n <= 5; ++n) qd2 = qd2 - o.q[n];
     D cva = qd2 * CVDRY;
 #pragma unroll
     for (int n = 1; n <= 5; ++n) cva = cva + o.q[n] * CVDRY;
-    o.tem = rhoge / (rhog * cva);
+    o.tem = quo(rhoge, rhog * cva);
   }
   o.rhog = rhog;
   o.rhoge = rhoge;

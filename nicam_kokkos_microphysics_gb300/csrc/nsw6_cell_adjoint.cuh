@@ -72,7 +72,7 @@ __device__ __forceinline__ void bmaxc(T a, T c, T g, T& ba, T& bb) {
   else ba += g;
 }
 // d sqrt(x) / dx from s = sqrt(x)
-__device__ __forceinline__ double bsqrt(double s) { return s > 0.0 ? 0.5 / s : 0.0; }
+__device__ __forceinline__ double bsqrt(double s) { return s > 0.0 ? quo(0.5, s) : 0.0; }
 __device__ __forceinline__ float bsqrt(float s) { return s > 0.0f ? 0.5f / s : 0.0f; }
 
 // How a call treats the forward's costly values (quotients, square roots,
@@ -144,11 +144,12 @@ __device__ __forceinline__ void nsw6_cell_adjoint(const ConstsT<R>& C, const M& 
   d2 -= rq[0];
   const D omd = 1.0 - d2;
   const D rhog = in.rhog * omd;
-  const D rrhog = NSW6_CK(D, 0, 1.0 / rhog);
+  const Divisor by_rhog(rhog);
+  const D rrhog = NSW6_CK(D, 0, rcp_of(by_rhog));
   D qn[6];
   qn[0] = in.q0;
 #pragma unroll
-  for (int n = 1; n <= 5; ++n) qn[n] = kMixed ? rq[n] * rrhog : div_rn(rq[n], rhog, rrhog);
+  for (int n = 1; n <= 5; ++n) qn[n] = kMixed ? rq[n] * rrhog : div_rn(rq[n], by_rhog);
   const D temp = in.tem;
   const D trh = temp * rhog;
   D dens, rhoge0, cv = CVDRY, pq = 0.0, dp = 0.0;
@@ -165,7 +166,7 @@ __device__ __forceinline__ void nsw6_cell_adjoint(const ConstsT<R>& C, const M& 
     dpR = densR * pqR;
     pre = dpR * R(temp);
   } else {
-    dens = NSW6_CK(D, 1, rhog / in.gsgam2);
+    dens = NSW6_CK(D, 1, quo(rhog, in.gsgam2));
     D qd = 1.0;
 #pragma unroll
     for (int n = 1; n <= 5; ++n) qd = qd - qn[n];
@@ -182,7 +183,7 @@ __device__ __forceinline__ void nsw6_cell_adjoint(const ConstsT<R>& C, const M& 
   // ---- psat / qsat (rate precision from here to the tendencies)
   const R tempR = R(temp);
   const R tmx = maxc(tempR, R(TEM_MIN));
-  const R rtem = NSW6_CK(R, 2, ONE / tmx);
+  const R rtem = NSW6_CK(R, 2, quo(ONE, tmx));
   const R al = C.LovR_liq * (C.RTEM00 - rtem);
   const R ai = C.LovR_ice * (C.RTEM00 - rtem);
   const R el = NSW6_CK(R, 3, mth.exp(al)), ei = NSW6_CK(R, 4, mth.exp(ai));
@@ -190,7 +191,7 @@ __device__ __forceinline__ void nsw6_cell_adjoint(const ConstsT<R>& C, const M& 
   const R psati = R(PSAT0) * ei;
   const R drv = densR * R(RVAP);
   const R drt = drv * tempR;
-  const R rdrt = NSW6_CK(R, 5, ONE / drt);
+  const R rdrt = NSW6_CK(R, 5, quo(ONE, drt));
   const R qsatl = psatl * rdrt;
   const R qsati = psati * rdrt;
 
@@ -198,9 +199,9 @@ __device__ __forceinline__ void nsw6_cell_adjoint(const ConstsT<R>& C, const M& 
   const R qv = maxz(R(qn[0])), qc = maxz(R(qn[1])), qr = maxz(R(qn[2]));
   const R qi = maxz(R(qn[3])), qs = maxz(R(qn[4])), qg = maxz(R(qn[5]));
   const R sld = maxc(qsatl, R(EPS)), sid = maxc(qsati, R(EPS));
-  const R Sliq = NSW6_CK(R, 6, qv / sld);
-  const R Sice = NSW6_CK(R, 7, qv / sid);
-  const R Rdens = NSW6_CK(R, 8, ONE / densR);
+  const R Sliq = NSW6_CK(R, 6, quo(qv, sld));
+  const R Sice = NSW6_CK(R, 7, quo(qv, sid));
+  const R Rdens = NSW6_CK(R, 8, quo(ONE, densR));
   const R rfa = R(DENS00) * Rdens;
   const R rho_fact = NSW6_CK(R, 9, sqrtR(rfa));
   const R temc = tempR - R(TEM00);
@@ -208,8 +209,9 @@ __device__ __forceinline__ void nsw6_cell_adjoint(const ConstsT<R>& C, const M& 
   const bool d1 = ge_c(qr, R(1.0E-4));
   const bool d2b = le_c(qr, R(1.0E-4)) && le_c(qs, R(1.0E-4));
   const bool sps = ge_c(Sice, ONE);
-  const R dqv_dt = per_dt(qv, dtR, rdtR), dqc_dt = per_dt(qc, dtR, rdtR), dqr_dt = per_dt(qr, dtR, rdtR);
-  const R dqi_dt = per_dt(qi, dtR, rdtR), dqs_dt = per_dt(qs, dtR, rdtR), dqg_dt = per_dt(qg, dtR, rdtR);
+  const DivisorT<R> by_dt(dtR);
+  const R dqv_dt = per_dt(qv, by_dt, rdtR), dqc_dt = per_dt(qc, by_dt, rdtR), dqr_dt = per_dt(qr, by_dt, rdtR);
+  const R dqi_dt = per_dt(qi, by_dt, rdtR), dqs_dt = per_dt(qs, by_dt, rdtR), dqg_dt = per_dt(qg, by_dt, rdtR);
 
   // rain slope parameter
   const bool rain = ge_c(qr, R(1.0E-12));
@@ -256,7 +258,7 @@ __device__ __forceinline__ void nsw6_cell_adjoint(const ConstsT<R>& C, const M& 
       mlb[i] = lb;
       mom[i] = NSW6_CK(R, 14 + i, mth.exp(fmaR(logX, lb, la)));
     }
-    RMOMs_Vt = NSW6_CK(R, 21, mom[5] / mom[2]);
+    RMOMs_Vt = NSW6_CK(R, 21, quo(mom[5], mom[2]));
   }
   const R MOMs_0 = mom[0], MOMs_1 = mom[1], MOMs_2 = Xs2;
   const R MOMs_0bs = mom[2], MOMs_1bs = mom[3], MOMs_2bs = mom[4], MOMs_2ds = mom[5];
@@ -370,12 +372,12 @@ __device__ __forceinline__ void nsw6_cell_adjoint(const ConstsT<R>& C, const M& 
   const R Ka = (R(2.428E-2) + R(7.47E-5) * temc);
   const R kd0 = (R(2.222E-5) + R(1.37E-7) * temc);
   const R kd1 = kd0 * R(PSTD);
-  const R kd2 = NSW6_CK(R, 29, kd1 / pre);
+  const R kd2 = NSW6_CK(R, 29, quo(kd1, pre));
   const R KdD = kd2 * densR;
   const R nu0 = (R(1.718E-5) + R(5.28E-8) * temc);
-  const R rNu = NSW6_CK(R, 30, densR / nu0);
+  const R rNu = NSW6_CK(R, 30, quo(densR, nu0));
   const R kat = Ka * tempR;
-  const R rKaT = NSW6_CK(R, 31, ONE / kat);
+  const R rKaT = NSW6_CK(R, 31, quo(ONE, kat));
   const R xi = KdD * qsati;
   const R gv1 = R(LHS0) * rKaT;
   const R gv2 = C.LovR_ice * rtem;
@@ -383,7 +385,7 @@ __device__ __forceinline__ void nsw6_cell_adjoint(const ConstsT<R>& C, const M& 
   const R gv4 = gv1 * gv3;
   const R gv5 = gv4 * xi;
   const R gv6 = gv5 + ONE;
-  const R Giv = NSW6_CK(R, 32, xi / gv6);
+  const R Giv = NSW6_CK(R, 32, quo(xi, gv6));
   const R gil_a = Ka * temc;
   const R Gil = gil_a * C.rLHF0;
   R Prevp = Z;
@@ -399,7 +401,7 @@ __device__ __forceinline__ void nsw6_cell_adjoint(const ConstsT<R>& C, const M& 
     gl4 = gl1 * gl3;
     gl5 = gl4 * xl;
     gl6 = gl5 + ONE;
-    Glv = NSW6_CK(R, 33, xl / gl6);
+    Glv = NSW6_CK(R, 33, quo(xl, gl6));
     vr1 = C.K_ventr1 * RLMDr_2;
     vr2 = C.Cr * fr;
     vr3 = vr2 * rNu;
@@ -428,7 +430,7 @@ __device__ __forceinline__ void nsw6_cell_adjoint(const ConstsT<R>& C, const M& 
     const R xm = xn_lo ? R(1.0E+3) : xn_a;
     xn_hi = gt_c(xm, R(1.0E+6));               // dmin(xm, 1e6) gives 1e6
     XNi = xn_hi ? R(1.0E+6) : xm;
-    XMi = NSW6_CK(R, 36, rhoqi / XNi);
+    XMi = NSW6_CK(R, 36, quo(rhoqi, XNi));
     di_s = NSW6_CK(R, 37, sqrtR(XMi));
     di_a = C.Di_a * di_s;
     di_cap = gt_c(di_a, C.Di_max);
@@ -534,7 +536,7 @@ __device__ __forceinline__ void nsw6_cell_adjoint(const ConstsT<R>& C, const M& 
       L.fac = ONE;
       L.ratio = false;
     } else {
-      const R r = NSW6_CK(R, slot, -dq / net);
+      const R r = NSW6_CK(R, slot, quo(-dq, net));
       L.ratio = !gt_c(r, ONE);
       L.fac = L.ratio ? r : ONE;
     }
@@ -652,7 +654,7 @@ __device__ __forceinline__ void nsw6_cell_adjoint(const ConstsT<R>& C, const M& 
     tem_o = NSW6_CK(D, 48, rhoge * rrhog * (1.0 / CVDRY));
   } else {
 #pragma unroll
-    for (int n = 1; n <= 5; ++n) q2[n] = div_rn(rq2[n], rhog, rrhog);
+    for (int n = 1; n <= 5; ++n) q2[n] = div_rn(rq2[n], by_rhog);
     D qd2 = 1.0;
 #pragma unroll
     for (int n = 1; n <= 5; ++n) qd2 = qd2 - q2[n];
@@ -660,7 +662,7 @@ __device__ __forceinline__ void nsw6_cell_adjoint(const ConstsT<R>& C, const M& 
 #pragma unroll
     for (int n = 1; n <= 5; ++n) cva = cva + q2[n] * CVDRY;
     rcva = rhog * cva;
-    tem_o = NSW6_CK(D, 48, rhoge / rcva);
+    tem_o = NSW6_CK(D, 48, quo(rhoge, rcva));
   }
   if constexpr (MODE == CA_SAVE) {
     // the outputs of nsw6_cell (the same operations on the same values)
@@ -668,10 +670,10 @@ __device__ __forceinline__ void nsw6_cell_adjoint(const ConstsT<R>& C, const M& 
     out->Vts = D(Vts);
     out->Vtg = D(Vtg);
     out->Vti = 0.0;
-    out->rceff = big ? D(r3 / r2) : 0.0;
+    out->rceff = big ? D(quo(r3, r2)) : 0.0;
     out->rctop = top ? out->rceff : UNDEF;
     out->tctop = top ? temp : UNDEF;
-    out->rceff_cld = cld ? D(r3_qc / r2_qc) : 0.0;
+    out->rceff_cld = cld ? D(quo(r3_qc, r2_qc)) : 0.0;
 #pragma unroll
     for (int n = 0; n < 6; ++n) {
       out->q[n] = q2[n];
@@ -699,7 +701,7 @@ __device__ __forceinline__ void nsw6_cell_adjoint(const ConstsT<R>& C, const M& 
       b_rhoge = fma(g, rrhog * (1.0 / CVDRY), b_rhoge);
       b_rhog = fma(-g * tem_o, rrhog, b_rhog);
     } else {
-      const D rr = 1.0 / rcva;
+      const D rr = quo(1.0, rcva);
       b_rhoge = fma(g, rr, b_rhoge);
       const D b_rcva = -g * tem_o * rr;
       b_rhog = fma(b_rcva, cva, b_rhog);
@@ -777,7 +779,7 @@ __device__ __forceinline__ void nsw6_cell_adjoint(const ConstsT<R>& C, const M& 
     R b_r2_qc = Z, b_r2_qr = Z, b_r3_qc = Z, b_r3_qr = Z;
     // rceff = big ? r3 / r2 : 0
     if (big) {
-      const R rr2 = ONE / r2;
+      const R rr2 = quo(ONE, r2);
       const R b_r3 = R(ob.rceff * sc) * rr2;
       const R b_r2 = -R(ob.rceff * sc) * (r3 * rr2) * rr2;
       b_r3_qc += b_r3;
@@ -789,7 +791,7 @@ __device__ __forceinline__ void nsw6_cell_adjoint(const ConstsT<R>& C, const M& 
     if (top) b_tempD += ob.tctop;
     // rceff_cld = cld ? r3_qc / r2_qc : 0
     if (cld) {
-      const R rr2 = ONE / r2_qc;
+      const R rr2 = quo(ONE, r2_qc);
       b_r3_qc = fmaR(R(ob.rceff_cld * sc), rr2, b_r3_qc);
       b_r2_qc = fmaR(-(R(ob.rceff_cld * sc) * (r3_qc * rr2)), rr2, b_r2_qc);
     }
@@ -801,7 +803,7 @@ __device__ __forceinline__ void nsw6_cell_adjoint(const ConstsT<R>& C, const M& 
     b_RLMDr_3 = fmaR(b_r2_qr, C.K_r2r, b_RLMDr_3);
     // r2_qc = K_r2c rf^2, rf = pow(xf3, 1/3)
     const R b_rf = b_r2_qc * C.K_r2c * R(2.0) * rf_qc;
-    const R b_xf3 = gt_z(xf3) ? b_rf * R(0.33333333) * rf_qc / xf3 : Z;
+    const R b_xf3 = gt_z(xf3) ? quo(b_rf * R(0.33333333) * rf_qc, xf3) : Z;
     b_rhoqc = fmaR(b_xf3 * C.coef_xf, C.K_xf, b_rhoqc);
   }
   // Vt outputs
@@ -843,7 +845,7 @@ __device__ __forceinline__ void nsw6_cell_adjoint(const ConstsT<R>& C, const M& 
       *bx[j] *= L.fac;
     }
     if (L.ratio) {   // fac = -dq / net
-      const R rnet = ONE / L.net;
+      const R rnet = quo(ONE, L.net);
       b_dq = fmaR(-b_fac, rnet, b_dq);
       const R b_net = b_fac * dq * (rnet * rnet);
       for (int j = 0; j < n; ++j) *bx[j] += sgn[j] * b_net;
@@ -1044,14 +1046,14 @@ __device__ __forceinline__ void nsw6_cell_adjoint(const ConstsT<R>& C, const M& 
       const R b_dia = b_Di;
       const R b_dis = b_dia * C.Di_a;
       const R b_XMi = b_dis * bsqrt(di_s);
-      const R rXNi = ONE / XNi;
+      const R rXNi = quo(ONE, XNi);
       b_rhoqi = fmaR(b_XMi, rXNi, b_rhoqi);
       b_XNi = fmaR(-(b_XMi * XMi), rXNi, b_XNi);
     }
     // XNi = min(max(5.38e7 pow(rhoqi, 0.75), 1e3), 1e6)
     if (!xn_hi && !xn_lo) {
       const R b_pow = b_XNi * R(5.38E+7);
-      if (gt_z(rhoqi)) b_rhoqi += b_pow * R(0.75) * xn_pow / rhoqi;
+      if (gt_z(rhoqi)) b_rhoqi += quo(b_pow * R(0.75) * xn_pow, rhoqi);
     }
   }
   if (rqi_on) {
@@ -1078,7 +1080,7 @@ __device__ __forceinline__ void nsw6_cell_adjoint(const ConstsT<R>& C, const M& 
     b_Cr = fmaR(b_vr2, fr, b_Cr);
     b_rho_fact = fmaR(b_vr2, C.Cr, b_rho_fact);
     // Glv = xl / (((LHV0 rKaT) (LovR_liq rtem - 1)) xl + 1)
-    const R rgl6 = ONE / gl6;
+    const R rgl6 = quo(ONE, gl6);
     const R b_xl0 = b_Glv * rgl6;
     const R b_gl6 = -b_Glv * Glv * rgl6;
     const R b_gl4 = b_gl6 * xl;
@@ -1103,7 +1105,7 @@ __device__ __forceinline__ void nsw6_cell_adjoint(const ConstsT<R>& C, const M& 
   }
   // Giv = xi / (((LHS0 rKaT) (LovR_ice rtem - 1)) xi + 1)
   {
-    const R rgv6 = ONE / gv6;
+    const R rgv6 = quo(ONE, gv6);
     const R b_xi0 = b_Giv * rgv6;
     const R b_gv6 = -b_Giv * Giv * rgv6;
     const R b_gv4 = b_gv6 * xi;
@@ -1120,7 +1122,7 @@ __device__ __forceinline__ void nsw6_cell_adjoint(const ConstsT<R>& C, const M& 
   }
   // rNu = dens / nu0, nu0 = 1.718e-5 + 5.28e-8 temc
   {
-    const R rnu0 = ONE / nu0;
+    const R rnu0 = quo(ONE, nu0);
     b_dens = fmaR(b_rNu, rnu0, b_dens);
     const R b_nu0 = -b_rNu * rNu * rnu0;
     b_temc = fmaR(b_nu0, R(5.28E-8), b_temc);
@@ -1129,7 +1131,7 @@ __device__ __forceinline__ void nsw6_cell_adjoint(const ConstsT<R>& C, const M& 
   {
     b_dens = fmaR(b_KdD, kd2, b_dens);
     const R b_kd2 = b_KdD * densR;
-    const R rpre = ONE / pre;
+    const R rpre = quo(ONE, pre);
     const R b_kd1 = b_kd2 * rpre;
     b_pre = fmaR(-(b_kd2 * kd2), rpre, b_pre);
     b_temc = fmaR(b_kd1 * R(PSTD), R(1.37E-7), b_temc);
@@ -1148,7 +1150,7 @@ __device__ __forceinline__ void nsw6_cell_adjoint(const ConstsT<R>& C, const M& 
   // Praut = K_aut pow(qc, 2.47)
   if (aut_on) {
     b_K_aut = fmaR(bPraut, aut_pow, b_K_aut);
-    if (gt_z(qc)) b_qc += bPraut * C.K_aut * R(2.47) * aut_pow / qc;
+    if (gt_z(qc)) b_qc += quo(bPraut * C.K_aut * R(2.47) * aut_pow, qc);
   }
   // rhoqc = (dens qc) 1000 (read by the effective radius)
   b_dens = fmaR(b_rhoqc * R(1000.0), qc, b_dens);
@@ -1253,7 +1255,7 @@ __device__ __forceinline__ void nsw6_cell_adjoint(const ConstsT<R>& C, const M& 
   if (prw_on) {
     const R b_pow = bPracw0 * R(67.0);
     if (gt_z(qcqr)) {
-      const R b_qcqr = b_pow * R(1.15) * prw_pow / qcqr;
+      const R b_qcqr = quo(b_pow * R(1.15) * prw_pow, qcqr);
       b_qc = fmaR(b_qcqr, qr, b_qc);
       b_qr = fmaR(b_qcqr, qc, b_qr);
     }
@@ -1326,7 +1328,7 @@ __device__ __forceinline__ void nsw6_cell_adjoint(const ConstsT<R>& C, const M& 
   // snow moments: Vts's RMOMs_Vt = mom5 / mom2; mom_i = exp(logX lb_i + la_i(tems)); MOMs_2 = Xs2
   R b_Xs2 = b_MOMs_2;
   if (snow) {
-    const R rm2 = ONE / mom[2];
+    const R rm2 = quo(ONE, mom[2]);
     b_mom[5] = fmaR(b_RMOMs_Vt, rm2, b_mom[5]);
     b_mom[2] = fmaR(-(b_RMOMs_Vt * RMOMs_Vt), rm2, b_mom[2]);
     R b_logX = Z, b_tems = Z;
@@ -1341,7 +1343,7 @@ __device__ __forceinline__ void nsw6_cell_adjoint(const ConstsT<R>& C, const M& 
       const R dlb = fmaR(fmaR(R(3.0) * b[3], tems, R(2.0) * b[2]), tems, b[1]);
       b_tems = fmaR(b_arg, (dla + logX * dlb), b_tems);
     }
-    b_Xs2 += b_logX / Xs2;
+    b_Xs2 += quo(b_logX, Xs2);
     if (tems_sel) b_temc += b_tems;
   }
   {
@@ -1386,12 +1388,12 @@ __device__ __forceinline__ void nsw6_cell_adjoint(const ConstsT<R>& C, const M& 
   b_dens = fmaR(-(b_Rdens * Rdens), Rdens, b_dens);
   // Sliq = qv / max(qsatl, EPS), Sice = qv / max(qsati, EPS)
   {
-    const R rsld = ONE / sld;
+    const R rsld = quo(ONE, sld);
     b_qv = fmaR(b_Sliq, rsld, b_qv);
     const R b_sld = -b_Sliq * Sliq * rsld;
     R dummy = Z;
     bmaxc(qsatl, R(EPS), b_sld, b_qsatl, dummy);
-    const R rsid = ONE / sid;
+    const R rsid = quo(ONE, sid);
     b_qv = fmaR(b_Sice, rsid, b_qv);
     const R b_sid = -b_Sice * Sice * rsid;
     bmaxc(qsati, R(EPS), b_sid, b_qsati, dummy);
@@ -1463,7 +1465,7 @@ __device__ __forceinline__ void nsw6_cell_adjoint(const ConstsT<R>& C, const M& 
       b_rq[n] = fma(b_qn[n], rrhog, b_rq[n]);
       b_rhogD = fma(-(b_qn[n] * qn[n]), rrhog, b_rhogD);
     }
-    const D rgs = 1.0 / in.gsgam2;
+    const D rgs = quo(1.0, in.gsgam2);
     b_rhogD = fma(b_densD, rgs, b_rhogD);
     ib.gsgam2 = fma(-b_densD * dens, rgs, ib.gsgam2);
   }

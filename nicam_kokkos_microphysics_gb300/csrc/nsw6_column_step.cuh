@@ -170,18 +170,18 @@ __device__ __forceinline__ int satadjust_t(const Consts& C, const FastMath& fm, 
   double qv[6];
 #pragma unroll
   for (int n = 0; n < 6; ++n) qv[n] = val(q[n]);
-  double rtem = 1.0 / (dmax(tv, TEM_MIN));
+  double rtem = quo(1.0, dmax(tv, TEM_MIN));
   double psat = PSAT0 * fm.exp(C.LovR_liq * (C.RTEM00 - rtem));
-  double qsat = psat / (rhov * RVAP * tv);
+  double qsat = quo(psat, rhov * RVAP * tv);
   if (!(qsumv - qsat > EPS)) return 0;
   bool converged = false;
   int ite;
   double tprev = tv;
   for (ite = 0; ite < itelim; ++ite) {
     tprev = tv;
-    rtem = 1.0 / (dmax(tv, TEM_MIN));
+    rtem = quo(1.0, dmax(tv, TEM_MIN));
     psat = PSAT0 * fm.exp(C.LovR_liq * (C.RTEM00 - rtem));
-    qsat = psat / (rhov * RVAP * tv);
+    qsat = quo(psat, rhov * RVAP * tv);
     qv[I_QV] = qsat;
     qv[I_QC] = qsumv - qsat;
     double cv = qdv * CVDRY;
@@ -190,7 +190,7 @@ __device__ __forceinline__ int satadjust_t(const Consts& C, const FastMath& fm, 
     const double emoist_new = tv * cv + qv[I_QV] * LHV0;
     const double dqsat_dT = C.LovR_liq * rtem * rtem * qsat;
     const double demoist_dT = cv + dqsat_dT * LHV0;
-    const double dtemp = (emoist_new - emv) / demoist_dT;
+    const double dtemp = quo(emoist_new - emv, demoist_dT);
     tv = tv - dtemp;
     if (fabs(dtemp) < C.dtemp_criteria) {
       converged = true;
@@ -209,12 +209,12 @@ __device__ __forceinline__ int satadjust_t(const Consts& C, const FastMath& fm, 
   // sum q[2..5]) CVdry, evaluated with T-typed inputs at the converged value
   const double ts = tprev;
   const T Tc = T(ts);
-  const T qsT = T(PSAT0) * T(fm.exp(C.LovR_liq * (C.RTEM00 - 1.0 / dmax(ts, TEM_MIN)))) / (rho_l * RVAP * Tc);
+  const T qsT = quo(T(PSAT0) * T(fm.exp(C.LovR_liq * (C.RTEM00 - quo(1.0, dmax(ts, TEM_MIN))))), rho_l * RVAP * Tc);
   T cvT = qd_l * CVDRY + (qsum - qsT) * CVDRY;
 #pragma unroll
   for (int n = 2; n <= 5; ++n) cvT = cvT + q[n] * CVDRY;
   const T F = Tc * cvT + qsT * LHV0 - ein_moist;
-  const double rts = 1.0 / ts;
+  const double rts = quo(1.0, ts);
   const double qs_v = val(qsT);
   const double dqs = qs_v * (C.LovR_liq * rts * rts - rts);   // d qsat / dT (T > TEM_MIN)
   const double cv_v = val(cvT);
@@ -251,12 +251,12 @@ __device__ __forceinline__ int satadjust_all_t(const Consts& C, const FastMath& 
 #pragma unroll
   for (int n = 0; n < 6; ++n) qv[n] = val(q[n]);
   {
-    const double rtem = 1.0 / (dmax(tv, TEM_MIN));
+    const double rtem = quo(1.0, dmax(tv, TEM_MIN));
     double psat = PSAT0 * fm.exp(C.LovR_liq * (C.RTEM00 - rtem));
-    const double alpha = dmin(dmax((tv - LL) / (UL - LL), 0.0), 1.0);
+    const double alpha = dmin(dmax(quo(tv - LL, UL - LL), 0.0), 1.0);
     const double psati = PSAT0 * fm.exp(C.LovR_ice * (C.RTEM00 - rtem));
     psat = psat * alpha + psati * (1.0 - alpha);
-    const double qsat = psat / (rhov * RVAP * tv);
+    const double qsat = quo(psat, rhov * RVAP * tv);
     if (!(qsumv - qsat > EPS)) return 0;
   }
   bool converged = false;
@@ -264,14 +264,14 @@ __device__ __forceinline__ int satadjust_all_t(const Consts& C, const FastMath& 
   double tprev = tv, alpha_s = 0.0, dalpha_s = 0.0, psatl_s = 0.0, psati_s = 0.0;
   for (ite = 0; ite < itelim; ++ite) {
     tprev = tv;
-    const double alpha = dmin(dmax((tv - LL) / (UL - LL), 0.0), 1.0);
-    const double rtem = 1.0 / (dmax(tv, TEM_MIN));
+    const double alpha = dmin(dmax(quo(tv - LL, UL - LL), 0.0), 1.0);
+    const double rtem = quo(1.0, dmax(tv, TEM_MIN));
     const double psatl = PSAT0 * fm.exp(C.LovR_liq * (C.RTEM00 - rtem));
     const double psati = PSAT0 * fm.exp(C.LovR_ice * (C.RTEM00 - rtem));
     const double psat = psatl * alpha + psati * (1.0 - alpha);
-    const double qsatl = psatl / (rhov * RVAP * tv);
-    const double qsati = psati / (rhov * RVAP * tv);
-    const double qsat = psat / (rhov * RVAP * tv);
+    const double qsatl = quo(psatl, rhov * RVAP * tv);
+    const double qsati = quo(psati, rhov * RVAP * tv);
+    const double qsat = quo(psat, rhov * RVAP * tv);
     qv[I_QV] = qsat;
     qv[I_QC] = (qsumv - qsat) * alpha;
     qv[I_QI] = (qsumv - qsat) * (1.0 - alpha);
@@ -279,16 +279,16 @@ __device__ __forceinline__ int satadjust_all_t(const Consts& C, const FastMath& 
 #pragma unroll
     for (int n = 1; n <= 5; ++n) cv = cv + qv[n] * CVDRY;
     const double emoist_new = tv * cv + qv[I_QV] * LHV0 - qv[I_QI] * LHF0;
-    const double dalpha_dT = (!(UL - tv < 0.0) && !(tv - LL < 0.0)) ? 1.0 / (UL - LL) : 0.0;
+    const double dalpha_dT = (!(UL - tv < 0.0) && !(tv - LL < 0.0)) ? quo(1.0, UL - LL) : 0.0;
     const double t2 = tv * tv;
-    const double dqsatl_dT = (C.LovR_liq / t2) * qsatl;
-    const double dqsati_dT = (C.LovR_ice / t2) * qsati;
+    const double dqsatl_dT = quo(C.LovR_liq, t2) * qsatl;
+    const double dqsati_dT = quo(C.LovR_ice, t2) * qsati;
     const double dqsat_dT = qsatl * dalpha_dT + dqsatl_dT * alpha - qsati * dalpha_dT + dqsati_dT * (1.0 - alpha);
     const double dqc_dT = (qsumv - qsat) * dalpha_dT - dqsat_dT * alpha;
     const double dqi_dT = -(qsumv - qsat) * dalpha_dT - dqsat_dT * (1.0 - alpha);
     const double dcv_dT = dqsat_dT * CVDRY + dqc_dT * CVDRY + dqi_dT * CVDRY;
     const double demoist_dT = tv * dcv_dT + cv + dqsat_dT * LHV0 - dqi_dT * LHF0;
-    const double dtemp = (emoist_new - emv) / demoist_dT;
+    const double dtemp = quo(emoist_new - emv, demoist_dT);
     alpha_s = alpha;
     dalpha_s = dalpha_dT;
     psatl_s = psatl;
@@ -312,7 +312,7 @@ __device__ __forceinline__ int satadjust_all_t(const Consts& C, const FastMath& 
   // saturation pressures held at their values there)
   const double ts = tprev;
   const T Tc = T(ts);
-  const T qsT = T(psatl_s * alpha_s + psati_s * (1.0 - alpha_s)) / (rho_l * RVAP * Tc);
+  const T qsT = quo(T(psatl_s * alpha_s + psati_s * (1.0 - alpha_s)), rho_l * RVAP * Tc);
   const T exc = qsum - qsT;
   const T qcT = exc * alpha_s, qiT = exc * (1.0 - alpha_s);
   T cvT = qd_l * CVDRY;
@@ -323,8 +323,8 @@ __device__ __forceinline__ int satadjust_all_t(const Consts& C, const FastMath& 
   cvT = cvT + q[5] * CVDRY;
   const T F = Tc * cvT + qsT * LHV0 - qiT * LHF0 - ein_moist;
   // exact T-slopes at ts
-  const double rts = 1.0 / ts;
-  const double qsl = psatl_s / (rhov * RVAP * ts), qsi = psati_s / (rhov * RVAP * ts);
+  const double rts = quo(1.0, ts);
+  const double qsl = quo(psatl_s, rhov * RVAP * ts), qsi = quo(psati_s, rhov * RVAP * ts);
   const double dqsl = qsl * (C.LovR_liq * rts * rts - rts), dqsi = qsi * (C.LovR_ice * rts * rts - rts);
   const double qs_v = val(qsT), exc_v = qsumv - qs_v;
   const double dqs = dqsl * alpha_s + dqsi * (1.0 - alpha_s) + (qsl - qsi) * dalpha_s;
@@ -450,16 +450,16 @@ __device__ void column_transport_phase(const Consts& C, const FastMath& fm, cons
     w.kinh[k] = T(0.0);
     w.kinv[k] = T(0.0);
     const bool interior = (k >= kmin && k <= kmax);
-    if (interior) w.rgs[k] = s.gam2[k] / s.gsgam2[k];
+    if (interior) w.rgs[k] = quo(s.gam2[k], s.gsgam2[k]);
     w.vi[k] = s.vx[k] * s.ix + s.vy[k] * s.iy + s.vz[k] * s.iz;
     w.vj[k] = s.vx[k] * s.jx + s.vy[k] * s.jy + s.vz[k] * s.jz;
     if (interior)
-      w.kinh[k] = 0.5 * (s.rhogvx[k] * s.rhogvx[k] + s.rhogvy[k] * s.rhogvy[k] + s.rhogvz[k] * s.rhogvz[k]) / s.rhog[k];
+      w.kinh[k] = quo(0.5 * (s.rhogvx[k] * s.rhogvx[k] + s.rhogvy[k] * s.rhogvy[k] + s.rhogvz[k] * s.rhogvz[k]), s.rhog[k]);
     if (k >= kmin + 1 && k <= kmax) {
-      const T c2w0 = afact[k] / s.gsgam2[k] * s.gsgam2h[k];
-      const T c2w1 = bfact[k] / s.gsgam2[k - 1] * s.gsgam2h[k];
+      const T c2w0 = quo(afact[k], s.gsgam2[k]) * s.gsgam2h[k];
+      const T c2w1 = quo(bfact[k], s.gsgam2[k - 1]) * s.gsgam2h[k];
       const T rw = s.rhogw[k];
-      w.kinv[k] = 0.5 * (rw * rw) / (c2w0 * s.rhog[k] + c2w1 * s.rhog[k - 1]);
+      w.kinv[k] = quo(0.5 * (rw * rw), c2w0 * s.rhog[k] + c2w1 * s.rhog[k - 1]);
     }
   }
 
@@ -500,7 +500,7 @@ __device__ void column_transport_phase(const Consts& C, const FastMath& fm, cons
         switch (f) {
           case 0:
             w.dq[t][k] = -d;
-            if (nq == I_QR) s.GPREC[k] = 0.0 + (-fk / dt);
+            if (nq == I_QR) s.GPREC[k] = 0.0 + (-quo(fk, dt));
             break;
           case 1: w.drhoe[k] = w.drhoe[k] - d; break;
           case 2: w.drhophi[k] = w.drhophi[k] - d; break;
@@ -512,15 +512,15 @@ __device__ void column_transport_phase(const Consts& C, const FastMath& fm, cons
           switch (f) {
             case 0:
               if (nq == I_QR) {
-                acc[0] = acc[0] - fk / dt;
+                acc[0] = acc[0] - quo(fk, dt);
               } else {
-                acc[1] = acc[1] - fk / dt;
-                acc[2] = acc[2] + fk * LHF0 / dt;
+                acc[1] = acc[1] - quo(fk, dt);
+                acc[2] = acc[2] + quo(fk * LHF0, dt);
               }
               break;
-            case 1: acc[3] = acc[3] - fk / dt; break;
-            case 2: acc[4] = acc[4] - fk / dt; break;
-            case 3: acc[5] = acc[5] - fk / dt; break;
+            case 1: acc[3] = acc[3] - quo(fk, dt); break;
+            case 2: acc[4] = acc[4] - quo(fk, dt); break;
+            case 3: acc[5] = acc[5] - quo(fk, dt); break;
             default: break;
           }
         }
@@ -530,7 +530,7 @@ __device__ void column_transport_phase(const Consts& C, const FastMath& fm, cons
     for (int k = 0; k < K; ++k) {
       T qh = T(0.0);
       if (k >= kmin + 1 && k <= kmax) {
-        qh = 0.5 * (s.q[nq][k] + s.q[nq][k - 1]) * (s.gam2h[k] / s.gsgam2h[k]);
+        qh = 0.5 * (s.q[nq][k] + s.q[nq][k - 1]) * quo(s.gam2h[k], s.gsgam2h[k]);
         w.kc[k] = (unsigned char)departure_cell_t(gzs, k, val(zdis0h[k]), bmn[3 + t][k], bmx[3 + t][k], kmin + 1,
                                                   kmax);
       }
@@ -591,16 +591,16 @@ __device__ void column_transport_phase(const Consts& C, const FastMath& fm, cons
     w.drhoe[k] = T(0.0);
     w.drhophi[k] = T(0.0);
     if (k >= kmin && k <= kmax) {
-      const T gh = s.gsgam2h[k + 1], rgh = 1.0 / gh;
+      const T gh = s.gsgam2h[k + 1], rgh = quo(1.0, gh);
       const T w2c0 = div_rn(cfact[k] * s.gsgam2[k], gh, rgh);
       const T w2c1 = div_rn(dfact[k] * s.gsgam2[k], gh, rgh);
       w.drhoe[k] = w.kinh[k] + (w2c0 * w.kinv[k + 1] + w2c1 * w.kinv[k]);
     }
     if (k >= kmin + 1 && k <= kmax) {
-      const T c2w0 = afact[k] / s.gsgam2[k] * s.gsgam2h[k];
-      const T c2w1 = bfact[k] / s.gsgam2[k - 1] * s.gsgam2h[k];
+      const T c2w0 = quo(afact[k], s.gsgam2[k]) * s.gsgam2h[k];
+      const T c2w1 = quo(bfact[k], s.gsgam2[k - 1]) * s.gsgam2h[k];
       const T rw = s.rhogw[k];
-      w.drhophi[k] = 0.5 * (rw * rw) / (c2w0 * s.rhog[k] + c2w1 * s.rhog[k - 1]);
+      w.drhophi[k] = quo(0.5 * (rw * rw), c2w0 * s.rhog[k] + c2w1 * s.rhog[k - 1]);
     }
   }
 
@@ -608,12 +608,12 @@ __device__ void column_transport_phase(const Consts& C, const FastMath& fm, cons
   for (int k = 0; k < K; ++k) {
     const bool interior = (k >= kmin && k <= kmax);
     const T rhog = s.rhog[k];
-    const T rrhog = 1.0 / rhog;
+    const T rrhog = quo(1.0, rhog);
     T rhoge = s.rhoge[k];
     if (interior) {
       const T rvx = s.rhogvx[k], rvy = s.rhogvy[k], rvz = s.rhogvz[k];
       const T tmp_h = div_rn(0.5 * (rvx * rvx + rvy * rvy + rvz * rvz), rhog, rrhog);
-      const T gh = s.gsgam2h[k + 1], rgh = 1.0 / gh;
+      const T gh = s.gsgam2h[k + 1], rgh = quo(1.0, gh);
       const T w2c0 = div_rn(cfact[k] * s.gsgam2[k], gh, rgh);
       const T w2c1 = div_rn(dfact[k] * s.gsgam2[k], gh, rgh);
       const T tmp = tmp_h + (w2c0 * w.drhophi[k + 1] + w2c1 * w.drhophi[k]);
@@ -625,7 +625,7 @@ __device__ void column_transport_phase(const Consts& C, const FastMath& fm, cons
 #pragma unroll
     for (int n = 0; n < 6; ++n) q[n] = div_rn(rq[n], rhog, rrhog);
     const T gsg = s.gsgam2[k];
-    T rho = rhog / gsg;
+    T rho = quo(rhog, gsg);
     const T ein = div_rn(rhoge, rhog, rrhog);
     T qd = T(1.0);
 #pragma unroll
@@ -637,7 +637,7 @@ __device__ void column_transport_phase(const Consts& C, const FastMath& fm, cons
       qdl = qdl - q[n];
     }
     cvt = cvt + qdl * CVDRY;
-    T tem = ein / cvt;
+    T tem = quo(ein, cvt);
     T pre = rho * tem * (qdl * RDRY + q[I_QV] * RVAP);
     const T ein_moist = ein + q[I_QV] * LHV0;
     const T qsum = q[I_QV] + q[I_QC];
@@ -647,7 +647,7 @@ __device__ void column_transport_phase(const Consts& C, const FastMath& fm, cons
 #pragma unroll
     for (int n = 1; n <= 5; ++n) cvtot = cvtot + q[n] * CVDRY;
     const T rho_l = rho;
-    tem = (ein_moist - q[I_QV] * LHV0) / cvtot;
+    tem = quo(ein_moist - q[I_QV] * LHV0, cvtot);
     if (interior) {
       int iters = 0;
       const int rc = satadjust_t(C, fm, itelim, ein_moist, qsum, rho_l, q, tem, &iters);
@@ -678,8 +678,8 @@ __device__ void column_transport_phase(const Consts& C, const FastMath& fm, cons
       rq[I_QV] = dmax(rq[I_QV], T(0.0));
       diffq -= rq[I_QV];
       rhog_o = rhog * (1.0 - diffq);
-      rho = rhog_o / gsg;
-      const T rrhog_o = 1.0 / rhog_o;
+      rho = quo(rhog_o, gsg);
+      const T rrhog_o = quo(1.0, rhog_o);
 #pragma unroll
       for (int n = 1; n <= 5; ++n) q[n] = div_rn(rq[n], rhog_o, rrhog_o);
       T qdf = T(1.0);

@@ -5,6 +5,7 @@
 #include <cstdint>
 
 #include "nsw6_fpcmp.cuh"
+#include "nsw6_soft.cuh"
 
 #ifndef __CUDACC__
 #define __host__
@@ -164,6 +165,7 @@ struct Problem {
   double dt, dt2, dt3;   // dt, pow(dt,2), pow(dt,3) as vadv1d_prep forms them (mod_vadv1d.cpp:265-266)
   double hdt2, sdt3;     // dt^2 / 2 and dt^3 / 6
   double rdt;            // 1 / dt
+  SoftDivisor by_dt;     // dt as a divisor (nsw6_soft.cuh)
   int itelim;
   int math_lib;                // 0 table-driven transcendentals, 1 CUDA libm
   int mixed;                   // 0 plain FP64 step, 1 mixed precision (FP32 process rates)

@@ -332,8 +332,9 @@ Consts make_consts(const nsw6_params& p) {
 }
 
 // Tables of the fixed-point exp2 and log2 (nsw6_soft.cuh, layout in
-// nsw6_fastmath.cuh), computed in extended precision.
-void build_fastmath_tables(double* tab) {
+// nsw6_fastmath.cuh), computed in extended precision, once per process (some
+// 0.8 ms where long double is emulated).
+void make_fastmath_tables(double* tab) {
   unsigned long long* t = reinterpret_cast<unsigned long long*>(tab);
   unsigned long long* lt = t + SOFT_EXP_N;
   unsigned short* ic = reinterpret_cast<unsigned short*>(lt + SOFT_LOG_N);
@@ -345,6 +346,15 @@ void build_fastmath_tables(double* tab) {
     ic[j] = (unsigned short)n;
     lt[j] = (unsigned long long)(-log2l((long double)n / 32768.0L) * 18446744073709551616.0L + 0.5L);
   }
+}
+
+void build_fastmath_tables(double* tab) {
+  struct Tables {
+    double t[FM_TABLE_DOUBLES];
+    Tables() { make_fastmath_tables(t); }
+  };
+  static const Tables made;
+  std::memcpy(tab, made.t, sizeof(made.t));
 }
 
 // GRD_Setup, mod_debug.cpp:92-187, plus GRD_gz_shift (mod_precip_transport.cpp:698-709).
@@ -478,6 +488,7 @@ int fill_problem(nsw6_handle* h, int lall, double* const* a, double dt, Problem&
   P.grid = h->d_grid;
   P.fmtab = h->d_fmtab;
   P.rdt = 1.0 / dt;
+  P.by_dt = soft_divisor(dt);
   P.math_lib = h->math_lib;
   P.mixed = h->mixed;
   P.opt = h->opt_active;

@@ -399,14 +399,15 @@ __device__ __forceinline__ double satadjust_newton(const Problem& P, const Const
     // satadjust_all, mod_satadjust.cpp:686-754 (CPovR = CVovR = 0, all CVW = CVdry)
     const double UL = C.sat_ulimit, LL = C.sat_llimit;
     for (ite = 0; ite < P.itelim; ++ite) {
-      const double alpha = dmin(dmax((tem - LL) / (UL - LL), 0.0), 1.0);
-      const double rtem = 1.0 / fp_max_pos(tem, TEM_MIN);
+      const double alpha = dmin(dmax(quo(tem - LL, UL - LL), 0.0), 1.0);
+      const double rtem = quo(1.0, fp_max_pos(tem, TEM_MIN));
       const double psatl = PSAT0 * mth.exp(C.LovR_liq * (C.RTEM00 - rtem));
       const double psati = PSAT0 * mth.exp(C.LovR_ice * (C.RTEM00 - rtem));
       const double psat = psatl * alpha + psati * (1.0 - alpha);
-      const double qsatl = psatl / (rho_l * RVAP * tem);
-      const double qsati = psati / (rho_l * RVAP * tem);
-      const double qsat = psat / (rho_l * RVAP * tem);
+      const Divisor by_rt(rho_l * RVAP * tem);
+      const double qsatl = soft_div(psatl, by_rt.s, by_rt.b);
+      const double qsati = soft_div(psati, by_rt.s, by_rt.b);
+      const double qsat = soft_div(psat, by_rt.s, by_rt.b);
       q[I_QV] = qsat;
       q[I_QC] = (qsum - qsat) * alpha;
       q[I_QI] = (qsum - qsat) * (1.0 - alpha);
@@ -414,16 +415,16 @@ __device__ __forceinline__ double satadjust_newton(const Problem& P, const Const
 #pragma unroll
       for (int n = 1; n <= 5; ++n) cv = cv + q[n] * CVDRY;
       const double emoist_new = tem * cv + q[I_QV] * LHV0 - q[I_QI] * LHF0;
-      const double dalpha_dT = (!(UL - tem < 0.0) && !(tem - LL < 0.0)) ? 1.0 / (UL - LL) : 0.0;
+      const double dalpha_dT = (!(UL - tem < 0.0) && !(tem - LL < 0.0)) ? quo(1.0, UL - LL) : 0.0;
       const double t2 = tem * tem;
-      const double dqsatl_dT = (C.LovR_liq / t2) * qsatl;
-      const double dqsati_dT = (C.LovR_ice / t2) * qsati;
+      const double dqsatl_dT = quo(C.LovR_liq, t2) * qsatl;
+      const double dqsati_dT = quo(C.LovR_ice, t2) * qsati;
       const double dqsat_dT = qsatl * dalpha_dT + dqsatl_dT * alpha - qsati * dalpha_dT + dqsati_dT * (1.0 - alpha);
       const double dqc_dT = (qsum - qsat) * dalpha_dT - dqsat_dT * alpha;
       const double dqi_dT = -(qsum - qsat) * dalpha_dT - dqsat_dT * (1.0 - alpha);
       const double dcv_dT = dqsat_dT * CVDRY + dqc_dT * CVDRY + dqi_dT * CVDRY;
       const double demoist_dT = tem * dcv_dT + cv + dqsat_dT * LHV0 - dqi_dT * LHF0;
-      const double dtemp = (emoist_new - ein_moist) / demoist_dT;
+      const double dtemp = quo(emoist_new - ein_moist, demoist_dT);
       tem = tem - dtemp;
       if (fp_abs_lt(dtemp, C.dtemp_criteria)) {
         converged = true;
@@ -433,9 +434,9 @@ __device__ __forceinline__ double satadjust_newton(const Problem& P, const Const
     }
   } else {
     for (ite = 0; ite < P.itelim; ++ite) {
-      const double rtem = 1.0 / fp_max_pos(tem, TEM_MIN);
+      const double rtem = quo(1.0, fp_max_pos(tem, TEM_MIN));
       const double psat = PSAT0 * mth.exp(C.LovR_liq * (C.RTEM00 - rtem));
-      const double qsat = psat / (rho_l * RVAP * tem);
+      const double qsat = quo(psat, rho_l * RVAP * tem);
       q[I_QV] = qsat;
       q[I_QC] = qsum - qsat;
       double cv = qd_l * CVDRY;
@@ -446,7 +447,7 @@ __device__ __forceinline__ double satadjust_newton(const Problem& P, const Const
       // dCVtot/dT = dqsat/dT (CVW(QV) - CVW(QC)) = 0 (all CVW = CVdry)
       const double dqsat_dT = C.LovR_liq * rtem * rtem * qsat;
       const double demoist_dT = cv + dqsat_dT * LHV0;
-      const double dtemp = (emoist_new - ein_moist) / demoist_dT;
+      const double dtemp = quo(emoist_new - ein_moist, demoist_dT);
       tem = tem - dtemp;
       if (fp_abs_lt(dtemp, C.dtemp_criteria)) {
         converged = true;
@@ -462,7 +463,7 @@ __device__ __forceinline__ double satadjust_newton(const Problem& P, const Const
 // The final state of one cell after the transport and KIN2EIN: thermodynamics,
 // saturation adjustment, negative filter and outputs (mod_mp_driver.cpp:
 // 555-612 with mod_thrmdyn.cpp, mod_satadjust.cpp:274-362 and
-// mod_mp_nsw6.cpp:1770-1831).  rhog, its reciprocal and rhoge (after KIN2EIN)
+// mod_mp_nsw6.cpp:1770-1831).  rhog, the divisor it makes and rhoge (after KIN2EIN)
 // are the cell's; the rest comes from the state arrays.  With newton = false
 // (the column kernel) a saturated interior cell is left as it is and true is
 // returned, for nsw6_satadj_kernel; every other cell is finished.  With
@@ -470,8 +471,9 @@ __device__ __forceinline__ double satadjust_newton(const Problem& P, const Const
 // formed, the Newton iteration runs and the cell is finished.
 template <class M, bool MIX, bool OPT>
 __device__ __forceinline__ bool final_cell(const Problem& P, const Consts& C, const M& mth, bool ice_adj, float lovr_f,
-                                           size_t i, size_t iq, size_t KG, bool interior, double rhog, double rrhog,
-                                           double rhoge, bool newton, int k, int g, int l) {
+                                           size_t i, size_t iq, size_t KG, bool interior, double rhog,
+                                           const Divisor& by_rhog, double rhoge, bool newton, int k, int g, int l) {
+  const double rrhog = MIX ? rcp_of(by_rhog) : 0.0;
   double rq[6], q[6];
 #pragma unroll
   for (int n = 0; n < 6; ++n) rq[n] = P.rhogq[iq + (size_t)n * KG];
@@ -480,10 +482,10 @@ __device__ __forceinline__ bool final_cell(const Problem& P, const Consts& C, co
   // in which one unit in the last place of qsum is already a relative error
   // of 1e-11 when qc is small.
 #pragma unroll
-  for (int n = 0; n < 6; ++n) q[n] = MIX ? rq[n] * rrhog : div_rn(rq[n], rhog, rrhog);
+  for (int n = 0; n < 6; ++n) q[n] = MIX ? rq[n] * rrhog : div_rn(rq[n], by_rhog);
   const double gsg = P.gsgam2[i];
-  double rho = rhog / gsg;
-  const double ein = MIX ? rhoge * rrhog : div_rn(rhoge, rhog, rrhog);
+  double rho = quo(rhog, gsg);
+  const double ein = MIX ? rhoge * rrhog : div_rn(rhoge, by_rhog);
   double qd = 1.0;
 #pragma unroll
   for (int n = 1; n <= 5; ++n) qd = qd - q[n];
@@ -499,7 +501,7 @@ __device__ __forceinline__ bool final_cell(const Problem& P, const Consts& C, co
       qdl = qdl - q[n];
     }
     cvt = cvt + qdl * CVDRY;
-    const double tem0 = ein / cvt;
+    const double tem0 = quo(ein, cvt);
     pre = rho * tem0 * (qdl * RDRY + q[I_QV] * RVAP);
   }
 
@@ -525,7 +527,7 @@ __device__ __forceinline__ bool final_cell(const Problem& P, const Consts& C, co
     if (n != I_QI || !ice_adj) cvtot = MIX ? cvtot + q[n] : cvtot + q[n] * CVDRY;
   if (MIX) cvtot = cvtot * CVDRY;
   const double rho_l = rho;
-  double tem = (ein_moist - q[I_QV] * LHV0) / cvtot;
+  double tem = quo(ein_moist - q[I_QV] * LHV0, cvtot);
   if (interior) {
     // satadjust_liq (mod_satadjust.cpp:771-896) or satadjust_all
     // (:620-769)
@@ -541,15 +543,15 @@ __device__ __forceinline__ bool final_cell(const Problem& P, const Consts& C, co
     // saturation only, sat_screen_liq); the FP64 test decides the rest.
     int sat = ice_adj ? -1 : sat_screen_liq(tem, rho_l, qsum, lovr_f);
     if (sat < 0) {
-      const double rtem = 1.0 / fp_max_pos(tem, TEM_MIN);
+      const double rtem = quo(1.0, fp_max_pos(tem, TEM_MIN));
       double psat = PSAT0 * mth.exp(C.LovR_liq * (C.RTEM00 - rtem));
       if (ice_adj) {
         const double alpha =
-            dmin(dmax((tem - C.sat_llimit) / (C.sat_ulimit - C.sat_llimit), 0.0), 1.0);
+            dmin(dmax(quo(tem - C.sat_llimit, C.sat_ulimit - C.sat_llimit), 0.0), 1.0);
         const double psati = PSAT0 * mth.exp(C.LovR_ice * (C.RTEM00 - rtem));
         psat = psat * alpha + psati * (1.0 - alpha);
       }
-      const double qsat = psat / (rho_l * RVAP * tem);
+      const double qsat = quo(psat, rho_l * RVAP * tem);
       sat = (qsum - qsat > EPS) ? 1 : 0;
     }
     if (sat) return true;
@@ -592,7 +594,7 @@ __device__ __forceinline__ bool final_cell(const Problem& P, const Consts& C, co
       const unsigned same = (0x34u | (ice_adj && newton ? 0u : 0x08u) | (newton ? 0u : 0x02u)) & ~clamped;
 #pragma unroll
       for (int n = 1; n <= 5; ++n)
-        if (!((same >> n) & 1u)) q[n] = MIX ? rq[n] * rrhog : div_rn(rq[n], rhog, rrhog);
+        if (!((same >> n) & 1u)) q[n] = MIX ? rq[n] * rrhog : div_rn(rq[n], by_rhog);
       // an unsaturated cell's q[QC] (and q[QI] in satadjust_all) is still +0
       const unsigned zero = newton ? 0u : (ice_adj ? 0x0Au : 0x02u);
       qdf = 1.0;
@@ -608,10 +610,11 @@ __device__ __forceinline__ bool final_cell(const Problem& P, const Consts& C, co
       }
     } else {
       rhog_o = rhog * (1.0 - diffq);
-      rho = rhog_o / gsg;
-      const double rrhog_o = 1.0 / rhog_o;
+      rho = quo(rhog_o, gsg);
+      const Divisor by_rhog_o(rhog_o);
+      const double rrhog_o = MIX ? rcp_of(by_rhog_o) : 0.0;
 #pragma unroll
-      for (int n = 1; n <= 5; ++n) q[n] = MIX ? rq[n] * rrhog_o : div_rn(rq[n], rhog_o, rrhog_o);
+      for (int n = 1; n <= 5; ++n) q[n] = MIX ? rq[n] * rrhog_o : div_rn(rq[n], by_rhog_o);
       qdf = 1.0;
 #pragma unroll
       for (int n = 1; n <= 5; ++n) qdf = qdf - q[n];
@@ -819,13 +822,10 @@ __global__ void __launch_bounds__(384, 2) nsw6_column_kernel(Problem P, Consts C
     const size_t i = off + (size_t)k * G + g;
     const size_t ic = (size_t)l * G + g;
     const bool interior = (k >= kmin && k <= kmax);
-    // gam2 / gsgam2, afact / gsgam2 and (below) the level above's bfact /
-    // gsgam2 from one reciprocal, correctly rounded; the reciprocal waits in
-    // S_BASE (free until the transport) for that level
+    // gam2 / gsgam2 and afact / gsgam2, correctly rounded
     const double gsg = P.gsgam2[i];
-    const double rgsg = 1.0 / gsg;
-    if (!MIX) F(S_BASE)[c] = rgsg;
-    if (interior) F(S_RGS)[c] = div_rn(P.gam2[i], gsg, rgsg);
+    const Divisor by_gsg(gsg);
+    if (interior) F(S_RGS)[c] = div_rn(P.gam2[i], by_gsg);
     if (MIX) {
       // the velocity components scale FP32 momentum sources only: FP32
       const float vx = (float)P.vx[i], vy = (float)P.vy[i], vz = (float)P.vz[i];
@@ -851,11 +851,11 @@ __global__ void __launch_bounds__(384, 2) nsw6_column_kernel(Problem P, Consts C
     F(S_VJ)[c] = vx * P.jx[ic] + vy * P.jy[ic] + vz * P.jz[ic];
     if (interior) {
       const double rvx = P.rhogvx[i], rvy = P.rhogvy[i], rvz = P.rhogvz[i];
-      F(S_KINH)[c] = 0.5 * (rvx * rvx + rvy * rvy + rvz * rvz) / P.rhog[i];
+      F(S_KINH)[c] = quo(0.5 * (rvx * rvx + rvy * rvy + rvz * rvz), P.rhog[i]);
     }
     if (k >= kmin + 1 && k <= kmax) {
-      r_c2w0[j] = div_rn(afact[k], gsg, rgsg) * P.gsgam2h[i];
-      r_rgsh[j] = P.gam2h[i] / P.gsgam2h[i];
+      r_c2w0[j] = div_rn(afact[k], by_gsg) * P.gsgam2h[i];
+      r_rgsh[j] = quo(P.gam2h[i], P.gsgam2h[i]);
     }
   }
   __syncthreads();
@@ -875,9 +875,9 @@ __global__ void __launch_bounds__(384, 2) nsw6_column_kernel(Problem P, Consts C
       continue;
     }
     const double c2w0 = r_c2w0[j];
-    const double c2w1 = div_rn(bfact[k], P.gsgam2[i - G], F(S_BASE)[c - COL_TG]) * P.gsgam2h[i];
+    const double c2w1 = div_rn(bfact[k], Divisor(P.gsgam2[i - G])) * P.gsgam2h[i];
     const double rw = P.rhogw[i];
-    F(S_KINV)[c] = 0.5 * (rw * rw) / (c2w0 * P.rhog[i] + c2w1 * P.rhog[i - G]);
+    F(S_KINV)[c] = quo(0.5 * (rw * rw), c2w0 * P.rhog[i] + c2w1 * P.rhog[i - G]);
     r_c2w1[j] = c2w1;
   }
   __syncthreads();
@@ -958,7 +958,7 @@ __global__ void __launch_bounds__(384, 2) nsw6_column_kernel(Problem P, Consts C
       switch (f) {
         case 0:
           F(dqs_slot)[c] = -d;
-          if (nq == I_QR) P.GPREC[off + (size_t)k * G + g] = plus_zero(div_rn(-fk, dt, P.rdt));
+          if (nq == I_QR) P.GPREC[off + (size_t)k * G + g] = plus_zero(soft_div_rn(-fk, P.by_dt, dt));
           break;
         case 1: F(S_DRHOE)[c] = F(S_DRHOE)[c] - d; break;
         case 2: F(S_DRHOPHI)[c] = F(S_DRHOPHI)[c] - d; break;
@@ -968,14 +968,14 @@ __global__ void __launch_bounds__(384, 2) nsw6_column_kernel(Problem P, Consts C
       }
       if (k == kmin) {
         double* acc = S.colacc;
-        const double fdt = div_rn(fk, dt, P.rdt);
+        const double fdt = soft_div_rn(fk, P.by_dt, dt);
         switch (f) {
           case 0:
             if (nq == I_QR) {
               acc[0 * COL_TG + gx] = acc[0 * COL_TG + gx] - fdt;
             } else {
               acc[1 * COL_TG + gx] = acc[1 * COL_TG + gx] - fdt;
-              acc[2 * COL_TG + gx] = acc[2 * COL_TG + gx] + div_rn(fk * LHF0, dt, P.rdt);
+              acc[2 * COL_TG + gx] = acc[2 * COL_TG + gx] + soft_div_rn(fk * LHF0, P.by_dt, dt);
             }
             break;
           case 1: acc[3 * COL_TG + gx] = acc[3 * COL_TG + gx] - fdt; break;
@@ -1052,7 +1052,7 @@ __global__ void __launch_bounds__(384, 2) nsw6_column_kernel(Problem P, Consts C
             }
             // the kinetic energy reaching the ground (precip_rhokin)
             if (k == kmin && f == 3)
-              S.colacc[5 * COL_TG + gx] = S.colacc[5 * COL_TG + gx] - div_rn((double)ff[c], dt, P.rdt);
+              S.colacc[5 * COL_TG + gx] = S.colacc[5 * COL_TG + gx] - soft_div_rn((double)ff[c], P.by_dt, dt);
           }
           if (f + 1 < 6) source(f + 1, c);
         }
@@ -1235,11 +1235,13 @@ __global__ void __launch_bounds__(384, 2) nsw6_column_kernel(Problem P, Consts C
       const size_t i = off + (size_t)k * G + g;
       const double rhog = F(S_RHOF)[c];
       if (k <= kmax) {
-        const double kin_h0 = (MIX ? (double)FF(S_KINH)[c] : F(S_KINH)[c]) / rhog;
-        double vx_t = P.rhogvx[i] / rhog, vy_t = P.rhogvy[i] / rhog, vz_t = P.rhogvz[i] / rhog;
+        const Divisor by_rhog(rhog);
+        const double kin_h0 = soft_div(MIX ? (double)FF(S_KINH)[c] : F(S_KINH)[c], by_rhog.s, rhog);
+        double vx_t = soft_div(P.rhogvx[i], by_rhog.s, rhog), vy_t = soft_div(P.rhogvy[i], by_rhog.s, rhog),
+               vz_t = soft_div(P.rhogvz[i], by_rhog.s, rhog);
         const double kin_h = 0.5 * (vx_t * vx_t + vy_t * vy_t + vz_t * vz_t);
         if (kin_h > 1.0E-20) {
-          const double r = sqrt(fabs(kin_h0 / kin_h));
+          const double r = sqrtR(fabs(quo(kin_h0, kin_h)));
           vx_t = vx_t * r;
           vy_t = vy_t * r;
           vz_t = vz_t * r;
@@ -1248,13 +1250,13 @@ __global__ void __launch_bounds__(384, 2) nsw6_column_kernel(Problem P, Consts C
         P.rhogvy[i] = vy_t * rhog;
         P.rhogvz[i] = vz_t * rhog;
       }
-      const double c2w0 = afact[k] / P.gsgam2[i] * P.gsgam2h[i];
-      const double c2w1 = bfact[k] / P.gsgam2[i - G] * P.gsgam2h[i];
+      const double c2w0 = quo(afact[k], P.gsgam2[i]) * P.gsgam2h[i];
+      const double c2w1 = quo(bfact[k], P.gsgam2[i - G]) * P.gsgam2h[i];
       const double rhogh = c2w0 * rhog + c2w1 * F(S_RHOF)[c - COL_TG];
-      const double kin_v0 = (MIX ? (double)FF(S_KINV)[c] : F(S_KINV)[c]) / rhogh;
-      double w_t = P.rhogw[i] / rhogh;
+      const double kin_v0 = quo(MIX ? (double)FF(S_KINV)[c] : F(S_KINV)[c], rhogh);
+      double w_t = quo(P.rhogw[i], rhogh);
       const double kin_v = 0.5 * (w_t * w_t);
-      if (kin_v > 1.0E-20) w_t = w_t * sqrt(fabs(kin_v0 / kin_v));
+      if (kin_v > 1.0E-20) w_t = w_t * sqrtR(fabs(quo(kin_v0, kin_v)));
       P.rhogw[i] = w_t * rhogh;
     }
   }
@@ -1295,16 +1297,16 @@ __global__ void __launch_bounds__(384, 2) nsw6_column_kernel(Problem P, Consts C
     const bool hk = (k >= kmin + 1 && k <= kmax);
     const double rw = hk ? F(S_DRHOGW)[c] : 0.0;
     if (k >= kmin && k <= kmax) {
-      const double gh = P.gsgam2h[i + G], rgh = 1.0 / gh;
-      const double w2c0 = div_rn(cfact[k] * P.gsgam2[i], gh, rgh);
-      const double w2c1 = div_rn(dfact[k] * P.gsgam2[i], gh, rgh);
+      const Divisor by_gh(P.gsgam2h[i + G]);
+      const double w2c0 = div_rn(cfact[k] * P.gsgam2[i], by_gh);
+      const double w2c1 = div_rn(dfact[k] * P.gsgam2[i], by_gh);
       F(S_DRHOE)[c] = F(S_KINH)[c] + (w2c0 * F(S_KINV)[c + COL_TG] + w2c1 * F(S_KINV)[c]);
       if (!OPT) {
         F(S_DRHOGW)[c] = w2c0;
         F(S_DRHOGV)[c] = w2c1;
       }
     }
-    if (hk) F(S_DRHOPHI)[c] = 0.5 * (rw * rw) / (r_c2w0[j] * F(S_RHOF)[c] + r_c2w1[j] * F(S_RHOF)[c - COL_TG]);
+    if (hk) F(S_DRHOPHI)[c] = quo(0.5 * (rw * rw), r_c2w0[j] * F(S_RHOF)[c] + r_c2w1[j] * F(S_RHOF)[c - COL_TG]);
   }
   __syncthreads();
 
@@ -1327,10 +1329,7 @@ __global__ void __launch_bounds__(384, 2) nsw6_column_kernel(Problem P, Consts C
     const size_t i = off + (size_t)k * G + g;
     const bool interior = (k >= kmin && k <= kmax);
     const double rhog = F(S_RHOF)[c];
-    // Quotients by a shared denominator are formed from one reciprocal with a
-    // Markstein correction step (div_rn): correctly rounded, as the reference's
-    // divisions, at a third of the cost.
-    const double rrhog = 1.0 / rhog;
+    const Divisor by_rhog(rhog);   // of the cell's quotients (correctly rounded, as the reference's divisions)
     double rhoge = P.rhoge[i];
     if (MIX && interior && !kin2kin) {
       // FP32 kinetic energies: the horizontal energy after the transport
@@ -1344,21 +1343,21 @@ __global__ void __launch_bounds__(384, 2) nsw6_column_kernel(Problem P, Consts C
       P.rhoge[i] = rhoge;   // a saturated cell's adjustment starts from here (final_cell overwrites the rest)
     } else if (interior && !kin2kin) {
       const double rvx = P.rhogvx[i], rvy = P.rhogvy[i], rvz = P.rhogvz[i];
-      const double tmp_h = div_rn(0.5 * (rvx * rvx + rvy * rvy + rvz * rvz), rhog, rrhog);
+      const double tmp_h = div_rn(0.5 * (rvx * rvx + rvy * rvy + rvz * rvz), by_rhog);
       double w2c0, w2c1;
       if (!OPT) {
         w2c0 = F(S_DRHOGW)[c];
         w2c1 = F(S_DRHOGV)[c];
       } else {
-        const double gh = P.gsgam2h[i + G], rgh = 1.0 / gh;
-        w2c0 = div_rn(cfact[k] * P.gsgam2[i], gh, rgh);
-        w2c1 = div_rn(dfact[k] * P.gsgam2[i], gh, rgh);
+        const Divisor by_gh(P.gsgam2h[i + G]);
+        w2c0 = div_rn(cfact[k] * P.gsgam2[i], by_gh);
+        w2c1 = div_rn(dfact[k] * P.gsgam2[i], by_gh);
       }
       const double tmp = tmp_h + (w2c0 * F(S_DRHOPHI)[c + COL_TG] + w2c1 * F(S_DRHOPHI)[c]);
       rhoge = rhoge + (F(S_DRHOE)[c] - tmp);
       P.rhoge[i] = rhoge;   // a saturated cell's adjustment starts from here (final_cell overwrites the rest)
     }
-    if (final_cell<M, MIX, OPT>(P, C, mth, ice_adj, lovr_f, i, offq + (size_t)k * G + g, KG, interior, rhog, rrhog,
+    if (final_cell<M, MIX, OPT>(P, C, mth, ice_adj, lovr_f, i, offq + (size_t)k * G + g, KG, interior, rhog, by_rhog,
                                 rhoge, false, k, g, l))
       qcell[atomicAdd(&nqueue, 1)] = c;
     if (k == kmin) {
@@ -1413,7 +1412,7 @@ __global__ void __launch_bounds__(SAT_THREADS) nsw6_satadj_kernel(Problem P, Con
     const size_t r = i - (size_t)l * KG;
     const int k = (int)(r / G), g = (int)(r - (size_t)k * G);
     const double rhog = P.rhog[i];
-    final_cell<M, MIX, OPT>(P, C, mth, ice_adj, lovr_f, i, (size_t)l * NQ * KG + r, KG, true, rhog, 1.0 / rhog,
+    final_cell<M, MIX, OPT>(P, C, mth, ice_adj, lovr_f, i, (size_t)l * NQ * KG + r, KG, true, rhog, Divisor(rhog),
                             P.rhoge[i], true, k, g, l);
   }
 }
