@@ -620,7 +620,7 @@ def main(argv=None) -> int:
         "vs_baseline": None, "dtype": "f32+f64" if mixed else "f64", "data": "synthetic (seeded NICAM-like state)",
         "config": workload_config(spec, args.precision, world),
         "e2e": e2e, "roofline": roofline, "cpu_baseline": cpu, "clocks": clocks,
-        "gpu_launches": 3 * args.steps,   # per step: nsw6_cell_kernel, nsw6_column_kernel, nsw6_satadj_kernel
+        "gpu_launches": 4 * args.steps,   # per step: nsw6_cell_kernel, nsw6_departure_kernel, nsw6_column_kernel, nsw6_satadj_kernel
     }
 
     if not args.no_extras and world == 1:

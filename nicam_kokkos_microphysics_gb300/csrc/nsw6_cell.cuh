@@ -35,6 +35,8 @@
 // reference's position.
 #pragma once
 
+#include <type_traits>
+
 #include "nsw6_common.cuh"
 #include "nsw6_soft.cuh"
 #include "nsw6_fastmath.cuh"
@@ -134,6 +136,8 @@ template <class T>
 __device__ __forceinline__ bool is_nonneg(const T& x) { return x >= T(0.0); }
 
 template <class T>
+__device__ __forceinline__ bool is_finite_nonneg(const T&) { return false; }   // (asked of doubles only)
+template <class T>
 __device__ __forceinline__ bool lt_z(const T& x) { return x < T(0.0); }
 template <class T>
 __device__ __forceinline__ bool gt_z(const T& x) { return x > T(0.0); }
@@ -204,6 +208,14 @@ template <class M, class R, class D = double, bool OPT = false>
 __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, double dt, double rdt,
                                           const CellInT<D>& in, CellOutT<D>& o) {
   constexpr bool kMixed = sizeof(R) == sizeof(float);
+  // The plain FP64 step leaves out what an absent species or the other side of
+  // 0 C makes an exact zero: x + 0 and 0 x need no FP64 instruction (16 to 19
+  // cycles of an SM each).  The cell kernel's warps hold cells of the same
+  // species and side of 0 C, so whole warps skip them; the results are the same
+  // bits.  The derivative types keep every term (a rate that is zero has
+  // partial derivatives), FP32 has cycles to spare: there nz(x) is true.
+  constexpr bool kPlain = std::is_same<R, double>::value && std::is_same<D, double>::value;
+  auto nz = [](const auto& x) { return !kPlain || !is_zero(x); };
   const R dtR = R(dt), rdtR = R(rdt);
   // ---- negative_filter, mod_mp_nsw6.cpp:1770-1831
   D rq[6];
@@ -212,16 +224,21 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
   D diffq = D(0.0);
 #pragma unroll
   for (int n = 2; n <= 5; ++n) {
-    diffq += rq[n];
+    if (nz(rq[n])) diffq += rq[n];
     rq[n] = maxz(rq[n]);
   }
 #pragma unroll
-  for (int n = 2; n <= 5; ++n) diffq -= rq[n];
-  rq[I_QV] += diffq;
+  for (int n = 2; n <= 5; ++n)
+    if (nz(rq[n])) diffq -= rq[n];
+  if (nz(diffq)) rq[I_QV] += diffq;
   diffq = rq[I_QV];
   rq[I_QV] = maxz(rq[I_QV]);
-  diffq -= rq[I_QV];
-  const D rhog = in.rhog * (1.0 - diffq);
+  // x - x is +0 for the vapour that is not negative (1 - 0 is 1, rhog 1 is rhog)
+  D rhog = in.rhog;
+  if (!kPlain || !is_finite_nonneg(diffq)) {
+    diffq -= rq[I_QV];
+    rhog = in.rhog * (1.0 - diffq);
+  }
   const DivisorT<D> by_rhog(rhog);
   D rrhog;   // mixed only
   if constexpr (kMixed) rrhog = rcp_of(by_rhog);
@@ -250,34 +267,48 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
     const D dens = quo(rhog, in.gsgam2);
     D qd = D(1.0);
 #pragma unroll
-    for (int n = 1; n <= 5; ++n) qd = qd - qn[n];
+    for (int n = 1; n <= 5; ++n)
+      if (nz(qn[n])) qd = qd - qn[n];
     D cv = qd * CVDRY;
 #pragma unroll
-    for (int n = 1; n <= 5; ++n) cv = cv + qn[n] * CVDRY;
+    for (int n = 1; n <= 5; ++n)
+      if (nz(qn[n])) cv = cv + qn[n] * CVDRY;
     rhoge = temp * rhog * cv;
     pre = R(dens * (qd * RDRY + qn[0] * RVAP) * temp);
     densR = R(dens);
   }
 
-  // ---- psat / qsat (CPovR = 0 under EIN_TYPE "SIMPLE": the power term is 1)
-  const R tempR = R(temp);
-  const R rtem = quo(R(1.0), maxc(tempR, R(TEM_MIN)));
-  const R psatl = R(PSAT0) * mth.exp(C.LovR_liq * (C.RTEM00 - rtem));
-  const R psati = R(PSAT0) * mth.exp(C.LovR_ice * (C.RTEM00 - rtem));
-  const R rdrt = quo(R(1.0), densR * R(RVAP) * tempR);
-  const R qsatl = psatl * rdrt;
-  const R qsati = psati * rdrt;
-
-  // ---- TagBigLoop, mod_mp_nsw6.cpp:902-1594
   const R Z = R(0.0), ONE = R(1.0);
   const R qv = maxz(R(qn[0])), qc = maxz(R(qn[1])), qr = maxz(R(qn[2]));
   const R qi = maxz(R(qn[3])), qs = maxz(R(qn[4])), qg = maxz(R(qn[5]));
-  const R Sliq = quo(qv, maxc(qsatl, R(EPS)));
-  const R Sice = quo(qv, maxc(qsati, R(EPS)));
-  const R Rdens = quo(ONE, densR);
-  const R rho_fact = sqrtR(R(DENS00) * Rdens);
+  const bool hc = nz(qc), hr = nz(qr), hi = nz(qi), hs = nz(qs), hg = nz(qg);   // the species the cell holds
+  const R tempR = R(temp);
   const R temc = tempR - R(TEM00);
   const bool warm = !lt_z(temc);  // iceflg = 0.5 - copysign(0.5, temc) == 0
+  const bool cold = !warm;        // iceflg == 1
+  const bool wcold = !kPlain || cold, wwarm = !kPlain || warm;   // work for cold (warm) cells
+
+  // ---- psat / qsat (CPovR = 0 under EIN_TYPE "SIMPLE": the power term is 1);
+  //      over liquid for the evaporation of rain, over ice for cold cells
+  R rtem = Z, rdrt = Z, qsatl = Z, qsati = Z, Sliq = Z, Sice = Z;
+  if (hr || wcold) {
+    rtem = quo(R(1.0), maxc(tempR, R(TEM_MIN)));
+    rdrt = quo(R(1.0), densR * R(RVAP) * tempR);
+  }
+  if (hr) {
+    const R psatl = R(PSAT0) * mth.exp(C.LovR_liq * (C.RTEM00 - rtem));
+    qsatl = psatl * rdrt;
+    Sliq = quo(qv, maxc(qsatl, R(EPS)));
+  }
+  if (wcold) {
+    const R psati = R(PSAT0) * mth.exp(C.LovR_ice * (C.RTEM00 - rtem));
+    qsati = psati * rdrt;
+    Sice = quo(qv, maxc(qsati, R(EPS)));
+  }
+
+  // ---- TagBigLoop, mod_mp_nsw6.cpp:902-1594
+  const R Rdens = quo(ONE, densR);
+  const R rho_fact = (hr || hs || hg) ? sqrtR(R(DENS00) * Rdens) : Z;
   const bool d1 = ge_c(qr, R(1.0E-4));                          // delta1
   const bool d2 = le_c(qr, R(1.0E-4)) && le_c(qs, R(1.0E-4));       // delta2
   const bool sps = ge_c(Sice, ONE);                              // spsati
@@ -311,7 +342,7 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
   // Roh and Satoh (2014) snow moments, :994-1057.  Each moment is
   // 10^loga * Xs2^b = exp(ln10 * loga + log(Xs2) * b), with loga and b
   // polynomials in tems whose coefficients per moment are folded on the host.
-  const R Xs2 = densR * qs * C.rAs;
+  const R Xs2 = hs ? densR * qs * C.rAs : Z;
   const bool roh = !OPT || C.opt_roh != Z;
   const bool snow = roh && ge_c(Xs2, R(1.0E-12));
   R mom[7] = {Z, Z, Z, Z, Z, Z, Z};  // MOMs_0, _1, _0bs, _1bs, _2bs, _2ds (= nm 2.25), _5ds_h
@@ -368,9 +399,10 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
   }
 
   // terminal velocity, :1072-1078
-  const R Vtr = C.K_vtr * rho_fact * RLMDr_dr;
-  const R Vts = C.K_vts * rho_fact * RMOMs_Vt;
-  const R Vtg = C.K_vtg * rho_fact * RLMDg_dg;
+  // (an absent species' is the zero of the product's sign)
+  const R Vtr = hr ? C.K_vtr * rho_fact * RLMDr_dr : sel(false, C.K_vtr);
+  const R Vts = hs ? C.K_vts * rho_fact * RMOMs_Vt : sel(false, C.K_vts);
+  const R Vtg = hg ? C.K_vtg * rho_fact * RLMDg_dg : sel(false, C.K_vtg);
   R Vti = Z;
   if constexpr (OPT) {
     // :1073-1075 with sw_constVti = 0 (CONST_Vti is UNDEF)
@@ -384,15 +416,18 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
 
   // nucleation, :1080-1085: Ni0 = max(exp(-0.1 temc), 1) * 1000 and
   // Qi0 = ice_nuc * Ni0^1.33 / dens, with log(Ni0) = ln 1000 + max(-0.1 temc, 0)
-  const R Qi0 = C.ice_nuc * mth.exp(R(1.33) * (C.ln1000 + maxz(R(-0.1) * temc))) * Rdens;
-  R Pigen = maxz(dmin(Qi0 - qi, qv - qsati)) * rdtR;
+  R Pigen = Z;
+  if (wcold) {
+    const R Qi0 = C.ice_nuc * mth.exp(R(1.33) * (C.ln1000 + maxz(R(-0.1) * temc))) * Rdens;
+    Pigen = maxz(dmin(Qi0 - qi, qv - qsati)) * rdtR;
+  }
 
   // accretion, :1087-1145
   // Esi_mod and betai, :1089, :1162: min(E, E exp(0.06 temc)) is E when temc >= 0
   // (exp >= 1 there) and E >= 0; both use the same exponential when
   // gamma_sacr == gamma_saut (both 6e-2 in this configuration).
   R Esi_mod = C.Esi, betai = C.beta_saut;
-  if (!(warm && is_nonneg(C.Esi) && is_nonneg(C.beta_saut))) {
+  if (hi && !(warm && is_nonneg(C.Esi) && is_nonneg(C.beta_saut))) {
     const R eg = mth.exp(C.gamma_sacr * temc);
     const R eb = (C.gamma_saut == C.gamma_sacr) ? eg : mth.exp(C.gamma_saut * temc);
     Esi_mod = dmin(C.Esi, C.Esi * eg);
@@ -400,35 +435,42 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
   }
   const bool kk = !OPT || C.opt_kk != Z;
   const R fr = rho_fact;
-  const R qcqr = qc * qr;
-  R Pracw = Z;
-  if (kk) {
-    if (ge_c(qcqr, R(1.0E-12))) Pracw = R(67.0) * mth.pow(qcqr, R(1.15));
-  } else {
-    Pracw = qc * C.K_raci * RLMDr_3dr * fr;   // Pracw_orig (Erw = Eri = 1)
+  R Pracw = Z, Psacw = Z, Pgacw = Z, Praci = Z, Psaci = Z, Piacr = Z, Psacr = Z, Pgacr = Z, Pracs = Z;
+  if (hc && hr) {
+    const R qcqr = qc * qr;
+    if (kk) {
+      if (ge_c(qcqr, R(1.0E-12))) Pracw = R(67.0) * mth.pow(qcqr, R(1.15));
+    } else {
+      Pracw = qc * C.K_raci * RLMDr_3dr * fr;   // Pracw_orig (Erw = Eri = 1)
+    }
   }
-  R Psacw = qc * C.K_sacw * MOMs_2ds * fr;
-  R Pgacw = qc * C.K_gacw * RLMDg_3dg * fr;
-  R Praci = qi * C.K_raci * RLMDr_3dr * fr;
-  R Psaci = qi * C.K_saci * Esi_mod * MOMs_2ds * fr;
-  R Piacr = qi * C.K_iacr * RLMDr_6dr * fr;
-  const R dvrs = fabsR(Vtr - Vts);
-  R Psacr = C.K_sacr * Rdens * dvrs *
+  if (hc && hs) Psacw = qc * C.K_sacw * MOMs_2ds * fr;
+  if (hc && hg) Pgacw = qc * C.K_gacw * RLMDg_3dg * fr;
+  if (hi && hr) {
+    Praci = qi * C.K_raci * RLMDr_3dr * fr;
+    Piacr = qi * C.K_iacr * RLMDr_6dr * fr;
+  }
+  if (hi && hs) Psaci = qi * C.K_saci * Esi_mod * MOMs_2ds * fr;
+  if (hr && hs) {
+    const R dvrs = fabsR(Vtr - Vts);
+    Psacr = C.K_sacr * Rdens * dvrs *
             (C.GAM_1br * RLMDr_1br * MOMs_2 + C.K_2gam2br * RLMDr_2br * MOMs_1 + C.GAM_3br * RLMDr_3br * MOMs_0);
-  R Pgacr = C.K_gacr * Rdens * fabsR(Vtg - Vtr) *
+    Pracs = C.K_racs * Rdens * dvrs * (R(2.0) * MOMs_0bs * RLMDr_3 + R(2.0) * MOMs_1bs * RLMDr_2 + MOMs_2bs * RLMDr);
+  }
+  if (hr && hg)
+    Pgacr = C.K_gacr * Rdens * fabsR(Vtg - Vtr) *
             (C.K_g13 * RLMDr_1br * RLMDg_3 + C.K_g22 * RLMDr_2br * RLMDg_2 + C.GAM_3br * RLMDr_3br * RLMDg);
-  R Pracs = C.K_racs * Rdens * dvrs * (R(2.0) * MOMs_0bs * RLMDr_3 + R(2.0) * MOMs_1bs * RLMDr_2 + MOMs_2bs * RLMDr);
   R Pgaci = Z, Pgacs = Z;   // Egi = Egs = 0 unless OPT
   if constexpr (OPT) {
-    Pgaci = qi * C.K_gaci * RLMDg_3dg * fr;
+    if (hi && hg) Pgaci = qi * C.K_gaci * RLMDg_3dg * fr;
     R Egs_mod = C.Egs;
-    if (!(warm && C.Egs >= Z)) Egs_mod = dmin(C.Egs, C.Egs * mth.exp(C.gamma_gacs * temc));
-    Pgacs = C.K_gacs * Rdens * Egs_mod * fabsR(Vtg - Vts) *
+    if (hs && hg && !(warm && C.Egs >= Z)) Egs_mod = dmin(C.Egs, C.Egs * mth.exp(C.gamma_gacs * temc));
+    if (hs && hg) Pgacs = C.K_gacs * Rdens * Egs_mod * fabsR(Vtg - Vts) *
             (R(2.0) * MOMs_0bs * RLMDg_3 + R(2.0) * MOMs_1bs * RLMDg_2 + MOMs_2bs * RLMDg);
   }
 
   // autoconversion, :1147-1172 (KK2000; only the second Praut_kk assignment is live)
-  const R rhoqc = densR * qc * R(1000.0);
+  const R rhoqc = hc ? densR * qc * R(1000.0) : Z;
   R Praut = Z;   // K_aut * pow(0, 2.47) = 0
   if (kk) {
     R K_aut = C.K_aut;
@@ -436,7 +478,7 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
       if (C.opt_indir != Z) K_aut = C.kk_aut * mth.pow(Nc, R(-1.79));
     }
     if (gt_z(qc)) Praut = K_aut * mth.pow(qc, R(2.47));
-  } else {
+  } else if (hc) {
     // Berry (1968), :1145-1147
     R Dc = C.Dc_berry;
     if constexpr (OPT) {
@@ -444,16 +486,23 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
     }
     Praut = quo(Rdens * R(1.67E-5) * rhoqc * rhoqc, R(5.0) + quo(R(3.66E-2) * Nc, Dc * rhoqc + R(EPS)));
   }
-  R Psaut = rate_on(betai * (qi - C.qicrt_saut));
+  R Psaut = Z;   // (without ice the limiter dqi_dt = 0 below would hold it there)
+  if (hi) Psaut = rate_on(betai * (qi - C.qicrt_saut));
 
   // evaporation, sublimation, melting and freezing, :1174-1247
-  const R Ka = (R(2.428E-2) + R(7.47E-5) * temc);
-  const R KdD = quo((R(2.222E-5) + R(1.37E-7) * temc) * R(PSTD), pre) * densR;   // Kd * dens
-  const R rNu = quo(densR, R(1.718E-5) + R(5.28E-8) * temc);               // 1 / Nu
-  const R rKaT = quo(ONE, Ka * tempR);
-  const R xi = KdD * qsati;
-  const R Giv = quo(xi, R(LHS0) * rKaT * (C.LovR_ice * rtem - ONE) * xi + ONE);
-  const R Gil = Ka * temc * C.rLHF0;
+  const bool falls = hr || hs || hg;
+  R Ka = Z, KdD = Z, rKaT = Z, Giv = Z, Gil = Z, rNu = Z;
+  if (falls || wcold) Ka = R(2.428E-2) + R(7.47E-5) * temc;
+  if (hr || wcold) {
+    KdD = quo((R(2.222E-5) + R(1.37E-7) * temc) * R(PSTD), pre) * densR;   // Kd * dens
+    rKaT = quo(ONE, Ka * tempR);
+  }
+  if (falls) rNu = quo(densR, R(1.718E-5) + R(5.28E-8) * temc);               // 1 / Nu
+  if (wcold) {
+    const R xi = KdD * qsati;
+    Giv = quo(xi, R(LHS0) * rKaT * (C.LovR_ice * rtem - ONE) * xi + ONE);
+  }
+  if ((hs || hg) && wwarm) Gil = Ka * temc * C.rLHF0;
   R Prevp = Z;
   if (rain) {
     const R xl = KdD * qsatl;
@@ -461,45 +510,58 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
     const R ventr = C.K_ventr1 * RLMDr_2 + C.K_ventr2 * sqrtR(C.Cr * fr * rNu * RLMDr_5dr);
     Prevp = C.K_revp * Rdens * (ONE - minc(Sliq, ONE)) * Glv * ventr;
   }
-  const R rhoqi = maxc(densR * qi, R(EPS));
-  // with no ice, rhoqi = EPS and XNi, Di take the constant values folded on the host
-  R XNi = C.XNi_eps, Di = C.Di_eps;
-  if (gt_c(rhoqi, R(EPS))) {
-    XNi = minc(maxc(R(5.38E+7) * mth.pow(rhoqi, R(0.75)), R(1.0E+3)), R(1.0E+6));
-    const R XMi = quo(rhoqi, XNi);
-    Di = minc(C.Di_a * sqrtR(XMi), C.Di_max);
+  // deposition and sublimation of ice (cold cells: the limiters keep it there)
+  R tmp, Pidep = Z, Pisub = Z;
+  if (wcold) {
+    const R rhoqi = hi ? maxc(densR * qi, R(EPS)) : R(EPS);
+    // with no ice, rhoqi = EPS and XNi, Di take the constant values folded on the host
+    R XNi = C.XNi_eps, Di = C.Di_eps;
+    if (gt_c(rhoqi, R(EPS))) {
+      XNi = minc(maxc(R(5.38E+7) * mth.pow(rhoqi, R(0.75)), R(1.0E+3)), R(1.0E+6));
+      const R XMi = quo(rhoqi, XNi);
+      Di = minc(C.Di_a * sqrtR(XMi), C.Di_max);
+    }
+    tmp = R(4.0) * Di * XNi * Rdens * (Sice - ONE) * Giv;
+    Pidep = sel(sps, tmp);
+    Pisub = sel(!sps, -tmp);
   }
-  R tmp = R(4.0) * Di * XNi * Rdens * (Sice - ONE) * Giv;
-  R Pidep = sel(sps, tmp);
-  R Pisub = sel(!sps, -tmp);
   const bool below40 = lt_z(temc + R(40.0));
   R Pihom = below40 ? dqc_dt : Z;
-  const R efrz = mth.exp(-C.A_frz * temc) - ONE;
-  R Pihtr = (!below40 && !warm) ? densR * (qc * qc) * C.K_ihtr * efrz : Z;
+  R efrz = Z;
+  if ((hc || hr) && wcold) efrz = mth.exp(-C.A_frz * temc) - ONE;
+  R Pihtr = Z;
+  if (hc && !below40 && !warm) Pihtr = densR * (qc * qc) * C.K_ihtr * efrz;
   R Pimlt = warm ? dqi_dt : Z;
   // ventilation of snow and graupel: without the species their moments /
   // slope terms are exact zeros and so is the sum (+0, skipped with its root)
-  const R vents = (is_zero(MOMs_1) && is_zero(MOMs_5ds_h)) ? Z : R(0.65) * MOMs_1 + C.K_vents2 * sqrtR(fr * rNu) * MOMs_5ds_h;
-  tmp = C.K_2pi * Rdens * (Sice - ONE) * Giv * vents;
-  R Psdep = sel(sps, tmp);
-  R Pssub = sel(!sps, -tmp);
-  R Psmlt = maxz(C.K_2pi * Rdens * Gil * vents + C.K_clf * temc * (Psacw + Psacr));
-  const R ventg = (is_zero(RLMDg_2) && is_zero(RLMDg_5dg)) ? Z
-                                                  : C.K_ventg1 * RLMDg_2 + C.K_ventg2 * sqrtR(C.Cg * fr * rNu * RLMDg_5dg);
-  tmp = C.K_gdep * Rdens * (Sice - ONE) * Giv * ventg;
-  R Pgdep = sel(sps, tmp);
-  R Pgsub = sel(!sps, -tmp);
-  R Pgmlt = maxz(C.K_gdep * Rdens * Gil * ventg + C.K_clf * temc * (Pgacw + Pgacr));
-  R Pgfrz = C.K_gfrz * Rdens * efrz * RLMDr_7;
+  R vents = Z, ventg = Z;
+  if (hs && !(is_zero(MOMs_1) && is_zero(MOMs_5ds_h)))
+    vents = R(0.65) * MOMs_1 + C.K_vents2 * sqrtR(fr * rNu) * MOMs_5ds_h;
+  R Psdep = Z, Pssub = Z, Psmlt = Z;
+  if (hs && wcold) {
+    tmp = C.K_2pi * Rdens * (Sice - ONE) * Giv * vents;
+    Psdep = sel(sps, tmp);
+    Pssub = sel(!sps, -tmp);
+  }
+  if (hs && wwarm) Psmlt = maxz(C.K_2pi * Rdens * Gil * vents + C.K_clf * temc * (Psacw + Psacr));
+  if (hg && !(is_zero(RLMDg_2) && is_zero(RLMDg_5dg)))
+    ventg = C.K_ventg1 * RLMDg_2 + C.K_ventg2 * sqrtR(C.Cg * fr * rNu * RLMDg_5dg);
+  R Pgdep = Z, Pgsub = Z, Pgmlt = Z, Pgfrz = Z;
+  if (hg && wcold) {
+    tmp = C.K_gdep * Rdens * (Sice - ONE) * Giv * ventg;
+    Pgdep = sel(sps, tmp);
+    Pgsub = sel(!sps, -tmp);
+  }
+  if (hg && wwarm) Pgmlt = maxz(C.K_gdep * Rdens * Gil * ventg + C.K_clf * temc * (Pgacw + Pgacr));
+  if (hr && wcold) Pgfrz = C.K_gfrz * Rdens * efrz * RLMDr_7;
 
   // Bergeron process (:1239-1247) with Bergeron_param (:1834-1890); it
   // contributes only when sw_bergeron = 1 (-30 <= temc <= 0, sw_expice = 0)
   // and iceflg = 1 (temc < 0)
   const bool expice = !OPT || C.opt_expice != Z;
-  const bool cold = !warm;   // iceflg == 1
   R Psfw = Z, Psfi = Z;
   if constexpr (OPT) {
-    if (!expice && cold && !(temc + R(30.0) < Z)) {
+    if (hi && !expice && cold && !(temc + R(30.0) < Z)) {
       const R tb = dmin(dmax(temc, R(-30.99)), Z);
       const int it = int(-val_of(tb));   // the table row: piecewise constant in tb
       const R fact = -(tb + R(it - 1));
@@ -518,7 +580,7 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
   Pidep = sel(cold && expice, min_nn(Pidep, dqv_dt));
   Psdep = sel(cold, min_nn(Psdep, dqv_dt));
   Pgdep = sel(cold, min_nn(Pgdep, dqv_dt));
-  Pracw = Pracw + sel(warm, Psacw) + sel(warm, Pgacw);
+  if (hc && wwarm) Pracw = Pracw + sel(warm, Psacw) + sel(warm, Pgacw);
   Praut = min_nn(Praut, dqc_dt);
   Pracw = min_nn(Pracw, dqc_dt);
   Pihom = sel(cold && expice, min_nn(Pihom, dqc_dt));
@@ -563,78 +625,126 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
   // nets the limiters form (same terms, same order) where no later scaling
   // changed their rates.  lc .. lg: the QC, QI, QR, QV, QS, QG limiter scaled
   // its rates.
-  bool lc, li, lr, lv, ls, lg;
-  R fac, net_c, net_i, net_r, net_s, net_g;
-  if constexpr (!OPT) {
-    net_c = +Pimlt - Praut - Pracw - Pihom - Pihtr - Psacw - Pgacw;  // [QC]
+  // An absent species' losses are zero (they scale with it, or their own
+  // limiter holds them at dq/dt = 0) and its limiter is 1 while its net is not
+  // negative.  Two losses can be negative, which no limiter holds: the Bergeron
+  // growth Psfw (extrapolated table weights) and, far below any temperature of
+  // the air, Pisub.
+  const bool bc = hc || (OPT && nz(Psfw));
+  const bool bi = hi || nz(Pisub);
+  bool lc = false, li = false, lr = false, lv = false, ls = false, lg = false;
+  R fac;
+  R net_c = +Pimlt;  // [QC]
+  if (bc) {
+    net_c = net_c - Praut - Pracw - Pihom - Pihtr - Psacw;
+    if constexpr (OPT) net_c = net_c - Psfw;
+    net_c = net_c - Pgacw;
     fac = limiter(net_c, dqc_dt);
     lc = !is_one(fac);
     if (lc) {
       Pimlt *= fac; Praut *= fac; Pracw *= fac; Pihom *= fac; Pihtr *= fac; Psacw *= fac; Pgacw *= fac;
+      if constexpr (OPT) Psfw *= fac;
     }
-    net_i = +Pigen + Pidep + Pihom + Pihtr - Pisub - Pimlt - Psaut - Praci_s - Psaci - Praci_g;  // [QI]
+  }
+  R net_i = Z;  // [QI]
+  if (wcold) net_i = +Pigen + Pidep;
+  if (hc && wcold) net_i = net_i + Pihom + Pihtr;
+  if (bi) {
+    net_i = net_i - Pisub - Pimlt - Psaut - Praci_s - Psaci;
+    if constexpr (OPT) net_i = net_i - Psfi;
+    net_i = net_i - Praci_g;
+    if constexpr (OPT) net_i = net_i - Pgaci;
+  }
+  if (bi || lt_z(net_i)) {
     fac = limiter(net_i, dqi_dt);
     li = !is_one(fac);
     if (li) {
       Pigen *= fac; Pidep *= fac; Pihom *= fac; Pihtr *= fac; Pisub *= fac; Pimlt *= fac; Psaut *= fac;
       Praci_s *= fac; Psaci *= fac; Praci_g *= fac;
-    }
-  } else {
-    net_c = +Pimlt - Praut - Pracw - Pihom - Pihtr - Psacw - Psfw - Pgacw;  // [QC]
-    fac = limiter(net_c, dqc_dt);
-    lc = !is_one(fac);
-    if (lc) {
-      Pimlt *= fac; Praut *= fac; Pracw *= fac; Pihom *= fac; Pihtr *= fac; Psacw *= fac; Psfw *= fac; Pgacw *= fac;
-    }
-    net_i = +Pigen + Pidep + Pihom + Pihtr - Pisub - Pimlt - Psaut - Praci_s - Psaci - Psfi - Praci_g - Pgaci;  // [QI]
-    fac = limiter(net_i, dqi_dt);
-    li = !is_one(fac);
-    if (li) {
-      Pigen *= fac; Pidep *= fac; Pihom *= fac; Pihtr *= fac; Pisub *= fac; Pimlt *= fac; Psaut *= fac;
-      Praci_s *= fac; Psaci *= fac; Psfi *= fac; Praci_g *= fac; Pgaci *= fac;
+      if constexpr (OPT) {
+        Psfi *= fac;
+        Pgaci *= fac;
+      }
     }
   }
-  net_r = +Praut + Pracw + Psmlt + Pgmlt - Prevp - Piacr_s - Psacr_s - Piacr_g - Psacr_g - Pgacr - Pgfrz;  // [QR]
-  fac = limiter(net_r, dqr_dt);
-  lr = !is_one(fac);
-  if (lr) {
-    Praut *= fac; Pracw *= fac; Psmlt *= fac; Pgmlt *= fac; Prevp *= fac; Piacr_s *= fac; Psacr_s *= fac;
-    Piacr_g *= fac; Psacr_g *= fac; Pgacr *= fac; Pgfrz *= fac;
+  R net_r = Z;  // [QR]
+  if (hc) net_r = +Praut + Pracw;
+  if (hs && wwarm) net_r = net_r + Psmlt;
+  if (hg && wwarm) net_r = net_r + Pgmlt;
+  if (hr) {
+    net_r = net_r - Prevp - Piacr_s - Psacr_s - Piacr_g - Psacr_g - Pgacr - Pgfrz;
   }
-  fac = limiter(+Prevp + Pisub + Pssub + Pgsub - Pigen - Pidep - Psdep - Pgdep, dqv_dt);  // [QV]
-  lv = !is_one(fac);
-  if (lv) {
-    Prevp *= fac; Pisub *= fac; Pssub *= fac; Pgsub *= fac; Pigen *= fac; Pidep *= fac; Psdep *= fac; Pgdep *= fac;
+  if (hr || lt_z(net_r)) {
+    fac = limiter(net_r, dqr_dt);
+    lr = !is_one(fac);
+    if (lr) {
+      Praut *= fac; Pracw *= fac; Psmlt *= fac; Pgmlt *= fac; Prevp *= fac; Piacr_s *= fac; Psacr_s *= fac;
+      Piacr_g *= fac; Psacr_g *= fac; Pgacr *= fac; Pgfrz *= fac;
+    }
   }
-  if constexpr (!OPT) {
-    net_s = +Psdep + Psacw + Piacr_s + Psacr_s + Psaut + Praci_s + Psaci - Pssub - Psmlt - Pracs;  // [QS]
+  R net_v = Z;  // [QV]
+  if (hr) net_v = +Prevp;
+  if (bi) net_v = net_v + Pisub;
+  if (hs) net_v = net_v + Pssub;
+  if (hg) net_v = net_v + Pgsub;
+  if (wcold) net_v = net_v - Pigen - Pidep;
+  if (hs && wcold) net_v = net_v - Psdep;
+  if (hg && wcold) net_v = net_v - Pgdep;
+  if (hr || wcold || lt_z(net_v)) {
+    fac = limiter(net_v, dqv_dt);
+    lv = !is_one(fac);
+    if (lv) {
+      Prevp *= fac; Pisub *= fac; Pssub *= fac; Pgsub *= fac; Pigen *= fac; Pidep *= fac; Psdep *= fac; Pgdep *= fac;
+    }
+  }
+  R net_s = Z;  // [QS]
+  if (hs) net_s = +Psdep + Psacw;
+  if constexpr (OPT) net_s = net_s + Psfw;
+  if (hr && hi) net_s = net_s + Piacr_s;
+  if (hr && hs) net_s = net_s + Psacr_s;
+  if (hi) {
+    net_s = net_s + Psaut + Praci_s + Psaci;
+    if constexpr (OPT) net_s = net_s + Psfi;
+  }
+  if (hs) {
+    net_s = net_s - Pssub - Psmlt - Pracs;
+    if constexpr (OPT) net_s = net_s - Pgacs;
+  }
+  if (hs || lt_z(net_s)) {
     fac = limiter(net_s, dqs_dt);
     ls = !is_one(fac);
     if (ls) {
       Psdep *= fac; Psacw *= fac; Piacr_s *= fac; Psacr_s *= fac; Psaut *= fac; Praci_s *= fac; Psaci *= fac;
       Pssub *= fac; Psmlt *= fac; Pracs *= fac;
+      if constexpr (OPT) {
+        Psfw *= fac;
+        Psfi *= fac;
+        Pgacs *= fac;
+      }
     }
-    net_g = +Pgdep + Pgacw + Piacr_g + Psacr_g + Pgacr + Pgfrz + Praci_g + Pracs - Pgsub - Pgmlt;  // [QG]
+  }
+  R net_g = Z;  // [QG]
+  if (hg) net_g = +Pgdep + Pgacw;
+  if (hr && hi) net_g = net_g + Piacr_g;
+  if (hr && hs) net_g = net_g + Psacr_g;
+  if (hr) net_g = net_g + Pgacr + Pgfrz;
+  if (hr && hi) net_g = net_g + Praci_g;
+  if constexpr (OPT) net_g = net_g + Pgaci;
+  if (hr && hs) net_g = net_g + Pracs;
+  if constexpr (OPT) net_g = net_g + Pgacs;
+  if (hg) {
+    net_g = net_g - Pgsub - Pgmlt;
+  }
+  if (hg || lt_z(net_g)) {
     fac = limiter(net_g, dqg_dt);
     lg = !is_one(fac);
     if (lg) {
       Pgdep *= fac; Pgacw *= fac; Piacr_g *= fac; Psacr_g *= fac; Pgacr *= fac; Pgfrz *= fac; Praci_g *= fac;
       Pracs *= fac; Pgsub *= fac; Pgmlt *= fac;
-    }
-  } else {
-    net_s = +Psdep + Psacw + Psfw + Piacr_s + Psacr_s + Psaut + Praci_s + Psaci + Psfi - Pssub - Psmlt - Pracs - Pgacs;
-    fac = limiter(net_s, dqs_dt);  // [QS]
-    ls = !is_one(fac);
-    if (ls) {
-      Psdep *= fac; Psacw *= fac; Psfw *= fac; Piacr_s *= fac; Psacr_s *= fac; Psaut *= fac; Praci_s *= fac;
-      Psaci *= fac; Psfi *= fac; Pssub *= fac; Psmlt *= fac; Pracs *= fac; Pgacs *= fac;
-    }
-    net_g = +Pgdep + Pgacw + Piacr_g + Psacr_g + Pgacr + Pgfrz + Praci_g + Pgaci + Pracs + Pgacs - Pgsub - Pgmlt;
-    fac = limiter(net_g, dqg_dt);  // [QG]
-    lg = !is_one(fac);
-    if (lg) {
-      Pgdep *= fac; Pgacw *= fac; Piacr_g *= fac; Psacr_g *= fac; Pgacr *= fac; Pgfrz *= fac; Praci_g *= fac;
-      Pgaci *= fac; Pracs *= fac; Pgacs *= fac; Pgsub *= fac; Pgmlt *= fac;
+      if constexpr (OPT) {
+        Pgaci *= fac;
+        Pgacs *= fac;
+      }
     }
   }
 
@@ -661,7 +771,12 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
   qi_t = max_nd(qi_t, dqi_dt);
   qs_t = max_nd(qs_t, dqs_dt);
   qg_t = max_nd(qg_t, dqg_dt);
-  const R qv_t = -(qc_t + qr_t + qi_t + qs_t + qg_t);
+  R q_t = qc_t;
+  if (nz(qr_t)) q_t = q_t + qr_t;
+  if (nz(qi_t)) q_t = q_t + qi_t;
+  if (nz(qs_t)) q_t = q_t + qs_t;
+  if (nz(qg_t)) q_t = q_t + qg_t;
+  const R qv_t = -q_t;
   D drq[6];
   if constexpr (kMixed) {
     // The tracer changes rhog q_t dt of the FP32 rates, formed in FP32 and
@@ -681,20 +796,26 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
     }
     drq[0] = -sum;
   } else {
-    drq[0] = rhog * D(qv_t) * dt;
-    drq[1] = rhog * D(qc_t) * dt;
-    drq[2] = rhog * D(qr_t) * dt;
-    drq[3] = rhog * D(qi_t) * dt;
-    drq[4] = rhog * D(qs_t) * dt;
-    drq[5] = rhog * D(qg_t) * dt;
+    const R qt[6] = {qv_t, qc_t, qr_t, qi_t, qs_t, qg_t};
+#pragma unroll
+    for (int n = 0; n < 6; ++n) {
+      drq[n] = D(qt[n]);
+      if (nz(qt[n])) drq[n] = rhog * D(qt[n]) * dt;
+    }
   }
   o.Vtr = D(Vtr);
   o.Vts = D(Vts);
   o.Vtg = D(Vtg);
   o.Vti = D(Vti);
 
-  // effective radius and cloud top, :1566-1592
-  {
+  // effective radius and cloud top, :1566-1592 (without cloud water and rain
+  // the radii are 0 and there is no top, on both sides of r2_min)
+  if (!(hc || hr)) {
+    o.rceff = D(0.0);
+    o.rceff_cld = D(0.0);
+    o.rctop = D(UNDEF);
+    o.tctop = D(UNDEF);
+  } else {
     const R r2_min = R(1.0E-10), q_min = R(1.0E-5);
     R K_xf = C.K_xf, K_r2c = C.K_r2c;
     if constexpr (OPT) {
@@ -720,8 +841,12 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
 
   // ---- TagUpdateRHOGQ / RHOGE / MassConc / TEM, mod_mp_nsw6.cpp:692-744
 #pragma unroll
-  for (int n = 0; n < 6; ++n) rq[n] += drq[n];
-  rhoge = rhoge - LHV0 * drq[I_QV] + LHF0 * drq[I_QI] + LHF0 * drq[I_QS] + LHF0 * drq[I_QG];
+  for (int n = 0; n < 6; ++n)
+    if (nz(drq[n])) rq[n] += drq[n];
+  if (nz(drq[I_QV])) rhoge = rhoge - LHV0 * drq[I_QV];
+  if (nz(drq[I_QI])) rhoge = rhoge + LHF0 * drq[I_QI];
+  if (nz(drq[I_QS])) rhoge = rhoge + LHF0 * drq[I_QS];
+  if (nz(drq[I_QG])) rhoge = rhoge + LHF0 * drq[I_QG];
   o.q[0] = qn[0];
   if constexpr (kMixed) {
     // q from the shared reciprocal, T = rhoge / (rhog CVdry) (cv = CVdry as above)
@@ -733,10 +858,12 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
     for (int n = 1; n <= 5; ++n) o.q[n] = div_rn(rq[n], by_rhog);
     D qd2 = D(1.0);
 #pragma unroll
-    for (int n = 1; n <= 5; ++n) qd2 = qd2 - o.q[n];
+    for (int n = 1; n <= 5; ++n)
+      if (nz(o.q[n])) qd2 = qd2 - o.q[n];
     D cva = qd2 * CVDRY;
 #pragma unroll
-    for (int n = 1; n <= 5; ++n) cva = cva + o.q[n] * CVDRY;
+    for (int n = 1; n <= 5; ++n)
+      if (nz(o.q[n])) cva = cva + o.q[n] * CVDRY;
     o.tem = quo(rhoge, rhog * cva);
   }
   o.rhog = rhog;
@@ -763,10 +890,11 @@ __device__ __forceinline__ R vadv_wh(const WP& wp, int j, int mkmin, int mkmax) 
 // instead of divisions.  zdis only decides which layer the departure point
 // lies in (an ulp-level change matters only within an ulp of an interface)
 // and scales the flux of the departure layer.
-// The same from the half-level velocities wh(j) themselves (an accessor).
-template <class R, class G, class WH>
-__device__ __forceinline__ R vadv_zdis_wh(const WH& wh, const G* rdz, const G* rdzs, int k, int mkmin, R dt, R hdt2,
-                                          R sdt3) {
+// The same from the half-level velocities wh(j) themselves (an accessor);
+// rdzs2(k) gives 2 rdzs[k].
+template <class R, class G, class WH, class TW>
+__device__ __forceinline__ R vadv_zdis_wh(const WH& wh, const G* rdz, const G* rdzs, const TW& rdzs2, int k, int mkmin,
+                                          R dt, R hdt2, R sdt3) {
   if (k == mkmin) {
     const R w0 = wh(mkmin), wpp = wh(mkmin + 1);
     return fmaR(-hdt2 * w0, (wpp - w0) * rdz[mkmin], dt * w0);
@@ -775,7 +903,7 @@ __device__ __forceinline__ R vadv_zdis_wh(const WH& wh, const G* rdz, const G* r
   const R w0 = wh(k);
   const R wpp = wh(k + 1);
   const R r = (wpp - wm) * rdzs[k];
-  const R c = R(2.0) * rdzs[k] * fmaR(wpp - w0, rdz[k], -(w0 - wm) * rdz[k - 1]);
+  const R c = rdzs2(k) * fmaR(wpp - w0, rdz[k], -(w0 - wm) * rdz[k - 1]);
   const R t3 = sdt3 * w0 * fmaR(w0, c, r * r);
   return fmaR(-hdt2 * w0, r, fmaR(dt, w0, t3));
 }
@@ -784,7 +912,7 @@ template <class R, class G, class WP>
 __device__ __forceinline__ R vadv_zdis(const WP& wp, const G* rdz, const G* rdzs, int k, int mkmin, int mkmax, R dt,
                                        R hdt2, R sdt3) {
   auto wh = [&](int j) { return vadv_wh<R>(wp, j, mkmin, mkmax); };
-  return vadv_zdis_wh<R>(wh, rdz, rdzs, k, mkmin, dt, hdt2, sdt3);
+  return vadv_zdis_wh<R>(wh, rdz, rdzs, [&](int j) { return R(2.0) * rdzs[j]; }, k, mkmin, dt, hdt2, sdt3);
 }
 
 }  // namespace nsw6

@@ -106,6 +106,10 @@ NSW6_FP_HD bool is_nonneg(double x) {                                           
   const long long b = fp_bits(x);
   return (b >= 0 && b <= FP_INF) || b == FP_SIGN;
 }
+NSW6_FP_HD bool is_finite_nonneg(double x) {                                             // 0 <= x < inf
+  const long long b = fp_bits(x);
+  return (unsigned long long)b < (unsigned long long)FP_INF || b == FP_SIGN;
+}
 NSW6_FP_HD bool is_zero(double x) { return fp_is_zero(x); }                              // x == 0
 NSW6_FP_HD bool lt_z(double x) {                                                         // x < 0
   return (unsigned long long)fp_bits(x) - 0x8000000000000001ull < 0x7FF0000000000000ull;

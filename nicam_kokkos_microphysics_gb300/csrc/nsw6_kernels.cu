@@ -1,16 +1,17 @@
 // GB300 (sm_103a) kernels of one NSW6 microphysics step, FP64.
 //
-// Three kernels per step (plus three memsets: the extrema buffers and the
-// saturated-cell list's count):
+// Four kernels per step:
 //
-//  nsw6_cell_kernel    one CTA = CELL_TG columns x all interior levels of one
+//  nsw6_cell_kernel    one CTA = a tile of consecutive interior cells of one
 //                      region.  Per cell: negative filter, saturation values,
 //                      Bergeron parameters, the NSW6 process rates, the
-//                      RHOGQ/RHOGE/TEM updates and the fall speeds.  Then, per
-//                      column, the sedimentation departure distances of
-//                      vadv1d_prep for QR/QS/QG on full and half levels and
-//                      their per-level extrema, reduced over the region with
-//                      exact order-preserving 64-bit atomics.
+//                      RHOGQ/RHOGE/TEM updates and the fall speeds.
+//
+//  nsw6_departure_kernel  one CTA = DEP_TG columns x all levels of one falling
+//                      tracer: the sedimentation departure distances of
+//                      vadv1d_prep on full and half levels and their per-level
+//                      extrema, reduced over the region with exact
+//                      order-preserving 64-bit atomics.
 //
 //  nsw6_column_kernel  one CTA = COL_TG columns x all levels, column state in
 //                      shared memory.  Departure cells, the 24 flux integrals of
@@ -24,8 +25,8 @@
 //                      (the saturation adjustment) and its final state.
 //
 // The only coupling between columns, the per-level max/min of the departure
-// distance over a region (mod_vadv1d.cpp:316-353), is what separates the two
-// kernels.
+// distance over a region (mod_vadv1d.cpp:316-353), is what separates the cell
+// phase (the first two kernels) from the column phase.
 #include <cfloat>
 #include <cuda_runtime.h>
 
@@ -63,105 +64,114 @@ __device__ __forceinline__ FloatMath make_math<FloatMath>(const double*) {
   return FloatMath{};
 }
 
-// Shared memory of the cell kernel: fall speeds [ntr][K][CELL_TG] (type R; 3
-// sedimenting tracers, 4 in the kernel with the scheme switches), the grid
-// block [GF_COUNT][K] and the fast-math tables (doubles), and for R = float
-// FP32 copies of the four reciprocal rows the departure distances use.
+// Cells of one CTA at most: the shared-memory keys and order take 3 B each.
+constexpr int CELL_TILE_MAX = 4096;
+
+// Fall speeds go from the cell kernel to the departure kernel in the 8-byte
+// words of the departure distances' own rows (row t of tracer t); FP32 speeds
+// as their bits.
+__device__ __forceinline__ double vt_word(double v) { return v; }
+__device__ __forceinline__ double vt_word(float v) { return __longlong_as_double((long long)__float_as_uint(v)); }
 template <class R>
-__host__ __device__ constexpr size_t cell_vts_doubles(int K, int nv = 3) {
-  return (nv * (size_t)K * CELL_TG * sizeof(R) + sizeof(double) - 1) / sizeof(double);
+__device__ __forceinline__ R vt_value(double w) {
+  if constexpr (sizeof(R) == sizeof(float)) return __uint_as_float((unsigned)__double_as_longlong(w));
+  else return w;
 }
 
-// OPT: the kernel with the scheme switches (FP64 only): the switched branches
-// of nsw6_cell, the CCN input, and the ice fall speed with its departure
-// distances when QI sediments.
+// Counts v (< 64; 64: cells to leave out) into bucket[] and returns the cell's
+// position in its bucket; one shared-memory atomic for each value that a warp
+// holds, not one a cell.
+__device__ __forceinline__ int bucket_add(int* bucket, int v) {
+  const unsigned lane = threadIdx.x & 31;
+  const unsigned peers = __match_any_sync(__activemask(), v);
+  const int leader = __ffs(peers) - 1;
+  int base = 0;
+  if ((int)lane == leader) base = atomicAdd(&bucket[v], __popc(peers));
+  return __shfl_sync(peers, base, leader) + __popc(peers & ((1u << lane) - 1u));
+}
+
+// One CTA: `tile` consecutive interior cells of one region in [k][g] order, the
+// cell physics and nothing that couples cells.  Bound by the FP64 pipe: what
+// helps is to leave work out, so the FP64 tile's cells are grouped by their
+// side of 0 C and by the hydrometeors they hold (a counting sort in shared
+// memory), in Gray-code order, so that a warp that straddles two groups does
+// the work of the larger one only.  A tile of many columns by few levels has
+// larger groups than one of 32 columns by all levels (the layout before, with
+// the departure distances in the same kernel).  The order only decides which
+// thread computes which cell.  One 16900 x 42 region, FP64, with the departure
+// kernel: 0.90 -> 0.67 ms (10.1 M -> 9.6 M FP64 warp instructions, of which this
+// kernel 7.1 M: its FP64 pipe is 75 % busy); 48 columns, which had two CTAs
+// here, 0.47 -> 0.29 ms for the whole step.
+//
+// OPT: the kernel with the scheme switches: the switched branches of nsw6_cell
+// and the CCN input.
 template <class M, class R, bool OPT = false>
-__global__ void __launch_bounds__(CELL_THREADS, 2) nsw6_cell_kernel(Problem P, ConstsT<R> C) {
+__global__ void __launch_bounds__(CELL_THREADS, 2) nsw6_cell_kernel(Problem P, ConstsT<R> C, int tile) {
   constexpr bool kMixed = sizeof(R) == sizeof(float);
-  constexpr int NV = OPT ? 4 : 3;            // fall-speed rows in shared memory
   const int ntr = OPT ? P.ntr : 3;          // sedimenting tracers of this call
   extern __shared__ double sm[];
-  const int G = P.gall, K = P.kall, kmin = P.kmin, kmax = P.kmax;
+  const int G = P.gall, kmin = P.kmin, kmax = P.kmax;
   const int l = blockIdx.y;
-  const int g0 = blockIdx.x * CELL_TG;
-  const size_t KG = (size_t)K * G;
-  const size_t off = (size_t)l * KG;
-  const size_t offq = (size_t)l * NQ * KG;
-  R* vts = reinterpret_cast<R*>(sm);                   // [ntr][K][CELL_TG] fall speeds, tracer order
-  // grid metrics and FastMath tables: staged in shared memory, or, in the
-  // kernel with the scheme switches for columns deeper than CELL_SMEM_KMAX,
-  // read from global memory (through L1)
-  const bool stage = !OPT || K <= CELL_SMEM_KMAX;
-  double* sgrid = sm + cell_vts_doubles<R>(K, NV);     // [GF_COUNT][K]
-  double* stab = sgrid + (stage ? GF_COUNT * K : 0);   // [FM_TABLE_DOUBLES]
-  const double* grid = stage ? sgrid : P.grid;
-  const double* tab = stage ? stab : P.fmtab;
-  float* gridf = reinterpret_cast<float*>(stab + (stage ? FM_TABLE_DOUBLES : 0));  // [4][K], mixed only
-  unsigned short* perm = reinterpret_cast<unsigned short*>(gridf + 4 * K);  // [nlev * CELL_TG], FP64 only
-  unsigned char* key = reinterpret_cast<unsigned char*>(perm + (K - 2) * CELL_TG);
-  R* whs = reinterpret_cast<R*>(                                          // [K][CELL_TG] half-level velocities
-      (reinterpret_cast<uintptr_t>(key + (K - 2) * CELL_TG) + 15) & ~(uintptr_t)15);
-  __shared__ int bucket[33];
+  const int first = blockIdx.x * tile;                 // of the region's interior cells
+  const int n = min(tile, (kmax - kmin + 1) * G - first);
+  const size_t KG = (size_t)P.kall * G;
+  const size_t off = (size_t)l * KG + (size_t)kmin * G + first;          // the tile's first cell
+  const size_t offq = (size_t)l * NQ * KG + (size_t)kmin * G + first;
+  const size_t offv = (size_t)l * 2 * ntr * KG + (size_t)kmin * G + first;
+  double* stab = sm;                                                     // [FM_TABLE_DOUBLES], FP64 only
+  unsigned short* perm = reinterpret_cast<unsigned short*>(stab + FM_TABLE_DOUBLES);   // [tile], FP64 only
+  unsigned char* key = reinterpret_cast<unsigned char*>(perm + tile);
+  __shared__ int bucket[64];
 
-  for (int c = threadIdx.x; c < NV * K * CELL_TG; c += blockDim.x) vts[c] = R(0.0);
-  if (stage) {
-    for (int c = threadIdx.x; c < GF_COUNT * K; c += blockDim.x) sgrid[c] = P.grid[c];
-    if (!kMixed)
-      for (int c = threadIdx.x; c < FM_TABLE_DOUBLES; c += blockDim.x) stab[c] = P.fmtab[c];
+  // the departure kernel's extrema and the column kernel's list start empty
+  {
+    const unsigned nkey = (unsigned)P.lall * 2 * ntr * P.kall;
+    const unsigned nthread = gridDim.x * gridDim.y * blockDim.x;
+    for (unsigned e = (blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x; e < nkey; e += nthread) {
+      P.zmax[e] = 0ull;
+      P.zmin[e] = ~0ull;
+      if (e == 0) P.satq[0] = 0u;
+    }
   }
-  if (kMixed) {
-    const int rows[4] = {GF_RDGZ, GF_RDGZH, GF_RDZS, GF_RDZSH};
-    for (int c = threadIdx.x; c < 4 * K; c += blockDim.x) gridf[c] = (float)P.grid[rows[c / K] * K + c % K];
-  }
-  __syncthreads();
-  const M mth = make_math<M>(tab);
-
-  const int nlev = kmax - kmin + 1;
-  const int ncell = nlev * CELL_TG;
-  // FP64: the tile's cells are grouped by the hydrometeors they hold (snow,
-  // rain, graupel, ice, cloud water: the blocks nsw6_cell skips when a species
-  // is absent), so that warps are uniform and skip those blocks together.  The
-  // order only decides which thread computes which cell.
-  int nvalid = ncell;
   if (!kMixed) {
-    for (int c = threadIdx.x; c < 33; c += blockDim.x) bucket[c] = 0;
+    for (int c = threadIdx.x; c < FM_TABLE_DOUBLES; c += blockDim.x) stab[c] = P.fmtab[c];
+    for (int c = threadIdx.x; c < 64; c += blockDim.x) bucket[c] = 0;
     __syncthreads();
-    for (int c = threadIdx.x; c < ncell; c += blockDim.x) {
-      const int k = kmin + c / CELL_TG;
-      const int g = g0 + c % CELL_TG;
-      int kk = 32;   // columns past the region's end go last
-      if (g < G) {
-        const size_t iq = offq + (size_t)k * G + g;
-        kk = (gt_z(P.rhogq[iq + (size_t)I_QS * KG]) ? 16 : 0) | (gt_z(P.rhogq[iq + (size_t)I_QR * KG]) ? 8 : 0) |
-             (gt_z(P.rhogq[iq + (size_t)I_QG * KG]) ? 4 : 0) | (gt_z(P.rhogq[iq + (size_t)I_QI * KG]) ? 2 : 0) |
-             (gt_z(P.rhogq[iq + (size_t)I_QC * KG]) ? 1 : 0);
-      }
+#pragma unroll 1
+    for (int c = threadIdx.x; c < n; c += blockDim.x) {
+      const double* rq = P.rhogq + offq + c;
+      int kk = (lt_c(P.tem[off + c], TEM00) ? 32 : 0) | (gt_z(rq[(size_t)I_QS * KG]) ? 16 : 0) |
+               (gt_z(rq[(size_t)I_QR * KG]) ? 8 : 0) | (gt_z(rq[(size_t)I_QG * KG]) ? 4 : 0) |
+               (gt_z(rq[(size_t)I_QI * KG]) ? 2 : 0) | (gt_z(rq[(size_t)I_QC * KG]) ? 1 : 0);
+      kk ^= kk >> 1;   // the key's place in Gray-code order
+      kk ^= kk >> 2;
+      kk ^= kk >> 4;
       key[c] = (unsigned char)kk;
-      atomicAdd(&bucket[kk], 1);
+      bucket_add(bucket, kk);
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-      int run = 0;
-      for (int b = 0; b < 33; ++b) {
-        const int n = bucket[b];
-        bucket[b] = run;
-        run += n;
+    if (threadIdx.x < 32) {   // exclusive prefix sums of the 64 counts
+      const int b0 = bucket[2 * threadIdx.x], b1 = bucket[2 * threadIdx.x + 1];
+      int run = b0 + b1;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, run, o);
+        if ((int)threadIdx.x >= o) run += v;
       }
+      bucket[2 * threadIdx.x] = run - b0 - b1;
+      bucket[2 * threadIdx.x + 1] = run - b1;
     }
     __syncthreads();
-    nvalid = bucket[32];   // cells of columns inside the region
-    __syncthreads();
-    for (int c = threadIdx.x; c < ncell; c += blockDim.x) perm[atomicAdd(&bucket[key[c]], 1)] = (unsigned short)c;
+#pragma unroll 1
+    for (int c = threadIdx.x; c < n; c += blockDim.x) perm[bucket_add(bucket, key[c])] = (unsigned short)c;
     __syncthreads();
   }
-  for (int j = threadIdx.x; j < nvalid; j += blockDim.x) {
+  const M mth = make_math<M>(stab);
+#pragma unroll 1
+  for (int j = threadIdx.x; j < n; j += blockDim.x) {
     const int c = kMixed ? j : perm[j];
-    const int k = kmin + c / CELL_TG;
-    const int gx = c % CELL_TG;
-    const int g = g0 + gx;
-    if (g >= G) continue;
-    const size_t i = off + (size_t)k * G + g;
-    const size_t iq = offq + (size_t)k * G + g;
+    const size_t i = off + c;
+    const size_t iq = offq + c;
     CellIn in;
     in.rhog = P.rhog[i];
     in.tem = P.tem[i];
@@ -181,100 +191,116 @@ __global__ void __launch_bounds__(CELL_THREADS, 2) nsw6_cell_kernel(Problem P, C
     for (int n = 1; n < 6; ++n) P.q[iq + (size_t)n * KG] = o.q[n];
     P.re_liquid[i] = o.rceff;
     P.re_cld[i] = o.rceff_cld;
-    // tracer order of the transport: QR, (QI,) QS, QG
-    vts[(0 * K + k) * CELL_TG + gx] = R(o.Vtr);
-    if (ntr == 4) vts[(1 * K + k) * CELL_TG + gx] = R(o.Vti);
-    vts[((ntr - 2) * K + k) * CELL_TG + gx] = R(o.Vts);
-    vts[((ntr - 1) * K + k) * CELL_TG + gx] = R(o.Vtg);
-    if (k == kmax) {
+    // fall speeds in the tracer order of the transport: QR, (QI,) QS, QG
+    double* vt = P.zdis + offv + c;
+    vt[0] = vt_word(R(o.Vtr));
+    if (ntr == 4) vt[KG] = vt_word(R(o.Vti));
+    vt[(size_t)(ntr - 2) * KG] = vt_word(R(o.Vts));
+    vt[(size_t)(ntr - 1) * KG] = vt_word(R(o.Vtg));
+    const int top = first + c - (kmax - kmin) * G;
+    if (top >= 0) {
       // The reference writes the cloud-top scalars from every level in parallel
       // (mod_mp_nsw6.cpp:1579-1592); the sequential order, in which the top
       // interior level is written last, is used.  TagUpdateCLD, :710-726.
-      const size_t ic = (size_t)l * G + g;
+      const size_t ic = (size_t)l * G + top;
       P.rctop[ic] = o.rctop;
       P.tctop[ic] = o.tctop;
       const double sw = (0.5 + copysign(0.5, o.tctop - TEM00));
       P.rwtop[ic] = (sw)*o.rctop + (1.0 - sw) * UNDEF;
     }
   }
+}
+
+// ------------------------------------------------------- departure distances
+// 0.5 x: the exponent one lower, where that is all there is to it
+__device__ __forceinline__ float half_of(float x) { return 0.5f * x; }
+__device__ __forceinline__ double half_of(double x) {
+  const long long b = __double_as_longlong(x);
+  if ((unsigned)(((b >> 52) & 0x7FF) - 2) < 2045u) return __longlong_as_double(b - (1ll << 52));
+  return (b << 1) == 0 ? x : 0.5 * x;
+}
+// the largest (smallest) key of a warp's lanes
+__device__ __forceinline__ unsigned long long warp_max(unsigned long long v) {
+  const unsigned hi = __reduce_max_sync(0xffffffffu, (unsigned)(v >> 32));
+  const unsigned lo = __reduce_max_sync(0xffffffffu, (unsigned)(v >> 32) == hi ? (unsigned)v : 0u);
+  return ((unsigned long long)hi << 32) | lo;
+}
+__device__ __forceinline__ unsigned long long warp_min(unsigned long long v) { return ~warp_max(~v); }
+
+// Departure distances (vadv1d_prep, mod_vadv1d.cpp:262-302) of one tracer on
+// full and half levels for DEP_TG columns, and their per-level extrema over the
+// region (order-preserving keys, exact atomics, so the order does not matter).
+// Row t of zdis holds the tracer's fall speeds on entry, the full-level
+// distances on return, row ntr + t the half-level ones.  One CTA reads all of
+// its columns' speeds before it writes.  Bound by the FP64 pipe: a half-level
+// velocity is the mean of two full-level ones, formed once, and the halvings
+// are integer operations.
+constexpr int DEP_TG = 32;
+constexpr int DEP_THREADS = 256;
+
+template <class R>
+__host__ __device__ constexpr size_t departure_smem_bytes(int K) {
+  return (size_t)K * sizeof(R) * (3 * DEP_TG + 6);
+}
+
+template <class R>
+__global__ void __launch_bounds__(DEP_THREADS) nsw6_departure_kernel(Problem P) {
+  extern __shared__ double sm[];
+  const int G = P.gall, K = P.kall, kmin = P.kmin, kmax = P.kmax, ntr = P.ntr;
+  const int g0 = blockIdx.x * DEP_TG, t = blockIdx.y, l = blockIdx.z;
+  const size_t KG = (size_t)K * G;
+  R* vt = reinterpret_cast<R*>(sm);     // [K][DEP_TG] fall speeds, zero outside the interior
+  R* wf = vt + K * DEP_TG;              // [K][DEP_TG] velocities on the full levels' interfaces
+  R* wh = wf + K * DEP_TG;              // [K][DEP_TG] and on the half levels'
+  R* grid = wh + K * DEP_TG;            // 1 / dz, 1 / (dz- + dz) and twice that, of full and half levels
+  double* z0 = P.zdis + ((size_t)l * 2 * ntr + t) * KG;
+  double* z1 = z0 + (size_t)ntr * KG;
+
+  const int rows[6] = {GF_RDGZ, GF_RDZS, GF_RDZS, GF_RDGZH, GF_RDZSH, GF_RDZSH};
+  for (int c = threadIdx.x; c < 6 * K; c += blockDim.x) {
+    const R v = R(P.grid[rows[c / K] * K + c % K]);
+    grid[c] = (c / K) % 3 == 2 ? R(2.0) * v : v;
+  }
+  const int gx = threadIdx.x % DEP_TG, g = g0 + gx, kw = threadIdx.x / DEP_TG, nw = blockDim.x / DEP_TG;
+#pragma unroll 4
+  for (int k = kw; k < K; k += nw)
+    vt[k * DEP_TG + gx] = (k >= kmin && k <= kmax && g < G) ? vt_value<R>(z0[(size_t)k * G + g]) : R(0.0);
+  __syncthreads();
+  // wh of vadv1d_prep from the speeds (full levels: mkmin = kmin)
+#pragma unroll 1
+  for (int k = kw; k < K; k += nw) {
+    const int c = k * DEP_TG + gx;
+    wf[c] = k > kmin && k <= kmax ? half_of(vt[c - DEP_TG] + vt[c]) : k == kmax + 1 ? vt[c - DEP_TG] : vt[c];
+  }
+  __syncthreads();
+  // half levels (mkmin = kmin + 1): the speeds there, Vtermh (mod_precip_transport.cpp:847-861), are the
+  // means just formed on [kmin + 1, kmax - 1] and zero elsewhere
+  auto vh = [&](int k) { return k > kmin && k < kmax ? wf[k * DEP_TG + gx] : R(0.0); };
+#pragma unroll 1
+  for (int k = kw; k < K; k += nw)
+    wh[k * DEP_TG + gx] = k > kmin + 1 && k <= kmax ? half_of(vh(k - 1) + vh(k)) : k == kmax + 1 ? vh(kmax) : vh(k);
   __syncthreads();
 
-  // Departure distances (vadv1d_prep) and their per-level region extrema.
-  // Row s = t + ntr*half: t = the sedimenting tracer; half = 0 full levels
-  // (mkmin = kmin, dz = dgz), 1 half levels (mkmin = kmin+1, dz = dgzh,
-  // wp = Vtermh).
-  const R* rdgz;
-  const R* rdgzh;
-  const R* rdzs;
-  const R* rdzsh;
-  if constexpr (kMixed) {
-    rdgz = gridf;
-    rdgzh = gridf + K;
-    rdzs = gridf + 2 * K;
-    rdzsh = gridf + 3 * K;
-  } else {
-    rdgz = grid + GF_RDGZ * K;
-    rdgzh = grid + GF_RDGZH * K;
-    rdzs = grid + GF_RDZS * K;
-    rdzsh = grid + GF_RDZSH * K;
-  }
-  const R dtR = R(P.dt), hdt2R = R(P.hdt2), sdt3R = R(P.sdt3);
-  // one row at a time: its half-level velocities wh(j) first (each is used by
-  // three departure distances), then the distances
-  const int nrow = 2 * ntr;
-  for (int s = 0; s < nrow; ++s) {
-    const int t = s % ntr;
-    const int half = s / ntr;
-    const int mkmin = half ? kmin + 1 : kmin;
-    for (int c = threadIdx.x; c < K * CELL_TG; c += blockDim.x) {
-      const int j = c / CELL_TG, gx = c % CELL_TG;
-      if (j < mkmin - 1 || j > kmax + 1) continue;
-      const R* col = vts + t * K * CELL_TG + gx;
-      R v;
-      if (!half) {
-        auto wp = [&](int jj) { return col[jj * CELL_TG]; };
-        v = vadv_wh<R>(wp, j, mkmin, kmax);
-      } else {
-        // Vtermh, mod_precip_transport.cpp:847-861
-        auto wp = [&](int jj) {
-          return (jj >= kmin + 1 && jj <= kmax - 1) ? R(0.5) * (col[jj * CELL_TG] + col[(jj - 1) * CELL_TG]) : R(0.0);
-        };
-        v = vadv_wh<R>(wp, j, mkmin, kmax);
-      }
-      whs[c] = v;
-    }
-    __syncthreads();
-  for (int c = threadIdx.x; c < K * CELL_TG; c += blockDim.x) {
-    const int k = c / CELL_TG;
-    const int gx = c % CELL_TG;
-    if (k < mkmin || k > kmax) continue;  // uniform across the warp (CELL_TG == 32)
-    const int g = g0 + gx;
+  const R dt = R(P.dt), hdt2 = R(P.hdt2), sdt3 = R(P.sdt3);
+#pragma unroll 1
+  for (int row = kw; row < 2 * K; row += nw) {   // one warp: one level of one of the two rows
+    const int half = row >= K ? 1 : 0, k = row - half * K, mkmin = kmin + half;
+    if (k < mkmin || k > kmax) continue;
+    const R* w = half ? wh : wf;
+    const R* gr = grid + 3 * half * K;
     const bool valid = g < G;
-    double z = 0.0;
-    if (valid) {
-      auto wh = [&](int j) { return whs[j * CELL_TG + gx]; };
-      z = half ? double(vadv_zdis_wh<R>(wh, rdgzh, rdzsh, k, mkmin, dtR, hdt2R, sdt3R))
-               : double(vadv_zdis_wh<R>(wh, rdgz, rdzs, k, mkmin, dtR, hdt2R, sdt3R));
-      P.zdis[((size_t)l * nrow + s) * KG + (size_t)k * G + g] = z;
-    }
+    auto wp = [&](int j) { return w[j * DEP_TG + gx]; };
+    const double z = double(vadv_zdis_wh<R>(wp, gr, gr + K, [&](int j) { return gr[2 * K + j]; }, k, mkmin, dt, hdt2, sdt3));
+    if (valid) (half ? z1 : z0)[(size_t)k * G + g] = z;
     // NaN never wins the reference's comparisons, so it is left out
     const bool use = valid && !is_nan_bits(z);
-    unsigned long long kmx = use ? order_key(z) : 0ull;
-    unsigned long long kmn = use ? order_key(z) : ~0ull;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const unsigned long long a = __shfl_xor_sync(0xffffffffu, kmx, o);
-      const unsigned long long b = __shfl_xor_sync(0xffffffffu, kmn, o);
-      kmx = a > kmx ? a : kmx;
-      kmn = b < kmn ? b : kmn;
-    }
-    if ((threadIdx.x & 31) == 0) {
-      const size_t e = ((size_t)l * nrow + s) * K + k;
+    const unsigned long long kmx = warp_max(use ? order_key(z) : 0ull);
+    const unsigned long long kmn = warp_min(use ? order_key(z) : ~0ull);
+    if (gx == 0) {
+      const size_t e = ((size_t)l * 2 * ntr + half * ntr + t) * K + k;
       if (kmx != 0ull) atomicMax(&P.zmax[e], kmx);
       if (kmn != ~0ull) atomicMin(&P.zmin[e], kmn);
     }
-  }
-    __syncthreads();
   }
 }
 
@@ -1439,13 +1465,41 @@ cudaError_t launch_math(int fn, const double* x, const double* y, double* out, i
 }
 
 // ------------------------------------------------------------------ launchers
-size_t cell_smem_bytes(int K, bool mixed, bool opt) {
-  const size_t vts = mixed ? cell_vts_doubles<float>(K, opt ? 4 : 3) : cell_vts_doubles<double>(K, opt ? 4 : 3);
-  const size_t staged = (!opt || K <= CELL_SMEM_KMAX) ? (size_t)GF_COUNT * K + FM_TABLE_DOUBLES : 0;
-  // fall speeds, grid, tables, the FP32 reciprocal rows, the cell order and keys
-  return sizeof(double) * (vts + staged) + sizeof(float) * 4 * K +
-         (sizeof(unsigned short) + 1) * (size_t)(K - 2) * CELL_TG + 16 +
-         (mixed ? sizeof(float) : sizeof(double)) * (size_t)K * CELL_TG;
+// Tile and threads of the cell kernel for `cells` interior cells of each of
+// lall regions.  Two CTAs of 256 threads fit an SM (128 registers); the tiles
+// share the cells out evenly over whole waves of them, so that no last wave is
+// nearly empty, and a call too small for that gets a cell a thread on as many
+// SMs as it has warps (a lone warp issues an FP64 instruction every 64 cycles,
+// four warps of an SM one every 16 to 19: fewer warps an SM cost nothing).
+struct CellShape {
+  int tile, threads, blocks;
+};
+static CellShape cell_shape(int cells, int lall) {
+  const int slots = 2 * 152;
+  CellShape s;
+  const long long total = (long long)cells * lall;
+  if (total <= (long long)slots * CELL_THREADS) {
+    const long long warps = (total + 31) / 32;
+    s.threads = (int)((warps + slots - 1) / slots) * 32;
+    s.tile = s.threads;
+  } else {
+    // whole waves of `slots` CTAs, each region's cells shared out alike
+    const int tile_goal = 2304;
+    const long long waves = (total + (long long)slots * tile_goal - 1) / ((long long)slots * tile_goal);
+    long long per = (waves * slots) / lall;   // CTAs of a region
+    if (per < 1) per = 1;
+    int tile = (int)((cells + per - 1) / per);
+    tile = (tile + 31) / 32 * 32;
+    if (tile > CELL_TILE_MAX) tile = CELL_TILE_MAX;
+    const int passes = (tile + CELL_THREADS - 1) / CELL_THREADS;
+    s.threads = ((tile + passes - 1) / passes + 31) / 32 * 32;
+    s.tile = tile;
+  }
+  s.blocks = (cells + s.tile - 1) / s.tile;
+  return s;
+}
+static size_t cell_smem_bytes(const CellShape& s, bool mixed) {
+  return mixed ? 0 : sizeof(double) * FM_TABLE_DOUBLES + 3 * (size_t)s.tile;
 }
 
 int column_tile(int K) { return K <= 64 ? 16 : 8; }
@@ -1470,22 +1524,31 @@ int column_threads(int K) {
 
 cudaError_t launch_prepare();
 
-// The cell kernel alone (FP64): used on a copy of a state to obtain the
+// The cell phase: the cell kernel and the departure distances.
+static cudaError_t launch_cells(const Problem& P, const Consts& C, cudaStream_t stream) {
+  const CellShape s = cell_shape((P.kmax - P.kmin + 1) * P.gall, P.lall);
+  const size_t sm = cell_smem_bytes(s, P.mixed != 0);
+  const dim3 g1(s.blocks, P.lall);
+  const int nt = s.threads;
+  if (P.opt && P.mixed) nsw6_cell_kernel<FloatMath, float, true><<<g1, nt, sm, stream>>>(P, consts_to_float(C), s.tile);
+  else if (P.opt) nsw6_cell_kernel<FastMath, double, true><<<g1, nt, sm, stream>>>(P, C, s.tile);
+  else if (P.mixed) nsw6_cell_kernel<FloatMath, float><<<g1, nt, sm, stream>>>(P, consts_to_float(C), s.tile);
+  else if (P.math_lib) nsw6_cell_kernel<LibMath, double><<<g1, nt, sm, stream>>>(P, C, s.tile);
+  else nsw6_cell_kernel<FastMath, double><<<g1, nt, sm, stream>>>(P, C, s.tile);
+  const dim3 g2((P.gall + DEP_TG - 1) / DEP_TG, P.ntr, P.lall);
+  if (P.mixed) nsw6_departure_kernel<float><<<g2, DEP_THREADS, departure_smem_bytes<float>(P.kall), stream>>>(P);
+  else nsw6_departure_kernel<double><<<g2, DEP_THREADS, departure_smem_bytes<double>(P.kall), stream>>>(P);
+  return cudaGetLastError();
+}
+
+// The cell phase alone (FP64): used on a copy of a state to obtain the
 // region extrema of the departure distances for the derivative kernels.
 cudaError_t launch_cell_only(const Problem& P, const Consts& C, cudaStream_t stream) {
-  const size_t nkey = (size_t)P.lall * 2 * P.ntr * P.kall;
-  cudaError_t e = cudaMemsetAsync(P.zmax, 0x00, nkey * sizeof(unsigned long long), stream);
+  const cudaError_t e = launch_prepare();
   if (e != cudaSuccess) return e;
-  e = cudaMemsetAsync(P.zmin, 0xff, nkey * sizeof(unsigned long long), stream);
-  if (e != cudaSuccess) return e;
-  e = launch_prepare();
-  if (e != cudaSuccess) return e;
-  dim3 g1((P.gall + CELL_TG - 1) / CELL_TG, P.lall);
-  if (P.opt)
-    nsw6_cell_kernel<FastMath, double, true><<<g1, CELL_THREADS, cell_smem_bytes(P.kall, false, true), stream>>>(P, C);
-  else
-    nsw6_cell_kernel<FastMath, double><<<g1, CELL_THREADS, cell_smem_bytes(P.kall, false, false), stream>>>(P, C);
-  return cudaGetLastError();
+  Problem F = P;
+  F.mixed = F.math_lib = 0;
+  return launch_cells(F, C, stream);
 }
 
 // Raises a kernel's dynamic shared-memory limit to what the device allows a
@@ -1508,10 +1571,8 @@ cudaError_t launch_prepare() {
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     const cudaError_t r[] = {
         e,
-        raise_smem_limit(nsw6_cell_kernel<FastMath, double>, optin),
-        raise_smem_limit(nsw6_cell_kernel<LibMath, double>, optin),
-        raise_smem_limit(nsw6_cell_kernel<FloatMath, float>, optin),
-        raise_smem_limit(nsw6_cell_kernel<FastMath, double, true>, optin),
+        raise_smem_limit(nsw6_departure_kernel<double>, optin),
+        raise_smem_limit(nsw6_departure_kernel<float>, optin),
         raise_smem_limit(nsw6_column_kernel<16, FastMath, false, true>, optin),
         raise_smem_limit(nsw6_column_kernel<8, FastMath, false, true>, optin),
         raise_smem_limit(nsw6_column_kernel<16, FastMath, false>, optin),
@@ -1520,7 +1581,6 @@ cudaError_t launch_prepare() {
         raise_smem_limit(nsw6_column_kernel<8, LibMath, false>, optin),
         raise_smem_limit(nsw6_column_kernel<16, FastMath, true>, optin),
         raise_smem_limit(nsw6_column_kernel<8, FastMath, true>, optin),
-        raise_smem_limit(nsw6_cell_kernel<FloatMath, float, true>, optin),
         raise_smem_limit(nsw6_column_kernel<16, FastMath, true, true>, optin),
         raise_smem_limit(nsw6_column_kernel<8, FastMath, true, true>, optin)};
     done = cudaSuccess;
@@ -1534,25 +1594,12 @@ cudaError_t launch_prepare() {
 // that only it reads may still be arriving while the cell kernel runs).
 cudaError_t launch_step(const Problem& P, const Consts& C, cudaStream_t stream, cudaEvent_t* ev,
                         cudaEvent_t before_column) {
-  const size_t nkey = (size_t)P.lall * 2 * P.ntr * P.kall;
   cudaError_t e = launch_prepare();
   if (e != cudaSuccess) return e;
-  e = cudaMemsetAsync(P.zmax, 0x00, nkey * sizeof(unsigned long long), stream);
-  if (e != cudaSuccess) return e;
-  e = cudaMemsetAsync(P.zmin, 0xff, nkey * sizeof(unsigned long long), stream);
-  if (e != cudaSuccess) return e;
-  e = cudaMemsetAsync(P.satq, 0, sizeof(unsigned), stream);
-  if (e != cudaSuccess) return e;
   const bool opt = P.opt != 0;
-  const size_t s1 = cell_smem_bytes(P.kall, P.mixed != 0, opt);
   const size_t s2 = column_smem_bytes(P.kall, opt);
-  dim3 g1((P.gall + CELL_TG - 1) / CELL_TG, P.lall);
   if (ev) cudaEventRecord(ev[0], stream);
-  if (opt && P.mixed) nsw6_cell_kernel<FloatMath, float, true><<<g1, CELL_THREADS, s1, stream>>>(P, consts_to_float(C));
-  else if (opt) nsw6_cell_kernel<FastMath, double, true><<<g1, CELL_THREADS, s1, stream>>>(P, C);
-  else if (P.mixed) nsw6_cell_kernel<FloatMath, float><<<g1, CELL_THREADS, s1, stream>>>(P, consts_to_float(C));
-  else if (P.math_lib) nsw6_cell_kernel<LibMath, double><<<g1, CELL_THREADS, s1, stream>>>(P, C);
-  else nsw6_cell_kernel<FastMath, double><<<g1, CELL_THREADS, s1, stream>>>(P, C);
+  if ((e = launch_cells(P, C, stream)) != cudaSuccess) return e;
   if (ev) cudaEventRecord(ev[1], stream);
   if (before_column && (e = cudaStreamWaitEvent(stream, before_column, 0)) != cudaSuccess) return e;
   const int tg = column_tile(P.kall);
