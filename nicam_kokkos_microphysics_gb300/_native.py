@@ -19,9 +19,10 @@ INCLUDE = PKG.parent / "include"
 LIBDIR = PKG / "_lib"
 LIB = LIBDIR / "libnsw6_gb300.so"
 
-SOURCES = ["nsw6_kernels.cu", "nsw6_deriv.cu", "nsw6_adjoint.cu", "nsw6_driver.cu"]
+SOURCES = ["nsw6_adjoint.cu", "nsw6_deriv.cu", "nsw6_kernels.cu", "nsw6_column_fp64.cu", "nsw6_column_mixed.cu",
+           "nsw6_column_fp64_switches.cu", "nsw6_column_mixed_switches.cu", "nsw6_driver.cu"]
 HEADERS = ["nsw6_common.cuh", "nsw6_cell.cuh", "nsw6_fastmath.cuh", "nsw6_fpcmp.cuh", "nsw6_soft.cuh",
-           "nsw6_ad.cuh", "nsw6_column_step.cuh", "nsw6_cell_adjoint.cuh"]
+           "nsw6_ad.cuh", "nsw6_column_step.cuh", "nsw6_column.cuh", "nsw6_cell_adjoint.cuh"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 # --fmad=false keeps every product and sum separately rounded, as the
 # reference's arithmetic is written; fused operations are spelled out

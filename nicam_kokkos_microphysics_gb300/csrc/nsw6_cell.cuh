@@ -184,13 +184,13 @@ __device__ __forceinline__ T max_nd(const T& a, const T& d) { return dmax(a, -d)
 // (and NaNs) are left to the FP64 test, as the reference computes it.
 // lovr_f = float(LovR_liq).
 __device__ __forceinline__ int sat_screen_liq(double tem, double rho, double qsum, float lovr_f) {
-  const float tf = float(tem);
+  const float tf = soft_d2f(tem);
   const float tcf = (tf < float(TEM_MIN)) ? float(TEM_MIN) : tf;   // float(max(tem, TEM_MIN))
   const float xf = lovr_f * ((tcf - float(TEM00)) / (tcf * float(TEM00)));
   if (!(fabsf(xf) <= 80.0f)) return -1;
-  const float qsf = (float(PSAT0) * expf(xf)) / (float(rho) * float(RVAP) * tf);
+  const float qsf = (float(PSAT0) * expf(xf)) / (soft_d2f(rho) * float(RVAP) * tf);
   if (!(qsf >= 1.0e-11f && qsf <= 1.0e30f)) return -1;
-  const float qq = float(qsum);
+  const float qq = soft_d2f(qsum);
   if (qq > qsf * 1.0001f) return 1;
   if (qq < qsf * 0.9999f) return 0;
   return -1;
