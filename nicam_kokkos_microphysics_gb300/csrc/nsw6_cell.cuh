@@ -216,6 +216,13 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
   // partial derivatives), FP32 has cycles to spare: there nz(x) is true.
   constexpr bool kPlain = std::is_same<R, double>::value && std::is_same<D, double>::value;
   auto nz = [](const auto& x) { return !kPlain || !is_zero(x); };
+  // First in a block that is left out.  A block without a call is made
+  // predicated instructions, and an FP64 instruction takes the pipe its 16 to
+  // 19 cycles with every lane's predicate off too (measured); around a call
+  // there is a branch.
+  auto only = [] {
+    if constexpr (kPlain) soft_branch();
+  };
   const R dtR = R(dt), rdtR = R(rdt);
   // ---- negative_filter, mod_mp_nsw6.cpp:1770-1831
   D rq[6];
@@ -224,13 +231,22 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
   D diffq = D(0.0);
 #pragma unroll
   for (int n = 2; n <= 5; ++n) {
-    if (nz(rq[n])) diffq += rq[n];
+    if (nz(rq[n])) {
+      only();
+      diffq += rq[n];
+    }
     rq[n] = maxz(rq[n]);
   }
 #pragma unroll
   for (int n = 2; n <= 5; ++n)
-    if (nz(rq[n])) diffq -= rq[n];
-  if (nz(diffq)) rq[I_QV] += diffq;
+    if (nz(rq[n])) {
+      only();
+      diffq -= rq[n];
+    }
+  if (nz(diffq)) {
+    only();
+    rq[I_QV] += diffq;
+  }
   diffq = rq[I_QV];
   rq[I_QV] = maxz(rq[I_QV]);
   // x - x is +0 for the vapour that is not negative (1 - 0 is 1, rhog 1 is rhog)
@@ -268,11 +284,17 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
     D qd = D(1.0);
 #pragma unroll
     for (int n = 1; n <= 5; ++n)
-      if (nz(qn[n])) qd = qd - qn[n];
+      if (nz(qn[n])) {
+        only();
+        qd = qd - qn[n];
+      }
     D cv = qd * CVDRY;
 #pragma unroll
     for (int n = 1; n <= 5; ++n)
-      if (nz(qn[n])) cv = cv + qn[n] * CVDRY;
+      if (nz(qn[n])) {
+        only();
+        cv = cv + qn[n] * CVDRY;
+      }
     rhoge = temp * rhog * cv;
     pre = R(dens * (qd * RDRY + qn[0] * RVAP) * temp);
     densR = R(dens);
@@ -292,15 +314,18 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
   //      over liquid for the evaporation of rain, over ice for cold cells
   R rtem = Z, rdrt = Z, qsatl = Z, qsati = Z, Sliq = Z, Sice = Z;
   if (hr || wcold) {
+    only();
     rtem = quo(R(1.0), maxc(tempR, R(TEM_MIN)));
     rdrt = quo(R(1.0), densR * R(RVAP) * tempR);
   }
   if (hr) {
+    only();
     const R psatl = R(PSAT0) * mth.exp(C.LovR_liq * (C.RTEM00 - rtem));
     qsatl = psatl * rdrt;
     Sliq = quo(qv, maxc(qsatl, R(EPS)));
   }
   if (wcold) {
+    only();
     const R psati = R(PSAT0) * mth.exp(C.LovR_ice * (C.RTEM00 - rtem));
     qsati = psati * rdrt;
     Sice = quo(qv, maxc(qsati, R(EPS)));
@@ -308,13 +333,22 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
 
   // ---- TagBigLoop, mod_mp_nsw6.cpp:902-1594
   const R Rdens = quo(ONE, densR);
-  const R rho_fact = (hr || hs || hg) ? sqrtR(R(DENS00) * Rdens) : Z;
+  R rho_fact = Z;
+  if (hr || hs || hg) {
+    only();
+    rho_fact = sqrtR(R(DENS00) * Rdens);
+  }
   const bool d1 = ge_c(qr, R(1.0E-4));                          // delta1
   const bool d2 = le_c(qr, R(1.0E-4)) && le_c(qs, R(1.0E-4));       // delta2
   const bool sps = ge_c(Sice, ONE);                              // spsati
   const DivisorT<R> by_dt(dtR);
-  const R dqv_dt = per_dt(qv, by_dt, rdtR), dqc_dt = per_dt(qc, by_dt, rdtR), dqr_dt = per_dt(qr, by_dt, rdtR);
-  const R dqi_dt = per_dt(qi, by_dt, rdtR), dqs_dt = per_dt(qs, by_dt, rdtR), dqg_dt = per_dt(qg, by_dt, rdtR);
+  R dqv_dt = Z, dqc_dt = Z, dqr_dt = Z, dqi_dt = Z, dqs_dt = Z, dqg_dt = Z;
+  if (hr || wcold) dqv_dt = per_dt(qv, by_dt, rdtR);   // (no other cell uses it)
+  if (hc) dqc_dt = per_dt(qc, by_dt, rdtR);
+  if (hr) dqr_dt = per_dt(qr, by_dt, rdtR);
+  if (hi) dqi_dt = per_dt(qi, by_dt, rdtR);
+  if (hs) dqs_dt = per_dt(qs, by_dt, rdtR);
+  if (hg) dqg_dt = per_dt(qg, by_dt, rdtR);
 
   // The blocks of a species that is absent are skipped: every quantity they
   // would compute is then exactly zero (the reference evaluates them with a
@@ -326,6 +360,7 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
   R RLMDr = Z, RLMDr_dr = Z, RLMDr_2 = Z, RLMDr_3 = Z, RLMDr_1br = Z, RLMDr_2br = Z, RLMDr_3br = Z, RLMDr_7 = Z;
   R RLMDr_3dr = Z, RLMDr_5dr = Z, RLMDr_6dr = Z;
   if (rain) {
+    only();
     RLMDr = sqrtR(sqrtR(densR * qr * C.K_rlmdr));
     RLMDr_dr = sqrtR(RLMDr);
     RLMDr_2 = RLMDr * RLMDr;
@@ -342,7 +377,11 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
   // Roh and Satoh (2014) snow moments, :994-1057.  Each moment is
   // 10^loga * Xs2^b = exp(ln10 * loga + log(Xs2) * b), with loga and b
   // polynomials in tems whose coefficients per moment are folded on the host.
-  const R Xs2 = hs ? densR * qs * C.rAs : Z;
+  R Xs2 = Z;
+  if (hs) {
+    only();
+    Xs2 = densR * qs * C.rAs;
+  }
   const bool roh = !OPT || C.opt_roh != Z;
   const bool snow = roh && ge_c(Xs2, R(1.0E-12));
   R mom[7] = {Z, Z, Z, Z, Z, Z, Z};  // MOMs_0, _1, _0bs, _1bs, _2bs, _2ds (= nm 2.25), _5ds_h
@@ -370,6 +409,7 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
     }
   }
   if (snow) {
+    only();
     const R tems = lt_negc(temc, R(-0.1)) ? temc : R(-0.1);   // min(-0.1, temc)
     const R logX = mth.log(Xs2);
 #pragma unroll
@@ -390,6 +430,7 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
   const bool graupel = ge_c(qg, R(1.0E-12));
   R RLMDg = Z, RLMDg_dg = Z, RLMDg_2 = Z, RLMDg_3 = Z, RLMDg_3dg = Z, RLMDg_5dg = Z;
   if (graupel) {
+    only();
     RLMDg = sqrtR(sqrtR(densR * qg * C.K_rlmdg));
     RLMDg_dg = sqrtR(RLMDg);
     RLMDg_2 = RLMDg * RLMDg;
@@ -400,9 +441,19 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
 
   // terminal velocity, :1072-1078
   // (an absent species' is the zero of the product's sign)
-  const R Vtr = hr ? C.K_vtr * rho_fact * RLMDr_dr : sel(false, C.K_vtr);
-  const R Vts = hs ? C.K_vts * rho_fact * RMOMs_Vt : sel(false, C.K_vts);
-  const R Vtg = hg ? C.K_vtg * rho_fact * RLMDg_dg : sel(false, C.K_vtg);
+  R Vtr = sel(false, C.K_vtr), Vts = sel(false, C.K_vts), Vtg = sel(false, C.K_vtg);
+  if (hr) {
+    only();
+    Vtr = C.K_vtr * rho_fact * RLMDr_dr;
+  }
+  if (hs) {
+    only();
+    Vts = C.K_vts * rho_fact * RMOMs_Vt;
+  }
+  if (hg) {
+    only();
+    Vtg = C.K_vtg * rho_fact * RLMDg_dg;
+  }
   R Vti = Z;
   if constexpr (OPT) {
     // :1073-1075 with sw_constVti = 0 (CONST_Vti is UNDEF)
@@ -418,6 +469,7 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
   // Qi0 = ice_nuc * Ni0^1.33 / dens, with log(Ni0) = ln 1000 + max(-0.1 temc, 0)
   R Pigen = Z;
   if (wcold) {
+    only();
     const R Qi0 = C.ice_nuc * mth.exp(R(1.33) * (C.ln1000 + maxz(R(-0.1) * temc))) * Rdens;
     Pigen = maxz(dmin(Qi0 - qi, qv - qsati)) * rdtR;
   }
@@ -428,6 +480,7 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
   // gamma_sacr == gamma_saut (both 6e-2 in this configuration).
   R Esi_mod = C.Esi, betai = C.beta_saut;
   if (hi && !(warm && is_nonneg(C.Esi) && is_nonneg(C.beta_saut))) {
+    only();
     const R eg = mth.exp(C.gamma_sacr * temc);
     const R eb = (C.gamma_saut == C.gamma_sacr) ? eg : mth.exp(C.gamma_saut * temc);
     Esi_mod = dmin(C.Esi, C.Esi * eg);
@@ -437,6 +490,7 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
   const R fr = rho_fact;
   R Pracw = Z, Psacw = Z, Pgacw = Z, Praci = Z, Psaci = Z, Piacr = Z, Psacr = Z, Pgacr = Z, Pracs = Z;
   if (hc && hr) {
+    only();
     const R qcqr = qc * qr;
     if (kk) {
       if (ge_c(qcqr, R(1.0E-12))) Pracw = R(67.0) * mth.pow(qcqr, R(1.15));
@@ -444,33 +498,59 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
       Pracw = qc * C.K_raci * RLMDr_3dr * fr;   // Pracw_orig (Erw = Eri = 1)
     }
   }
-  if (hc && hs) Psacw = qc * C.K_sacw * MOMs_2ds * fr;
-  if (hc && hg) Pgacw = qc * C.K_gacw * RLMDg_3dg * fr;
+  if (hc && hs) {
+    only();
+    Psacw = qc * C.K_sacw * MOMs_2ds * fr;
+  }
+  if (hc && hg) {
+    only();
+    Pgacw = qc * C.K_gacw * RLMDg_3dg * fr;
+  }
   if (hi && hr) {
+    only();
     Praci = qi * C.K_raci * RLMDr_3dr * fr;
     Piacr = qi * C.K_iacr * RLMDr_6dr * fr;
   }
-  if (hi && hs) Psaci = qi * C.K_saci * Esi_mod * MOMs_2ds * fr;
+  if (hi && hs) {
+    only();
+    Psaci = qi * C.K_saci * Esi_mod * MOMs_2ds * fr;
+  }
   if (hr && hs) {
+    only();
     const R dvrs = fabsR(Vtr - Vts);
     Psacr = C.K_sacr * Rdens * dvrs *
             (C.GAM_1br * RLMDr_1br * MOMs_2 + C.K_2gam2br * RLMDr_2br * MOMs_1 + C.GAM_3br * RLMDr_3br * MOMs_0);
     Pracs = C.K_racs * Rdens * dvrs * (R(2.0) * MOMs_0bs * RLMDr_3 + R(2.0) * MOMs_1bs * RLMDr_2 + MOMs_2bs * RLMDr);
   }
-  if (hr && hg)
+  if (hr && hg) {
+    only();
     Pgacr = C.K_gacr * Rdens * fabsR(Vtg - Vtr) *
             (C.K_g13 * RLMDr_1br * RLMDg_3 + C.K_g22 * RLMDr_2br * RLMDg_2 + C.GAM_3br * RLMDr_3br * RLMDg);
+  }
   R Pgaci = Z, Pgacs = Z;   // Egi = Egs = 0 unless OPT
   if constexpr (OPT) {
-    if (hi && hg) Pgaci = qi * C.K_gaci * RLMDg_3dg * fr;
+    if (hi && hg) {
+      only();
+      Pgaci = qi * C.K_gaci * RLMDg_3dg * fr;
+    }
     R Egs_mod = C.Egs;
-    if (hs && hg && !(warm && C.Egs >= Z)) Egs_mod = dmin(C.Egs, C.Egs * mth.exp(C.gamma_gacs * temc));
-    if (hs && hg) Pgacs = C.K_gacs * Rdens * Egs_mod * fabsR(Vtg - Vts) *
+    if (hs && hg && !(warm && C.Egs >= Z)) {
+      only();
+      Egs_mod = dmin(C.Egs, C.Egs * mth.exp(C.gamma_gacs * temc));
+    }
+    if (hs && hg) {
+      only();
+      Pgacs = C.K_gacs * Rdens * Egs_mod * fabsR(Vtg - Vts) *
             (R(2.0) * MOMs_0bs * RLMDg_3 + R(2.0) * MOMs_1bs * RLMDg_2 + MOMs_2bs * RLMDg);
+    }
   }
 
   // autoconversion, :1147-1172 (KK2000; only the second Praut_kk assignment is live)
-  const R rhoqc = hc ? densR * qc * R(1000.0) : Z;
+  R rhoqc = Z;
+  if (hc) {
+    only();
+    rhoqc = densR * qc * R(1000.0);
+  }
   R Praut = Z;   // K_aut * pow(0, 2.47) = 0
   if (kk) {
     R K_aut = C.K_aut;
@@ -479,6 +559,7 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
     }
     if (gt_z(qc)) Praut = K_aut * mth.pow(qc, R(2.47));
   } else if (hc) {
+    only();
     // Berry (1968), :1145-1147
     R Dc = C.Dc_berry;
     if constexpr (OPT) {
@@ -487,24 +568,39 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
     Praut = quo(Rdens * R(1.67E-5) * rhoqc * rhoqc, R(5.0) + quo(R(3.66E-2) * Nc, Dc * rhoqc + R(EPS)));
   }
   R Psaut = Z;   // (without ice the limiter dqi_dt = 0 below would hold it there)
-  if (hi) Psaut = rate_on(betai * (qi - C.qicrt_saut));
+  if (hi) {
+    only();
+    Psaut = rate_on(betai * (qi - C.qicrt_saut));
+  }
 
   // evaporation, sublimation, melting and freezing, :1174-1247
   const bool falls = hr || hs || hg;
   R Ka = Z, KdD = Z, rKaT = Z, Giv = Z, Gil = Z, rNu = Z;
-  if (falls || wcold) Ka = R(2.428E-2) + R(7.47E-5) * temc;
+  if (falls || wcold) {
+    only();
+    Ka = R(2.428E-2) + R(7.47E-5) * temc;
+  }
   if (hr || wcold) {
+    only();
     KdD = quo((R(2.222E-5) + R(1.37E-7) * temc) * R(PSTD), pre) * densR;   // Kd * dens
     rKaT = quo(ONE, Ka * tempR);
   }
-  if (falls) rNu = quo(densR, R(1.718E-5) + R(5.28E-8) * temc);               // 1 / Nu
+  if (falls) {
+    only();
+    rNu = quo(densR, R(1.718E-5) + R(5.28E-8) * temc);   // 1 / Nu
+  }
   if (wcold) {
+    only();
     const R xi = KdD * qsati;
     Giv = quo(xi, R(LHS0) * rKaT * (C.LovR_ice * rtem - ONE) * xi + ONE);
   }
-  if ((hs || hg) && wwarm) Gil = Ka * temc * C.rLHF0;
+  if ((hs || hg) && wwarm) {
+    only();
+    Gil = Ka * temc * C.rLHF0;
+  }
   R Prevp = Z;
   if (rain) {
+    only();
     const R xl = KdD * qsatl;
     const R Glv = quo(xl, R(LHV0) * rKaT * (C.LovR_liq * rtem - ONE) * xl + ONE);
     const R ventr = C.K_ventr1 * RLMDr_2 + C.K_ventr2 * sqrtR(C.Cr * fr * rNu * RLMDr_5dr);
@@ -513,7 +609,12 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
   // deposition and sublimation of ice (cold cells: the limiters keep it there)
   R tmp, Pidep = Z, Pisub = Z;
   if (wcold) {
-    const R rhoqi = hi ? maxc(densR * qi, R(EPS)) : R(EPS);
+    only();
+    R rhoqi = R(EPS);
+    if (hi) {
+      only();
+      rhoqi = maxc(densR * qi, R(EPS));
+    }
     // with no ice, rhoqi = EPS and XNi, Di take the constant values folded on the host
     R XNi = C.XNi_eps, Di = C.Di_eps;
     if (gt_c(rhoqi, R(EPS))) {
@@ -528,32 +629,53 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
   const bool below40 = lt_z(temc + R(40.0));
   R Pihom = below40 ? dqc_dt : Z;
   R efrz = Z;
-  if ((hc || hr) && wcold) efrz = mth.exp(-C.A_frz * temc) - ONE;
+  if ((hc || hr) && wcold) {
+    only();
+    efrz = mth.exp(-C.A_frz * temc) - ONE;
+  }
   R Pihtr = Z;
-  if (hc && !below40 && !warm) Pihtr = densR * (qc * qc) * C.K_ihtr * efrz;
+  if (hc && !below40 && !warm) {
+    only();
+    Pihtr = densR * (qc * qc) * C.K_ihtr * efrz;
+  }
   R Pimlt = warm ? dqi_dt : Z;
   // ventilation of snow and graupel: without the species their moments /
   // slope terms are exact zeros and so is the sum (+0, skipped with its root)
   R vents = Z, ventg = Z;
-  if (hs && !(is_zero(MOMs_1) && is_zero(MOMs_5ds_h)))
+  if (hs && !(is_zero(MOMs_1) && is_zero(MOMs_5ds_h))) {
+    only();
     vents = R(0.65) * MOMs_1 + C.K_vents2 * sqrtR(fr * rNu) * MOMs_5ds_h;
+  }
   R Psdep = Z, Pssub = Z, Psmlt = Z;
   if (hs && wcold) {
+    only();
     tmp = C.K_2pi * Rdens * (Sice - ONE) * Giv * vents;
     Psdep = sel(sps, tmp);
     Pssub = sel(!sps, -tmp);
   }
-  if (hs && wwarm) Psmlt = maxz(C.K_2pi * Rdens * Gil * vents + C.K_clf * temc * (Psacw + Psacr));
-  if (hg && !(is_zero(RLMDg_2) && is_zero(RLMDg_5dg)))
+  if (hs && wwarm) {
+    only();
+    Psmlt = maxz(C.K_2pi * Rdens * Gil * vents + C.K_clf * temc * (Psacw + Psacr));
+  }
+  if (hg && !(is_zero(RLMDg_2) && is_zero(RLMDg_5dg))) {
+    only();
     ventg = C.K_ventg1 * RLMDg_2 + C.K_ventg2 * sqrtR(C.Cg * fr * rNu * RLMDg_5dg);
+  }
   R Pgdep = Z, Pgsub = Z, Pgmlt = Z, Pgfrz = Z;
   if (hg && wcold) {
+    only();
     tmp = C.K_gdep * Rdens * (Sice - ONE) * Giv * ventg;
     Pgdep = sel(sps, tmp);
     Pgsub = sel(!sps, -tmp);
   }
-  if (hg && wwarm) Pgmlt = maxz(C.K_gdep * Rdens * Gil * ventg + C.K_clf * temc * (Pgacw + Pgacr));
-  if (hr && wcold) Pgfrz = C.K_gfrz * Rdens * efrz * RLMDr_7;
+  if (hg && wwarm) {
+    only();
+    Pgmlt = maxz(C.K_gdep * Rdens * Gil * ventg + C.K_clf * temc * (Pgacw + Pgacr));
+  }
+  if (hr && wcold) {
+    only();
+    Pgfrz = C.K_gfrz * Rdens * efrz * RLMDr_7;
+  }
 
   // Bergeron process (:1239-1247) with Bergeron_param (:1834-1890); it
   // contributes only when sw_bergeron = 1 (-30 <= temc <= 0, sw_expice = 0)
@@ -562,6 +684,7 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
   R Psfw = Z, Psfi = Z;
   if constexpr (OPT) {
     if (hi && !expice && cold && !(temc + R(30.0) < Z)) {
+      only();
       const R tb = dmin(dmax(temc, R(-30.99)), Z);
       const int it = int(-val_of(tb));   // the table row: piecewise constant in tb
       const R fact = -(tb + R(it - 1));
@@ -576,50 +699,71 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
   }
 
   // limiters, :1249-1296 (iceflg selects; sw_expice = 1 unless OPT; Pgaut = 0)
-  Pigen = sel(cold && expice, min_nn(Pigen, dqv_dt));
-  Pidep = sel(cold && expice, min_nn(Pidep, dqv_dt));
-  Psdep = sel(cold, min_nn(Psdep, dqv_dt));
-  Pgdep = sel(cold, min_nn(Pgdep, dqv_dt));
-  if (hc && wwarm) Pracw = Pracw + sel(warm, Psacw) + sel(warm, Pgacw);
-  Praut = min_nn(Praut, dqc_dt);
-  Pracw = min_nn(Pracw, dqc_dt);
-  Pihom = sel(cold && expice, min_nn(Pihom, dqc_dt));
-  Pihtr = sel(cold && expice, min_nn(Pihtr, dqc_dt));
-  Psacw = sel(cold, min_nn(Psacw, dqc_dt));
-  if constexpr (OPT) Psfw = sel(cold, min_nn(Psfw, dqc_dt));
-  Pgacw = sel(cold, min_nn(Pgacw, dqc_dt));
-  Prevp = min_nn(Prevp, dqr_dt);
-  Piacr = sel(cold, min_nn(Piacr, dqr_dt));
-  Psacr = sel(cold, min_nn(Psacr, dqr_dt));
-  Pgacr = sel(cold, min_nn(Pgacr, dqr_dt));
-  Pgfrz = sel(cold, min_nn(Pgfrz, dqr_dt));
-  Pisub = sel(cold && expice, min_nn(Pisub, dqi_dt));
-  Pimlt = sel(warm && expice, min_nn(Pimlt, dqi_dt));
-  Psaut = sel(cold, min_nn(Psaut, dqi_dt));
-  Praci = sel(cold, min_nn(Praci, dqi_dt));
-  Psaci = sel(cold, min_nn(Psaci, dqi_dt));
-  if constexpr (OPT) {
-    Psfi = sel(cold, min_nn(Psfi, dqi_dt));
-    Pgaci = sel(cold, min_nn(Pgaci, dqi_dt));
+  R Piacr_s = Z, Piacr_g = Z, Praci_s = Z, Praci_g = Z, Psacr_s = Z, Psacr_g = Z;
+  if (wcold) {
+    only();
+    Pigen = sel(cold && expice, min_nn(Pigen, dqv_dt));
+    Pidep = sel(cold && expice, min_nn(Pidep, dqv_dt));
+    Pisub = sel(cold && expice, min_nn(Pisub, dqi_dt));
   }
-  Pssub = sel(cold, min_nn(Pssub, dqs_dt));
-  Psmlt = sel(warm, min_nn(Psmlt, dqs_dt));
-  Pracs = sel(cold, min_nn(Pracs, dqs_dt));
-  if constexpr (OPT) Pgacs = min_nn(Pgacs, dqs_dt);
-  Pgsub = sel(cold, min_nn(Pgsub, dqg_dt));
-  Pgmlt = sel(warm, min_nn(Pgmlt, dqg_dt));
-  R Piacr_s = sel(!d1, Piacr);
-  R Piacr_g = sel(d1, Piacr);
-  R Praci_s = sel(!d1, Praci);
-  R Praci_g = sel(d1, Praci);
-  R Psacr_s = sel(d2, Psacr);
-  R Psacr_g = sel(!d2, Psacr);
-  Pracs = sel(!d2, Pracs);
+  if (hc) {
+    only();
+    if (wwarm) Pracw = Pracw + sel(warm, Psacw) + sel(warm, Pgacw);
+    Praut = min_nn(Praut, dqc_dt);
+    Pracw = min_nn(Pracw, dqc_dt);
+    Pihom = sel(cold && expice, min_nn(Pihom, dqc_dt));
+    Pihtr = sel(cold && expice, min_nn(Pihtr, dqc_dt));
+    Psacw = sel(cold, min_nn(Psacw, dqc_dt));
+    Pgacw = sel(cold, min_nn(Pgacw, dqc_dt));
+  }
+  if constexpr (OPT) Psfw = sel(cold, min_nn(Psfw, dqc_dt));
+  if (hr) {
+    only();
+    Prevp = min_nn(Prevp, dqr_dt);
+    Piacr = sel(cold, min_nn(Piacr, dqr_dt));
+    Psacr = sel(cold, min_nn(Psacr, dqr_dt));
+    Pgacr = sel(cold, min_nn(Pgacr, dqr_dt));
+    Pgfrz = sel(cold, min_nn(Pgfrz, dqr_dt));
+  }
+  if (hi) {
+    only();
+    Pimlt = sel(warm && expice, min_nn(Pimlt, dqi_dt));
+    Psaut = sel(cold, min_nn(Psaut, dqi_dt));
+    Praci = sel(cold, min_nn(Praci, dqi_dt));
+    Psaci = sel(cold, min_nn(Psaci, dqi_dt));
+    if constexpr (OPT) {
+      Psfi = sel(cold, min_nn(Psfi, dqi_dt));
+      Pgaci = sel(cold, min_nn(Pgaci, dqi_dt));
+    }
+    Piacr_s = sel(!d1, Piacr);
+    Piacr_g = sel(d1, Piacr);
+    Praci_s = sel(!d1, Praci);
+    Praci_g = sel(d1, Praci);
+  }
+  if (hs) {
+    only();
+    Pssub = sel(cold, min_nn(Pssub, dqs_dt));
+    Psdep = sel(cold, min_nn(Psdep, dqv_dt));
+    Psmlt = sel(warm, min_nn(Psmlt, dqs_dt));
+    Pracs = sel(cold, min_nn(Pracs, dqs_dt));
+    if constexpr (OPT) Pgacs = min_nn(Pgacs, dqs_dt);
+    Psacr_s = sel(d2, Psacr);
+    Psacr_g = sel(!d2, Psacr);
+    Pracs = sel(!d2, Pracs);
+  }
+  if (hg) {
+    only();
+    Pgsub = sel(cold, min_nn(Pgsub, dqg_dt));
+    Pgdep = sel(cold, min_nn(Pgdep, dqv_dt));
+    Pgmlt = sel(warm, min_nn(Pgmlt, dqg_dt));
+  }
 
   // loss limiters, :1298-1477: fac = 1 when production >= loss - EPS,
   // else min(-dq/dt / net, 1) (the reference's (net - fac_sw) is net there)
   auto limiter = [&](R net, R dq) {
-    return is_nonneg(net + R(EPS)) ? ONE : dmin(quo(-dq, net), ONE);
+    if (kPlain && is_nonneg(net)) return ONE;
+    only();
+    return is_nonneg(net + R(EPS)) ? ONE : minc(quo(-dq, net), ONE);
   };
   // Scaling by fac = 1 is exact and skipped.  The tendencies below are the
   // nets the limiters form (same terms, same order) where no later scaling
@@ -636,29 +780,40 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
   R fac;
   R net_c = +Pimlt;  // [QC]
   if (bc) {
+    only();
     net_c = net_c - Praut - Pracw - Pihom - Pihtr - Psacw;
     if constexpr (OPT) net_c = net_c - Psfw;
     net_c = net_c - Pgacw;
     fac = limiter(net_c, dqc_dt);
     lc = !is_one(fac);
     if (lc) {
+      only();
       Pimlt *= fac; Praut *= fac; Pracw *= fac; Pihom *= fac; Pihtr *= fac; Psacw *= fac; Pgacw *= fac;
       if constexpr (OPT) Psfw *= fac;
     }
   }
   R net_i = Z;  // [QI]
-  if (wcold) net_i = +Pigen + Pidep;
-  if (hc && wcold) net_i = net_i + Pihom + Pihtr;
+  if (wcold) {
+    only();
+    net_i = +Pigen + Pidep;
+  }
+  if (hc && wcold) {
+    only();
+    net_i = net_i + Pihom + Pihtr;
+  }
   if (bi) {
+    only();
     net_i = net_i - Pisub - Pimlt - Psaut - Praci_s - Psaci;
     if constexpr (OPT) net_i = net_i - Psfi;
     net_i = net_i - Praci_g;
     if constexpr (OPT) net_i = net_i - Pgaci;
   }
   if (bi || lt_z(net_i)) {
+    only();
     fac = limiter(net_i, dqi_dt);
     li = !is_one(fac);
     if (li) {
+      only();
       Pigen *= fac; Pidep *= fac; Pihom *= fac; Pihtr *= fac; Pisub *= fac; Pimlt *= fac; Psaut *= fac;
       Praci_s *= fac; Psaci *= fac; Praci_g *= fac;
       if constexpr (OPT) {
@@ -668,52 +823,100 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
     }
   }
   R net_r = Z;  // [QR]
-  if (hc) net_r = +Praut + Pracw;
-  if (hs && wwarm) net_r = net_r + Psmlt;
-  if (hg && wwarm) net_r = net_r + Pgmlt;
+  if (hc) {
+    only();
+    net_r = +Praut + Pracw;
+  }
+  if (hs && wwarm) {
+    only();
+    net_r = net_r + Psmlt;
+  }
+  if (hg && wwarm) {
+    only();
+    net_r = net_r + Pgmlt;
+  }
   if (hr) {
+    only();
     net_r = net_r - Prevp - Piacr_s - Psacr_s - Piacr_g - Psacr_g - Pgacr - Pgfrz;
   }
   if (hr || lt_z(net_r)) {
+    only();
     fac = limiter(net_r, dqr_dt);
     lr = !is_one(fac);
     if (lr) {
+      only();
       Praut *= fac; Pracw *= fac; Psmlt *= fac; Pgmlt *= fac; Prevp *= fac; Piacr_s *= fac; Psacr_s *= fac;
       Piacr_g *= fac; Psacr_g *= fac; Pgacr *= fac; Pgfrz *= fac;
     }
   }
   R net_v = Z;  // [QV]
-  if (hr) net_v = +Prevp;
-  if (bi) net_v = net_v + Pisub;
-  if (hs) net_v = net_v + Pssub;
-  if (hg) net_v = net_v + Pgsub;
-  if (wcold) net_v = net_v - Pigen - Pidep;
-  if (hs && wcold) net_v = net_v - Psdep;
-  if (hg && wcold) net_v = net_v - Pgdep;
+  if (hr) {
+    only();
+    net_v = +Prevp;
+  }
+  if (bi) {
+    only();
+    net_v = net_v + Pisub;
+  }
+  if (hs) {
+    only();
+    net_v = net_v + Pssub;
+  }
+  if (hg) {
+    only();
+    net_v = net_v + Pgsub;
+  }
+  if (wcold) {
+    only();
+    net_v = net_v - Pigen - Pidep;
+  }
+  if (hs && wcold) {
+    only();
+    net_v = net_v - Psdep;
+  }
+  if (hg && wcold) {
+    only();
+    net_v = net_v - Pgdep;
+  }
   if (hr || wcold || lt_z(net_v)) {
+    only();
     fac = limiter(net_v, dqv_dt);
     lv = !is_one(fac);
     if (lv) {
+      only();
       Prevp *= fac; Pisub *= fac; Pssub *= fac; Pgsub *= fac; Pigen *= fac; Pidep *= fac; Psdep *= fac; Pgdep *= fac;
     }
   }
   R net_s = Z;  // [QS]
-  if (hs) net_s = +Psdep + Psacw;
+  if (hs) {
+    only();
+    net_s = +Psdep + Psacw;
+  }
   if constexpr (OPT) net_s = net_s + Psfw;
-  if (hr && hi) net_s = net_s + Piacr_s;
-  if (hr && hs) net_s = net_s + Psacr_s;
+  if (hr && hi) {
+    only();
+    net_s = net_s + Piacr_s;
+  }
+  if (hr && hs) {
+    only();
+    net_s = net_s + Psacr_s;
+  }
   if (hi) {
+    only();
     net_s = net_s + Psaut + Praci_s + Psaci;
     if constexpr (OPT) net_s = net_s + Psfi;
   }
   if (hs) {
+    only();
     net_s = net_s - Pssub - Psmlt - Pracs;
     if constexpr (OPT) net_s = net_s - Pgacs;
   }
   if (hs || lt_z(net_s)) {
+    only();
     fac = limiter(net_s, dqs_dt);
     ls = !is_one(fac);
     if (ls) {
+      only();
       Psdep *= fac; Psacw *= fac; Piacr_s *= fac; Psacr_s *= fac; Psaut *= fac; Praci_s *= fac; Psaci *= fac;
       Pssub *= fac; Psmlt *= fac; Pracs *= fac;
       if constexpr (OPT) {
@@ -724,21 +927,42 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
     }
   }
   R net_g = Z;  // [QG]
-  if (hg) net_g = +Pgdep + Pgacw;
-  if (hr && hi) net_g = net_g + Piacr_g;
-  if (hr && hs) net_g = net_g + Psacr_g;
-  if (hr) net_g = net_g + Pgacr + Pgfrz;
-  if (hr && hi) net_g = net_g + Praci_g;
+  if (hg) {
+    only();
+    net_g = +Pgdep + Pgacw;
+  }
+  if (hr && hi) {
+    only();
+    net_g = net_g + Piacr_g;
+  }
+  if (hr && hs) {
+    only();
+    net_g = net_g + Psacr_g;
+  }
+  if (hr) {
+    only();
+    net_g = net_g + Pgacr + Pgfrz;
+  }
+  if (hr && hi) {
+    only();
+    net_g = net_g + Praci_g;
+  }
   if constexpr (OPT) net_g = net_g + Pgaci;
-  if (hr && hs) net_g = net_g + Pracs;
+  if (hr && hs) {
+    only();
+    net_g = net_g + Pracs;
+  }
   if constexpr (OPT) net_g = net_g + Pgacs;
   if (hg) {
+    only();
     net_g = net_g - Pgsub - Pgmlt;
   }
   if (hg || lt_z(net_g)) {
+    only();
     fac = limiter(net_g, dqg_dt);
     lg = !is_one(fac);
     if (lg) {
+      only();
       Pgdep *= fac; Pgacw *= fac; Piacr_g *= fac; Psacr_g *= fac; Pgacr *= fac; Pgfrz *= fac; Praci_g *= fac;
       Pracs *= fac; Pgsub *= fac; Pgmlt *= fac;
       if constexpr (OPT) {
@@ -752,19 +976,44 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
   // or after it scaled one of its rates: QC's by QC, QI, QR, QS, QG; QI's by
   // QI, QV, QS, QG; QR's by QR, QV, QS, QG; QS's by QS, QG; QG's by QG.
   R qc_t = net_c, qr_t = net_r, qi_t = net_i, qs_t = net_s, qg_t = net_g;
-  if (lr | lv | ls | lg) qr_t = +Praut + Pracw + Psmlt + Pgmlt - Prevp - Piacr_s - Psacr_s - Piacr_g - Psacr_g - Pgacr - Pgfrz;
+  if (lr | lv | ls | lg) {
+    only();
+    qr_t = +Praut + Pracw + Psmlt + Pgmlt - Prevp - Piacr_s - Psacr_s - Piacr_g - Psacr_g - Pgacr - Pgfrz;
+  }
   if constexpr (!OPT) {
-    if (lc | li | lr | ls | lg) qc_t = +Pimlt - Praut - Pracw - Pihom - Pihtr - Psacw - Pgacw;
-    if (li | lv | ls | lg) qi_t = +Pigen + Pidep + Pihom + Pihtr - Pisub - Pimlt - Psaut - Praci_s - Psaci - Praci_g;
-    if (ls | lg) qs_t = +Psdep + Psacw + Piacr_s + Psacr_s + Psaut + Praci_s + Psaci - Pssub - Psmlt - Pracs;
-    if (lg) qg_t = +Pgdep + Pgacw + Piacr_g + Psacr_g + Pgacr + Pgfrz + Praci_g + Pracs - Pgsub - Pgmlt;
+    if (lc | li | lr | ls | lg) {
+      only();
+      qc_t = +Pimlt - Praut - Pracw - Pihom - Pihtr - Psacw - Pgacw;
+    }
+    if (li | lv | ls | lg) {
+      only();
+      qi_t = +Pigen + Pidep + Pihom + Pihtr - Pisub - Pimlt - Psaut - Praci_s - Psaci - Praci_g;
+    }
+    if (ls | lg) {
+      only();
+      qs_t = +Psdep + Psacw + Piacr_s + Psacr_s + Psaut + Praci_s + Psaci - Pssub - Psmlt - Pracs;
+    }
+    if (lg) {
+      only();
+      qg_t = +Pgdep + Pgacw + Piacr_g + Psacr_g + Pgacr + Pgfrz + Praci_g + Pracs - Pgsub - Pgmlt;
+    }
   } else {
-    if (lc | li | lr | ls | lg) qc_t = +Pimlt - Praut - Pracw - Pihom - Pihtr - Psacw - Psfw - Pgacw;
-    if (li | lv | ls | lg)
+    if (lc | li | lr | ls | lg) {
+      only();
+      qc_t = +Pimlt - Praut - Pracw - Pihom - Pihtr - Psacw - Psfw - Pgacw;
+    }
+    if (li | lv | ls | lg) {
+      only();
       qi_t = +Pigen + Pidep + Pihom + Pihtr - Pisub - Pimlt - Psaut - Praci_s - Psaci - Psfi - Praci_g - Pgaci;
-    if (ls | lg)
+    }
+    if (ls | lg) {
+      only();
       qs_t = +Psdep + Psacw + Psfw + Piacr_s + Psacr_s + Psaut + Praci_s + Psaci + Psfi - Pssub - Psmlt - Pracs - Pgacs;
-    if (lg) qg_t = +Pgdep + Pgacw + Piacr_g + Psacr_g + Pgacr + Pgfrz + Praci_g + Pgaci + Pracs + Pgacs - Pgsub - Pgmlt;
+    }
+    if (lg) {
+      only();
+      qg_t = +Pgdep + Pgacw + Piacr_g + Psacr_g + Pgacr + Pgfrz + Praci_g + Pgaci + Pracs + Pgacs - Pgsub - Pgmlt;
+    }
   }
   qc_t = max_nd(qc_t, dqc_dt);
   qr_t = max_nd(qr_t, dqr_dt);
@@ -772,10 +1021,22 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
   qs_t = max_nd(qs_t, dqs_dt);
   qg_t = max_nd(qg_t, dqg_dt);
   R q_t = qc_t;
-  if (nz(qr_t)) q_t = q_t + qr_t;
-  if (nz(qi_t)) q_t = q_t + qi_t;
-  if (nz(qs_t)) q_t = q_t + qs_t;
-  if (nz(qg_t)) q_t = q_t + qg_t;
+  if (nz(qr_t)) {
+    only();
+    q_t = q_t + qr_t;
+  }
+  if (nz(qi_t)) {
+    only();
+    q_t = q_t + qi_t;
+  }
+  if (nz(qs_t)) {
+    only();
+    q_t = q_t + qs_t;
+  }
+  if (nz(qg_t)) {
+    only();
+    q_t = q_t + qg_t;
+  }
   const R qv_t = -q_t;
   D drq[6];
   if constexpr (kMixed) {
@@ -800,7 +1061,10 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
 #pragma unroll
     for (int n = 0; n < 6; ++n) {
       drq[n] = D(qt[n]);
-      if (nz(qt[n])) drq[n] = rhog * D(qt[n]) * dt;
+      if (nz(qt[n])) {
+        only();
+        drq[n] = rhog * D(qt[n]) * dt;
+      }
     }
   }
   o.Vtr = D(Vtr);
@@ -811,6 +1075,7 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
   // effective radius and cloud top, :1566-1592 (without cloud water and rain
   // the radii are 0 and there is no top, on both sides of r2_min)
   if (!(hc || hr)) {
+    only();
     o.rceff = D(0.0);
     o.rceff_cld = D(0.0);
     o.rctop = D(UNDEF);
@@ -842,11 +1107,26 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
   // ---- TagUpdateRHOGQ / RHOGE / MassConc / TEM, mod_mp_nsw6.cpp:692-744
 #pragma unroll
   for (int n = 0; n < 6; ++n)
-    if (nz(drq[n])) rq[n] += drq[n];
-  if (nz(drq[I_QV])) rhoge = rhoge - LHV0 * drq[I_QV];
-  if (nz(drq[I_QI])) rhoge = rhoge + LHF0 * drq[I_QI];
-  if (nz(drq[I_QS])) rhoge = rhoge + LHF0 * drq[I_QS];
-  if (nz(drq[I_QG])) rhoge = rhoge + LHF0 * drq[I_QG];
+    if (nz(drq[n])) {
+      only();
+      rq[n] += drq[n];
+    }
+  if (nz(drq[I_QV])) {
+    only();
+    rhoge = rhoge - LHV0 * drq[I_QV];
+  }
+  if (nz(drq[I_QI])) {
+    only();
+    rhoge = rhoge + LHF0 * drq[I_QI];
+  }
+  if (nz(drq[I_QS])) {
+    only();
+    rhoge = rhoge + LHF0 * drq[I_QS];
+  }
+  if (nz(drq[I_QG])) {
+    only();
+    rhoge = rhoge + LHF0 * drq[I_QG];
+  }
   o.q[0] = qn[0];
   if constexpr (kMixed) {
     // q from the shared reciprocal, T = rhoge / (rhog CVdry) (cv = CVdry as above)
@@ -859,11 +1139,17 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
     D qd2 = D(1.0);
 #pragma unroll
     for (int n = 1; n <= 5; ++n)
-      if (nz(o.q[n])) qd2 = qd2 - o.q[n];
+      if (nz(o.q[n])) {
+        only();
+        qd2 = qd2 - o.q[n];
+      }
     D cva = qd2 * CVDRY;
 #pragma unroll
     for (int n = 1; n <= 5; ++n)
-      if (nz(o.q[n])) cva = cva + o.q[n] * CVDRY;
+      if (nz(o.q[n])) {
+        only();
+        cva = cva + o.q[n] * CVDRY;
+      }
     o.tem = quo(rhoge, rhog * cva);
   }
   o.rhog = rhog;

@@ -87,9 +87,10 @@ __device__ __forceinline__ int bucket_add(int* bucket, int v) {
 // larger groups than one of 32 columns by all levels (the layout before, with
 // the departure distances in the same kernel).  The order only decides which
 // thread computes which cell.  One 16900 x 42 region, FP64, with the departure
-// kernel: 0.90 -> 0.67 ms (10.1 M -> 9.6 M FP64 warp instructions, of which this
-// kernel 7.1 M: its FP64 pipe is 75 % busy); 48 columns, which had two CTAs
-// here, 0.47 -> 0.29 ms for the whole step.
+// kernel: 0.90 -> 0.67 ms; 48 columns, which had two CTAs here, 0.47 -> 0.29 ms
+// for the whole step.  What is left out is branched around since: this kernel
+// then took 0.45 -> 0.34 ms (6.1 M -> 3.7 M FP64 warp instructions; its FP64
+// pipe is 60 % busy, next to it come waits for instructions).
 //
 // OPT: the kernel with the scheme switches: the switched branches of nsw6_cell
 // and the CCN input.
@@ -156,7 +157,13 @@ __global__ void __launch_bounds__(CELL_THREADS, 2) nsw6_cell_kernel(Problem P, C
   }
   const M mth = make_math<M>(stab);
 #pragma unroll 1
-  for (int j = threadIdx.x; j < n; j += blockDim.x) {
+  for (int j0 = 0; j0 < n; j0 += blockDim.x) {
+    // FP64: the CTA's warps go through neighbouring groups together, so that
+    // they run the same parts of the code (its 120 KB do not fit the
+    // instruction caches)
+    if (!kMixed) __syncthreads();
+    const int j = j0 + threadIdx.x;
+    if (j >= n) continue;
     const int c = kMixed ? j : perm[j];
     const size_t i = off + c;
     const size_t iq = offq + c;

@@ -115,6 +115,9 @@ NSW6_FP_HD float soft_rsqrt_seed(float x) {
 #endif
 }
 
+// An empty call: the block it stands in is branched around, not predicated.
+NSW6_SLOW void soft_branch() { asm volatile(""); }
+
 constexpr u64 SOFT_MANT = 0x000FFFFFFFFFFFFFull;
 constexpr u64 SOFT_ONE = 0x0010000000000000ull;
 
