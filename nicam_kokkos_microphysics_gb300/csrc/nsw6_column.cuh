@@ -108,8 +108,8 @@ __device__ __forceinline__ R flux_rest(const R* dz, int k, int kc, R zdis0, int 
 }
 // |f| >= EPS on the integer pipe (NaN fails, as the comparison does)
 __device__ __forceinline__ double flux_filter(double f) {
-  const long long ab = __double_as_longlong(f) & 0x7fffffffffffffffLL;
-  return (ab >= EPS_BITS && ab <= 0x7ff0000000000000LL) ? f : 0.0;
+  const unsigned long long ab = (unsigned long long)__double_as_longlong(f) & 0x7fffffffffffffffull;
+  return ab - (unsigned long long)EPS_BITS <= 0x7ff0000000000000ull - (unsigned long long)EPS_BITS ? f : 0.0;
 }
 __device__ __forceinline__ float flux_filter(float f) { return fabsf(f) >= (float)EPS ? f : 0.0f; }
 // n sources src[m] (columns of the tile) into f[m]
@@ -323,6 +323,7 @@ __device__ __forceinline__ bool final_cell(const Problem& P, const Consts& C, co
   rq[I_QC] = rhog * q[I_QC];
   if (ice_adj) rq[I_QI] = rhog * q[I_QI];
   if (!interior) {   // interior levels: rhoge comes from the negative filter below
+    soft_branch();
     cvtot = qd * CVDRY;
 #pragma unroll
     for (int n = 1; n <= 5; ++n) cvtot = cvtot + q[n] * CVDRY;
@@ -574,7 +575,6 @@ __global__ void __launch_bounds__(COL_THREADS_MAX, 2) nsw6_column_kernel(Problem
     r_rgs[j] = r_rgsh[j] = r_c2w0[j] = r_c2w1[j] = 0.0;
     r_rgshf[j] = r_c2w0f[j] = r_c2w1f[j] = 0.0f;
     if (c >= ncell) continue;
-    const int k = c / COL_TG, gx = c % COL_TG, g = g0 + gx;
     for (int s = S_KINH; s <= S_DQG; ++s) F(s)[c] = 0.0;   // (a slot's two FP32 halves are zero as well)
     if (OPT) F(S_DQI)[c] = 0.0;
     F(S_VI)[c] = 0.0;
@@ -694,7 +694,10 @@ __global__ void __launch_bounds__(COL_THREADS_MAX, 2) nsw6_column_kernel(Problem
       if (own) {
         const size_t i = (size_t)k * G + g;
         const double b0 = rhogq_n[i];
-        if (!fp_is_zero(b0)) bq[j] = b0 * r_rgs[j];
+        if (!fp_is_zero(b0)) {
+          soft_branch();
+          bq[j] = b0 * r_rgs[j];
+        }
         if (k >= kmin && k <= kmax) {
           const double z = zdis0[i];
           kc[j] = departure_cell(gzh, zkey, k, z, bmn_f[k], bmx_f[k], kmin, kmax);
@@ -705,8 +708,13 @@ __global__ void __launch_bounds__(COL_THREADS_MAX, 2) nsw6_column_kernel(Problem
       const double b = bq[j];
       const bool holds = own && !fp_is_zero(b);
       if (c < ncell) {
+        double e = 0.0;
+        if (holds) {
+          soft_branch();
+          e = b * CVDRY * P.tem[off + (size_t)k * G + g];
+        }
         F(S_RHOF)[c] = b;
-        F(S_RHOF2)[c] = holds ? b * CVDRY * P.tem[off + (size_t)k * G + g] : 0.0;
+        F(S_RHOF2)[c] = e;
       }
       note(held[t], c, holds);
     }
@@ -723,6 +731,7 @@ __global__ void __launch_bounds__(COL_THREADS_MAX, 2) nsw6_column_kernel(Problem
     // kinetic energy, momentum along i and j
     auto source = [&](int f, int c, double b) {
       if (fp_is_zero(b)) return 0.0;
+      soft_branch();
       const int k = c / COL_TG, g = g0 + c % COL_TG;
       const size_t i = off + (size_t)k * G + g;
       switch (f) {
@@ -738,13 +747,16 @@ __global__ void __launch_bounds__(COL_THREADS_MAX, 2) nsw6_column_kernel(Problem
       if (g >= G || k < kmin || k > kmax) return;
       const double fk = fl[c], fk1 = fl[c + COL_TG];
       const bool none = fp_is_zero(fk) && fp_is_zero(fk1);
-      const double d = none ? 0.0 : (fk1 - fk) * rdgz[k];
+      double d = 0.0;
+      const int s = f == 1 ? S_DRHOE : f == 2 ? S_DRHOPHI : f == 3 ? S_DKINH : f == 4 ? S_DRHOGU : S_DRHOGV;
+      if (!none) {
+        soft_branch();
+        d = (fk1 - fk) * rdgz[k];
+        if (f != 0) F(s)[c] = F(s)[c] - d;
+      }
       if (f == 0) {
         F(dqs_slot)[c] = none ? 0.0 : -d;
         if (nq == I_QR) P.GPREC[off + (size_t)k * G + g] = fp_is_zero(fk) ? 0.0 : soft_div_rn(-fk, P.by_dt, dt);
-      } else if (!none) {
-        const int s = f == 1 ? S_DRHOE : f == 2 ? S_DRHOPHI : f == 3 ? S_DKINH : f == 4 ? S_DRHOGU : S_DRHOGV;
-        F(s)[c] = F(s)[c] - d;
       }
       if (k == kmin && !fp_is_zero(fk)) {
         double* acc = S.colacc;
@@ -776,6 +788,7 @@ __global__ void __launch_bounds__(COL_THREADS_MAX, 2) nsw6_column_kernel(Problem
         const int k = c / COL_TG, gx = c % COL_TG;
         double fl[2] = {0.0, 0.0};
         if ((act >> j) & 1u) {
+          soft_branch();
           const double* const src[2] = {F(S_RHOF) + gx, F(S_RHOF2) + gx};
           // (the reference passes the full levels' upper bound to the half levels too)
           flux_integrals<COL_TG, 2>(src, dz, k, kc[j], rest[j], bmn[k], bmx_f[k], fl);
@@ -804,9 +817,15 @@ __global__ void __launch_bounds__(COL_THREADS_MAX, 2) nsw6_column_kernel(Problem
           FF(S_RHOF)[c] = __fmul_rn(qh, FF(S_KINV)[c]);
           FF(S_RHOF)[ncell + c] = __fmul_rn(qh, FF(S_DKINV)[ncell + c]);   // rhogw before the transport
         } else {
-          const double qh = some ? 0.5 * (qa + qb) * r_rgsh[j] : 0.0;
-          F(S_RHOF)[c] = some ? qh * F(S_KINV)[c] : 0.0;
-          F(S_RHOF2)[c] = some ? qh * P.rhogw[off + (size_t)k * G + g] : 0.0;
+          double s0 = 0.0, s1 = 0.0;
+          if (some) {
+            soft_branch();
+            const double qh = 0.5 * (qa + qb) * r_rgsh[j];
+            s0 = qh * F(S_KINV)[c];
+            s1 = qh * P.rhogw[off + (size_t)k * G + g];
+          }
+          F(S_RHOF)[c] = s0;
+          F(S_RHOF2)[c] = s1;
         }
         qs = some ? 1.0 : 0.0;
       } else if (c < ncell) {
@@ -843,7 +862,12 @@ __global__ void __launch_bounds__(COL_THREADS_MAX, 2) nsw6_column_kernel(Problem
         divergence(1, c, F(S_F2));
         const double b = bq[j];
         F(S_RHOF)[c] = source(2, c, b);
-        F(S_RHOF2)[c] = fp_is_zero(b) ? 0.0 : q_n[(size_t)k * G + g] * r_rgs[j] * F(S_KINH)[c];
+        double e = 0.0;
+        if (!fp_is_zero(b)) {
+          soft_branch();
+          e = q_n[(size_t)k * G + g] * r_rgs[j] * F(S_KINH)[c];
+        }
+        F(S_RHOF2)[c] = e;
       }
       __syncthreads();
       flux_pair(false);   // potential and horizontal kinetic energy
@@ -879,8 +903,11 @@ __global__ void __launch_bounds__(COL_THREADS_MAX, 2) nsw6_column_kernel(Problem
         const int k = c / COL_TG, g = g0 + c % COL_TG;
         if (c >= ncell || g >= G || k < kmin + 1 || k > kmax) continue;
         const double a1 = F(S_F)[c], a0 = F(S_F)[c - COL_TG], b1 = F(S_F2)[c], b0 = F(S_F2)[c - COL_TG];
-        if (!(fp_is_zero(a1) && fp_is_zero(a0))) F(S_DKINV)[c] = F(S_DKINV)[c] - (a1 - a0) * rdgzh[k];
-        if (!(fp_is_zero(b1) && fp_is_zero(b0))) F(S_DRHOGW)[c] = F(S_DRHOGW)[c] - (b1 - b0) * rdgzh[k];
+        if (!(fp_is_zero(a1) && fp_is_zero(a0) && fp_is_zero(b1) && fp_is_zero(b0))) {
+          soft_branch();
+          F(S_DKINV)[c] = F(S_DKINV)[c] - (a1 - a0) * rdgzh[k];
+          F(S_DRHOGW)[c] = F(S_DRHOGW)[c] - (b1 - b0) * rdgzh[k];
+        }
       }
       continue;   // the next tracer's sources go to S_RHOF, which nobody reads now
     }
@@ -1024,6 +1051,7 @@ __global__ void __launch_bounds__(COL_THREADS_MAX, 2) nsw6_column_kernel(Problem
     const double zz = P.z[i];
     auto add = [&](int n, double dq) {
       if (fp_is_zero(dq)) return;
+      soft_branch();
       P.rhogq[iq + (size_t)n * KG] = P.rhogq[iq + (size_t)n * KG] + dq;
       rhog = rhog + dq;
       rhoge = rhoge - dq * GRAV * zz;

@@ -218,8 +218,10 @@ __device__ __forceinline__ long long cmp_key(double x) {
   if (b == (long long)0x8000000000000000ULL) b = 0;
   return b < 0 ? (b ^ 0x7fffffffffffffffLL) : b;
 }
+// (by the two words: of the 64-bit form the compiler makes an FP64 comparison)
 __device__ __forceinline__ bool is_nan_bits(double x) {
-  return (__double_as_longlong(x) & 0x7fffffffffffffffLL) > 0x7ff0000000000000LL;
+  const unsigned hi = (unsigned)__double2hiint(x) & 0x7fffffffu;
+  return hi > 0x7ff00000u || (hi == 0x7ff00000u && __double2loint(x) != 0);
 }
 constexpr long long EPS_BITS = 0x3caffffff4178da3LL;   // bit pattern of EPS = 2.220446E-16
 

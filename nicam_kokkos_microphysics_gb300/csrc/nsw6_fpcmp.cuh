@@ -84,7 +84,13 @@ NSW6_FP_HD bool fp_is_zero(double x) {
 }
 
 // x is +-inf or NaN (x * 0 != 0)
-NSW6_FP_HD bool fp_not_finite(double x) { return (fp_bits(x) & FP_ABS) >= FP_INF; }
+NSW6_FP_HD bool fp_not_finite(double x) {
+#ifdef __CUDA_ARCH__
+  return ((unsigned)__double2hiint(x) & 0x7FF00000u) == 0x7FF00000u;
+#else
+  return (fp_bits(x) & FP_ABS) >= FP_INF;
+#endif
+}
 
 // x is a positive normal number (not zero, subnormal, infinite or NaN)
 NSW6_FP_HD bool fp_pos_normal(double x) {

@@ -208,11 +208,12 @@ __global__ void __launch_bounds__(CELL_THREADS, 2) nsw6_cell_kernel(Problem P, C
 
 // ------------------------------------------------------- departure distances
 // 0.5 x: the exponent one lower, where that is all there is to it
+NSW6_SLOW double soft_slow_half(double x) { return 0.5 * x; }
 __device__ __forceinline__ float half_of(float x) { return 0.5f * x; }
 __device__ __forceinline__ double half_of(double x) {
   const long long b = __double_as_longlong(x);
   if ((unsigned)(((b >> 52) & 0x7FF) - 2) < 2045u) return __longlong_as_double(b - (1ll << 52));
-  return (b << 1) == 0 ? x : 0.5 * x;
+  return fp_is_zero(x) ? x : soft_slow_half(x);
 }
 // the largest (smallest) key of a warp's lanes
 __device__ __forceinline__ unsigned long long warp_max(unsigned long long v) {
@@ -227,34 +228,45 @@ __device__ __forceinline__ unsigned long long warp_min(unsigned long long v) { r
 // region (order-preserving keys, exact atomics, so the order does not matter).
 // Row t of zdis holds the tracer's fall speeds on entry, the full-level
 // distances on return, row ntr + t the half-level ones.  One CTA reads all of
-// its columns' speeds before it writes.  Bound by the FP64 pipe: a half-level
-// velocity is the mean of two full-level ones, formed once, and the halvings
-// are integer operations.
+// its columns' speeds before it writes.  Bound by the FP64 pipe (82 % busy): a
+// half-level velocity is the mean of two full-level ones, formed once, the
+// halvings are integer operations, a warp walks consecutive levels and forms
+// their differences once, and levels without the tracer are branched around.
+// One 16900 x 42 region, FP64: 0.165 -> 0.118 ms (2.5 M -> 1.75 M FP64 warp
+// instructions).
 constexpr int DEP_TG = 32;
 constexpr int DEP_THREADS = 256;
 
 template <class R>
 __host__ __device__ constexpr size_t departure_smem_bytes(int K) {
-  return (size_t)K * sizeof(R) * (3 * DEP_TG + 6);
+  return (size_t)K * sizeof(R) * (3 * DEP_TG + 8);
 }
 
 template <class R>
 __global__ void __launch_bounds__(DEP_THREADS) nsw6_departure_kernel(Problem P) {
   extern __shared__ double sm[];
+  constexpr bool kMixed = sizeof(R) == sizeof(float);
   const int G = P.gall, K = P.kall, kmin = P.kmin, kmax = P.kmax, ntr = P.ntr;
   const int g0 = blockIdx.x * DEP_TG, t = blockIdx.y, l = blockIdx.z;
   const size_t KG = (size_t)K * G;
   R* vt = reinterpret_cast<R*>(sm);     // [K][DEP_TG] fall speeds, zero outside the interior
   R* wf = vt + K * DEP_TG;              // [K][DEP_TG] velocities on the full levels' interfaces
   R* wh = wf + K * DEP_TG;              // [K][DEP_TG] and on the half levels'
-  R* grid = wh + K * DEP_TG;            // 1 / dz, 1 / (dz- + dz) and twice that, of full and half levels
+  // 1 / dz, 1 / (dz- + dz) and, FP32, twice that or, FP64, twice that over dz and over dz-, of full and half levels
+  R* grid = wh + K * DEP_TG;
   double* z0 = P.zdis + ((size_t)l * 2 * ntr + t) * KG;
   double* z1 = z0 + (size_t)ntr * KG;
 
-  const int rows[6] = {GF_RDGZ, GF_RDZS, GF_RDZS, GF_RDGZH, GF_RDZSH, GF_RDZSH};
-  for (int c = threadIdx.x; c < 6 * K; c += blockDim.x) {
-    const R v = R(P.grid[rows[c / K] * K + c % K]);
-    grid[c] = (c / K) % 3 == 2 ? R(2.0) * v : v;
+  for (int c = threadIdx.x; c < 2 * K; c += blockDim.x) {
+    const int half = c / K, k = c % K;
+    const double* rdz = P.grid + (half ? GF_RDGZH : GF_RDGZ) * K;
+    const double* rdzs = P.grid + (half ? GF_RDZSH : GF_RDZS) * K;
+    R* row = grid + 4 * half * K + k;
+    row[0] = R(rdz[k]);
+    row[K] = R(rdzs[k]);
+    const R s2 = R(2.0) * R(rdzs[k]);
+    row[2 * K] = kMixed ? s2 : s2 * R(rdz[k]);
+    row[3 * K] = (kMixed || k == 0) ? R(0.0) : s2 * R(rdz[k - 1]);
   }
   const int gx = threadIdx.x % DEP_TG, g = g0 + gx, kw = threadIdx.x / DEP_TG, nw = blockDim.x / DEP_TG;
 #pragma unroll 4
@@ -277,15 +289,48 @@ __global__ void __launch_bounds__(DEP_THREADS) nsw6_departure_kernel(Problem P) 
   __syncthreads();
 
   const R dt = R(P.dt), hdt2 = R(P.hdt2), sdt3 = R(P.sdt3);
+  // a warp: consecutive levels of one of the two rows, so that a difference of
+  // two levels is formed once
+  const int share = (2 * K + nw - 1) / nw;
+  const bool valid = g < G;
+  R w0 = R(0.0), w1 = R(0.0), dn = R(0.0);   // w at k and k + 1, w(k) - w(k - 1)
+  int at = -1;                               // the row those are of
 #pragma unroll 1
-  for (int row = kw; row < 2 * K; row += nw) {   // one warp: one level of one of the two rows
+  for (int row = kw * share; row < min((kw + 1) * share, 2 * K); ++row) {
     const int half = row >= K ? 1 : 0, k = row - half * K, mkmin = kmin + half;
     if (k < mkmin || k > kmax) continue;
-    const R* w = half ? wh : wf;
-    const R* gr = grid + 3 * half * K;
-    const bool valid = g < G;
-    auto wp = [&](int j) { return w[j * DEP_TG + gx]; };
-    const double z = double(vadv_zdis_wh<R>(wp, gr, gr + K, [&](int j) { return gr[2 * K + j]; }, k, mkmin, dt, hdt2, sdt3));
+    const R* w = (half ? wh : wf) + gx;
+    const R* gr = grid + 4 * half * K;
+    double z;
+    if constexpr (kMixed) {
+      auto wp = [&](int j) { return w[j * DEP_TG]; };
+      z = soft_f2d(vadv_zdis_f<R>(wp, gr, gr + K, [&](int j) { return gr[2 * K + j]; }, k, mkmin, dt, hdt2, sdt3));
+    } else {
+      const R wm = k > mkmin ? w[(k - 1) * DEP_TG] : R(0.0);
+      if (at == row - 1) {
+        w0 = w1;
+      } else {
+        w0 = w[k * DEP_TG];
+        dn = w0 - wm;
+      }
+      w1 = w[(k + 1) * DEP_TG];
+      at = row;
+      z = w0;
+      if (__any_sync(0xffffffffu, !(fp_is_zero(wm) && fp_is_zero(w0) && fp_is_zero(w1)))) {
+        soft_branch();   // (levels without the tracer are branched around)
+        const R up = w1 - w0;
+        if (k == mkmin) {
+          soft_branch();
+          z = fmaR(-hdt2 * w0, up * gr[k], dt * w0);
+        } else {
+          soft_branch();
+          z = vadv_zdis_d<R, R>(w0, up, dn, w1 - wm, gr[K + k], gr[2 * K + k], gr[3 * K + k], dt, hdt2, sdt3);
+        }
+        dn = up;
+      } else {
+        dn = R(0.0);
+      }
+    }
     if (valid) (half ? z1 : z0)[(size_t)k * G + g] = z;
     // NaN never wins the reference's comparisons, so it is left out
     const bool use = valid && !is_nan_bits(z);
