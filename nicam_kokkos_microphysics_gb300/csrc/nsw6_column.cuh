@@ -231,21 +231,25 @@ __device__ __forceinline__ double satadjust_newton(const Problem& P, const Const
 // returned, for nsw6_satadj_kernel; every other cell is finished.  With
 // newton = true (that kernel) the cell is saturated: the same values are
 // formed, the Newton iteration runs and the cell is finished.
+// A value loaded here and not sunk to its use: the loads of a pass are in
+// flight together before its first call of a soft routine, across which none moves.
+__device__ __forceinline__ void loaded(double x) { asm volatile("" ::"d"(x)); }
+
 template <class M, bool MIX, bool OPT>
 __device__ __forceinline__ bool final_cell(const Problem& P, const Consts& C, const M& mth, bool ice_adj, float lovr_f,
                                            size_t i, size_t iq, size_t KG, bool interior, double rhog,
-                                           const Divisor& by_rhog, double rhoge, bool newton, int k, int g, int l) {
+                                           const Divisor& by_rhog, double rhoge, double (&rq)[6], double gsg,
+                                           bool newton, int k, int g, int l) {
   const double rrhog = MIX ? rcp_of(by_rhog) : 0.0;
-  double rq[6], q[6];
+  double q[6];
 #pragma unroll
-  for (int n = 0; n < 6; ++n) rq[n] = plus_zero(P.rhogq[iq + (size_t)n * KG]);
+  for (int n = 0; n < 6; ++n) rq[n] = plus_zero(rq[n]);
   // These quotients must be correctly rounded: the saturation adjustment
   // forms qc = qsum - qsat from them, a difference of nearly equal numbers
   // in which one unit in the last place of qsum is already a relative error
   // of 1e-11 when qc is small.
 #pragma unroll
   for (int n = 0; n < 6; ++n) q[n] = MIX ? rq[n] * rrhog : div_rn(rq[n], by_rhog);
-  const double gsg = P.gsgam2[i];
   double rho = quo(rhog, gsg);
   const double ein = MIX ? rhoge * rrhog : div_rn(rhoge, by_rhog);
   double qd = 1.0;
@@ -440,7 +444,12 @@ __device__ __forceinline__ bool final_cell(const Problem& P, const Consts& C, co
 // they draw on hold nothing of the tracer does none of it (rain above the
 // freezing level).  One 16900 x 42 region, FP64: 0.56 -> 0.47 ms (7.1 M -> 6.4 M
 // FP64 warp instructions), ten regions in mixed precision
-// 5.75 -> 5.18 ms a step.
+// 5.75 -> 5.18 ms a step.  A pass's loads go first, ahead of the calls of the
+// soft routines (no load moves across one, so each would wait for memory by
+// itself) and, where registers allow, ahead of the barrier before the pass; the
+// final passes take the state from shared memory where their thread has just
+// formed it: ten regions 5.11 -> 4.46 ms in mixed precision (a third of whose
+// stalls were for memory), 9.35 -> 9.19 ms in FP64.
 //
 // Threads of a CTA at most, two of which an SM holds (80 registers a thread).
 constexpr int COL_THREADS_MAX = 384;
@@ -590,40 +599,42 @@ __global__ void __launch_bounds__(COL_THREADS_MAX, 2) nsw6_column_kernel(Problem
     const size_t i = off + (size_t)k * G + g;
     const size_t ic = (size_t)l * G + g;
     const bool interior = (k >= kmin && k <= kmax);
+    const double gsg = P.gsgam2[i], gm = P.gam2[i], gsh = P.gsgam2h[i], gmh = P.gam2h[i], rg = P.rhog[i];
+    const double vxd = P.vx[i], vyd = P.vy[i], vzd = P.vz[i];
+    const double rvx = P.rhogvx[i], rvy = P.rhogvy[i], rvz = P.rhogvz[i], rwd = MIX ? P.rhogw[i] : 0.0;
+    loaded(gsg), loaded(gm), loaded(gsh), loaded(gmh), loaded(rg), loaded(vxd), loaded(vyd), loaded(vzd);
+    loaded(rvx), loaded(rvy), loaded(rvz);
+    if (MIX) loaded(rwd);
     // gam2 / gsgam2 and afact / gsgam2, correctly rounded
-    const double gsg = P.gsgam2[i];
     const Divisor by_gsg(gsg);
-    if (interior) r_rgs[j] = div_rn(P.gam2[i], by_gsg);
+    if (interior) r_rgs[j] = div_rn(gm, by_gsg);
     if (MIX) {
       // the velocity components scale FP32 momentum sources only: FP32
-      const float vx = soft_d2f(P.vx[i]), vy = soft_d2f(P.vy[i]), vz = soft_d2f(P.vz[i]);
+      const float vx = soft_d2f(vxd), vy = soft_d2f(vyd), vz = soft_d2f(vzd);
       FF(S_VI)[c] = __fmaf_rn(vz, uvf[2 * COL_TG + gx], __fmaf_rn(vy, uvf[1 * COL_TG + gx], __fmul_rn(vx, uvf[gx])));
       FF(S_VJ)[c] =
           __fmaf_rn(vz, uvf[5 * COL_TG + gx], __fmaf_rn(vy, uvf[4 * COL_TG + gx], __fmul_rn(vx, uvf[3 * COL_TG + gx])));
-      const float gsgf = soft_d2f(gsg), ghf = soft_d2f(P.gsgam2h[i]), rhogf = soft_d2f(P.rhog[i]);
+      const float gsgf = soft_d2f(gsg), ghf = soft_d2f(gsh), rhogf = soft_d2f(rg);
       FF(S_VI)[ncell + c] = ghf;
       FF(S_VJ)[ncell + c] = gsgf;
       FF(S_KINH)[ncell + c] = rhogf;
       if (interior) {
         FF(S_KINV)[ncell + c] = soft_d2f(r_rgs[j]);
-        FF(S_KINH)[c] = kin_h_f(soft_d2f(P.rhogvx[i]), soft_d2f(P.rhogvy[i]), soft_d2f(P.rhogvz[i]), rhogf);
+        FF(S_KINH)[c] = kin_h_f(soft_d2f(rvx), soft_d2f(rvy), soft_d2f(rvz), rhogf);
       }
       if (k >= kmin + 1 && k <= kmax) {
         r_c2w0f[j] = __fmul_rn(__fdiv_rn(aff[k], gsgf), ghf);
-        r_rgshf[j] = __fdiv_rn(soft_d2f(P.gam2h[i]), ghf);
+        r_rgshf[j] = __fdiv_rn(soft_d2f(gmh), ghf);
+        FF(S_DKINV)[ncell + c] = soft_d2f(rwd);
       }
       continue;
     }
-    const double vx = P.vx[i], vy = P.vy[i], vz = P.vz[i];
-    F(S_VI)[c] = vx * P.ix[ic] + vy * P.iy[ic] + vz * P.iz[ic];
-    F(S_VJ)[c] = vx * P.jx[ic] + vy * P.jy[ic] + vz * P.jz[ic];
-    if (interior) {
-      const double rvx = P.rhogvx[i], rvy = P.rhogvy[i], rvz = P.rhogvz[i];
-      F(S_KINH)[c] = quo(0.5 * (rvx * rvx + rvy * rvy + rvz * rvz), P.rhog[i]);
-    }
+    F(S_VI)[c] = vxd * P.ix[ic] + vyd * P.iy[ic] + vzd * P.iz[ic];
+    F(S_VJ)[c] = vxd * P.jx[ic] + vyd * P.jy[ic] + vzd * P.jz[ic];
+    if (interior) F(S_KINH)[c] = quo(0.5 * (rvx * rvx + rvy * rvy + rvz * rvz), rg);
     if (k >= kmin + 1 && k <= kmax) {
-      r_c2w0[j] = div_rn(afact[k], by_gsg) * P.gsgam2h[i];
-      r_rgsh[j] = quo(P.gam2h[i], P.gsgam2h[i]);
+      r_c2w0[j] = div_rn(afact[k], by_gsg) * gsh;
+      r_rgsh[j] = quo(gmh, gsh);
     }
   }
   __syncthreads();
@@ -636,16 +647,16 @@ __global__ void __launch_bounds__(COL_THREADS_MAX, 2) nsw6_column_kernel(Problem
     const size_t i = off + (size_t)k * G + g;
     if (MIX) {
       const float c2w1 = __fmul_rn(__fdiv_rn(bff[k], FF(S_VJ)[ncell + c - COL_TG]), FF(S_VI)[ncell + c]);
-      const float rw = soft_d2f(P.rhogw[i]);
-      FF(S_DKINV)[ncell + c] = rw;
+      const float rw = FF(S_DKINV)[ncell + c];
       FF(S_KINV)[c] = kin_v_f(rw, r_c2w0f[j], c2w1, FF(S_KINH)[ncell + c], FF(S_KINH)[ncell + c - COL_TG]);
       r_c2w1f[j] = c2w1;
       continue;
     }
     const double c2w0 = r_c2w0[j];
-    const double c2w1 = div_rn(bfact[k], Divisor(P.gsgam2[i - G])) * P.gsgam2h[i];
-    const double rw = P.rhogw[i];
-    F(S_KINV)[c] = quo(0.5 * (rw * rw), c2w0 * P.rhog[i] + c2w1 * P.rhog[i - G]);
+    const double gsgm = P.gsgam2[i - G], gsh = P.gsgam2h[i], rw = P.rhogw[i], rg = P.rhog[i], rgm = P.rhog[i - G];
+    loaded(gsgm), loaded(gsh), loaded(rw), loaded(rg), loaded(rgm);
+    const double c2w1 = div_rn(bfact[k], Divisor(gsgm)) * gsh;
+    F(S_KINV)[c] = quo(0.5 * (rw * rw), c2w0 * rg + c2w1 * rgm);
     r_c2w1[j] = c2w1;
   }
   // (the vertical kinetic energies are next read by their own threads, after barriers by others)
@@ -679,9 +690,37 @@ __global__ void __launch_bounds__(COL_THREADS_MAX, 2) nsw6_column_kernel(Problem
     const double* rhogq_n = P.rhogq + offq + (size_t)nq * KG;
     const double* q_n = P.q + offq + (size_t)nq * KG;
     unsigned act = 0;   // bit j: the cell draws on levels that hold something
+    double ld0[NJ], ld1[NJ], ld2[NJ], ld3[NJ];   // a pass's loads
+    // loads of the half levels' pass: departure distance, q of the two levels (and rhogw)
+    auto load_half = [&]() {
+#pragma unroll
+      for (int j = 0; j < NJ; ++j) {
+        const int c = threadIdx.x + j * blockDim.x;
+        const int k = c / COL_TG, g = g0 + c % COL_TG;
+        if (c >= ncell || g >= G || k < kmin + 1 || k > kmax) continue;
+        const size_t i = (size_t)k * G + g;
+        ld0[j] = zdis0h[i];
+        ld1[j] = q_n[i];
+        ld2[j] = q_n[i - G];
+        if (!MIX) ld3[j] = P.rhogw[off + i];
+        loaded(ld0[j]), loaded(ld1[j]), loaded(ld2[j]);
+        if (!MIX) loaded(ld3[j]);
+      }
+    };
 
     // departure cells (full levels), rhoq = rhogq * rgs, which is the source of
     // the first flux (the mass flux), and the source of the second (energy)
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) {
+      const int c = threadIdx.x + j * blockDim.x;
+      const int k = c / COL_TG, g = g0 + c % COL_TG;
+      if (c >= ncell || g >= G) continue;
+      const size_t i = (size_t)k * G + g;
+      ld0[j] = rhogq_n[i];
+      ld1[j] = zdis0[i];
+      ld2[j] = P.tem[off + i];
+      loaded(ld0[j]), loaded(ld1[j]), loaded(ld2[j]);
+    }
 #pragma unroll
     for (int j = 0; j < NJ; ++j) {
       const int c = threadIdx.x + j * blockDim.x;
@@ -692,14 +731,13 @@ __global__ void __launch_bounds__(COL_THREADS_MAX, 2) nsw6_column_kernel(Problem
       kc[j] = kmin;
       const bool own = c < ncell && g < G;
       if (own) {
-        const size_t i = (size_t)k * G + g;
-        const double b0 = rhogq_n[i];
+        const double b0 = ld0[j];
         if (!fp_is_zero(b0)) {
           soft_branch();
           bq[j] = b0 * r_rgs[j];
         }
         if (k >= kmin && k <= kmax) {
-          const double z = zdis0[i];
+          const double z = ld1[j];
           kc[j] = departure_cell(gzh, zkey, k, z, bmn_f[k], bmx_f[k], kmin, kmax);
           rest[j] = flux_rest(dgz, k, kc[j], z, bmn_f[k], bmx_f[k]);
           if (MIX) restf[j] = flux_rest(dgzf, k, kc[j], soft_d2f(z), bmn_f[k], bmx_f[k]);
@@ -711,7 +749,7 @@ __global__ void __launch_bounds__(COL_THREADS_MAX, 2) nsw6_column_kernel(Problem
         double e = 0.0;
         if (holds) {
           soft_branch();
-          e = b * CVDRY * P.tem[off + (size_t)k * G + g];
+          e = b * CVDRY * ld2[j];
         }
         F(S_RHOF)[c] = b;
         F(S_RHOF2)[c] = e;
@@ -727,15 +765,13 @@ __global__ void __launch_bounds__(COL_THREADS_MAX, 2) nsw6_column_kernel(Problem
         act |= 1u << j;
     }
 
-    // sources 2 .. 5 (mod_precip_transport.cpp:776-808): potential energy, horizontal
-    // kinetic energy, momentum along i and j
-    auto source = [&](int f, int c, double b) {
+    // sources 2 .. 5 (mod_precip_transport.cpp:776-808): potential energy (of the cell's z),
+    // horizontal kinetic energy, momentum along i and j
+    auto source = [&](int f, int c, double b, double z) {
       if (fp_is_zero(b)) return 0.0;
       soft_branch();
-      const int k = c / COL_TG, g = g0 + c % COL_TG;
-      const size_t i = off + (size_t)k * G + g;
       switch (f) {
-        case 2: return b * GRAV * P.z[i];
+        case 2: return b * GRAV * z;
         case 4: return b * F(S_VI)[c];
         default: return b * F(S_VJ)[c];
       }
@@ -805,11 +841,11 @@ __global__ void __launch_bounds__(COL_THREADS_MAX, 2) nsw6_column_kernel(Problem
       const bool hv = c < ncell && g < G && k >= kmin + 1 && k <= kmax;
       double qs = 0.0;
       if (hv) {
-        const double z = zdis0h[(size_t)k * G + g];
+        const double z = ld0[j];
         kc[j] = departure_cell(gzs, zkey + K, k, z, bmn_h[k], bmx_h[k], kmin + 1, kmax);
         if (MIX) restf[j] = flux_rest(dgzhf, k, kc[j], soft_d2f(z), bmn_h[k], bmx_f[k]);
         else rest[j] = flux_rest(dgzh, k, kc[j], z, bmn_h[k], bmx_f[k]);
-        const double qa = q_n[(size_t)k * G + g], qb = q_n[(size_t)(k - 1) * G + g];
+        const double qa = ld1[j], qb = ld2[j];
         const bool some = !(fp_is_zero(qa) && fp_is_zero(qb));
         if (MIX) {
           // qh scales the FP32 sources of the two half-level fluxes only: FP32
@@ -822,7 +858,7 @@ __global__ void __launch_bounds__(COL_THREADS_MAX, 2) nsw6_column_kernel(Problem
             soft_branch();
             const double qh = 0.5 * (qa + qb) * r_rgsh[j];
             s0 = qh * F(S_KINV)[c];
-            s1 = qh * P.rhogw[off + (size_t)k * G + g];
+            s1 = qh * ld3[j];
           }
           F(S_RHOF)[c] = s0;
           F(S_RHOF2)[c] = s1;
@@ -851,21 +887,30 @@ __global__ void __launch_bounds__(COL_THREADS_MAX, 2) nsw6_column_kernel(Problem
     };
 
     flux_pair(false);   // mass and internal energy
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) {
+      const int c = threadIdx.x + j * blockDim.x;
+      const int k = c / COL_TG, g = g0 + c % COL_TG;
+      if (c >= ncell || g >= G) continue;
+      const size_t i = (size_t)k * G + g;
+      ld0[j] = P.z[off + i];
+      ld1[j] = q_n[i];
+      loaded(ld0[j]), loaded(ld1[j]);
+    }
     __syncthreads();
     if (!MIX) {
 #pragma unroll
       for (int j = 0; j < NJ; ++j) {
         const int c = threadIdx.x + j * blockDim.x;
         if (c >= ncell) continue;
-        const int k = c / COL_TG, g = g0 + c % COL_TG;
         divergence(0, c, F(S_F));
         divergence(1, c, F(S_F2));
         const double b = bq[j];
-        F(S_RHOF)[c] = source(2, c, b);
+        F(S_RHOF)[c] = source(2, c, b, ld0[j]);
         double e = 0.0;
         if (!fp_is_zero(b)) {
           soft_branch();
-          e = q_n[(size_t)k * G + g] * r_rgs[j] * F(S_KINH)[c];
+          e = ld1[j] * r_rgs[j] * F(S_KINH)[c];
         }
         F(S_RHOF2)[c] = e;
       }
@@ -878,11 +923,12 @@ __global__ void __launch_bounds__(COL_THREADS_MAX, 2) nsw6_column_kernel(Problem
         if (c >= ncell) continue;
         divergence(2, c, F(S_F));
         divergence(3, c, F(S_F2));
-        F(S_RHOF)[c] = source(4, c, bq[j]);
-        F(S_RHOF2)[c] = source(5, c, bq[j]);
+        F(S_RHOF)[c] = source(4, c, bq[j], 0.0);
+        F(S_RHOF2)[c] = source(5, c, bq[j], 0.0);
       }
       __syncthreads();
       flux_pair(false);   // momentum along i and j
+      load_half();
       __syncthreads();
 #pragma unroll
       for (int j = 0; j < NJ; ++j) {
@@ -923,13 +969,12 @@ __global__ void __launch_bounds__(COL_THREADS_MAX, 2) nsw6_column_kernel(Problem
       if (c >= ncell) continue;
       divergence(0, c, F(S_F));
       divergence(1, c, F(S_F2));
-      F(S_RHOF)[c] = source(2, c, bq[j]);
+      F(S_RHOF)[c] = source(2, c, bq[j], ld0[j]);
       // (S_RHOF2's doubles were read before the last barrier)
-      const int k = c / COL_TG, g = g0 + c % COL_TG;
       float r3 = 0.0f, r4 = 0.0f, r5 = 0.0f;
       if (!fp_is_zero(bq[j])) {
         const float bf = soft_d2f(bq[j]);
-        r3 = __fmul_rn(__fmul_rn(soft_d2f(q_n[(size_t)k * G + g]), FF(S_KINV)[ncell + c]), FF(S_KINH)[c]);
+        r3 = __fmul_rn(__fmul_rn(soft_d2f(ld1[j]), FF(S_KINV)[ncell + c]), FF(S_KINH)[c]);
         r4 = __fmul_rn(bf, FF(S_VI)[c]);
         r5 = __fmul_rn(bf, FF(S_VJ)[c]);
       }
@@ -956,6 +1001,7 @@ __global__ void __launch_bounds__(COL_THREADS_MAX, 2) nsw6_column_kernel(Problem
       fluxf[1][c] = ff[1];
       fluxf[2][c] = ff[2];
     }
+    load_half();
     __syncthreads();
 #pragma unroll
     for (int j = 0; j < NJ; ++j) {
@@ -1012,7 +1058,14 @@ __global__ void __launch_bounds__(COL_THREADS_MAX, 2) nsw6_column_kernel(Problem
     const size_t i = off + (size_t)k * G + g;
     const size_t ic = (size_t)l * G + g;
     const size_t iq = offq + (size_t)k * G + g;
-    double rhoge = P.rhoge[i];
+    double rhoge = P.rhoge[i], rhog = P.rhog[i], rw = P.rhogw[i];
+    double rvx = P.rhogvx[i], rvy = P.rhogvy[i], rvz = P.rhogvz[i];
+    const double zz = P.z[i];
+    const double rqr = P.rhogq[iq + (size_t)I_QR * KG], rqs = P.rhogq[iq + (size_t)I_QS * KG],
+                 rqg = P.rhogq[iq + (size_t)I_QG * KG], rqi = OPT ? P.rhogq[iq + (size_t)I_QI * KG] : 0.0;
+    loaded(rhoge), loaded(rhog), loaded(rw), loaded(rvx), loaded(rvy), loaded(rvz), loaded(zz);
+    loaded(rqr), loaded(rqs), loaded(rqg);
+    if (OPT) loaded(rqi);
     const double de = F(S_DRHOE)[c], dphi = F(S_DRHOPHI)[c];
     if (!fp_is_zero(de)) rhoge = rhoge + de;
     if (!fp_is_zero(dphi)) rhoge = rhoge + dphi;
@@ -1027,43 +1080,49 @@ __global__ void __launch_bounds__(COL_THREADS_MAX, 2) nsw6_column_kernel(Problem
       // the FP32 momentum tendencies along the FP32 unit vectors, added to the FP64 state
       const float du = FF(S_DRHOGU)[c], dv = FF(S_DRHOGV)[c];
       if (du != 0.0f || dv != 0.0f) {
-        P.rhogvx[i] = P.rhogvx[i] + soft_f2d(__fmaf_rn(dv, uvf[3 * COL_TG + gx], __fmul_rn(du, uvf[gx])));
-        P.rhogvy[i] = P.rhogvy[i] + soft_f2d(__fmaf_rn(dv, uvf[4 * COL_TG + gx], __fmul_rn(du, uvf[1 * COL_TG + gx])));
-        P.rhogvz[i] = P.rhogvz[i] + soft_f2d(__fmaf_rn(dv, uvf[5 * COL_TG + gx], __fmul_rn(du, uvf[2 * COL_TG + gx])));
+        P.rhogvx[i] = rvx = rvx + soft_f2d(__fmaf_rn(dv, uvf[3 * COL_TG + gx], __fmul_rn(du, uvf[gx])));
+        P.rhogvy[i] = rvy = rvy + soft_f2d(__fmaf_rn(dv, uvf[4 * COL_TG + gx], __fmul_rn(du, uvf[1 * COL_TG + gx])));
+        P.rhogvz[i] = rvz = rvz + soft_f2d(__fmaf_rn(dv, uvf[5 * COL_TG + gx], __fmul_rn(du, uvf[2 * COL_TG + gx])));
       }
     } else {
       const double du = F(S_DRHOGU)[c], dv = F(S_DRHOGV)[c];
       if (!(fp_is_zero(du) && fp_is_zero(dv))) {
-        P.rhogvx[i] = P.rhogvx[i] + du * P.ix[ic] + dv * P.jx[ic];
-        P.rhogvy[i] = P.rhogvy[i] + du * P.iy[ic] + dv * P.jy[ic];
-        P.rhogvz[i] = P.rhogvz[i] + du * P.iz[ic] + dv * P.jz[ic];
+        P.rhogvx[i] = rvx = rvx + du * P.ix[ic] + dv * P.jx[ic];
+        P.rhogvy[i] = rvy = rvy + du * P.iy[ic] + dv * P.jy[ic];
+        P.rhogvz[i] = rvz = rvz + du * P.iz[ic] + dv * P.jz[ic];
       }
     }
     const double dw = MIX ? soft_f2d(FF(S_DRHOGW)[c]) : F(S_DRHOGW)[c];
-    double rw = P.rhogw[i];
     if (!fp_is_zero(dw)) {
       rw = rw + dw;
       P.rhogw[i] = rw;
     }
     if (!MIX) F(S_DRHOGW)[c] = rw;   // MIX: the FP32 view of this slot is still being read
     // tracers in order QV..QG (QV, QC and QI add exact zeros; the -0 that makes a +0 is left to final_cell)
-    double rhog = P.rhog[i];
-    const double zz = P.z[i];
-    auto add = [&](int n, double dq) {
+    auto add = [&](int n, double rq, double dq) {
       if (fp_is_zero(dq)) return;
       soft_branch();
-      P.rhogq[iq + (size_t)n * KG] = P.rhogq[iq + (size_t)n * KG] + dq;
+      P.rhogq[iq + (size_t)n * KG] = rq + dq;
       rhog = rhog + dq;
       rhoge = rhoge - dq * GRAV * zz;
     };
-    add(I_QR, F(S_DQR)[c]);
-    if (OPT && ntr == 4) add(I_QI, F(S_DQI)[c]);
-    add(I_QS, F(S_DQS)[c]);
-    add(I_QG, F(S_DQG)[c]);
+    add(I_QR, rqr, F(S_DQR)[c]);
+    if (OPT && ntr == 4) add(I_QI, rqi, F(S_DQI)[c]);
+    add(I_QS, rqs, F(S_DQS)[c]);
+    add(I_QG, rqg, F(S_DQG)[c]);
     P.rhog[i] = rhog;
-    P.rhoge[i] = rhoge;
     F(S_RHOF)[c] = rhog;
-    if (MIX) FF(S_KINH)[ncell + c] = soft_d2f(rhog);   // rhog after the transport, for the FP32 kinetic energies
+    F(S_DQR)[c] = rhoge;   // for the final pass
+    // (the horizontal kinetic energy of the updated state times rhog)
+    if (!MIX && !kin2kin && k >= kmin && k <= kmax) F(S_DKINH)[c] = 0.5 * (rvx * rvx + rvy * rvy + rvz * rvz);
+    if (MIX) {
+      const float rhogf = soft_d2f(rhog);
+      FF(S_KINH)[ncell + c] = rhogf;   // rhog after the transport, for the FP32 kinetic energies
+      FF(S_DKINV)[c] = soft_d2f(rw);   // and rhogw
+      // the horizontal kinetic energy carried by the transport less that of the updated state
+      if (!kin2kin && k >= kmin && k <= kmax)
+        FF(S_KINH)[c] = FF(S_KINH)[c] - kin_h_f(soft_d2f(rvx), soft_d2f(rvy), soft_d2f(rvz), rhogf);
+    }
   }
   __syncthreads();
 
@@ -1122,8 +1181,7 @@ __global__ void __launch_bounds__(COL_THREADS_MAX, 2) nsw6_column_kernel(Problem
       // W2Cfact of the interior cells in the two halves of S_DRHOE
       float dkv = 0.0f;
       if (g < G && k >= kmin + 1 && k <= kmax) {
-        const size_t i = off + (size_t)k * G + g;
-        dkv = FF(S_KINV)[c] - kin_v_f(soft_d2f(P.rhogw[i]), r_c2w0f[j], r_c2w1f[j], FF(S_KINH)[ncell + c],
+        dkv = FF(S_KINV)[c] - kin_v_f(FF(S_DKINV)[c], r_c2w0f[j], r_c2w1f[j], FF(S_KINH)[ncell + c],
                                       FF(S_KINH)[ncell + c - COL_TG]);
       }
       FF(S_DRHOPHI)[c] = dkv;
@@ -1173,22 +1231,25 @@ __global__ void __launch_bounds__(COL_THREADS_MAX, 2) nsw6_column_kernel(Problem
     if (g >= G) continue;
     const size_t i = off + (size_t)k * G + g;
     const bool interior = (k >= kmin && k <= kmax);
+    const size_t iq = offq + (size_t)k * G + g;
+    double rq[6];
+#pragma unroll
+    for (int n = 0; n < 6; ++n) loaded(rq[n] = P.rhogq[iq + (size_t)n * KG]);
+    const double gsg = P.gsgam2[i];
+    loaded(gsg);
     const double rhog = F(S_RHOF)[c];
     const Divisor by_rhog(rhog);   // of the cell's quotients (correctly rounded, as the reference's divisions)
-    double rhoge = P.rhoge[i];
+    double rhoge = F(S_DQR)[c];
     if (MIX && interior && !kin2kin) {
       // FP32 kinetic energies: the horizontal energy after the transport
       // against before (with its tendency), the vertical energies' changes
       // weighted by W2Cfact; their sum enters the FP64 internal energy
-      const float kh = kin_h_f(soft_d2f(P.rhogvx[i]), soft_d2f(P.rhogvy[i]), soft_d2f(P.rhogvz[i]), FF(S_KINH)[ncell + c]);
-      const float dke = (FF(S_KINH)[c] - kh) +
+      const float dke = FF(S_KINH)[c] +
                         __fmaf_rn(FF(S_DRHOE)[c], FF(S_DRHOPHI)[c + COL_TG],
                                   __fmul_rn(FF(S_DRHOE)[ncell + c], FF(S_DRHOPHI)[c]));
       if (dke != 0.0f) rhoge = rhoge + soft_f2d(dke);
-      P.rhoge[i] = rhoge;   // a saturated cell's adjustment starts from here (final_cell overwrites the rest)
     } else if (interior && !kin2kin) {
-      const double rvx = P.rhogvx[i], rvy = P.rhogvy[i], rvz = P.rhogvz[i];
-      const double tmp_h = div_rn(0.5 * (rvx * rvx + rvy * rvy + rvz * rvz), by_rhog);
+      const double tmp_h = div_rn(F(S_DKINH)[c], by_rhog);
       double w2c0, w2c1;
       if (!OPT) {
         w2c0 = F(S_DRHOGW)[c];
@@ -1200,11 +1261,12 @@ __global__ void __launch_bounds__(COL_THREADS_MAX, 2) nsw6_column_kernel(Problem
       }
       const double tmp = tmp_h + (w2c0 * F(S_DRHOPHI)[c + COL_TG] + w2c1 * F(S_DRHOPHI)[c]);
       rhoge = rhoge + (F(S_DRHOE)[c] - tmp);
-      P.rhoge[i] = rhoge;   // a saturated cell's adjustment starts from here (final_cell overwrites the rest)
     }
-    if (final_cell<ColumnMath, MIX, OPT>(P, C, mth, ice_adj, lovr_f, i, offq + (size_t)k * G + g, KG, interior, rhog, by_rhog,
-                                rhoge, false, k, g, l))
+    if (final_cell<ColumnMath, MIX, OPT>(P, C, mth, ice_adj, lovr_f, i, iq, KG, interior, rhog, by_rhog, rhoge, rq, gsg,
+                                         false, k, g, l)) {
+      P.rhoge[i] = rhoge;   // its adjustment starts from here
       qcell[atomicAdd(&nqueue, 1)] = c;
+    }
     if (k == kmin) {
       const size_t ic = (size_t)l * G + g;
       const size_t r0 = (size_t)l * G + g, r1 = P.prec_ld + r0;
@@ -1257,8 +1319,13 @@ __global__ void __launch_bounds__(SAT_THREADS) nsw6_satadj_kernel(Problem P, Con
     const size_t r = i - (size_t)l * KG;
     const int k = (int)(r / G), g = (int)(r - (size_t)k * G);
     const double rhog = P.rhog[i];
-    final_cell<ColumnMath, MIX, OPT>(P, C, mth, ice_adj, lovr_f, i, (size_t)l * NQ * KG + r, KG, true, rhog, Divisor(rhog),
-                            P.rhoge[i], true, k, g, l);
+    const size_t iq = (size_t)l * NQ * KG + r;
+    const double rhoge = P.rhoge[i], gsg = P.gsgam2[i];
+    double rq[6];
+#pragma unroll
+    for (int n = 0; n < 6; ++n) loaded(rq[n] = P.rhogq[iq + (size_t)n * KG]);
+    final_cell<ColumnMath, MIX, OPT>(P, C, mth, ice_adj, lovr_f, i, iq, KG, true, rhog, Divisor(rhog), rhoge, rq, gsg, true,
+                                     k, g, l);
   }
 }
 
