@@ -20,12 +20,16 @@
 
 #include <type_traits>
 
+#include "nsw6_cell.cuh"
 #include "nsw6_common.cuh"
 #include "nsw6_fastmath.cuh"
 
 namespace nsw6 {
 
 // ------------------------------------------------------------------ Dual
+// The tangents take fused multiply-adds, the values the step's operations.
+// What carries no tangent (literals, the constants that no parameter enters)
+// stays a double.  With both, 4096 columns' cell phase went @TLMCELL@.
 struct Dual {
   double v, d;
   __device__ __forceinline__ Dual() : v(0.0), d(0.0) {}
@@ -33,13 +37,44 @@ struct Dual {
   __device__ __forceinline__ Dual(double x, double dx) : v(x), d(dx) {}
 };
 
+// The scheme constants with the parameters' tangents: these members hide the
+// doubles of the same names.
+struct DualConsts : Consts {
+  Dual beta_saut, qicrt_saut, Cr, Cs, Cg, ice_nuc, kk_aut;
+  Dual K_vtr, K_raci, K_iacr, K_vts, K_sacw, K_saci, K_vents2, K_vtg, K_gacw, K_aut;
+};
+template <>
+struct ScalarOf<Dual> {
+  using constant = double;
+  using consts = DualConsts;
+};
+
 __device__ __forceinline__ Dual operator+(const Dual& a, const Dual& b) { return Dual(a.v + b.v, a.d + b.d); }
 __device__ __forceinline__ Dual operator-(const Dual& a, const Dual& b) { return Dual(a.v - b.v, a.d - b.d); }
-__device__ __forceinline__ Dual operator*(const Dual& a, const Dual& b) { return Dual(a.v * b.v, a.d * b.v + a.v * b.d); }
+__device__ __forceinline__ Dual operator*(const Dual& a, const Dual& b) {
+  return Dual(a.v * b.v, __fma_rn(a.d, b.v, a.v * b.d));
+}
 __device__ __forceinline__ Dual operator/(const Dual& a, const Dual& b) {
   const SoftDivisor by = soft_divisor(b.v);
   const double q = soft_div(a.v, by, b.v);
-  return Dual(q, soft_div(a.d - q * b.d, by, b.v));
+  return Dual(q, soft_div(__fma_rn(-q, b.d, a.d), by, b.v));
+}
+// With a constant: its tangent, an exact zero, costs nothing (the compiler may
+// not drop a product with 0.0 or a sum with it).
+__device__ __forceinline__ Dual operator+(const Dual& a, double b) { return Dual(a.v + b, a.d); }
+__device__ __forceinline__ Dual operator+(double a, const Dual& b) { return Dual(a + b.v, b.d); }
+__device__ __forceinline__ Dual operator-(const Dual& a, double b) { return Dual(a.v - b, a.d); }
+__device__ __forceinline__ Dual operator-(double a, const Dual& b) { return Dual(a - b.v, -b.d); }
+__device__ __forceinline__ Dual operator*(const Dual& a, double b) { return Dual(a.v * b, a.d * b); }
+__device__ __forceinline__ Dual operator*(double a, const Dual& b) { return Dual(a * b.v, a * b.d); }
+__device__ __forceinline__ Dual operator/(const Dual& a, double b) {
+  const SoftDivisor by = soft_divisor(b);
+  return Dual(soft_div(a.v, by, b), soft_div(a.d, by, b));
+}
+__device__ __forceinline__ Dual operator/(double a, const Dual& b) {
+  const SoftDivisor by = soft_divisor(b.v);
+  const double q = soft_div(a, by, b.v);
+  return Dual(q, soft_div(-q * b.d, by, b.v));
 }
 __device__ __forceinline__ Dual operator-(const Dual& a) { return Dual(-a.v, -a.d); }
 __device__ __forceinline__ Dual operator+(const Dual& a) { return a; }
@@ -61,11 +96,23 @@ __device__ __forceinline__ double with_value(double, double v) { return v; }
 // f(x) with value fv and derivative dfdx at x.
 __device__ __forceinline__ Dual dep(double fv, const Dual& x, double dfdx) { return Dual(fv, dfdx * x.d); }
 __device__ __forceinline__ Dual dep2(double fv, const Dual& x, double dx, const Dual& y, double dy) {
-  return Dual(fv, dx * x.d + dy * y.d);
+  return Dual(fv, __fma_rn(dx, x.d, dy * y.d));
 }
 
 __device__ __forceinline__ Dual fmaR(const Dual& a, const Dual& b, const Dual& c) {
-  return Dual(__fma_rn(a.v, b.v, c.v), a.d * b.v + a.v * b.d + c.d);
+  return Dual(__fma_rn(a.v, b.v, c.v), __fma_rn(a.d, b.v, __fma_rn(a.v, b.d, c.d)));
+}
+__device__ __forceinline__ Dual fmaR(double a, const Dual& b, const Dual& c) {
+  return Dual(__fma_rn(a, b.v, c.v), __fma_rn(a, b.d, c.d));
+}
+__device__ __forceinline__ Dual fmaR(const Dual& a, double b, const Dual& c) { return fmaR(b, a, c); }
+__device__ __forceinline__ Dual fmaR(double a, const Dual& b, double c) { return Dual(__fma_rn(a, b.v, c), a * b.d); }
+__device__ __forceinline__ Dual fmaR(const Dual& a, double b, double c) { return fmaR(b, a, c); }
+__device__ __forceinline__ Dual fmaR(const Dual& a, const Dual& b, double c) {
+  return Dual(__fma_rn(a.v, b.v, c), __fma_rn(a.d, b.v, a.v * b.d));
+}
+__device__ __forceinline__ Dual per_dt(const Dual& q, const Divisor& dt, double) {
+  return Dual(div_rn(q.v, dt), div_rn(q.d, dt));
 }
 __device__ __forceinline__ Dual sqrtR(const Dual& x) {
   const double s = soft_sqrt(x.v);

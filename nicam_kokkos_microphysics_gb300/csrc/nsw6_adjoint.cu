@@ -189,6 +189,22 @@ struct In<RVar> {
   __device__ RVar x(int a, size_t i) const { return put(LK_X, a, i, io.x.a[a][i]); }
 };
 
+// Forward mode: the stored value and its tangent.
+template <>
+struct In<Dual> {
+  const StageIO& io;
+  int l, g;
+  __device__ Dual w(int f, int kk) const {
+    const size_t i = f * io.NC + io.L.f(l, kk, g);
+    return Dual(io.W[i], io.WB[i]);
+  }
+  __device__ Dual y(int f, int kk) const {
+    const size_t i = f * io.NC + io.L.f(l, kk, g);
+    return Dual(io.Y[i], io.YB[i]);
+  }
+  __device__ Dual x(int a, size_t i) const { return Dual(io.x.a[a][i], io.xb.a[a][i]); }
+};
+
 // State fields the column phase reads: the cell phase's output at interior
 // levels, the caller's array at the halo levels.
 template <class T>
@@ -759,7 +775,8 @@ __global__ void adj_bounds_kernel(Problem P, int* bnd) {
 // departure distances over the region (vadv1d_prep, mod_vadv1d.cpp:316-353)
 // reduce within the block: one 64-bit atomic per block and row, on
 // order-preserving keys (exact, independent of the order of the atomics).
-template <bool MIX>
+// T = Dual: S1 in forward mode, the tangents of its outputs into WB.
+template <bool MIX, class T = double>
 __global__ void __launch_bounds__(STAGE_THREADS) adj_s1_fwd_kernel(StageIO io) {
   __shared__ double grid[GF_COUNT * MAX_KALL];
   __shared__ float grf[MIX ? 4 * MAX_KALL : 1];   // MIX: rdgz, rdgzh, rdzs, rdzsh in FP32
@@ -777,12 +794,13 @@ __global__ void __launch_bounds__(STAGE_THREADS) adj_s1_fwd_kernel(StageIO io) {
   double z[2 * MAX_TR] = {0, 0, 0, 0, 0, 0, 0, 0};
   if (valid) {
     const size_t c = io.L.f(l, k, g);
-    const In<double> in{io, l, g};
-    stage1<double, MIX>(
+    const In<T> in{io, l, g};
+    stage1<T, MIX>(
         in, grid, k,
-        [&](int f, double v) {
-          io.W[f * io.NC + c] = v;
-          if (f < nrow) z[f] = v;
+        [&](int f, const T& v) {
+          io.W[f * io.NC + c] = val(v);
+          if constexpr (std::is_same<T, Dual>::value) io.WB[f * io.NC + c] = v.d;
+          if (f < nrow) z[f] = val(v);
         },
         grf);
   }
@@ -2045,26 +2063,11 @@ __global__ void __launch_bounds__(128) adj_cell_hw_kernel(Problem P, ConstsT<R> 
 // The same stages in forward mode (T = Dual): every cell of every column in
 // parallel.  StageIO's adjoint arrays hold the tangents here: xb the step's
 // argument tangents (read as inputs, written as outputs), YB the cell
-// outputs' tangents, WB the work fields' tangents.  The values of the work
-// fields and the flux bounds come from the forward kernels above.  The last
-// two stages also write the step's output values: the stage functions make
+// outputs' tangents, WB the work fields' tangents.  Each stage writes values
+// and tangents: the forward kernels above beside them were 190 of 1690 us at
+// 4096 columns.  The last two stages also write the step's output values: the stage functions make
 // the production kernels' operations on the same values, so they are those
 // kernels' outputs bit for bit (tested against the step).
-template <>
-struct In<Dual> {
-  const StageIO& io;
-  int l, g;
-  __device__ Dual w(int f, int kk) const {
-    const size_t i = f * io.NC + io.L.f(l, kk, g);
-    return Dual(io.W[i], io.WB[i]);
-  }
-  __device__ Dual y(int f, int kk) const {
-    const size_t i = f * io.NC + io.L.f(l, kk, g);
-    return Dual(io.Y[i], io.YB[i]);
-  }
-  __device__ Dual x(int a, size_t i) const { return Dual(io.x.a[a][i], io.xb.a[a][i]); }
-};
-
 // Cell phase in forward mode: the FP64 cell physics over Dual (parameter
 // tangents through the folded constants), its outputs' values into Y and
 // tangents into YB.  The constants (one copy per block) sit in shared memory.
@@ -2072,8 +2075,8 @@ template <bool OPT>
 __global__ void __launch_bounds__(128) tlm_cell_kernel(StageIO io, Consts C, const double* params,
                                                        const double* dparams) {
   __shared__ double tab[FM_TABLE_DOUBLES];
-  __shared__ __align__(16) unsigned char ct_raw[sizeof(ConstsT<Dual>)];
-  ConstsT<Dual>& CT = *reinterpret_cast<ConstsT<Dual>*>(ct_raw);
+  __shared__ __align__(16) unsigned char ct_raw[sizeof(DualConsts)];
+  DualConsts& CT = *reinterpret_cast<DualConsts*>(ct_raw);
   const Problem& P = io.P;
   for (int c = threadIdx.x; c < FM_TABLE_DOUBLES; c += blockDim.x) tab[c] = P.fmtab[c];
   if (threadIdx.x == 0) {
@@ -2126,19 +2129,6 @@ __global__ void __launch_bounds__(128) tlm_cell_kernel(StageIO io, Consts C, con
   }
 }
 
-// S1 in forward mode: the work fields' tangents.
-__global__ void __launch_bounds__(STAGE_THREADS) tlm_s1_kernel(StageIO io) {
-  __shared__ double grid[GF_COUNT * MAX_KALL];
-  for (int c = threadIdx.x; c < GF_COUNT * io.P.kall; c += blockDim.x) grid[c] = io.P.grid[c];
-  __syncthreads();
-  for (size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x; c < io.NC; c += (size_t)gridDim.x * blockDim.x) {
-    int g, k, l;
-    io.L.split(c, l, k, g);
-    const In<Dual> in{io, l, g};
-    stage1<Dual>(in, grid, k, [&](int f, const Dual& v) { io.WB[f * io.NC + c] = v.d; });
-  }
-}
-
 // S2 in forward mode (a work item per cell and flux).
 __global__ void __launch_bounds__(STAGE_THREADS) tlm_s2_kernel(StageIO io) {
   __shared__ double grid[GF_COUNT * MAX_KALL];
@@ -2150,12 +2140,14 @@ __global__ void __launch_bounds__(STAGE_THREADS) tlm_s2_kernel(StageIO io) {
       int g, k, l;
       io.L.split(c, l, k, g);
       const In<Dual> in{io, l, g};
-      io.WB[(W_F + j) * io.NC + c] = stage2<Dual>(in, grid, k, j).d;
+      const Dual F = stage2<Dual>(in, grid, k, j);
+      io.W[(W_F + j) * io.NC + c] = F.v;
+      io.WB[(W_F + j) * io.NC + c] = F.d;
     }
 }
 
-// S3 in forward mode: work-field tangents, and the values and tangents of the
-// step's momentum, GPREC and surface outputs.
+// S3 in forward mode: the work fields, and the step's momentum, GPREC and
+// surface outputs.
 __global__ void __launch_bounds__(STAGE_THREADS) tlm_s3_kernel(StageIO io) {
   __shared__ double grid[GF_COUNT * MAX_KALL];
   for (int c = threadIdx.x; c < GF_COUNT * io.P.kall; c += blockDim.x) grid[c] = io.P.grid[c];
@@ -2175,7 +2167,11 @@ __global__ void __launch_bounds__(STAGE_THREADS) tlm_s3_kernel(StageIO io) {
     // GPREC: from the surface-ward flux at the interior levels, 0 elsewhere
     if (k < io.P.kmin || k > io.P.kmax) out(A_GPREC, c, Dual(0.0));
     stage3<Dual>(
-        in, grid, k, [&](int f, const Dual& v) { io.WB[f * io.NC + c] = v.d; },
+        in, grid, k,
+        [&](int f, const Dual& v) {
+          io.W[f * io.NC + c] = v.v;
+          io.WB[f * io.NC + c] = v.d;
+        },
         [&](int f, const Dual& v) {
           if (io.kin2kin && f != SF_GPREC) return;   // S4 gives the momenta
           const int a = f == SF_RVX ? A_rhogvx : f == SF_RVY ? A_rhogvy : f == SF_RVZ ? A_rhogvz
@@ -2280,9 +2276,9 @@ cudaError_t launch_adj_cell_hw(const Problem& P, const Consts& C, const ArgPtrs&
 }
 
 // The tangent-linear step in stages: the cell phase in forward mode (Y and
-// its tangents), the column phase's forward values and flux bounds, then its
-// stages in forward mode writing the step's outputs into x and their tangents
-// into dx.  Y holds 2 x ADJ_Y_FIELDS fields (values, tangents); work as for
+// its tangents), S1 in forward mode and the flux bounds its values give, then
+// the other stages, the last two writing the step's outputs into x and their
+// tangents into dx.  Y holds 2 x ADJ_Y_FIELDS fields (values, tangents); work as for
 // the adjoint.
 cudaError_t launch_tlm_staged(const Problem& P, const Consts& C, const ArgPtrs& x, const ArgPtrs& dx,
                               const double* params, const double* dparams, double* Y, double* work, int* bnd,
@@ -2308,12 +2304,9 @@ cudaError_t launch_tlm_staged(const Problem& P, const Consts& C, const ArgPtrs& 
     tlm_cell_kernel<true><<<152 * 4, 128, 0, stream>>>(io, C, params, dparams);
   else
     tlm_cell_kernel<false><<<152 * 4, 128, 0, stream>>>(io, C, params, dparams);
-  adj_s1_fwd_kernel<false><<<dim3((P.gall + STAGE_THREADS - 1) / STAGE_THREADS, P.kall, P.lall), STAGE_THREADS, 0, stream>>>(
-      io);
+  const dim3 levels((P.gall + STAGE_THREADS - 1) / STAGE_THREADS, P.kall, P.lall);
+  adj_s1_fwd_kernel<false, Dual><<<levels, STAGE_THREADS, 0, stream>>>(io);
   adj_bounds_kernel<<<(int)((nkey + 127) / 128), 128, 0, stream>>>(P, bnd);
-  adj_s2_fwd_kernel<<<152 * 8, STAGE_THREADS, 0, stream>>>(io);
-  adj_s3_fwd_kernel<<<152 * 8, STAGE_THREADS, 0, stream>>>(io);
-  tlm_s1_kernel<<<152 * 8, STAGE_THREADS, 0, stream>>>(io);
   tlm_s2_kernel<<<152 * 8, STAGE_THREADS, 0, stream>>>(io);
   tlm_s3_kernel<<<152 * 8, STAGE_THREADS, 0, stream>>>(io);
   tlm_s4_kernel<<<152 * 4, STAGE_THREADS, 0, stream>>>(io, C);

@@ -43,6 +43,13 @@
 
 namespace nsw6 {
 
+// Of the scalar R: the type of what has no derivative, and the scheme constants.
+template <class R>
+struct ScalarOf {
+  using constant = R;
+  using consts = ConstsT<R>;
+};
+
 template <class D>
 struct CellInT {
   D rhog, tem, gsgam2, q0;
@@ -205,8 +212,9 @@ __device__ __forceinline__ int sat_screen_liq(double tem, double rho, double qsu
 // tangent-linear and adjoint kernels instantiate R = D with their derivative
 // types (nsw6_ad.cuh).
 template <class M, class R, class D = double, bool OPT = false>
-__device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, double dt, double rdt,
+__device__ __forceinline__ void nsw6_cell(const typename ScalarOf<R>::consts& C, const M& mth, double dt, double rdt,
                                           const CellInT<D>& in, CellOutT<D>& o) {
+  using K = typename ScalarOf<R>::constant;
   constexpr bool kMixed = sizeof(R) == sizeof(float);
   // The plain FP64 step leaves out what an absent species or the other side of
   // 0 C makes an exact zero: x + 0 and 0 x need no FP64 instruction (16 to 19
@@ -223,7 +231,7 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
   auto only = [] {
     if constexpr (kPlain) soft_branch();
   };
-  const R dtR = R(dt), rdtR = R(rdt);
+  const K dtR = K(dt), rdtR = K(rdt);
   // ---- negative_filter, mod_mp_nsw6.cpp:1770-1831
   D rq[6];
 #pragma unroll
@@ -278,7 +286,7 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
     R qdR = R(1.0);
 #pragma unroll
     for (int n = 1; n <= 5; ++n) qdR = qdR - R(qn[n]);
-    pre = densR * (qdR * R(RDRY) + R(qn[0]) * R(RVAP)) * R(temp);
+    pre = densR * (qdR * K(RDRY) + R(qn[0]) * K(RVAP)) * R(temp);
   } else {
     const D dens = quo(rhog, in.gsgam2);
     D qd = D(1.0);
@@ -305,7 +313,7 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
   const R qi = maxz(R(qn[3])), qs = maxz(R(qn[4])), qg = maxz(R(qn[5]));
   const bool hc = nz(qc), hr = nz(qr), hi = nz(qi), hs = nz(qs), hg = nz(qg);   // the species the cell holds
   const R tempR = R(temp);
-  const R temc = tempR - R(TEM00);
+  const R temc = tempR - K(TEM00);
   const bool warm = !lt_z(temc);  // iceflg = 0.5 - copysign(0.5, temc) == 0
   const bool cold = !warm;        // iceflg == 1
   const bool wcold = !kPlain || cold, wwarm = !kPlain || warm;   // work for cold (warm) cells
@@ -315,33 +323,33 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
   R rtem = Z, rdrt = Z, qsatl = Z, qsati = Z, Sliq = Z, Sice = Z;
   if (hr || wcold) {
     only();
-    rtem = quo(R(1.0), maxc(tempR, R(TEM_MIN)));
-    rdrt = quo(R(1.0), densR * R(RVAP) * tempR);
+    rtem = quo(K(1.0), maxc(tempR, R(TEM_MIN)));
+    rdrt = quo(K(1.0), densR * K(RVAP) * tempR);
   }
   if (hr) {
     only();
-    const R psatl = R(PSAT0) * mth.exp(C.LovR_liq * (C.RTEM00 - rtem));
+    const R psatl = K(PSAT0) * mth.exp(C.LovR_liq * (C.RTEM00 - rtem));
     qsatl = psatl * rdrt;
     Sliq = quo(qv, maxc(qsatl, R(EPS)));
   }
   if (wcold) {
     only();
-    const R psati = R(PSAT0) * mth.exp(C.LovR_ice * (C.RTEM00 - rtem));
+    const R psati = K(PSAT0) * mth.exp(C.LovR_ice * (C.RTEM00 - rtem));
     qsati = psati * rdrt;
     Sice = quo(qv, maxc(qsati, R(EPS)));
   }
 
   // ---- TagBigLoop, mod_mp_nsw6.cpp:902-1594
-  const R Rdens = quo(ONE, densR);
+  const R Rdens = quo(K(1.0), densR);
   R rho_fact = Z;
   if (hr || hs || hg) {
     only();
-    rho_fact = sqrtR(R(DENS00) * Rdens);
+    rho_fact = sqrtR(K(DENS00) * Rdens);
   }
   const bool d1 = ge_c(qr, R(1.0E-4));                          // delta1
   const bool d2 = le_c(qr, R(1.0E-4)) && le_c(qs, R(1.0E-4));       // delta2
   const bool sps = ge_c(Sice, ONE);                              // spsati
-  const DivisorT<R> by_dt(dtR);
+  const DivisorT<K> by_dt(dtR);
   R dqv_dt = Z, dqc_dt = Z, dqr_dt = Z, dqi_dt = Z, dqs_dt = Z, dqg_dt = Z;
   if (hr || wcold) dqv_dt = per_dt(qv, by_dt, rdtR);   // (no other cell uses it)
   if (hc) dqc_dt = per_dt(qc, by_dt, rdtR);
@@ -414,8 +422,8 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
     const R logX = mth.log(Xs2);
 #pragma unroll
     for (int i = 0; i < 7; ++i) {
-      const R* a = C.roh_a + 4 * i;
-      const R* b = C.roh_b + 4 * i;
+      const K* a = C.roh_a + 4 * i;
+      const K* b = C.roh_b + 4 * i;
       const R la = fmaR(fmaR(fmaR(a[3], tems, a[2]), tems, a[1]), tems, a[0]);
       const R lb = fmaR(fmaR(fmaR(b[3], tems, b[2]), tems, b[1]), tems, b[0]);
       mom[i] = mth.exp(fmaR(logX, lb, la));
@@ -457,12 +465,12 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
   R Vti = Z;
   if constexpr (OPT) {
     // :1073-1075 with sw_constVti = 0 (CONST_Vti is UNDEF)
-    if (C.opt_qised != Z && qi >= R(1.0E-8)) Vti = R(-3.29) * mth.exp(mth.log(densR * qi) * R(0.16));
+    if (C.opt_qised != Z && qi >= R(1.0E-8)) Vti = K(-3.29) * mth.exp(mth.log(densR * qi) * K(0.16));
   }
   // cloud number (TagAerosolT / TagAerosolF, :676-684)
   R Nc = C.Nc_def;
   if constexpr (OPT) {
-    if (C.opt_indir != Z) Nc = dmax(R(in.unccn) * R(1.0E-6), C.Nc_def);
+    if (C.opt_indir != Z) Nc = dmax(R(in.unccn) * K(1.0E-6), C.Nc_def);
   }
 
   // nucleation, :1080-1085: Ni0 = max(exp(-0.1 temc), 1) * 1000 and
@@ -470,7 +478,7 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
   R Pigen = Z;
   if (wcold) {
     only();
-    const R Qi0 = C.ice_nuc * mth.exp(R(1.33) * (C.ln1000 + maxz(R(-0.1) * temc))) * Rdens;
+    const R Qi0 = C.ice_nuc * mth.exp(K(1.33) * (C.ln1000 + maxz(K(-0.1) * temc))) * Rdens;
     Pigen = maxz(dmin(Qi0 - qi, qv - qsati)) * rdtR;
   }
 
@@ -493,7 +501,7 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
     only();
     const R qcqr = qc * qr;
     if (kk) {
-      if (ge_c(qcqr, R(1.0E-12))) Pracw = R(67.0) * mth.pow(qcqr, R(1.15));
+      if (ge_c(qcqr, R(1.0E-12))) Pracw = K(67.0) * mth.pow(qcqr, R(1.15));
     } else {
       Pracw = qc * C.K_raci * RLMDr_3dr * fr;   // Pracw_orig (Erw = Eri = 1)
     }
@@ -520,7 +528,7 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
     const R dvrs = fabsR(Vtr - Vts);
     Psacr = C.K_sacr * Rdens * dvrs *
             (C.GAM_1br * RLMDr_1br * MOMs_2 + C.K_2gam2br * RLMDr_2br * MOMs_1 + C.GAM_3br * RLMDr_3br * MOMs_0);
-    Pracs = C.K_racs * Rdens * dvrs * (R(2.0) * MOMs_0bs * RLMDr_3 + R(2.0) * MOMs_1bs * RLMDr_2 + MOMs_2bs * RLMDr);
+    Pracs = C.K_racs * Rdens * dvrs * (K(2.0) * MOMs_0bs * RLMDr_3 + K(2.0) * MOMs_1bs * RLMDr_2 + MOMs_2bs * RLMDr);
   }
   if (hr && hg) {
     only();
@@ -541,7 +549,7 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
     if (hs && hg) {
       only();
       Pgacs = C.K_gacs * Rdens * Egs_mod * fabsR(Vtg - Vts) *
-            (R(2.0) * MOMs_0bs * RLMDg_3 + R(2.0) * MOMs_1bs * RLMDg_2 + MOMs_2bs * RLMDg);
+            (K(2.0) * MOMs_0bs * RLMDg_3 + K(2.0) * MOMs_1bs * RLMDg_2 + MOMs_2bs * RLMDg);
     }
   }
 
@@ -549,7 +557,7 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
   R rhoqc = Z;
   if (hc) {
     only();
-    rhoqc = densR * qc * R(1000.0);
+    rhoqc = densR * qc * K(1000.0);
   }
   R Praut = Z;   // K_aut * pow(0, 2.47) = 0
   if (kk) {
@@ -563,9 +571,9 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
     // Berry (1968), :1145-1147
     R Dc = C.Dc_berry;
     if constexpr (OPT) {
-      if (C.opt_indir != Z) Dc = R(0.146) - R(5.964E-2) * mth.log(quo(Nc, R(2000.0)));
+      if (C.opt_indir != Z) Dc = K(0.146) - K(5.964E-2) * mth.log(quo(Nc, R(2000.0)));
     }
-    Praut = quo(Rdens * R(1.67E-5) * rhoqc * rhoqc, R(5.0) + quo(R(3.66E-2) * Nc, Dc * rhoqc + R(EPS)));
+    Praut = quo(Rdens * K(1.67E-5) * rhoqc * rhoqc, K(5.0) + quo(K(3.66E-2) * Nc, Dc * rhoqc + K(EPS)));
   }
   R Psaut = Z;   // (without ice the limiter dqi_dt = 0 below would hold it there)
   if (hi) {
@@ -578,21 +586,21 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
   R Ka = Z, KdD = Z, rKaT = Z, Giv = Z, Gil = Z, rNu = Z;
   if (falls || wcold) {
     only();
-    Ka = R(2.428E-2) + R(7.47E-5) * temc;
+    Ka = K(2.428E-2) + K(7.47E-5) * temc;
   }
   if (hr || wcold) {
     only();
-    KdD = quo((R(2.222E-5) + R(1.37E-7) * temc) * R(PSTD), pre) * densR;   // Kd * dens
-    rKaT = quo(ONE, Ka * tempR);
+    KdD = quo((K(2.222E-5) + K(1.37E-7) * temc) * K(PSTD), pre) * densR;   // Kd * dens
+    rKaT = quo(K(1.0), Ka * tempR);
   }
   if (falls) {
     only();
-    rNu = quo(densR, R(1.718E-5) + R(5.28E-8) * temc);   // 1 / Nu
+    rNu = quo(densR, K(1.718E-5) + K(5.28E-8) * temc);   // 1 / Nu
   }
   if (wcold) {
     only();
     const R xi = KdD * qsati;
-    Giv = quo(xi, R(LHS0) * rKaT * (C.LovR_ice * rtem - ONE) * xi + ONE);
+    Giv = quo(xi, K(LHS0) * rKaT * (C.LovR_ice * rtem - K(1.0)) * xi + K(1.0));
   }
   if ((hs || hg) && wwarm) {
     only();
@@ -602,9 +610,9 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
   if (rain) {
     only();
     const R xl = KdD * qsatl;
-    const R Glv = quo(xl, R(LHV0) * rKaT * (C.LovR_liq * rtem - ONE) * xl + ONE);
+    const R Glv = quo(xl, K(LHV0) * rKaT * (C.LovR_liq * rtem - K(1.0)) * xl + K(1.0));
     const R ventr = C.K_ventr1 * RLMDr_2 + C.K_ventr2 * sqrtR(C.Cr * fr * rNu * RLMDr_5dr);
-    Prevp = C.K_revp * Rdens * (ONE - minc(Sliq, ONE)) * Glv * ventr;
+    Prevp = C.K_revp * Rdens * (K(1.0) - minc(Sliq, ONE)) * Glv * ventr;
   }
   // deposition and sublimation of ice (cold cells: the limiters keep it there)
   R tmp, Pidep = Z, Pisub = Z;
@@ -618,20 +626,20 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
     // with no ice, rhoqi = EPS and XNi, Di take the constant values folded on the host
     R XNi = C.XNi_eps, Di = C.Di_eps;
     if (gt_c(rhoqi, R(EPS))) {
-      XNi = minc(maxc(R(5.38E+7) * mth.pow(rhoqi, R(0.75)), R(1.0E+3)), R(1.0E+6));
+      XNi = minc(maxc(K(5.38E+7) * mth.pow(rhoqi, R(0.75)), R(1.0E+3)), R(1.0E+6));
       const R XMi = quo(rhoqi, XNi);
-      Di = minc(C.Di_a * sqrtR(XMi), C.Di_max);
+      Di = minc(C.Di_a * sqrtR(XMi), R(C.Di_max));
     }
-    tmp = R(4.0) * Di * XNi * Rdens * (Sice - ONE) * Giv;
+    tmp = K(4.0) * Di * XNi * Rdens * (Sice - K(1.0)) * Giv;
     Pidep = sel(sps, tmp);
     Pisub = sel(!sps, -tmp);
   }
-  const bool below40 = lt_z(temc + R(40.0));
+  const bool below40 = lt_z(temc + K(40.0));
   R Pihom = below40 ? dqc_dt : Z;
   R efrz = Z;
   if ((hc || hr) && wcold) {
     only();
-    efrz = mth.exp(-C.A_frz * temc) - ONE;
+    efrz = mth.exp(-C.A_frz * temc) - K(1.0);
   }
   R Pihtr = Z;
   if (hc && !below40 && !warm) {
@@ -644,12 +652,12 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
   R vents = Z, ventg = Z;
   if (hs && !(is_zero(MOMs_1) && is_zero(MOMs_5ds_h))) {
     only();
-    vents = R(0.65) * MOMs_1 + C.K_vents2 * sqrtR(fr * rNu) * MOMs_5ds_h;
+    vents = K(0.65) * MOMs_1 + C.K_vents2 * sqrtR(fr * rNu) * MOMs_5ds_h;
   }
   R Psdep = Z, Pssub = Z, Psmlt = Z;
   if (hs && wcold) {
     only();
-    tmp = C.K_2pi * Rdens * (Sice - ONE) * Giv * vents;
+    tmp = C.K_2pi * Rdens * (Sice - K(1.0)) * Giv * vents;
     Psdep = sel(sps, tmp);
     Pssub = sel(!sps, -tmp);
   }
@@ -664,7 +672,7 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
   R Pgdep = Z, Pgsub = Z, Pgmlt = Z, Pgfrz = Z;
   if (hg && wcold) {
     only();
-    tmp = C.K_gdep * Rdens * (Sice - ONE) * Giv * ventg;
+    tmp = C.K_gdep * Rdens * (Sice - K(1.0)) * Giv * ventg;
     Pgdep = sel(sps, tmp);
     Pgsub = sel(!sps, -tmp);
   }
@@ -683,14 +691,14 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
   const bool expice = !OPT || C.opt_expice != Z;
   R Psfw = Z, Psfi = Z;
   if constexpr (OPT) {
-    if (hi && !expice && cold && !(temc + R(30.0) < Z)) {
+    if (hi && !expice && cold && !(temc + K(30.0) < Z)) {
       only();
       const R tb = dmin(dmax(temc, R(-30.99)), Z);
       const int it = int(-val_of(tb));   // the table row: piecewise constant in tb
       const R fact = -(tb + R(it - 1));
-      const R a2 = (ONE - fact) * C.berg_a2[it] + fact * C.berg_a2[it + 1];
+      const R a2 = (K(1.0) - fact) * C.berg_a2[it] + fact * C.berg_a2[it + 1];
       const R ma2 = ONE - a2;
-      const R a1 = ((ONE - fact) * C.berg_a1[it] + fact * C.berg_a1[it + 1]) * mth.pow(R(1.0E-3), ma2);
+      const R a1 = ((K(1.0) - fact) * C.berg_a1[it] + fact * C.berg_a1[it + 1]) * mth.pow(R(1.0E-3), ma2);
       const R dt1 = quo(mth.exp(C.log_mi50 * ma2) - mth.exp(C.log_mi40 * ma2), a1 * ma2);
       const R Ni50 = quo(qi * dtR, C.mi50 * dt1);
       Psfw = Ni50 * (a1 * mth.pow(C.mi50, a2) + C.K_berg_w * densR * qc);
@@ -763,7 +771,7 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
   auto limiter = [&](R net, R dq) {
     if (kPlain && is_nonneg(net)) return ONE;
     only();
-    return is_nonneg(net + R(EPS)) ? ONE : minc(quo(-dq, net), ONE);
+    return is_nonneg(net + K(EPS)) ? ONE : minc(quo(-dq, net), ONE);
   };
   // Scaling by fac = 1 is exact and skipped.  The tendencies below are the
   // nets the limiters form (same terms, same order) where no later scaling
@@ -1086,10 +1094,10 @@ __device__ __forceinline__ void nsw6_cell(const ConstsT<R>& C, const M& mth, dou
     if constexpr (OPT) {
       if (C.opt_indir != Z) {
         K_xf = quo(R(1.0E-9), Nc);
-        K_r2c = C.coef_dgam * (Nc * R(1.0E+6));
+        K_r2c = C.coef_dgam * (Nc * K(1.0E+6));
       }
     }
-    const R rf_qc = mth.pow(C.coef_xf * (rhoqc * K_xf) + R(EPS), R(0.33333333));
+    const R rf_qc = mth.pow(C.coef_xf * (rhoqc * K_xf) + K(EPS), R(0.33333333));
     const R r2_qc = K_r2c * (rf_qc * rf_qc);
     const R r2_qr = C.K_r2r * RLMDr_3;
     const R r3_qc = C.coef_xf * densR * qc;

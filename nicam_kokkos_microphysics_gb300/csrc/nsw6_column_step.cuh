@@ -55,10 +55,14 @@ struct ColWork {
 // (beta_saut, qicrt_saut, Cr, Cs, Cg, ice_nuc, kk_aut); values as built on the
 // host, derivatives of the factors folded from them (make_consts).
 template <class T>
-__device__ __forceinline__ void consts_with_params(const Consts& c, const T* p, ConstsT<T>& r) {
-  const double* src = reinterpret_cast<const double*>(&c);
-  T* dst = reinterpret_cast<T*>(&r);
-  for (size_t i = 0; i < sizeof(Consts) / sizeof(double); ++i) dst[i] = T(src[i]);
+__device__ __forceinline__ void consts_with_params(const Consts& c, const T* p, typename ScalarOf<T>::consts& r) {
+  if constexpr (std::is_same<T, Dual>::value) {
+    static_cast<Consts&>(r) = c;
+  } else {
+    const double* src = reinterpret_cast<const double*>(&c);
+    T* dst = reinterpret_cast<T*>(&r);
+    for (size_t i = 0; i < sizeof(Consts) / sizeof(double); ++i) dst[i] = T(src[i]);
+  }
   r.beta_saut = p[0];
   r.qicrt_saut = p[1];
   r.Cr = p[2];
@@ -343,7 +347,7 @@ __device__ __forceinline__ int satadjust_all_t(const Consts& C, const FastMath& 
 // The cell phase of one column: nsw6_cell on every interior level (as
 // nsw6_cell_kernel), leaving the fall speeds in w.vt.
 template <class T, class M>
-__device__ void column_cell_phase(const ConstsT<T>& CT, const M& mth, int K, double dt, double rdt,
+__device__ void column_cell_phase(const typename ScalarOf<T>::consts& CT, const M& mth, int K, double dt, double rdt,
                                   ColState<T>& s, ColWork<T>& w) {
   const int kmin = 1, kmax = K - 2;
   for (int t = 0; t < 3; ++t)
@@ -392,7 +396,7 @@ __device__ void column_transport_phase(const Consts& C, const FastMath& fm, cons
 // (values), CT: the same as T (with the parameter derivatives).  err: first
 // error of the column.
 template <class T, class M>
-__device__ void column_step(const ConstsT<T>& CT, const Consts& C, const M& mth, const FastMath& fm,
+__device__ void column_step(const typename ScalarOf<T>::consts& CT, const Consts& C, const M& mth, const FastMath& fm,
                             const double* gr, int K, double dt, double rdt, double hdt2, double sdt3, int itelim,
                             const int (*bmn)[KA], const int (*bmx)[KA], ColState<T>& s, ColWork<T>& w, int* err,
                             int* err_k, int* err_it) {

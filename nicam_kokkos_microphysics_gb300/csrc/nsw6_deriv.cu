@@ -163,7 +163,7 @@ __global__ void __launch_bounds__(AD_THREADS) nsw6_tlm_kernel(Problem P, Consts 
   if (g >= P.gall) return;
   Dual p[7];
   for (int i = 0; i < 7; ++i) p[i] = Dual(params[i], dparams ? dparams[i] : 0.0);
-  ConstsT<Dual> CT;
+  DualConsts CT;
   consts_with_params(C, p, CT);
   ColState<Dual> s;
   ColWork<Dual> w;
