@@ -349,36 +349,95 @@ __device__ void stage1(const In<T>& in, const double* gr, int k, const O& out, c
   }
 }
 
-// S2: flux j (tracer j / 8, source j % 8) of cell (l, k, g).
-template <class T>
-__device__ T stage2(const In<T>& in, const double* gr, int k, int j) {
-  const Problem& P = in.io.P;
-  const int K = P.kall, kmin = P.kmin, kmax = P.kmax;
-  const int t = j / 8, f = j % 8;
-  const bool full = f < 6;
-  const int mkmin = full ? kmin : kmin + 1;
-  if (k < mkmin || k > kmax) return T(0.0);
-  const int r = full ? t : P.ntr + t;
-  const int* bmn = in.io.bnd + ((size_t)in.l * 2 + 0) * 2 * MAX_TR * K;
-  const int* bmx = in.io.bnd + ((size_t)in.l * 2 + 1) * 2 * MAX_TR * K;
+// S2: the range of a cell's flux integrals of tracer t on full or half levels
+// and its departure cell (discrete, held at the forward's values); ok: the
+// level has fluxes there.
+struct FluxSpan {
+  bool ok, span;
+  int lo, hi, kc, r;
+};
+__device__ __forceinline__ FluxSpan flux_span(const StageIO& io, const double* gr, int l, int k, int t, bool half,
+                                              size_t c) {
+  const Problem& P = io.P;
+  const int K = P.kall, mkmin = half ? P.kmin + 1 : P.kmin;
+  FluxSpan s{};
+  s.ok = k >= mkmin && k <= P.kmax;
+  if (!s.ok) return s;
+  s.r = half ? P.ntr + t : t;
+  const int* bmn = io.bnd + ((size_t)l * 2 + 0) * 2 * MAX_TR * K;
+  const int* bmx = io.bnd + ((size_t)l * 2 + 1) * 2 * MAX_TR * K;
   // the integral's range: the half levels use the full-level kcell_max
   // (mod_precip_transport.cpp:890, 892)
-  const int lo = bmn[r * K + k];
-  const int hi = bmx[t * K + k];
-  const double* zh = gr + (full ? GF_GZH : GF_GZSHIFT) * K;
-  const double* dz = gr + (full ? GF_DGZ : GF_DGZH) * K;
-  const double zv = in.io.W[(W_ZDIS + r) * in.io.NC + in.io.L.f(in.l, k, in.g)];
-  const int kc = departure_cell_t(zh, k, zv, lo, bmx[r * K + k], mkmin, kmax);
-  const int src = W_RHOF + 8 * t + f;
-  T acc = T(0.0);
-  T zdis = in.w(W_ZDIS + r, k);
-  if (!(lo == k && hi == k)) {
-    for (int k2 = lo; k2 <= hi; ++k2)
-      acc = fmaR(in.w(src, k2), T(k2 > kc ? dz[k2] : (k2 < kc ? -dz[k2] : 0.0)), acc);
-    if (hi != kc) zdis = zdis - T(hi > kc ? dz[hi] : -dz[hi]);
+  s.lo = bmn[s.r * K + k];
+  s.hi = bmx[t * K + k];
+  s.span = !(s.lo == k && s.hi == k);
+  s.kc = departure_cell_t(gr + (half ? GF_GZSHIFT : GF_GZH) * K, k, io.W[(W_ZDIS + s.r) * io.NC + c], s.lo,
+                          bmx[s.r * K + k], mkmin, P.kmax);
+  return s;
+}
+
+// |acc| >= EPS (NaN: false), of the values, on the integer pipe
+__device__ __forceinline__ bool flux_kept(double acc) {
+  const unsigned long long ab = (unsigned long long)__double_as_longlong(acc) & 0x7fffffffffffffffull;
+  return ab - (unsigned long long)EPS_BITS <= 0x7ff0000000000000ull - (unsigned long long)EPS_BITS;
+}
+
+// S2: N fluxes f0 .. of tracer t (0..5 full, 6..7 half levels) of cell (l, k,
+// g); zdis: the departure distance less the last layer of the range
+// (flux_rest_t).
+template <class T>
+__device__ __forceinline__ T flux_rest_t(const In<T>& in, const double* dz, int k, const FluxSpan& s) {
+  T zdis = in.w(W_ZDIS + s.r, k);
+  if (s.span && s.hi != s.kc) zdis = zdis - (s.hi > s.kc ? dz[s.hi] : -dz[s.hi]);
+  return zdis;
+}
+template <int N, class T>
+__device__ __forceinline__ void stage2_fluxes(const In<T>& in, const double* dz, int t, int f0, const FluxSpan& s,
+                                              const T& zdis, T (&acc)[N]) {
+  const int src = W_RHOF + 8 * t + f0;
+#pragma unroll
+  for (int f = 0; f < N; ++f) acc[f] = T(0.0);
+  if (s.span)
+#pragma unroll 1
+    for (int k2 = s.lo; k2 <= s.hi; ++k2) {
+      const double w = k2 > s.kc ? dz[k2] : (k2 < s.kc ? -dz[k2] : 0.0);
+#pragma unroll
+      for (int f = 0; f < N; ++f) acc[f] = fmaR(in.w(src + f, k2), w, acc[f]);
+    }
+#pragma unroll
+  for (int f = 0; f < N; ++f) {
+    acc[f] = fmaR(in.w(src + f, s.kc), zdis, acc[f]);
+    if (!flux_kept(val(acc[f]))) acc[f] = T(0.0);
   }
-  acc = fmaR(in.w(src, kc), zdis, acc);
-  return fabsR(acc) >= T(EPS) ? acc : T(0.0);
+}
+// flux j = 8 t + f by itself (the recorded form)
+template <class T>
+__device__ T stage2(const In<T>& in, const double* gr, int k, int j) {
+  const int t = j / 8, f = j % 8;
+  const bool half = f >= 6;
+  const FluxSpan s = flux_span(in.io, gr, in.l, k, t, half, in.io.L.f(in.l, k, in.g));
+  if (!s.ok) return T(0.0);
+  const double* dz = gr + (half ? GF_DGZH : GF_DGZ) * in.io.P.kall;
+  T F[1];
+  stage2_fluxes(in, dz, t, f, s, flux_rest_t(in, dz, k, s), F);
+  return F[0];
+}
+// the eight fluxes of tracer t, which share the departure cells: o(f, flux)
+template <class T, class O>
+__device__ __forceinline__ void stage2_tracer(const In<T>& in, const double* gr, int k, int t, size_t c, const O& o) {
+  auto level = [&](auto& F, bool half) {
+    constexpr int N = sizeof(F) / sizeof(T);
+    const FluxSpan s = flux_span(in.io, gr, in.l, k, t, half, c);
+    const double* dz = gr + (half ? GF_DGZH : GF_DGZ) * in.io.P.kall;
+#pragma unroll
+    for (int f = 0; f < N; ++f) F[f] = T(0.0);
+    if (s.ok) stage2_fluxes(in, dz, t, half ? 6 : 0, s, flux_rest_t(in, dz, k, s), F);
+#pragma unroll
+    for (int f = 0; f < N; ++f) o((half ? 6 : 0) + f, F[f]);
+  };
+  T F[6], H[2];
+  level(F, false);
+  level(H, true);
 }
 
 // S3: divergences, surface fluxes and the updated state of cell (l, k, g).
@@ -836,18 +895,20 @@ __global__ void __launch_bounds__(STAGE_THREADS) adj_s1_fwd_kernel(StageIO io) {
   }
 }
 
-// Forward of S2 (a work item per cell and flux).
+// Forward of S2: a work item per cell and tracer.  Bound by the integer work of
+// the departure cells, which the tracer's fluxes share: an item per flux, its
+// heights compared on the FP64 pipe, took 57 us at 4096 x 42 cells, this 30
+// (in forward mode 77 -> 43 us, the reverse sweep 73 -> 46 us).
 __global__ void __launch_bounds__(STAGE_THREADS) adj_s2_fwd_kernel(StageIO io) {
   __shared__ double grid[GF_COUNT * MAX_KALL];
   for (int c = threadIdx.x; c < GF_COUNT * io.P.kall; c += blockDim.x) grid[c] = io.P.grid[c];
   __syncthreads();
-  const int nj = 8 * io.P.ntr;
-  for (int j = 0; j < nj; ++j)
+  for (int t = 0; t < io.P.ntr; ++t)
     for (size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x; c < io.NC; c += (size_t)gridDim.x * blockDim.x) {
       int g, k, l;
       io.L.split(c, l, k, g);
       const In<double> in{io, l, g};
-      io.W[(W_F + j) * io.NC + c] = stage2<double>(in, grid, k, j);
+      stage2_tracer<double>(in, grid, k, t, c, [&](int f, double F) { io.W[(W_F + 8 * t + f) * io.NC + c] = F; });
     }
 }
 
@@ -1755,52 +1816,48 @@ __global__ void __launch_bounds__(STAGE_THREADS) adj_s2_hw_kernel(StageIO io) {
   for (int i = threadIdx.x; i < GF_COUNT * io.P.kall; i += blockDim.x) grid[i] = io.P.grid[i];
   __syncthreads();
   const Problem& P = io.P;
-  const int K = P.kall, kmin = P.kmin, kmax = P.kmax;
+  const int K = P.kall, ntr = P.ntr;
   const size_t NC = io.NC, G = io.L.G;
-  const int ntr = P.ntr;
-  const size_t n = NC * ntr;
-  for (size_t w = (size_t)blockIdx.x * blockDim.x + threadIdx.x; w < n; w += (size_t)gridDim.x * blockDim.x) {
-    const size_t c = w % NC;
-    const int t = (int)(w / NC);
-    const int k = (int)((c / G) % K), l = (int)(c / (G * K));
-    if (k < kmin || k > kmax) continue;
-    const int* bmn = io.bnd + ((size_t)l * 2 + 0) * 2 * MAX_TR * K;
-    const int* bmx = io.bnd + ((size_t)l * 2 + 1) * 2 * MAX_TR * K;
-    for (int half = 0; half < 2; ++half) {
-      const int mkmin = half ? kmin + 1 : kmin;
-      if (k < mkmin) continue;
-      const int f0 = half ? 6 : 0, f1 = half ? 8 : 6;
-      bool any = false;
-      for (int f = f0; f < f1; ++f)
-        any = any || (io.WB[(W_F + 8 * t + f) * NC + c] != 0.0 && io.W[(W_F + 8 * t + f) * NC + c] != 0.0);
-      if (!any) continue;
-      const int r = half ? ntr + t : t;
-      const int lo = bmn[r * K + k];
-      const int hi = bmx[t * K + k];
-      const double* zh = grid + (half ? GF_GZSHIFT : GF_GZH) * K;
-      const double* dz = grid + (half ? GF_DGZH : GF_DGZ) * K;
-      const double zv = io.W[(W_ZDIS + r) * NC + c];
-      const int kc = departure_cell_t(zh, k, zv, lo, bmx[r * K + k], mkmin, kmax);
-      const bool span = !(lo == k && hi == k);
-      double zd = zv;
-      if (span && hi != kc) zd = zd - (hi > kc ? dz[hi] : -dz[hi]);
-      double b_z = 0.0;
-      for (int f = f0; f < f1; ++f) {
-        const double gF = io.WB[(W_F + 8 * t + f) * NC + c];
-        if (gF == 0.0 || io.W[(W_F + 8 * t + f) * NC + c] == 0.0) continue;
-        const int src = W_RHOF + 8 * t + f;
-        double* bs = io.WB + (size_t)src * NC + (c - (size_t)k * G);   // level 0 of this column
-        if (span)
-          for (int k2 = lo; k2 <= hi; ++k2) {
-            if (k2 == kc) continue;
-            atomicAdd(bs + (size_t)k2 * G, gF * (k2 > kc ? dz[k2] : -dz[k2]));
-          }
-        if (zd != 0.0) atomicAdd(bs + (size_t)kc * G, gF * zd);
-        b_z = fma(gF, io.W[(size_t)src * NC + (c - (size_t)k * G) + (size_t)kc * G], b_z);
+  for (int t = 0; t < ntr; ++t)
+    for (size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x; c < NC; c += (size_t)gridDim.x * blockDim.x) {
+      int g, k, l;
+      io.L.split(c, l, k, g);
+      if (k < P.kmin || k > P.kmax) continue;
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        const int f0 = half ? 6 : 0, nf = half ? 2 : 6;
+        double gF[6];
+        bool any = false;
+#pragma unroll
+        for (int f = 0; f < nf; ++f) {
+          // a flux below EPS was left out, and its adjoint goes nowhere
+          const double b = io.WB[(W_F + 8 * t + f0 + f) * NC + c];
+          gF[f] = fp_is_zero(io.W[(W_F + 8 * t + f0 + f) * NC + c]) ? 0.0 : b;
+          any = any || !fp_is_zero(gF[f]);
+        }
+        if (!any) continue;
+        const FluxSpan s = flux_span(io, grid, l, k, t, half, c);
+        if (!s.ok) continue;
+        const double* dz = grid + (half ? GF_DGZH : GF_DGZ) * K;
+        double zd = io.W[(W_ZDIS + s.r) * NC + c];
+        if (s.span && s.hi != s.kc) zd = zd - (s.hi > s.kc ? dz[s.hi] : -dz[s.hi]);
+        double b_z = 0.0;
+#pragma unroll
+        for (int f = 0; f < nf; ++f) {
+          if (fp_is_zero(gF[f])) continue;
+          const int src = W_RHOF + 8 * t + f0 + f;
+          double* bs = io.WB + (size_t)src * NC + (c - (size_t)k * G);   // level 0 of this column
+          if (s.span)
+            for (int k2 = s.lo; k2 <= s.hi; ++k2) {
+              if (k2 == s.kc) continue;
+              atomicAdd(bs + (size_t)k2 * G, gF[f] * (k2 > s.kc ? dz[k2] : -dz[k2]));
+            }
+          if (!fp_is_zero(zd)) atomicAdd(bs + (size_t)s.kc * G, gF[f] * zd);
+          b_z = fma(gF[f], io.W[(size_t)src * NC + (c - (size_t)k * G) + (size_t)s.kc * G], b_z);
+        }
+        io.WB[(W_ZDIS + s.r) * NC + c] += b_z;
       }
-      io.WB[(W_ZDIS + r) * NC + c] += b_z;
     }
-  }
 }
 
 // Adjoint of S1, recorded on a tape (adjoint mode 1): seeds from S2's and S3's adjoints (WB).
@@ -2129,20 +2186,20 @@ __global__ void __launch_bounds__(128) tlm_cell_kernel(StageIO io, Consts C, con
   }
 }
 
-// S2 in forward mode (a work item per cell and flux).
+// S2 in forward mode (a work item per cell and tracer).
 __global__ void __launch_bounds__(STAGE_THREADS) tlm_s2_kernel(StageIO io) {
   __shared__ double grid[GF_COUNT * MAX_KALL];
   for (int c = threadIdx.x; c < GF_COUNT * io.P.kall; c += blockDim.x) grid[c] = io.P.grid[c];
   __syncthreads();
-  const int nj = 8 * io.P.ntr;
-  for (int j = 0; j < nj; ++j)
+  for (int t = 0; t < io.P.ntr; ++t)
     for (size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x; c < io.NC; c += (size_t)gridDim.x * blockDim.x) {
       int g, k, l;
       io.L.split(c, l, k, g);
       const In<Dual> in{io, l, g};
-      const Dual F = stage2<Dual>(in, grid, k, j);
-      io.W[(W_F + j) * io.NC + c] = F.v;
-      io.WB[(W_F + j) * io.NC + c] = F.d;
+      stage2_tracer<Dual>(in, grid, k, t, c, [&](int f, const Dual& F) {
+        io.W[(W_F + 8 * t + f) * io.NC + c] = F.v;
+        io.WB[(W_F + 8 * t + f) * io.NC + c] = F.d;
+      });
     }
 }
 

@@ -145,10 +145,16 @@ __device__ __forceinline__ int departure_cell_t(const double* zh, int k, double 
     kc = k;
   } else {
     kc = 0;
+    // (compared on the integer pipe; a NaN fails every comparison)
     const double dep = zh[k] - zdis;
+    const long long dk = cmp_key(dep);
+    const bool nan = is_nan_bits(dep);
+    long long zk = cmp_key(zh[bmn]);
     for (int k2 = bmn; k2 <= bmx; ++k2) {
-      const bool s1 = dep >= zh[k2];
-      const bool s2 = zh[k2 + 1] >= dep;
+      const long long zu = cmp_key(zh[k2 + 1]);
+      const bool s1 = !nan && dk >= zk;
+      const bool s2 = !nan && zu >= dk;
+      zk = zu;
       const int tmp = (s1 == s2) ? k2 : -k2;
       kc = kc > tmp ? kc : tmp;
     }
