@@ -266,7 +266,7 @@ __device__ void stage1(const In<T>& in, const double* gr, int k, const O& out, c
   float vtf[MIX ? MAX_TR : 1][5];
   if constexpr (MIX)
     for (int t = 0; t < ntr; ++t)
-      for (int j = 0; j < 5; ++j) vtf[t][j] = float(vt[t][j]);
+      for (int j = 0; j < 5; ++j) vtf[t][j] = as<float>(vt[t][j]);
   for (int r = 0; r < 2 * ntr; ++r) {
     const int t = r % ntr, half = r / ntr;
     const int mkmin = half ? kmin + 1 : kmin;
@@ -283,7 +283,7 @@ __device__ void stage1(const In<T>& in, const double* gr, int k, const O& out, c
           auto wp = [&](int j) { return (j >= kmin + 1 && j <= kmax - 1) ? 0.5f * (col(j) + col(j - 1)) : 0.0f; };
           zf = vadv_zdis<float>(wp, grf + K, grf + 3 * K, k, mkmin, kmax, dtf, hdt2f, sdt3f);
         }
-        z = T(double(zf));
+        z = T(soft_f2d(zf));
       }
       out(W_ZDIS + r, z);
       continue;
@@ -1493,10 +1493,12 @@ __global__ void __launch_bounds__(STAGE_THREADS) adj_s1_hw_kernel(StageIO io) {
       if (fp_is_zero(bz[0]) && fp_is_zero(bz[1])) continue;
       const int fv = sed_tracer(t, ntr).vt;
       double vt[5], bvt[5] = {0.0, 0.0, 0.0, 0.0, 0.0};   // fall speeds at k - 3 .. k + 1, their adjoints
+      float vtf[5];
 #pragma unroll
       for (int j = 0; j < 5; ++j) {
         const int kk = k - 3 + j;
         vt[j] = (kk >= kmin && kk <= kmax) ? Y(fv, c + (size_t)(j - 3) * G) : 0.0;
+        if (MIX) vtf[j] = soft_d2f(vt[j]);
       }
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
@@ -1509,7 +1511,7 @@ __global__ void __launch_bounds__(STAGE_THREADS) adj_s1_hw_kernel(StageIO io) {
           float wp[4];
 #pragma unroll
           for (int d = -2; d <= 1; ++d)
-            wp[d + 2] = !half ? float(vt[d + 3]) : inside(d) ? 0.5f * (float(vt[d + 3]) + float(vt[d + 2])) : 0.0f;
+            wp[d + 2] = !half ? vtf[d + 3] : inside(d) ? 0.5f * (vtf[d + 3] + vtf[d + 2]) : 0.0f;
           auto at = [&](int j) { return j <= k - 2 ? wp[0] : j == k - 1 ? wp[1] : j == k ? wp[2] : wp[3]; };
           auto wh = [&](int j) { return vadv_wh<float>(at, j, mkmin, kmax); };
           const float wm = k > mkmin ? wh(k - 1) : 0.0f;
@@ -2015,9 +2017,15 @@ struct CellMath<float> {
 // slot-major over the cells), both from the hand-written forward.  check: also
 // evaluate nsw6_cell and report a cell whose outputs differ in any bit
 // (status ERR_ADJ_CHECK, iters = the first output field that differs).
+// The cell kernels of the derivatives hold three CTAs an SM (168 registers a
+// thread, four at 128 where the rates are FP32), which costs no spills to speak
+// of; at 255 registers and two, their warps waited for one another's FP64
+// results: 4096 x 42 cells 220 -> 190 us here, 504 -> 471 in the sweep, 457 ->
+// 420 in forward mode, 16900 x 42 in mixed precision 144 -> 102 us here.  (One
+// CTA more spills a kilobyte a thread.)
 constexpr int ERR_ADJ_CHECK = 7;
 template <class R>
-__global__ void __launch_bounds__(128) adj_cell_save_kernel(Problem P, ConstsT<R> C, ArgPtrs x, double* Y, double* ck,
+__global__ void __launch_bounds__(128, sizeof(R) == 4 ? 4 : 3) adj_cell_save_kernel(Problem P, ConstsT<R> C, ArgPtrs x, double* Y, double* ck,
                                                             int check) {
   __shared__ double tab[FM_TABLE_DOUBLES];
   if constexpr (sizeof(R) == sizeof(double)) {
@@ -2090,7 +2098,7 @@ __global__ void __launch_bounds__(128) adj_cell_save_kernel(Problem P, ConstsT<R
 // The cell phase's adjoint, hand-written, from the checkpoint ck of
 // adj_cell_save_kernel.
 template <class R>
-__global__ void __launch_bounds__(128) adj_cell_hw_kernel(Problem P, ConstsT<R> C, ArgPtrs x, ArgPtrs xb,
+__global__ void __launch_bounds__(128, 3) adj_cell_hw_kernel(Problem P, ConstsT<R> C, ArgPtrs x, ArgPtrs xb,
                                                           const double* YB, double* pbar, double* ck) {
   __shared__ double tab[FM_TABLE_DOUBLES];
   __shared__ double red[7][128];
@@ -2160,7 +2168,7 @@ __global__ void __launch_bounds__(128) adj_cell_hw_kernel(Problem P, ConstsT<R> 
 // tangents through the folded constants), its outputs' values into Y and
 // tangents into YB.  The constants (one copy per block) sit in shared memory.
 template <bool OPT>
-__global__ void __launch_bounds__(128) tlm_cell_kernel(StageIO io, Consts C, const double* params,
+__global__ void __launch_bounds__(128, 3) tlm_cell_kernel(StageIO io, Consts C, const double* params,
                                                        const double* dparams) {
   __shared__ double tab[FM_TABLE_DOUBLES];
   __shared__ __align__(16) unsigned char ct_raw[sizeof(DualConsts)];
@@ -2357,9 +2365,9 @@ int adj_stage_slots() { return 152 * 4 * STAGE_THREADS; }
 cudaError_t launch_adj_cell_hw(const Problem& P, const Consts& C, const ArgPtrs& x, const ArgPtrs& xb, const double* YB,
                                double* pbar, double* ck, int mixed, cudaStream_t stream) {
   if (mixed)
-    adj_cell_hw_kernel<float><<<152 * 2, 128, 0, stream>>>(P, consts_to_float(C), x, xb, YB, pbar, ck);
+    adj_cell_hw_kernel<float><<<152 * 3, 128, 0, stream>>>(P, consts_to_float(C), x, xb, YB, pbar, ck);
   else
-    adj_cell_hw_kernel<double><<<152 * 2, 128, 0, stream>>>(P, C, x, xb, YB, pbar, ck);
+    adj_cell_hw_kernel<double><<<152 * 3, 128, 0, stream>>>(P, C, x, xb, YB, pbar, ck);
   return cudaGetLastError();
 }
 
@@ -2389,9 +2397,9 @@ cudaError_t launch_tlm_staged(const Problem& P, const Consts& C, const ArgPtrs& 
   if ((e = cudaMemsetAsync(P.zmax, 0x00, nkey * sizeof(unsigned long long), stream)) != cudaSuccess) return e;
   if ((e = cudaMemsetAsync(P.zmin, 0xff, nkey * sizeof(unsigned long long), stream)) != cudaSuccess) return e;
   if (P.opt)
-    tlm_cell_kernel<true><<<152 * 4, 128, 0, stream>>>(io, C, params, dparams);
+    tlm_cell_kernel<true><<<152 * 3, 128, 0, stream>>>(io, C, params, dparams);
   else
-    tlm_cell_kernel<false><<<152 * 4, 128, 0, stream>>>(io, C, params, dparams);
+    tlm_cell_kernel<false><<<152 * 3, 128, 0, stream>>>(io, C, params, dparams);
   const dim3 levels((P.gall + STAGE_THREADS - 1) / STAGE_THREADS, P.kall, P.lall);
   adj_s1_fwd_kernel<false, Dual><<<levels, STAGE_THREADS, 0, stream>>>(io);
   adj_bounds_kernel<<<(int)((nkey + 127) / 128), 128, 0, stream>>>(P, bnd);
@@ -2410,7 +2418,7 @@ cudaError_t launch_adj_cell_save(const Problem& P, const Consts& C, const ArgPtr
   if (mixed)
     adj_cell_save_kernel<float><<<152 * 4, 128, 0, stream>>>(P, consts_to_float(C), x, Y, ck, check);
   else
-    adj_cell_save_kernel<double><<<152 * 4, 128, 0, stream>>>(P, C, x, Y, ck, check);
+    adj_cell_save_kernel<double><<<152 * 3, 128, 0, stream>>>(P, C, x, Y, ck, check);
   return cudaGetLastError();
 }
 

@@ -68,6 +68,16 @@ struct CellOutT {
 using CellIn = CellInT<double>;
 using CellOut = CellOutT<double>;
 
+// x as the scalar T: between FP64 and FP32 on the integer pipe (a conversion
+// instruction takes the FP64 pipe 16 cycles of an SM, and the mixed cell phase
+// makes 21 a cell: a third of its FP64 time).
+template <class T, class S>
+__device__ __forceinline__ T as(const S& x) {
+  if constexpr (std::is_same<T, float>::value && std::is_same<S, double>::value) return soft_d2f(x);
+  else if constexpr (std::is_same<T, double>::value && std::is_same<S, float>::value) return soft_f2d(x);
+  else return T(x);
+}
+
 // Scalar helpers overloaded on the precision of the process rates (FP64 in
 // the plain path, FP32 in the mixed path).
 __device__ __forceinline__ double fmaR(double a, double b, double c) { return __fma_rn(a, b, c); }
@@ -282,11 +292,11 @@ __device__ __forceinline__ void nsw6_cell(const typename ScalarOf<R>::consts& C,
     // qd CVdry + sum q CVW is CVdry up to its roundings.  Density and
     // pressure scale FP32 rates only: FP32.
     rhoge = temp * rhog * CVDRY;
-    densR = R(rhog) / R(in.gsgam2);
+    densR = as<R>(rhog) / as<R>(in.gsgam2);
     R qdR = R(1.0);
 #pragma unroll
-    for (int n = 1; n <= 5; ++n) qdR = qdR - R(qn[n]);
-    pre = densR * (qdR * K(RDRY) + R(qn[0]) * K(RVAP)) * R(temp);
+    for (int n = 1; n <= 5; ++n) qdR = qdR - as<R>(qn[n]);
+    pre = densR * (qdR * K(RDRY) + as<R>(qn[0]) * K(RVAP)) * as<R>(temp);
   } else {
     const D dens = quo(rhog, in.gsgam2);
     D qd = D(1.0);
@@ -305,14 +315,14 @@ __device__ __forceinline__ void nsw6_cell(const typename ScalarOf<R>::consts& C,
       }
     rhoge = temp * rhog * cv;
     pre = R(dens * (qd * RDRY + qn[0] * RVAP) * temp);
-    densR = R(dens);
+    densR = as<R>(dens);
   }
 
   const R Z = R(0.0), ONE = R(1.0);
-  const R qv = maxz(R(qn[0])), qc = maxz(R(qn[1])), qr = maxz(R(qn[2]));
-  const R qi = maxz(R(qn[3])), qs = maxz(R(qn[4])), qg = maxz(R(qn[5]));
+  const R qv = maxz(as<R>(qn[0])), qc = maxz(as<R>(qn[1])), qr = maxz(as<R>(qn[2]));
+  const R qi = maxz(as<R>(qn[3])), qs = maxz(as<R>(qn[4])), qg = maxz(as<R>(qn[5]));
   const bool hc = nz(qc), hr = nz(qr), hi = nz(qi), hs = nz(qs), hg = nz(qg);   // the species the cell holds
-  const R tempR = R(temp);
+  const R tempR = as<R>(temp);
   const R temc = tempR - K(TEM00);
   const bool warm = !lt_z(temc);  // iceflg = 0.5 - copysign(0.5, temc) == 0
   const bool cold = !warm;        // iceflg == 1
@@ -470,7 +480,7 @@ __device__ __forceinline__ void nsw6_cell(const typename ScalarOf<R>::consts& C,
   // cloud number (TagAerosolT / TagAerosolF, :676-684)
   R Nc = C.Nc_def;
   if constexpr (OPT) {
-    if (C.opt_indir != Z) Nc = dmax(R(in.unccn) * K(1.0E-6), C.Nc_def);
+    if (C.opt_indir != Z) Nc = dmax(as<R>(in.unccn) * K(1.0E-6), C.Nc_def);
   }
 
   // nucleation, :1080-1085: Ni0 = max(exp(-0.1 temc), 1) * 1000 and
@@ -1054,13 +1064,13 @@ __device__ __forceinline__ void nsw6_cell(const typename ScalarOf<R>::consts& C,
     // of the same size as the reference's; FP32 rates would leave one 10^9
     // times larger), and the vapour takes the balance so that total water
     // stays exact.
-    const R rgdt = R(rhog * dt);
+    const R rgdt = as<R>(rhog * dt);
     const R qt[6] = {qv_t, qc_t, qr_t, qi_t, qs_t, qg_t};
     const R lim[6] = {dqv_dt, dqc_dt, dqr_dt, dqi_dt, dqs_dt, dqg_dt};
     D sum = D(0.0);
 #pragma unroll
     for (int n = 1; n <= 5; ++n) {
-      drq[n] = (qt[n] <= -lim[n] && lim[n] > Z) ? -rq[n] : D(qt[n] * rgdt);
+      drq[n] = (qt[n] <= -lim[n] && lim[n] > Z) ? -rq[n] : as<D>(qt[n] * rgdt);
       sum += drq[n];
     }
     drq[0] = -sum;
@@ -1068,17 +1078,17 @@ __device__ __forceinline__ void nsw6_cell(const typename ScalarOf<R>::consts& C,
     const R qt[6] = {qv_t, qc_t, qr_t, qi_t, qs_t, qg_t};
 #pragma unroll
     for (int n = 0; n < 6; ++n) {
-      drq[n] = D(qt[n]);
+      drq[n] = as<D>(qt[n]);
       if (nz(qt[n])) {
         only();
-        drq[n] = rhog * D(qt[n]) * dt;
+        drq[n] = rhog * as<D>(qt[n]) * dt;
       }
     }
   }
-  o.Vtr = D(Vtr);
-  o.Vts = D(Vts);
-  o.Vtg = D(Vtg);
-  o.Vti = D(Vti);
+  o.Vtr = as<D>(Vtr);
+  o.Vts = as<D>(Vts);
+  o.Vtg = as<D>(Vtg);
+  o.Vti = as<D>(Vti);
 
   // effective radius and cloud top, :1566-1592 (without cloud water and rain
   // the radii are 0 and there is no top, on both sides of r2_min)
@@ -1106,10 +1116,10 @@ __device__ __forceinline__ void nsw6_cell(const typename ScalarOf<R>::consts& C,
     const bool big = ge_c(r2, r2_min);
     const R rceff = big ? quo(r3_qc + r3_qr, r2) : Z;
     const bool top = !big && ge_c(qc + qr, q_min);
-    o.rceff = D(rceff);
-    o.rctop = top ? D(rceff) : D(UNDEF);
+    o.rceff = as<D>(rceff);
+    o.rctop = top ? as<D>(rceff) : D(UNDEF);
     o.tctop = top ? temp : D(UNDEF);
-    o.rceff_cld = ge_c(r2_qc, r2_min) ? D(quo(r3_qc, r2_qc)) : D(0.0);
+    o.rceff_cld = ge_c(r2_qc, r2_min) ? as<D>(quo(r3_qc, r2_qc)) : D(0.0);
   }
 
   // ---- TagUpdateRHOGQ / RHOGE / MassConc / TEM, mod_mp_nsw6.cpp:692-744

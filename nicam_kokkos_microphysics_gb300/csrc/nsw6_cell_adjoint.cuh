@@ -157,14 +157,14 @@ __device__ __forceinline__ void nsw6_cell_adjoint(const ConstsT<R>& C, const M& 
   if constexpr (kMixed) {
     // as nsw6_cell: cv = CVdry (every CVW is CVdry), density and pressure in FP32
     rhoge0 = trh * CVDRY;
-    densR = NSW6_CK(R, 1, R(rhog) / R(in.gsgam2));
-    dens = D(densR);
+    densR = NSW6_CK(R, 1, as<R>(rhog) / as<R>(in.gsgam2));
+    dens = as<D>(densR);
     R qdR = ONE;
 #pragma unroll
-    for (int n = 1; n <= 5; ++n) qdR = qdR - R(qn[n]);
-    pqR = qdR * R(RDRY) + R(qn[0]) * R(RVAP);
+    for (int n = 1; n <= 5; ++n) qdR = qdR - as<R>(qn[n]);
+    pqR = qdR * R(RDRY) + as<R>(qn[0]) * R(RVAP);
     dpR = densR * pqR;
-    pre = dpR * R(temp);
+    pre = dpR * as<R>(temp);
   } else {
     dens = NSW6_CK(D, 1, quo(rhog, in.gsgam2));
     D qd = 1.0;
@@ -177,11 +177,11 @@ __device__ __forceinline__ void nsw6_cell_adjoint(const ConstsT<R>& C, const M& 
     pq = qd * RDRY + qn[0] * RVAP;
     dp = dens * pq;
     pre = R(dp * temp);
-    densR = R(dens);
+    densR = as<R>(dens);
   }
 
   // ---- psat / qsat (rate precision from here to the tendencies)
-  const R tempR = R(temp);
+  const R tempR = as<R>(temp);
   const R tmx = maxc(tempR, R(TEM_MIN));
   const R rtem = NSW6_CK(R, 2, quo(ONE, tmx));
   const R al = C.LovR_liq * (C.RTEM00 - rtem);
@@ -196,8 +196,8 @@ __device__ __forceinline__ void nsw6_cell_adjoint(const ConstsT<R>& C, const M& 
   const R qsati = psati * rdrt;
 
   // ---- TagBigLoop
-  const R qv = maxz(R(qn[0])), qc = maxz(R(qn[1])), qr = maxz(R(qn[2]));
-  const R qi = maxz(R(qn[3])), qs = maxz(R(qn[4])), qg = maxz(R(qn[5]));
+  const R qv = maxz(as<R>(qn[0])), qc = maxz(as<R>(qn[1])), qr = maxz(as<R>(qn[2]));
+  const R qi = maxz(as<R>(qn[3])), qs = maxz(as<R>(qn[4])), qg = maxz(as<R>(qn[5]));
   const R sld = maxc(qsatl, R(EPS)), sid = maxc(qsati, R(EPS));
   const R Sliq = NSW6_CK(R, 6, quo(qv, sld));
   const R Sice = NSW6_CK(R, 7, quo(qv, sid));
@@ -607,19 +607,19 @@ __device__ __forceinline__ void nsw6_cell_adjoint(const ConstsT<R>& C, const M& 
   bool exh[6] = {false, false, false, false, false, false};
   if constexpr (kMixed) {
     // formed in FP32 as in nsw6_cell: qt (rhog dt)
-    const R rgdt = R(rhog * dt);
+    const R rgdt = as<R>(rhog * dt);
     const R lim[6] = {dqv_dt, dqc_dt, dqr_dt, dqi_dt, dqs_dt, dqg_dt};
     D sum = 0.0;
 #pragma unroll
     for (int n = 1; n <= 5; ++n) {
       exh[n] = qt[n] <= -lim[n] && lim[n] > Z;
-      drq[n] = exh[n] ? -rq[n] : D(qt[n] * rgdt);
+      drq[n] = exh[n] ? -rq[n] : as<D>(qt[n] * rgdt);
       sum += drq[n];
     }
     drq[0] = -sum;
   } else {
 #pragma unroll
-    for (int n = 0; n < 6; ++n) drq[n] = rhog * D(qt[n]) * dt;
+    for (int n = 0; n < 6; ++n) drq[n] = rhog * as<D>(qt[n]) * dt;
   }
   D rq2[6];
 #pragma unroll
@@ -666,14 +666,14 @@ __device__ __forceinline__ void nsw6_cell_adjoint(const ConstsT<R>& C, const M& 
   }
   if constexpr (MODE == CA_SAVE) {
     // the outputs of nsw6_cell (the same operations on the same values)
-    out->Vtr = D(Vtr);
-    out->Vts = D(Vts);
-    out->Vtg = D(Vtg);
+    out->Vtr = as<D>(Vtr);
+    out->Vts = as<D>(Vts);
+    out->Vtg = as<D>(Vtg);
     out->Vti = 0.0;
-    out->rceff = big ? D(quo(r3, r2)) : 0.0;
+    out->rceff = big ? as<D>(quo(r3, r2)) : 0.0;
     out->rctop = top ? out->rceff : UNDEF;
     out->tctop = top ? temp : UNDEF;
-    out->rceff_cld = cld ? D(quo(r3_qc, r2_qc)) : 0.0;
+    out->rceff_cld = cld ? as<D>(quo(r3_qc, r2_qc)) : 0.0;
 #pragma unroll
     for (int n = 0; n < 6; ++n) {
       out->q[n] = q2[n];
@@ -744,7 +744,7 @@ __device__ __forceinline__ void nsw6_cell_adjoint(const ConstsT<R>& C, const M& 
 #pragma unroll
   for (int n = 0; n < 6; ++n) {
     const D b_rqt = b_drq[n] * dt;
-    b_rhog = fma(b_rqt, D(qt[n]), b_rhog);
+    b_rhog = fma(b_rqt, as<D>(qt[n]), b_rhog);
     b_qtD[n] = b_rqt * rhog;
   }
   // ---- rate precision from here to the psat block.  The sweep is linear in
@@ -1405,8 +1405,8 @@ __device__ __forceinline__ void nsw6_cell_adjoint(const ConstsT<R>& C, const M& 
 #pragma unroll
     for (int n = 0; n < 6; ++n) {
       R b = Z, dummy = Z;
-      bmaxz(R(qn[n]), bq[n], b, dummy);
-      b_qn[n] = D(b) * isc;
+      bmaxz(as<R>(qn[n]), bq[n], b, dummy);
+      b_qn[n] = as<D>(b) * isc;
     }
   }
   // psat / qsat: qsat = psat (1 / ((dens RVAP) temp)), psat = PSAT0 exp(LovR (RTEM00 - rtem))
@@ -1423,18 +1423,18 @@ __device__ __forceinline__ void nsw6_cell_adjoint(const ConstsT<R>& C, const M& 
     bmaxc(tempR, R(TEM_MIN), b_tmx, b_temp, dummy);
   }
   // ---- FP64 from here: pre = (dens (qd RDRY + qn0 RVAP)) temp
-  D b_densD = D(b_dens) * isc;
-  b_tempD += D(b_temp) * isc;
+  D b_densD = as<D>(b_dens) * isc;
+  b_tempD += as<D>(b_temp) * isc;
   D b_rhogD = b_rhog;
   if constexpr (kMixed) {
     // pre = (densR pq) temp, pq = qd RDRY + qn0 RVAP, qd = 1 - sum qn (FP32)
-    const R tR = R(temp);
-    b_tempD = fma(D(b_pre * dpR), isc, b_tempD);
+    const R tR = as<R>(temp);
+    b_tempD = fma(as<D>(b_pre * dpR), isc, b_tempD);
     const R b_dp = b_pre * tR;
-    b_densD = fma(D(b_dp * pqR), isc, b_densD);
+    b_densD = fma(as<D>(b_dp * pqR), isc, b_densD);
     const R b_pq = b_dp * densR;
-    const D b_qd = D(b_pq * R(RDRY)) * isc;
-    b_qn[0] = fma(D(b_pq * R(RVAP)), isc, b_qn[0]);
+    const D b_qd = as<D>(b_pq * R(RDRY)) * isc;
+    b_qn[0] = fma(as<D>(b_pq * R(RVAP)), isc, b_qn[0]);
 #pragma unroll
     for (int n = 1; n <= 5; ++n) b_qn[n] -= b_qd;
     // rhoge0 = (temp rhog) CVdry
@@ -1442,7 +1442,7 @@ __device__ __forceinline__ void nsw6_cell_adjoint(const ConstsT<R>& C, const M& 
     b_tempD = fma(b_trh, rhog, b_tempD);
     b_rhogD = fma(b_trh, temp, b_rhogD);
   } else {
-    const D b_preD = D(b_pre) * isc;
+    const D b_preD = as<D>(b_pre) * isc;
     b_tempD = fma(b_preD, dp, b_tempD);
     const D b_dp = b_preD * temp;
     b_densD = fma(b_dp, pq, b_densD);
@@ -1491,25 +1491,25 @@ __device__ __forceinline__ void nsw6_cell_adjoint(const ConstsT<R>& C, const M& 
                  C.Cs;
     const R p4 = (b_K_vtg * C.K_vtg + b_K_gacw * C.K_gacw) / C.Cg + b_Cg;
     const R p6 = b_K_aut * C.K_aut / C.kk_aut;
-    pb[0] += D(b_beta) * isc;
-    pb[1] += D(b_qicrt) * isc;
-    pb[2] += D(p2) * isc;
-    pb[3] += D(p3) * isc;
-    pb[4] += D(p4) * isc;
-    pb[5] += D(b_icenuc) * isc;
-    pb[6] += D(p6) * isc;
+    pb[0] += as<D>(b_beta) * isc;
+    pb[1] += as<D>(b_qicrt) * isc;
+    pb[2] += as<D>(p2) * isc;
+    pb[3] += as<D>(p3) * isc;
+    pb[4] += as<D>(p4) * isc;
+    pb[5] += as<D>(b_icenuc) * isc;
+    pb[6] += as<D>(p6) * isc;
     return;
   }
-  pb[0] += D(b_beta) * isc;
-  pb[1] += D(b_qicrt) * isc;
-  pb[2] += ((D(b_K_vtr) * D(C.K_vtr) + D(b_K_raci) * D(C.K_raci) + D(b_K_iacr) * D(C.K_iacr)) * (1.0 / D(C.Cr)) +
-            D(b_Cr)) * isc;
-  pb[3] += (D(b_K_vts) * D(C.K_vts) + D(b_K_sacw) * D(C.K_sacw) + D(b_K_saci) * D(C.K_saci) +
-            D(b_K_vents2) * 0.5 * D(C.K_vents2)) *
+  pb[0] += as<D>(b_beta) * isc;
+  pb[1] += as<D>(b_qicrt) * isc;
+  pb[2] += ((as<D>(b_K_vtr) * D(C.K_vtr) + as<D>(b_K_raci) * D(C.K_raci) + as<D>(b_K_iacr) * D(C.K_iacr)) * (1.0 / D(C.Cr)) +
+            as<D>(b_Cr)) * isc;
+  pb[3] += (as<D>(b_K_vts) * D(C.K_vts) + as<D>(b_K_sacw) * D(C.K_sacw) + as<D>(b_K_saci) * D(C.K_saci) +
+            as<D>(b_K_vents2) * 0.5 * D(C.K_vents2)) *
            (1.0 / D(C.Cs)) * isc;
-  pb[4] += ((D(b_K_vtg) * D(C.K_vtg) + D(b_K_gacw) * D(C.K_gacw)) * (1.0 / D(C.Cg)) + D(b_Cg)) * isc;
-  pb[5] += D(b_icenuc) * isc;
-  pb[6] += D(b_K_aut) * D(C.K_aut) / D(C.kk_aut) * isc;
+  pb[4] += ((as<D>(b_K_vtg) * D(C.K_vtg) + as<D>(b_K_gacw) * D(C.K_gacw)) * (1.0 / D(C.Cg)) + as<D>(b_Cg)) * isc;
+  pb[5] += as<D>(b_icenuc) * isc;
+  pb[6] += as<D>(b_K_aut) * D(C.K_aut) / D(C.kk_aut) * isc;
 }
 
 #undef NSW6_CK

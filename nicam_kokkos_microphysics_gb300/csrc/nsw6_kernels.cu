@@ -95,7 +95,7 @@ __device__ __forceinline__ int bucket_add(int* bucket, int v) {
 // OPT: the kernel with the scheme switches: the switched branches of nsw6_cell
 // and the CCN input.
 template <class M, class R, bool OPT = false>
-__global__ void __launch_bounds__(CELL_THREADS, 2) nsw6_cell_kernel(Problem P, ConstsT<R> C, int tile) {
+__global__ void __launch_bounds__(CELL_THREADS, sizeof(R) == 4 ? 3 : 2) nsw6_cell_kernel(Problem P, ConstsT<R> C, int tile) {
   constexpr bool kMixed = sizeof(R) == sizeof(float);
   const int ntr = OPT ? P.ntr : 3;          // sedimenting tracers of this call
   extern __shared__ double sm[];
@@ -375,8 +375,10 @@ cudaError_t launch_math(int fn, const double* x, const double* y, double* out, i
 struct CellShape {
   int tile, threads, blocks;
 };
-static CellShape cell_shape(int cells, int lall) {
-  const int slots = 2 * 152;
+static CellShape cell_shape(int cells, int lall, bool mixed) {
+  // CTAs the chip holds: in mixed precision, 80 registers a thread without
+  // spills, three an SM (ten regions 4.46 -> 4.41 ms a step; FP64 at 80 spills)
+  const int slots = (mixed ? 3 : 2) * 152;
   CellShape s;
   const long long total = (long long)cells * lall;
   if (total <= (long long)slots * CELL_THREADS) {
@@ -407,7 +409,7 @@ cudaError_t launch_prepare();
 
 // The cell phase: the cell kernel and the departure distances.
 static cudaError_t launch_cells(const Problem& P, const Consts& C, cudaStream_t stream) {
-  const CellShape s = cell_shape((P.kmax - P.kmin + 1) * P.gall, P.lall);
+  const CellShape s = cell_shape((P.kmax - P.kmin + 1) * P.gall, P.lall, P.mixed != 0);
   const size_t sm = cell_smem_bytes(s, P.mixed != 0);
   const dim3 g1(s.blocks, P.lall);
   const int nt = s.threads;
