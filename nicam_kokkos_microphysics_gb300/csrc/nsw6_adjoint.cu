@@ -965,7 +965,7 @@ __global__ void __launch_bounds__(STAGE_THREADS) adj_s4_kernel(StageIO io, Const
 // converged value as satadjust_t does: with F(T) = T cv(T) + qsat(T) LHV0 -
 // Emoist, dT = -dF / F_T at the last iterate.  Adjoints go to S3's outputs at
 // this level and its neighbours and to the metric factors, atomically.
-__global__ void __launch_bounds__(STAGE_THREADS) adj_s4_hw_kernel(StageIO io, Consts C, int pass) {
+__global__ void __launch_bounds__(STAGE_THREADS, 4) adj_s4_hw_kernel(StageIO io, Consts C, int pass) {
   __shared__ double grid[GF_COUNT * MAX_KALL];
   __shared__ double tab[FM_TABLE_DOUBLES];
   stage_smem(io.P, grid, tab);
@@ -1447,7 +1447,7 @@ __device__ __forceinline__ void zdis_wh_bar(R wm, R w0, R wpp, const R* rdz, con
 // MIX: the departure distances are the mixed step's (FP32, stage1): their
 // adjoint coefficients in FP32 at the FP32 values, times the FP64 adjoint.
 template <bool MIX>
-__global__ void __launch_bounds__(STAGE_THREADS) adj_s1_hw_kernel(StageIO io) {
+__global__ void __launch_bounds__(STAGE_THREADS, 5) adj_s1_hw_kernel(StageIO io) {
   __shared__ double grid[GF_COUNT * MAX_KALL];
   __shared__ float grf[MIX ? 4 * MAX_KALL : 1];   // MIX: rdgz, rdgzh, rdzs, rdzsh in FP32
   for (int i = threadIdx.x; i < GF_COUNT * io.P.kall; i += blockDim.x) grid[i] = io.P.grid[i];
@@ -2018,11 +2018,11 @@ struct CellMath<float> {
 // evaluate nsw6_cell and report a cell whose outputs differ in any bit
 // (status ERR_ADJ_CHECK, iters = the first output field that differs).
 // The cell kernels of the derivatives hold three CTAs an SM (168 registers a
-// thread, four at 128 where the rates are FP32), which costs no spills to speak
-// of; at 255 registers and two, their warps waited for one another's FP64
-// results: 4096 x 42 cells 220 -> 190 us here, 504 -> 471 in the sweep, 457 ->
-// 420 in forward mode, 16900 x 42 in mixed precision 144 -> 102 us here.  (One
-// CTA more spills a kilobyte a thread.)
+// thread, four at 128 in this kernel where the rates are FP32).  That spills
+// 0.3 to 2.4 kB a thread, but at 255 registers and two CTAs the warps were too
+// few to cover the FP64 pipe's latency: 4096 x 42 cells 220 -> 190 us here, 504
+// -> 471 in the sweep, 457 -> 420 in forward mode, 16900 x 42 in mixed
+// precision 144 -> 102 us here.
 constexpr int ERR_ADJ_CHECK = 7;
 template <class R>
 __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 4 : 3) adj_cell_save_kernel(Problem P, ConstsT<R> C, ArgPtrs x, double* Y, double* ck,
@@ -2244,7 +2244,7 @@ __global__ void __launch_bounds__(STAGE_THREADS) tlm_s2_kernel(StageIO io) {
 
 // S3 in forward mode: the work fields, and the step's momentum, GPREC and
 // surface outputs.
-__global__ void __launch_bounds__(STAGE_THREADS) tlm_s3_kernel(StageIO io) {
+__global__ void __launch_bounds__(STAGE_THREADS, 6) tlm_s3_kernel(StageIO io) {
   __shared__ double grid[GF_COUNT * MAX_KALL];
   for (int c = threadIdx.x; c < GF_COUNT * io.P.kall; c += blockDim.x) grid[c] = io.P.grid[c];
   __syncthreads();
@@ -2291,7 +2291,7 @@ __global__ void __launch_bounds__(STAGE_THREADS) tlm_s3_kernel(StageIO io) {
 // the outputs the cell phase gives directly (effective radii, cloud top) and
 // of those the step sets to constants (the mp_driver epilogue,
 // mod_mp_driver.cpp:555-612; zero tangents).
-__global__ void __launch_bounds__(STAGE_THREADS) tlm_s4_kernel(StageIO io, Consts C) {
+__global__ void __launch_bounds__(STAGE_THREADS, 4) tlm_s4_kernel(StageIO io, Consts C) {
   __shared__ double grid[GF_COUNT * MAX_KALL];
   __shared__ double tab[FM_TABLE_DOUBLES];
   stage_smem(io.P, grid, tab);
@@ -2404,7 +2404,7 @@ cudaError_t launch_tlm_staged(const Problem& P, const Consts& C, const ArgPtrs& 
   adj_s1_fwd_kernel<false, Dual><<<levels, STAGE_THREADS, 0, stream>>>(io);
   adj_bounds_kernel<<<(int)((nkey + 127) / 128), 128, 0, stream>>>(P, bnd);
   tlm_s2_kernel<<<152 * 8, STAGE_THREADS, 0, stream>>>(io);
-  tlm_s3_kernel<<<152 * 8, STAGE_THREADS, 0, stream>>>(io);
+  tlm_s3_kernel<<<152 * 6, STAGE_THREADS, 0, stream>>>(io);
   tlm_s4_kernel<<<152 * 4, STAGE_THREADS, 0, stream>>>(io, C);
   return cudaGetLastError();
 }
@@ -2481,9 +2481,9 @@ cudaError_t launch_adj_column_staged(const Problem& P, const Consts& C, const Ar
   if (recorded)
     adj_s1_kernel<<<blocks, STAGE_THREADS, 0, stream>>>(io, tm);
   else if (mixed)
-    adj_s1_hw_kernel<true><<<152 * 4, STAGE_THREADS, 0, stream>>>(io);
+    adj_s1_hw_kernel<true><<<152 * 5, STAGE_THREADS, 0, stream>>>(io);
   else
-    adj_s1_hw_kernel<false><<<152 * 4, STAGE_THREADS, 0, stream>>>(io);
+    adj_s1_hw_kernel<false><<<152 * 5, STAGE_THREADS, 0, stream>>>(io);
   return cudaGetLastError();
 }
 
