@@ -964,7 +964,10 @@ __global__ void __launch_bounds__(STAGE_THREADS) adj_s4_kernel(StageIO io, Const
 // reverse sweep.  The Newton temperature is differentiated implicitly at its
 // converged value as satadjust_t does: with F(T) = T cv(T) + qsat(T) LHV0 -
 // Emoist, dT = -dF / F_T at the last iterate.  Adjoints go to S3's outputs at
-// this level and its neighbours and to the metric factors, atomically.
+// this level and its neighbours and to the metric factors, atomically.  Bound by
+// the FP64 pipe; four CTAs an SM, as the grid has (at 168 registers three were
+// resident and the fourth ran alone after them), took 4096 x 42 cells from 127
+// to 105 us, 16900 x 42 in mixed precision from 15.3 to 14.6 ms over four steps.
 __global__ void __launch_bounds__(STAGE_THREADS, 4) adj_s4_hw_kernel(StageIO io, Consts C, int pass) {
   __shared__ double grid[GF_COUNT * MAX_KALL];
   __shared__ double tab[FM_TABLE_DOUBLES];

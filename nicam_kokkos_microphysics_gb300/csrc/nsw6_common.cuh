@@ -231,9 +231,16 @@ __host__ __device__ __forceinline__ double dmax(double a, double b) { return (a 
 // Order-preserving map double -> uint64 (total order, -0 < +0), used for exact
 // atomic max/min of the per-level departure-distance extrema.
 __host__ __device__ __forceinline__ unsigned long long order_key(double v) {
+#ifdef __CUDA_ARCH__
+  // (by the two words: of the 64-bit form the compiler makes FP64 negations)
+  const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
+  const unsigned neg = (unsigned)((int)hi >> 31);   // all ones for a negative number
+  return ((unsigned long long)(hi ^ (neg | 0x80000000u)) << 32) | (lo ^ neg);
+#else
   union { double d; unsigned long long u; } c;
   c.d = v;
   return (c.u >> 63) ? ~c.u : (c.u | 0x8000000000000000ull);
+#endif
 }
 __host__ __device__ __forceinline__ double key_value(unsigned long long k) {
   union { double d; unsigned long long u; } c;
