@@ -143,6 +143,14 @@ template <class T>
 __device__ __forceinline__ T per_dt(const T& q, const DivisorT<T>& dt, const T&) { return div_rn(q, dt); }
 __device__ __forceinline__ float per_dt(float q, const DivisorT<float>&, float rdt) { return q * rdt; }
 
+// -x; a double's by the word that has its sign (a negation that no FP64
+// instruction takes as its operand is one of its own on that pipe).
+template <class T>
+__device__ __forceinline__ T neg_of(const T& x) { return -x; }
+__device__ __forceinline__ double neg_of(double x) {
+  return __hiloint2double(__double2hiint(x) ^ (int)0x80000000, __double2loint(x));
+}
+
 // The comparisons of the cell physics with constants and the min / max they
 // select: for doubles the integer-pipe forms of nsw6_fpcmp.cuh (an FP64
 // comparison takes an FP64-pipe slot, as an FMA does); the other types compare
@@ -781,7 +789,7 @@ __device__ __forceinline__ void nsw6_cell(const typename ScalarOf<R>::consts& C,
   auto limiter = [&](R net, R dq) {
     if (kPlain && is_nonneg(net)) return ONE;
     only();
-    return is_nonneg(net + K(EPS)) ? ONE : minc(quo(-dq, net), ONE);
+    return is_nonneg(net + K(EPS)) ? ONE : minc(quo(neg_of(dq), net), ONE);
   };
   // Scaling by fac = 1 is exact and skipped.  The tendencies below are the
   // nets the limiters form (same terms, same order) where no later scaling
@@ -1055,7 +1063,7 @@ __device__ __forceinline__ void nsw6_cell(const typename ScalarOf<R>::consts& C,
     only();
     q_t = q_t + qg_t;
   }
-  const R qv_t = -q_t;
+  const R qv_t = neg_of(q_t);
   D drq[6];
   if constexpr (kMixed) {
     // The tracer changes rhog q_t dt of the FP32 rates, formed in FP32 and

@@ -167,7 +167,12 @@ NSW6_FP_HD bool lt_nd(double a, double d) {                                     
   return ba < 0 && ma > (fp_bits(d) & FP_ABS) && ma <= FP_INF;
 }
 NSW6_FP_HD double max_nd(double a, double d) {                                          // max(a, -d)
+#ifdef __CUDA_ARCH__
+  // (by the word that has the sign: of the 64-bit form the compiler makes an FP64 negation)
+  return lt_nd(a, d) ? __hiloint2double(__double2hiint(d) ^ (int)0x80000000, __double2loint(d)) : a;
+#else
   return lt_nd(a, d) ? fp_from_bits(fp_bits(d) ^ FP_SIGN) : a;
+#endif
 }
 
 // x + 0.0: -0 becomes +0, every other value stays (a NaN keeps its payload,
