@@ -59,23 +59,23 @@ CELL_KERNEL_BYTES_PER_CELL = (10 + 17) * 8
 # cells): DRAM bytes read + written, and the FP64 thread instructions the
 # kernel executes -- DFMA, DADD, DMUL and all instructions of the FP64 pipe
 # (compares, min/max and conversions included) -- per interior cell (cell
-# kernel) or per cell (column phase).  The column phase is nsw6_column_kernel
-# and nsw6_satadj_kernel (the saturated cells), timed together as one
-# interval; its figures are the two kernels' sums.
-CELL_KERNEL_TRAFFIC_PER_CELL = {"fp64": 229.0, "mixed": 172.4}
-COLUMN_KERNEL_TRAFFIC_PER_CELL = {"fp64": 379.8 + 30.0, "mixed": 386.4 + 30.0}
+# kernel) or per cell (column phase).  The cell phase is nsw6_cell_kernel and
+# nsw6_departure_kernel, the column phase nsw6_column_kernel and
+# nsw6_satadj_kernel (the saturated cells), each timed together as one
+# interval; the figures are the two kernels' sums.
+CELL_KERNEL_TRAFFIC_PER_CELL = {"fp64": 395.0 + 24.0, "mixed": 147.7 + 24.0}
+COLUMN_KERNEL_TRAFFIC_PER_CELL = {"fp64": 382.0 + 30.0, "mixed": 386.3 + 30.0}
 FP64_EXECUTED = {
-    "nsw6_cell_kernel": {"fp64": {"dfma": 353.9, "dadd": 258.8, "dmul": 273.0, "pipe": 901.5},
-                         "mixed": {"dfma": 5.0, "dadd": 43.0, "dmul": 20.1, "pipe": 91.9}},
-    "nsw6_column_kernel": {"fp64": {"dfma": 113.8 + 9.9, "dadd": 137.4 + 6.0, "dmul": 144.8 + 5.4,
-                                    "pipe": 403.0 + 21.6},
-                           "mixed": {"dfma": 37.3 + 9.0, "dadd": 69.0 + 5.8, "dmul": 55.8 + 6.2,
-                                     "pipe": 208.5 + 21.4}},
+    "nsw6_cell_kernel": {"fp64": {"dfma": 38.4 + 16.8, "dadd": 104.7 + 15.0, "dmul": 80.4 + 17.3,
+                                  "pipe": 239.6 + 49.2},
+                         "mixed": {"dfma": 0.0, "dadd": 26.3, "dmul": 20.1, "pipe": 52.4 + 2.2}},
+    "nsw6_column_kernel": {"fp64": {"dfma": 19.7, "dadd": 102.2 + 5.4, "dmul": 84.1 + 4.2, "pipe": 222.0 + 9.9},
+                           "mixed": {"dfma": 6.4, "dadd": 51.9 + 5.2, "dmul": 34.5 + 4.4, "pipe": 98.3 + 9.6}},
 }
 # FP64-pipe activity (fraction of active cycles) of each kernel in the same
-# captures (cold, serialised launches; the column kernel alone).
-FP64_PIPE_ACTIVE = {"nsw6_cell_kernel": {"fp64": 0.839, "mixed": 0.656},
-                    "nsw6_column_kernel": {"fp64": 0.732, "mixed": 0.585}}
+# captures (cold, serialised launches; the cell and the column kernel alone).
+FP64_PIPE_ACTIVE = {"nsw6_cell_kernel": {"fp64": 0.707, "mixed": 0.723},
+                    "nsw6_column_kernel": {"fp64": 0.721, "mixed": 0.494}}
 # FP64 op weights in flop equivalents (an FMA counts 2): the cost of CUDA's FP64
 # divide, sqrt, exp, log and pow relative to DFMA, measured once on a GB300 with
 # the throughput probe (probe/nsw6_probe.cu) and frozen here.
@@ -386,8 +386,9 @@ def time_end_to_end(drv, spec: StateSpec, st: dict, steps: int, world: int, dist
 
 
 def roofline_of(kernel_ms: dict, spec: StateSpec, precision: str, rates, aw) -> dict:
-    """FP64 roofline of the dominant kernel.  Both kernels are bound by the
-    FP64 pipe, which issues one DFMA, DADD, DMUL, compare, min/max or
+    """FP64 roofline of the dominant kernel.  The FP64 kernels are bound by the
+    FP64 pipe first (quotients, roots and transcendentals run on the integer
+    pipe, which issues beside it), which issues one DFMA, DADD, DMUL, compare, min/max or
     conversion per thread and slot.  achieved = the FP64-pipe thread
     instructions the kernel executes per launch (ncu, per cell, times the
     cells of a launch) / its mean CUDA-event duration, counted at 2 flops each
@@ -427,6 +428,8 @@ def roofline_of(kernel_ms: dict, spec: StateSpec, precision: str, rates, aw) -> 
                               "sm__thread_inst_executed_pipe_fp64_pred_on per cell on one 16900 x 42 region, "
                               "profiles/fp64_work_16900x42.md, times the cells of the launch), 2 flops each",
            "kernels": per,
+           "cell_phase": "nsw6_cell_kernel above times the cell phase: nsw6_cell_kernel and "
+                         "nsw6_departure_kernel (the departure distances), one CUDA-event interval",
            "column_phase": "nsw6_column_kernel above times the column phase: nsw6_column_kernel and "
                            "nsw6_satadj_kernel (the saturated cells' Newton iteration), one CUDA-event interval",
            "hbm": {"cell_kernel_gbs": hbm_cell, "cell_kernel_frac": hbm_cell / peaks["hbm_gbs"],

@@ -265,8 +265,8 @@ int nsw6_host_copy_bytes(const nsw6_handle* h, int lall, unsigned long long* h2d
 
 /* nsteps consecutive steps of mp_driver_argv (device pointers) on the same
  * arrays, the state evolving in place as in the reference harness's
- * SET_iteration loop (src/main.cpp:261-319).  The step (three memsets and the
- * three kernels) is captured once into a CUDA graph on a stream of the handle
+ * SET_iteration loop (src/main.cpp:261-319).  The step (four kernels) is
+ * captured once into a CUDA graph on a stream of the handle
  * and replayed nsteps times on the handle's stream; the graph is kept and
  * re-captured when the arrays, lall, dt, the parameters or the precision /
  * math / itelim settings change.  The status word is checked once, after the

@@ -4,7 +4,7 @@
 // 335-613) and the set-up routines the reference runs through globals:
 // GRD_Setup (mod_debug.cpp:92-187), SATURATION_Setup (mod_satadjust.cpp:24-47)
 // and mp_nsw6_init (mod_mp_nsw6.cpp:276-434).  All device memory a step needs
-// is allocated in nsw6_create; a step enqueues three memsets and three kernels.
+// is allocated in nsw6_create; a step enqueues four kernels.
 #include <algorithm>
 #include <climits>
 #include <cmath>
