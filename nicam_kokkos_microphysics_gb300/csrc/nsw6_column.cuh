@@ -1297,18 +1297,26 @@ __global__ void __launch_bounds__(COL_THREADS_MAX, 2) nsw6_column_kernel(Problem
 // The saturated cells the column kernel listed (P.satq): the cell's state
 // after KIN2EIN is formed again exactly as there, the saturation-adjustment
 // Newton iteration runs and the cell is finished (final_cell).  One thread per
-// cell, grid-stride over the list, whose length only the device knows.
-constexpr int SAT_THREADS = 128;
-constexpr int SAT_BLOCKS = 152 * 8;
+// cell, grid-stride over the list, whose length only the device knows.  Bound by
+// the latency of the iteration's chain where the list is short, by the FP64 pipe
+// where it is long: CTAs of one warp spread a short list over all SMs (with 128
+// threads some had twice the warps of others), the tables through L1.  Twelve
+// mixed steps of 2500 x 42 1.593 -> 1.561 ms, one region's FP64 step 1.037 ->
+// 1.030 ms, ten regions the same.
+constexpr int SAT_THREADS = 32;
+// CTAs: enough for a sixteenth of the cells (some 4 percent are saturated) in
+// one sweep, so that the last ones level out; at least 8 an SM, for a small call
+// that is saturated throughout, and no more than 64, whose start costs.
+inline int sat_blocks(long long cells) {
+  const long long n = cells / (16 * SAT_THREADS);
+  return (int)(n < 152 * 8 ? 152 * 8 : n > 152 * 64 ? 152 * 64 : n);
+}
 
 template <bool MIX, bool OPT>
 __global__ void __launch_bounds__(SAT_THREADS) nsw6_satadj_kernel(Problem P, Consts C) {
-  __shared__ double tab[FM_TABLE_DOUBLES];
   const unsigned n = P.satq[0];
   if (blockIdx.x * blockDim.x >= n) return;
-  for (int t = threadIdx.x; t < FM_TABLE_DOUBLES; t += blockDim.x) tab[t] = P.fmtab[t];
-  __syncthreads();
-  const ColumnMath mth{FastMath(tab), P.math_lib != 0};
+  const ColumnMath mth{FastMath(P.fmtab), P.math_lib != 0};
   const int G = P.gall;
   const size_t KG = (size_t)P.kall * G;
   const bool ice_adj = OPT && C.opt_expice == 0.0;
@@ -1400,7 +1408,7 @@ cudaError_t run_column(const Problem& P, const Consts& C, cudaStream_t stream) {
   const size_t sm = column_smem_bytes(P.kall, s.tg, OPT);
   if (!with_column_kernel<MIX, OPT>(s.tg, s.nj, [&](auto k) { k<<<grid, s.threads, sm, stream>>>(P, C); }))
     return cudaErrorInvalidConfiguration;
-  nsw6_satadj_kernel<MIX, OPT><<<SAT_BLOCKS, SAT_THREADS, 0, stream>>>(P, C);
+  nsw6_satadj_kernel<MIX, OPT><<<sat_blocks((long long)P.lall * P.kall * P.gall), SAT_THREADS, 0, stream>>>(P, C);
   return cudaGetLastError();
 }
 
