@@ -376,7 +376,9 @@ NSW6_CALL double soft_log(u64 b, SoftTables T) {
   const u64 mm = l ? m : soft_pair(w2, w1);              // (a shift by 32 is one by 0)
   u64 p = soft_mulhi64(mm, 0xB17217F7D1CF79ABull);
   if (!(p >> 63)) { p <<= 1; ++z; }
-  return fp_from_bits((long long)((((p + 0x400ull) >> 11) + ((u64)(u32)(31 - z + 1022) << 52)) |
+  // (p + 0x400 would run over for p next to 2^64, a logarithm just below a
+  // power of two; rounded so, the carry goes into the exponent)
+  return fp_from_bits((long long)(((p >> 11) + ((u32)(p >> 10) & 1u) + ((u64)(u32)(31 - z + 1022) << 52)) |
                                   ((u64)((u32)I & 0x80000000u) << 32)));
 }
 
