@@ -329,12 +329,22 @@ __device__ __forceinline__ void nsw6_cell(const typename ScalarOf<R>::consts& C,
   const R Z = R(0.0), ONE = R(1.0);
   const R qv = maxz(as<R>(qn[0])), qc = maxz(as<R>(qn[1])), qr = maxz(as<R>(qn[2]));
   const R qi = maxz(as<R>(qn[3])), qs = maxz(as<R>(qn[4])), qg = maxz(as<R>(qn[5]));
-  const bool hc = nz(qc), hr = nz(qr), hi = nz(qi), hs = nz(qs), hg = nz(qg);   // the species the cell holds
+  // A zero times an infinity or a NaN is no zero: a cell where one may arise
+  // keeps every term.  The pressure is a product of everything the rates draw
+  // on (but the cloud number): where it is a positive normal number, so are
+  // its factors finite and the density not zero.
+  bool whole = !kPlain;
+  if constexpr (kPlain) {
+    whole = !fp_pos_normal(pre);
+    if constexpr (OPT) whole = whole || (C.opt_indir != 0.0 && fp_not_finite(in.unccn));
+  }
+  const bool hc = whole || nz(qc), hr = whole || nz(qr), hi = whole || nz(qi), hs = whole || nz(qs),
+             hg = whole || nz(qg);   // the species the cell holds
   const R tempR = as<R>(temp);
   const R temc = tempR - K(TEM00);
   const bool warm = !lt_z(temc);  // iceflg = 0.5 - copysign(0.5, temc) == 0
   const bool cold = !warm;        // iceflg == 1
-  const bool wcold = !kPlain || cold, wwarm = !kPlain || warm;   // work for cold (warm) cells
+  const bool wcold = whole || cold, wwarm = whole || warm;   // work for cold (warm) cells
 
   // ---- psat / qsat (CPovR = 0 under EIN_TYPE "SIMPLE": the power term is 1);
   //      over liquid for the evaporation of rain, over ice for cold cells
