@@ -569,6 +569,12 @@ __global__ void __launch_bounds__(COL_THREADS_MAX, 2) nsw6_column_kernel(Problem
   const float* bff = gf + 5 * K;
   const float* cff = gf + 6 * K;
   const float* dff = gf + 7 * K;
+  // Bit j (8 + j): a factor of the cell's sources (of its half level's) is an
+  // infinity or a NaN, which a zero mass does not make a zero: the products are
+  // formed all the same, and a NaN flux is filtered out.  (A level with nothing
+  // else adds nothing to a flux, so the levels held and `act` leave it out.)
+  unsigned odd = 0;
+  auto infinite = [](float x) { return (soft_float_bits(x) & 0x7F800000u) == 0x7F800000u; };
 
   // ---- metric factors, kinetic energy, zeroed accumulators
   //      (mod_precip_transport.cpp:715-770, cnvvar_rhogkin_in mod_debug.cpp:269-330)
@@ -611,27 +617,35 @@ __global__ void __launch_bounds__(COL_THREADS_MAX, 2) nsw6_column_kernel(Problem
     if (MIX) {
       // the velocity components scale FP32 momentum sources only: FP32
       const float vx = soft_d2f(vxd), vy = soft_d2f(vyd), vz = soft_d2f(vzd);
-      FF(S_VI)[c] = __fmaf_rn(vz, uvf[2 * COL_TG + gx], __fmaf_rn(vy, uvf[1 * COL_TG + gx], __fmul_rn(vx, uvf[gx])));
-      FF(S_VJ)[c] =
+      const float vi = __fmaf_rn(vz, uvf[2 * COL_TG + gx], __fmaf_rn(vy, uvf[1 * COL_TG + gx], __fmul_rn(vx, uvf[gx])));
+      const float vj =
           __fmaf_rn(vz, uvf[5 * COL_TG + gx], __fmaf_rn(vy, uvf[4 * COL_TG + gx], __fmul_rn(vx, uvf[3 * COL_TG + gx])));
+      float rgs = 0.0f, kin = 0.0f;
+      FF(S_VI)[c] = vi;
+      FF(S_VJ)[c] = vj;
       const float gsgf = soft_d2f(gsg), ghf = soft_d2f(gsh), rhogf = soft_d2f(rg);
       FF(S_VI)[ncell + c] = ghf;
       FF(S_VJ)[ncell + c] = gsgf;
       FF(S_KINH)[ncell + c] = rhogf;
       if (interior) {
-        FF(S_KINV)[ncell + c] = soft_d2f(r_rgs[j]);
-        FF(S_KINH)[c] = kin_h_f(soft_d2f(rvx), soft_d2f(rvy), soft_d2f(rvz), rhogf);
+        FF(S_KINV)[ncell + c] = rgs = soft_d2f(r_rgs[j]);
+        FF(S_KINH)[c] = kin = kin_h_f(soft_d2f(rvx), soft_d2f(rvy), soft_d2f(rvz), rhogf);
       }
       if (k >= kmin + 1 && k <= kmax) {
         r_c2w0f[j] = __fmul_rn(__fdiv_rn(aff[k], gsgf), ghf);
         r_rgshf[j] = __fdiv_rn(soft_d2f(gmh), ghf);
         FF(S_DKINV)[ncell + c] = soft_d2f(rwd);
       }
+      if (infinite(vi) || infinite(vj) || infinite(rgs) || infinite(kin)) odd |= 1u << j;
       continue;
     }
-    F(S_VI)[c] = vxd * P.ix[ic] + vyd * P.iy[ic] + vzd * P.iz[ic];
-    F(S_VJ)[c] = vxd * P.jx[ic] + vyd * P.jy[ic] + vzd * P.jz[ic];
-    if (interior) F(S_KINH)[c] = quo(0.5 * (rvx * rvx + rvy * rvy + rvz * rvz), rg);
+    const double vi = vxd * P.ix[ic] + vyd * P.iy[ic] + vzd * P.iz[ic];
+    const double vj = vxd * P.jx[ic] + vyd * P.jy[ic] + vzd * P.jz[ic];
+    F(S_VI)[c] = vi;
+    F(S_VJ)[c] = vj;
+    double kin = 0.0;
+    if (interior) F(S_KINH)[c] = kin = quo(0.5 * (rvx * rvx + rvy * rvy + rvz * rvz), rg);
+    if (fp_not_finite(vi) || fp_not_finite(vj) || fp_not_finite(r_rgs[j]) || fp_not_finite(kin)) odd |= 1u << j;
     if (k >= kmin + 1 && k <= kmax) {
       r_c2w0[j] = div_rn(afact[k], by_gsg) * gsh;
       r_rgsh[j] = quo(gmh, gsh);
@@ -648,7 +662,9 @@ __global__ void __launch_bounds__(COL_THREADS_MAX, 2) nsw6_column_kernel(Problem
     if (MIX) {
       const float c2w1 = __fmul_rn(__fdiv_rn(bff[k], FF(S_VJ)[ncell + c - COL_TG]), FF(S_VI)[ncell + c]);
       const float rw = FF(S_DKINV)[ncell + c];
-      FF(S_KINV)[c] = kin_v_f(rw, r_c2w0f[j], c2w1, FF(S_KINH)[ncell + c], FF(S_KINH)[ncell + c - COL_TG]);
+      const float kin = kin_v_f(rw, r_c2w0f[j], c2w1, FF(S_KINH)[ncell + c], FF(S_KINH)[ncell + c - COL_TG]);
+      FF(S_KINV)[c] = kin;
+      if (infinite(kin) || infinite(r_rgshf[j])) odd |= 0x100u << j;   // (an infinite rw gives no finite kin)
       r_c2w1f[j] = c2w1;
       continue;
     }
@@ -656,7 +672,9 @@ __global__ void __launch_bounds__(COL_THREADS_MAX, 2) nsw6_column_kernel(Problem
     const double gsgm = P.gsgam2[i - G], gsh = P.gsgam2h[i], rw = P.rhogw[i], rg = P.rhog[i], rgm = P.rhog[i - G];
     loaded(gsgm), loaded(gsh), loaded(rw), loaded(rg), loaded(rgm);
     const double c2w1 = div_rn(bfact[k], Divisor(gsgm)) * gsh;
-    F(S_KINV)[c] = quo(0.5 * (rw * rw), c2w0 * rg + c2w1 * rgm);
+    const double kin = quo(0.5 * (rw * rw), c2w0 * rg + c2w1 * rgm);
+    F(S_KINV)[c] = kin;
+    if (fp_not_finite(kin) || fp_not_finite(r_rgsh[j])) odd |= 0x100u << j;   // (an infinite rw gives no finite kin)
     r_c2w1[j] = c2w1;
   }
   // (the vertical kinetic energies are next read by their own threads, after barriers by others)
@@ -732,7 +750,8 @@ __global__ void __launch_bounds__(COL_THREADS_MAX, 2) nsw6_column_kernel(Problem
       const bool own = c < ncell && g < G;
       if (own) {
         const double b0 = ld0[j];
-        if (!fp_is_zero(b0)) {
+        if (fp_not_finite(ld2[j])) odd |= 1u << j;
+        if (!fp_is_zero(b0) || ((odd >> j) & 1u)) {
           soft_branch();
           bq[j] = b0 * r_rgs[j];
         }
@@ -747,7 +766,7 @@ __global__ void __launch_bounds__(COL_THREADS_MAX, 2) nsw6_column_kernel(Problem
       const bool holds = own && !fp_is_zero(b);
       if (c < ncell) {
         double e = 0.0;
-        if (holds) {
+        if (holds || ((odd >> j) & 1u)) {
           soft_branch();
           e = b * CVDRY * ld2[j];
         }
@@ -767,8 +786,9 @@ __global__ void __launch_bounds__(COL_THREADS_MAX, 2) nsw6_column_kernel(Problem
 
     // sources 2 .. 5 (mod_precip_transport.cpp:776-808): potential energy (of the cell's z),
     // horizontal kinetic energy, momentum along i and j
-    auto source = [&](int f, int c, double b, double z) {
-      if (fp_is_zero(b)) return 0.0;
+    auto source = [&](int f, int c, int j, double z) {
+      const double b = bq[j];
+      if (fp_is_zero(b) && !((odd >> j) & 1u)) return 0.0;
       soft_branch();
       switch (f) {
         case 2: return b * GRAV * z;
@@ -846,15 +866,15 @@ __global__ void __launch_bounds__(COL_THREADS_MAX, 2) nsw6_column_kernel(Problem
         if (MIX) restf[j] = flux_rest(dgzhf, k, kc[j], soft_d2f(z), bmn_h[k], bmx_f[k]);
         else rest[j] = flux_rest(dgzh, k, kc[j], z, bmn_h[k], bmx_f[k]);
         const double qa = ld1[j], qb = ld2[j];
-        const bool some = !(fp_is_zero(qa) && fp_is_zero(qb));
+        const bool some = !(fp_is_zero(qa) && fp_is_zero(qb)), full = some || ((odd >> (8 + j)) & 1u);
         if (MIX) {
           // qh scales the FP32 sources of the two half-level fluxes only: FP32
-          const float qh = some ? 0.5f * (soft_d2f(qa) + soft_d2f(qb)) * r_rgshf[j] : 0.0f;
+          const float qh = full ? 0.5f * (soft_d2f(qa) + soft_d2f(qb)) * r_rgshf[j] : 0.0f;
           FF(S_RHOF)[c] = __fmul_rn(qh, FF(S_KINV)[c]);
           FF(S_RHOF)[ncell + c] = __fmul_rn(qh, FF(S_DKINV)[ncell + c]);   // rhogw before the transport
         } else {
           double s0 = 0.0, s1 = 0.0;
-          if (some) {
+          if (full) {
             soft_branch();
             const double qh = 0.5 * (qa + qb) * r_rgsh[j];
             s0 = qh * F(S_KINV)[c];
@@ -896,6 +916,7 @@ __global__ void __launch_bounds__(COL_THREADS_MAX, 2) nsw6_column_kernel(Problem
       ld0[j] = P.z[off + i];
       ld1[j] = q_n[i];
       loaded(ld0[j]), loaded(ld1[j]);
+      if (fp_not_finite(ld0[j])) odd |= 1u << j;
     }
     __syncthreads();
     if (!MIX) {
@@ -905,10 +926,9 @@ __global__ void __launch_bounds__(COL_THREADS_MAX, 2) nsw6_column_kernel(Problem
         if (c >= ncell) continue;
         divergence(0, c, F(S_F));
         divergence(1, c, F(S_F2));
-        const double b = bq[j];
-        F(S_RHOF)[c] = source(2, c, b, ld0[j]);
+        F(S_RHOF)[c] = source(2, c, j, ld0[j]);
         double e = 0.0;
-        if (!fp_is_zero(b)) {
+        if (!fp_is_zero(bq[j]) || ((odd >> j) & 1u)) {
           soft_branch();
           e = ld1[j] * r_rgs[j] * F(S_KINH)[c];
         }
@@ -923,8 +943,8 @@ __global__ void __launch_bounds__(COL_THREADS_MAX, 2) nsw6_column_kernel(Problem
         if (c >= ncell) continue;
         divergence(2, c, F(S_F));
         divergence(3, c, F(S_F2));
-        F(S_RHOF)[c] = source(4, c, bq[j], 0.0);
-        F(S_RHOF2)[c] = source(5, c, bq[j], 0.0);
+        F(S_RHOF)[c] = source(4, c, j, 0.0);
+        F(S_RHOF2)[c] = source(5, c, j, 0.0);
       }
       __syncthreads();
       flux_pair(false);   // momentum along i and j
@@ -969,10 +989,10 @@ __global__ void __launch_bounds__(COL_THREADS_MAX, 2) nsw6_column_kernel(Problem
       if (c >= ncell) continue;
       divergence(0, c, F(S_F));
       divergence(1, c, F(S_F2));
-      F(S_RHOF)[c] = source(2, c, bq[j], ld0[j]);
+      F(S_RHOF)[c] = source(2, c, j, ld0[j]);
       // (S_RHOF2's doubles were read before the last barrier)
       float r3 = 0.0f, r4 = 0.0f, r5 = 0.0f;
-      if (!fp_is_zero(bq[j])) {
+      if (!fp_is_zero(bq[j]) || ((odd >> j) & 1u)) {
         const float bf = soft_d2f(bq[j]);
         r3 = __fmul_rn(__fmul_rn(soft_d2f(ld1[j]), FF(S_KINV)[ncell + c]), FF(S_KINH)[c]);
         r4 = __fmul_rn(bf, FF(S_VI)[c]);
@@ -1052,9 +1072,10 @@ __global__ void __launch_bounds__(COL_THREADS_MAX, 2) nsw6_column_kernel(Problem
   // ---- apply the tendencies (mod_precip_transport.cpp:956-989); a zero
   //      tendency leaves its field as it is
 #pragma unroll 1
-  for (int c = threadIdx.x; c < ncell; c += blockDim.x) {
+  for (int c = threadIdx.x; c < ncell; c += blockDim.x, odd >>= 1) {
     const int k = c / COL_TG, gx = c % COL_TG, g = g0 + gx;
     if (g >= G) continue;
+    const bool full = odd & 1u;   // a zero tendency times an infinity or a NaN is none
     const size_t i = off + (size_t)k * G + g;
     const size_t ic = (size_t)l * G + g;
     const size_t iq = offq + (size_t)k * G + g;
@@ -1079,14 +1100,14 @@ __global__ void __launch_bounds__(COL_THREADS_MAX, 2) nsw6_column_kernel(Problem
     if (MIX) {
       // the FP32 momentum tendencies along the FP32 unit vectors, added to the FP64 state
       const float du = FF(S_DRHOGU)[c], dv = FF(S_DRHOGV)[c];
-      if (du != 0.0f || dv != 0.0f) {
+      if (du != 0.0f || dv != 0.0f || full) {
         P.rhogvx[i] = rvx = rvx + soft_f2d(__fmaf_rn(dv, uvf[3 * COL_TG + gx], __fmul_rn(du, uvf[gx])));
         P.rhogvy[i] = rvy = rvy + soft_f2d(__fmaf_rn(dv, uvf[4 * COL_TG + gx], __fmul_rn(du, uvf[1 * COL_TG + gx])));
         P.rhogvz[i] = rvz = rvz + soft_f2d(__fmaf_rn(dv, uvf[5 * COL_TG + gx], __fmul_rn(du, uvf[2 * COL_TG + gx])));
       }
     } else {
       const double du = F(S_DRHOGU)[c], dv = F(S_DRHOGV)[c];
-      if (!(fp_is_zero(du) && fp_is_zero(dv))) {
+      if (!(fp_is_zero(du) && fp_is_zero(dv)) || full) {
         P.rhogvx[i] = rvx = rvx + du * P.ix[ic] + dv * P.jx[ic];
         P.rhogvy[i] = rvy = rvy + du * P.iy[ic] + dv * P.jy[ic];
         P.rhogvz[i] = rvz = rvz + du * P.iz[ic] + dv * P.jz[ic];
@@ -1100,7 +1121,7 @@ __global__ void __launch_bounds__(COL_THREADS_MAX, 2) nsw6_column_kernel(Problem
     if (!MIX) F(S_DRHOGW)[c] = rw;   // MIX: the FP32 view of this slot is still being read
     // tracers in order QV..QG (QV, QC and QI add exact zeros; the -0 that makes a +0 is left to final_cell)
     auto add = [&](int n, double rq, double dq) {
-      if (fp_is_zero(dq)) return;
+      if (fp_is_zero(dq) && !full) return;
       soft_branch();
       P.rhogq[iq + (size_t)n * KG] = rq + dq;
       rhog = rhog + dq;

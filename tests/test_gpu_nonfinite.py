@@ -55,3 +55,13 @@ def differences(field, variant, options, dt):
 def test_poisoned_cells(field, variant, options):
     bad = differences(field, variant, options, 10.0)
     assert not bad, bad
+
+
+# five minutes: departure distances of several layers, so fluxes draw on poisoned levels without the tracer
+@pytest.mark.parametrize("field,options", [(f, o) for f in ("tem", "q", "vx", "ix", "unccn") for o in (None, ALL_SWITCHES)] +
+                         [("rhogw", ALL_SWITCHES), ("gsgam2h", ALL_SWITCHES)],
+                         ids=lambda p: p if isinstance(p, str) else "switches" if p else "reference")
+@pytest.mark.parametrize("variant", ["convective", "cold"])
+def test_poisoned_levels(field, variant, options):
+    bad = differences(field, variant, options, 300.0)
+    assert not bad, bad
