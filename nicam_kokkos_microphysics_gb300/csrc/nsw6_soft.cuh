@@ -26,7 +26,9 @@
 // 0.80 ms (one 16900 x 42 region).
 //
 // Every routine compiles for the host too, where tests/test_softfp.py compares
-// it with the host's IEEE arithmetic and with 128-bit references.
+// it with the host's IEEE arithmetic and with extended-precision references;
+// tests/test_gpu_softfp.py compares the quotients, roots and conversions on the
+// device, whose seeds are the special-function unit's.
 #pragma once
 
 #include <cmath>
@@ -95,14 +97,20 @@ NSW6_FP_HD u32 soft_float_bits(float f) {
   return b;
 #endif
 }
-// 1 / x and 1 / sqrt(x) to about 2^-22, the special-function unit's
+// 1 / x and 1 / sqrt(x), the special-function unit's (PTX: rcp.approx.ftz.f32
+// within one unit in the last place, rsqrt.approx.ftz.f32 within 2^-22.9
+// relative).  The host has them correctly rounded, moved by NSW6_SEED_ULPS
+// units (a test sets it) where the device's may be.
+#ifndef NSW6_SEED_ULPS
+#define NSW6_SEED_ULPS 0
+#endif
 NSW6_FP_HD float soft_rcp_seed(float x) {
 #ifdef __CUDA_ARCH__
   float y;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 #else
-  return 1.0f / x;
+  return soft_as_float(soft_float_bits(1.0f / x) + (u32)(NSW6_SEED_ULPS));
 #endif
 }
 NSW6_FP_HD float soft_rsqrt_seed(float x) {
@@ -111,7 +119,7 @@ NSW6_FP_HD float soft_rsqrt_seed(float x) {
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 #else
-  return (float)(1.0 / std::sqrt((double)x));
+  return soft_as_float(soft_float_bits((float)(1.0 / std::sqrt((double)x))) + (u32)(NSW6_SEED_ULPS));
 #endif
 }
 
@@ -157,9 +165,11 @@ struct SoftDivisor {
 };
 
 // One Newton step from the special-function unit's reciprocal: with b the top
-// 32 bits of m, r0 = 2^32 / b' for a b' just above b / 2^31, and
+// 32 bits of m, r0 = 2^32 / b' for a b' 2^-22 above b / 2^31, and
 // r = r0 + r0 (1 - b r0) in floor arithmetic is at most 2^63 / b and at least
-// that less 3, so r is within 3 of 2^84 / m and below 2^32.
+// that less 3, so r is within 3 of 2^84 / m and below 2^32.  y = 1 / b' has to
+// stay below 1, where r0 has its top bit: for b = 2^31 it is 1 - 2^-22, four
+// units in the last place below, and the unit is within one.
 NSW6_FP_HD SoftDivisor soft_divisor(double b) {
   const u64 bits = (u64)fp_bits(b);
   SoftDivisor d;
@@ -167,7 +177,7 @@ NSW6_FP_HD SoftDivisor soft_divisor(double b) {
   d.e = (int)((soft_hi(bits) >> 20) & 0x7FFu);
   d.s = soft_hi(bits) & 0x80000000u;
   const u32 b32 = (u32)(d.m >> 21);                      // [2^31, 2^32)
-  const float y = soft_rcp_seed(soft_as_float((b32 >> 8) + 0x3F000001u));   // 1 / (b32 / 2^31 + 2^-23)
+  const float y = soft_rcp_seed(soft_as_float((b32 >> 8) + 0x3F000002u));   // 1 / (b32 / 2^31 + 2^-22)
   const u32 r0 = (soft_float_bits(fmaxf(y, 0.5f)) << 8) | 0x80000000u;      // y in [0.5, 1)
   const long long err = (long long)(0x8000000000000000ull - (u64)b32 * r0);   // below 2^43 in size
   d.r = r0 + (u32)(int)(((long long)(int)(r0 >> 1) * (long long)(int)(err >> 13)) >> 49);
@@ -249,7 +259,8 @@ NSW6_CALL double soft_sqrt(double x) {
   const u32 odd = mh >> 31;                              // f >= 2: its float has the higher exponent
   const float f = soft_as_float(odd ? (((mh >> 8) & 0x007FFFFFu) | 0x40000000u)
                                     : (((mh >> 7) & 0x007FFFFFu) | 0x3F800000u));
-  const int y = (int)(soft_rsqrt_seed(f) * 2147483520.0f);        // 2^31 / sqrt(f), below 2^31
+  // 2^31 / sqrt(f), below 2^31 (the unit may give more than 1 for f = 1)
+  const int y = (int)(fminf(soft_rsqrt_seed(f), 1.0f) * 2147483520.0f);
   const u64 p = (u64)mh * (u32)y;                        // 2^61 sqrt(f)
   u32 s = (p >> 62) ? 0xFFFFFFFFu : (u32)(p >> 30);      // 2^31 sqrt(f) to 2^11
   long long r = (long long)(M - (u64)s * s);             // below 2^44 in size
