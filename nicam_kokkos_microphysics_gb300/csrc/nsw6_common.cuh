@@ -210,42 +210,9 @@ struct TapeMem {
   int nslot, cap, count_only;
 };
 
-// Comparisons of doubles on the integer pipe (the FP64 pipe is the scarce one
-// on GB300): for non-NaN a and b, a >= b exactly when cmp_key(a) >=
-// cmp_key(b), with -0 and +0 equal.
-__device__ __forceinline__ long long cmp_key(double x) {
-  long long b = __double_as_longlong(x);
-  if (b == (long long)0x8000000000000000ULL) b = 0;
-  return b < 0 ? (b ^ 0x7fffffffffffffffLL) : b;
-}
-// (by the two words: of the 64-bit form the compiler makes an FP64 comparison)
-__device__ __forceinline__ bool is_nan_bits(double x) {
-  const unsigned hi = (unsigned)__double2hiint(x) & 0x7fffffffu;
-  return hi > 0x7ff00000u || (hi == 0x7ff00000u && __double2loint(x) != 0);
-}
 constexpr long long EPS_BITS = 0x3caffffff4178da3LL;   // bit pattern of EPS = 2.220446E-16
 
 __host__ __device__ __forceinline__ double dmin(double a, double b) { return (b < a) ? b : a; }  // Kokkos::min
 __host__ __device__ __forceinline__ double dmax(double a, double b) { return (a < b) ? b : a; }  // Kokkos::max
-
-// Order-preserving map double -> uint64 (total order, -0 < +0), used for exact
-// atomic max/min of the per-level departure-distance extrema.
-__host__ __device__ __forceinline__ unsigned long long order_key(double v) {
-#ifdef __CUDA_ARCH__
-  // (by the two words: of the 64-bit form the compiler makes FP64 negations)
-  const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
-  const unsigned neg = (unsigned)((int)hi >> 31);   // all ones for a negative number
-  return ((unsigned long long)(hi ^ (neg | 0x80000000u)) << 32) | (lo ^ neg);
-#else
-  union { double d; unsigned long long u; } c;
-  c.d = v;
-  return (c.u >> 63) ? ~c.u : (c.u | 0x8000000000000000ull);
-#endif
-}
-__host__ __device__ __forceinline__ double key_value(unsigned long long k) {
-  union { double d; unsigned long long u; } c;
-  c.u = (k >> 63) ? (k & 0x7fffffffffffffffull) : ~k;
-  return c.d;
-}
 
 }  // namespace nsw6

@@ -36,6 +36,35 @@ NSW6_FP_HD long long fp_bits(double x) {
 #endif
 }
 
+// The two words of a double, and the double of two words.  Where one word
+// decides, or each by itself, the forms below go by words: of the same test on
+// the 64-bit pattern the compiler makes an FP64 instruction, 16 to 19 cycles of
+// an SM's FP64 pipe (see each).
+NSW6_FP_HD unsigned fp_hi(double x) {
+#ifdef __CUDA_ARCH__
+  return (unsigned)__double2hiint(x);
+#else
+  return (unsigned)((unsigned long long)fp_bits(x) >> 32);
+#endif
+}
+NSW6_FP_HD unsigned fp_lo(double x) {
+#ifdef __CUDA_ARCH__
+  return (unsigned)__double2loint(x);
+#else
+  return (unsigned)fp_bits(x);
+#endif
+}
+NSW6_FP_HD double fp_of_words(unsigned hi, unsigned lo) {
+#ifdef __CUDA_ARCH__
+  return __hiloint2double((int)hi, (int)lo);
+#else
+  const unsigned long long b = ((unsigned long long)hi << 32) | lo;
+  double x;
+  std::memcpy(&x, &b, sizeof x);
+  return x;
+#endif
+}
+
 NSW6_FP_HD long long fp_key(long long b) { return b ^ ((b >> 63) & FP_ABS); }
 
 // a < b
@@ -72,24 +101,17 @@ NSW6_FP_HD bool fp_lt_pos(double x, double c) {
 // max(x, c) as Kokkos::max, (x < c) ? c : x, for a constant c > 0
 NSW6_FP_HD double fp_max_pos(double x, double c) { return fp_lt_pos(x, c) ? c : x; }
 
-// x == 0 (either zero).  On the device by the two words: the compiler makes an
-// FP64 comparison of the 64-bit form ((bits & FP_ABS) == 0), which takes the
-// FP64 pipe 16 cycles.
-NSW6_FP_HD bool fp_is_zero(double x) {
-#ifdef __CUDA_ARCH__
-  return (((unsigned)__double2hiint(x) << 1) | (unsigned)__double2loint(x)) == 0u;
-#else
-  return (fp_bits(x) & FP_ABS) == 0;
-#endif
-}
+// x == 0 (either zero), by words: the 64-bit form ((bits & FP_ABS) == 0) was 92
+// FP64-pipe instructions a cell of the column kernel
+NSW6_FP_HD bool fp_is_zero(double x) { return ((fp_hi(x) << 1) | fp_lo(x)) == 0u; }
 
 // x is +-inf or NaN (x * 0 != 0)
-NSW6_FP_HD bool fp_not_finite(double x) {
-#ifdef __CUDA_ARCH__
-  return ((unsigned)__double2hiint(x) & 0x7FF00000u) == 0x7FF00000u;
-#else
-  return (fp_bits(x) & FP_ABS) >= FP_INF;
-#endif
+NSW6_FP_HD bool fp_not_finite(double x) { return (fp_hi(x) & 0x7FF00000u) == 0x7FF00000u; }
+
+// x is NaN
+NSW6_FP_HD bool is_nan_bits(double x) {
+  const unsigned hi = fp_hi(x) & 0x7FFFFFFFu;
+  return hi > 0x7FF00000u || (hi == 0x7FF00000u && fp_lo(x) != 0u);
 }
 
 // x is a positive normal number (not zero, subnormal, infinite or NaN)
@@ -167,16 +189,31 @@ NSW6_FP_HD bool lt_nd(double a, double d) {                                     
   return ba < 0 && ma > (fp_bits(d) & FP_ABS) && ma <= FP_INF;
 }
 NSW6_FP_HD double max_nd(double a, double d) {                                          // max(a, -d)
-#ifdef __CUDA_ARCH__
-  // (by the word that has the sign: of the 64-bit form the compiler makes an FP64 negation)
-  return lt_nd(a, d) ? __hiloint2double(__double2hiint(d) ^ (int)0x80000000, __double2loint(d)) : a;
-#else
-  return lt_nd(a, d) ? fp_from_bits(fp_bits(d) ^ FP_SIGN) : a;
-#endif
+  return lt_nd(a, d) ? fp_of_words(fp_hi(d) ^ 0x80000000u, fp_lo(d)) : a;
 }
 
 // x + 0.0: -0 becomes +0, every other value stays (a NaN keeps its payload,
 // where an FP64 addition gives the canonical NaN)
 NSW6_FP_HD double plus_zero(double x) { return fp_bits(x) == FP_SIGN ? 0.0 : x; }
+
+// Keys in the order of the doubles.  cmp_key: for non-NaN a and b, a >= b
+// exactly when cmp_key(a) >= cmp_key(b), with -0 and +0 equal.
+NSW6_FP_HD long long cmp_key(double x) {
+  long long b = fp_bits(x);
+  if (b == FP_SIGN) b = 0;
+  return b < 0 ? (b ^ FP_ABS) : b;
+}
+// Order-preserving map double -> uint64 (total order, -0 < +0), used for exact
+// atomic max/min of the per-level departure-distance extrema, and back.  By
+// words: the 64-bit form's OR and NOT with the sign were two FP64-pipe
+// instructions a row of the departure kernel.
+NSW6_FP_HD unsigned long long order_key(double v) {
+  const unsigned hi = fp_hi(v), lo = fp_lo(v);
+  const unsigned neg = (unsigned)((int)hi >> 31);   // all ones for a negative number
+  return ((unsigned long long)(hi ^ (neg | 0x80000000u)) << 32) | (lo ^ neg);
+}
+NSW6_FP_HD double key_value(unsigned long long k) {
+  return fp_from_bits((long long)((k >> 63) ? (k & 0x7FFFFFFFFFFFFFFFull) : ~k));
+}
 
 }  // namespace nsw6
