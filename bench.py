@@ -63,19 +63,19 @@ CELL_KERNEL_BYTES_PER_CELL = (10 + 17) * 8
 # nsw6_departure_kernel, the column phase nsw6_column_kernel and
 # nsw6_satadj_kernel (the saturated cells), each timed together as one
 # interval; the figures are the two kernels' sums.
-CELL_KERNEL_TRAFFIC_PER_CELL = {"fp64": 395.0 + 24.0, "mixed": 147.7 + 24.0}
-COLUMN_KERNEL_TRAFFIC_PER_CELL = {"fp64": 382.0 + 30.0, "mixed": 386.3 + 30.0}
+CELL_KERNEL_TRAFFIC_PER_CELL = {"fp64": 385.4 + 24.1, "mixed": 148.2 + 24.0}
+COLUMN_KERNEL_TRAFFIC_PER_CELL = {"fp64": 384.3 + 30.9, "mixed": 386.6 + 30.9}
 FP64_EXECUTED = {
-    "nsw6_cell_kernel": {"fp64": {"dfma": 38.4 + 16.8, "dadd": 104.7 + 15.0, "dmul": 80.4 + 17.3,
-                                  "pipe": 239.6 + 49.2},
+    "nsw6_cell_kernel": {"fp64": {"dfma": 38.4 + 16.8, "dadd": 96.9 + 15.0, "dmul": 80.5 + 17.3,
+                                  "pipe": 231.8 + 49.2},
                          "mixed": {"dfma": 0.0, "dadd": 26.3, "dmul": 20.1, "pipe": 52.4 + 2.2}},
-    "nsw6_column_kernel": {"fp64": {"dfma": 19.7, "dadd": 102.2 + 5.4, "dmul": 84.1 + 4.2, "pipe": 222.0 + 9.9},
-                           "mixed": {"dfma": 6.4, "dadd": 51.9 + 5.2, "dmul": 34.5 + 4.4, "pipe": 98.3 + 9.6}},
+    "nsw6_column_kernel": {"fp64": {"dfma": 19.7, "dadd": 102.2 + 5.4, "dmul": 84.1 + 3.9, "pipe": 222.0 + 9.6},
+                           "mixed": {"dfma": 6.4, "dadd": 51.9 + 5.2, "dmul": 34.5 + 4.2, "pipe": 98.3 + 9.3}},
 }
 # FP64-pipe activity (fraction of active cycles) of each kernel in the same
 # captures (cold, serialised launches; the cell and the column kernel alone).
-FP64_PIPE_ACTIVE = {"nsw6_cell_kernel": {"fp64": 0.707, "mixed": 0.723},
-                    "nsw6_column_kernel": {"fp64": 0.721, "mixed": 0.494}}
+FP64_PIPE_ACTIVE = {"nsw6_cell_kernel": {"fp64": 0.697, "mixed": 0.720},
+                    "nsw6_column_kernel": {"fp64": 0.707, "mixed": 0.487}}
 # FP64 op weights in flop equivalents (an FMA counts 2): the cost of CUDA's FP64
 # divide, sqrt, exp, log and pow relative to DFMA, measured once on a GB300 with
 # the throughput probe (probe/nsw6_probe.cu) and frozen here.

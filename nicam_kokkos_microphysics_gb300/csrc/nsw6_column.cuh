@@ -222,19 +222,19 @@ __device__ __forceinline__ double satadjust_newton(const Problem& P, const Const
   return tem;
 }
 
-// The final state of one cell after the transport and KIN2EIN: thermodynamics,
-// saturation adjustment, negative filter and outputs (mod_mp_driver.cpp:
-// 555-612 with mod_thrmdyn.cpp, mod_satadjust.cpp:274-362 and
-// mod_mp_nsw6.cpp:1770-1831).  rhog, the divisor it makes and rhoge (after KIN2EIN)
-// are the cell's; the rest comes from the state arrays.  With newton = false
-// (the column kernel) a saturated interior cell is left as it is and true is
-// returned, for nsw6_satadj_kernel; every other cell is finished.  With
-// newton = true (that kernel) the cell is saturated: the same values are
-// formed, the Newton iteration runs and the cell is finished.
 // A value loaded here and not sunk to its use: the loads of a pass are in
 // flight together before its first call of a soft routine, across which none moves.
 __device__ __forceinline__ void loaded(double x) { asm volatile("" ::"d"(x)); }
 
+// The final state of one cell after the transport and KIN2EIN: thermodynamics,
+// saturation adjustment, negative filter and outputs (mod_mp_driver.cpp:
+// 555-612 with mod_thrmdyn.cpp, mod_satadjust.cpp:274-362 and
+// mod_mp_nsw6.cpp:1770-1831) from the cell's rhog and the divisor it makes, rhoge
+// (after KIN2EIN), tracers and gsgam2.  With newton = false
+// (the column kernel) a saturated interior cell is left as it is and true is
+// returned, for nsw6_satadj_kernel; every other cell is finished.  With
+// newton = true (that kernel) the cell is saturated: the same values are
+// formed, the Newton iteration runs and the cell is finished.
 template <class M, bool MIX, bool OPT>
 __device__ __forceinline__ bool final_cell(const Problem& P, const Consts& C, const M& mth, bool ice_adj, float lovr_f,
                                            size_t i, size_t iq, size_t KG, bool interior, double rhog,
@@ -1245,7 +1245,7 @@ __global__ void __launch_bounds__(COL_THREADS_MAX, 2) nsw6_column_kernel(Problem
   if (threadIdx.x == 0) nqueue = 0;
   __syncthreads();
   const float lovr_f = float(C.LovR_liq);
-  int* qcell = reinterpret_cast<int*>(F(S_RHOF2));   // the tile's saturated cells (S_BASE is dead by now)
+  int* qcell = reinterpret_cast<int*>(F(S_RHOF2));   // the tile's saturated cells (S_RHOF2 is dead by now)
 #pragma unroll 1
   for (int c = threadIdx.x; c < ncell; c += blockDim.x) {
     const int k = c / COL_TG, gx = c % COL_TG, g = g0 + gx;
@@ -1314,7 +1314,7 @@ __global__ void __launch_bounds__(COL_THREADS_MAX, 2) nsw6_column_kernel(Problem
   }
 }
 
-// ------------------------------------------------------------------ kernel 3
+// ------------------------------------------------------ saturation adjustment
 // The saturated cells the column kernel listed (P.satq): the cell's state
 // after KIN2EIN is formed again exactly as there, the saturation-adjustment
 // Newton iteration runs and the cell is finished (final_cell).  One thread per
@@ -1325,9 +1325,13 @@ __global__ void __launch_bounds__(COL_THREADS_MAX, 2) nsw6_column_kernel(Problem
 // mixed steps of 2500 x 42 1.593 -> 1.561 ms, one region's FP64 step 1.037 ->
 // 1.030 ms, ten regions the same.
 constexpr int SAT_THREADS = 32;
-// CTAs: enough for a sixteenth of the cells (some 4 percent are saturated) in
-// one sweep, so that the last ones level out; at least 8 an SM, for a small call
-// that is saturated throughout, and no more than 64, whose start costs.
+// CTAs: enough for a sixteenth of the cells in one sweep, so that the last ones
+// level out (some 4 percent are saturated in ordinary weather); at least 8 an
+// SM, for a small call that is saturated throughout, and no more than 64, whose
+// start costs.  Any number of saturated cells is handled, the loop strides over
+// the list; where 37 percent are (a state 1.6 times as moist) a region's call
+// takes two or three uneven sweeps, 1144 us in FP64 and 667 in mixed precision
+// where 64 CTAs an SM take 1123 and 650; ten regions take the same.
 inline int sat_blocks(long long cells) {
   const long long n = cells / (16 * SAT_THREADS);
   return (int)(n < 152 * 8 ? 152 * 8 : n > 152 * 64 ? 152 * 64 : n);

@@ -37,8 +37,8 @@ constexpr double DENS00 = 1.28;    // mod_mp_nsw6.cpp:8
 constexpr int NQ = 6;
 constexpr int I_QV = 0, I_QC = 1, I_QR = 2, I_QI = 3, I_QS = 4, I_QG = 5;
 
-// Geometry: the cell kernel's threads; the column kernel gives one CTA 16
-// (kall <= 64) or 8 columns x all levels.
+// The cell kernel's threads at most (cell_shape; the column kernel's tiles of
+// 16, 8 or 4 columns: column_shape).
 constexpr int CELL_THREADS = 256;
 constexpr int MAX_KALL = 160;
 

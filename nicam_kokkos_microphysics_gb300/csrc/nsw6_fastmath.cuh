@@ -12,8 +12,9 @@
 // doubles had 96 %, 95 % and 2 units for pow.  One 16900 x 42 region, FP64:
 // step 2.134 -> 1.944 ms.
 //
-// The tables (7 KB) are built on the host in extended precision and staged in
-// shared memory by every CTA.
+// The tables (7 KB) are built on the host in extended precision.  The cell and
+// derivative kernels stage them in shared memory; the column and saturation
+// kernels, few of whose cells ask for them, read them through L1.
 #pragma once
 
 #include <cstdint>

@@ -233,7 +233,7 @@ __device__ __forceinline__ unsigned long long warp_min(unsigned long long v) { r
 // halvings are integer operations, a warp walks consecutive levels and forms
 // their differences once, and levels without the tracer are branched around.
 // One 16900 x 42 region, FP64: 0.165 -> 0.118 ms (2.5 M -> 1.75 M FP64 warp
-// instructions).
+// instructions), with the extrema's keys by words 0.083 (1.04 M).
 constexpr int DEP_TG = 32;
 constexpr int DEP_THREADS = 256;
 
